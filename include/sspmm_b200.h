@@ -60,6 +60,16 @@ int sspmm_f16_f16_batched(int m_vec, int vec_length, int N, int K, int batch, co
                           int64_t out_stride, void* stream);
 
 /*
+ * The three calls above for a caller that knows the vector count nvec = row_offsets[m_vec] (the compression returns it):
+ * nothing is read back or remembered and the call never synchronises.  nvec decides which kernel runs and how the work is
+ * cut, never the result: a count that is only an upper bound (the length of column_indices) will do.  fp16 or fp32 output;
+ * batch and strides as in sspmm_f16_f16_batched.
+ */
+int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nvec, const int* row_indices, const int* row_offsets,
+                  const int* column_indices, const void* values_f16, int64_t values_stride, const void* rhs_f16, int64_t rhs_stride,
+                  void* out, int64_t out_stride, int out_is_f16, void* stream);
+
+/*
  * Same product as sspmm_f16_f16, for callers that must not allocate device memory when they call:
  * a server that gave all device memory to its own arena at start-up, or a latency-critical loop
  * in which an allocation could fail or stall other streams.  No counterpart in the reference (its
@@ -93,7 +103,8 @@ int sspmm_f16_f16_noalloc(int m_vec, int vec_length, int N, int K, const int* ro
  *     and the row-gather kernel is used;
  *   - the block kernel takes K * m_vec*V * 2 bytes (a dense transposed copy of A), plus fp32
  *     partial tiles when it splits K, from cudaMallocAsync on `stream` and returns them with
- *     cudaFreeAsync; the row-gather kernel does the same for the partial tiles of split long rows;
+ *     cudaFreeAsync; the row-gather kernel does the same for the partial tiles of split long rows, and
+ *     either for an aligned copy of rhs when N is not a multiple of 8 or rhs not on a 16-byte boundary;
  *   - once per device the release threshold of the device's default memory pool is raised to 1 GiB
  *     so that this scratch is not returned to the system at every synchronisation.
  * Callers that must not allocate or synchronise at call time use a plan (below), or

@@ -78,23 +78,21 @@ static long long lookup_nvec(const int* row_offsets, int m_vec, cudaStream_t st)
     return h;
 }
 
-// Modelled times (seconds) of the two tensor-core kernels; constants from measurements on B200.
-// Gather kernel: one work item per (vector row, 128 output columns); an item costs about 1 us plus
-// 0.9 us per 64 gathered rows while items are few (latency of the gather chain), and the whole kernel
-// never beats 4 TB/s of gathered bytes.  Block kernel: expansion + dense GEMM, about 9 us of fixed cost
-// (two or three dependent launches).
+// Modelled times (seconds) of the two kernels, fitted to a sweep of shapes (64 to 2048 rows, K 64 to 4608, N 8 to 8192,
+// sparsity 0.5 to 0.98, both V) measured on B200 in graph replays.  Row-gather kernel: launch and one chain of look-ups,
+// then 2 * nvec * N bytes of gathers at 8.3 TB/s.  Block kernel: two launches, the dense copy of A written and read, the
+// longer of its K loop's latency and its dense flops, and a third launch when few tiles make it cut K.  The last term is
+// what the host pays for the scratch and the extra launches.  At the crossing (512 x 512, sparsity 0.5, V = 8): N = 128
+// 5.4 against 9.3 us, N = 1024 11.1 against 9.4 us.
 static bool block_kernel_is_faster(long long nvec, const SpmmArgs& a) {
     const double n = (double)a.N * a.batch;
     const double mp = (double)a.m_vec * a.V;
     const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;
-    const double items = (double)a.m_vec * ((a.N + 127) / 128) * a.batch;
-    const double waves = (items + sms - 1) / sms >= 1.0 ? (double)(long long)((items + sms - 1) / sms) : 1.0;
-    const double steps = (double)nvec / (a.m_vec > 0 ? a.m_vec : 1) / 64.0;
-    const double t_chain = waves * (1.0e-6 + steps * 0.9e-6);
-    const double t_stream = 2.0 * (double)nvec * n / 4.0e12;
-    const double t_gather = 3e-6 + (t_chain > t_stream ? t_chain : t_stream);
-    const double t_block = 2.0 * mp * a.K * n / 6.0e14 + 4.0 * mp * a.K / 3e12 + 9e-6;
-    return t_block < t_gather;
+    const double t_rows = 3.7e-6 + 2.0 * (double)nvec * n / 8.3e12;
+    const double depth = 1.0e-9 * a.K, flops = 2.0 * mp * a.K * n / 1.25e15;
+    const bool cuts_k = a.K >= 512 && (mp + 127) / 128 * ((a.N + 255) / 256) * a.batch < sms;
+    const double t_block = 6.0e-6 + (cuts_k ? 2.8e-6 : 0.0) + 4.0 * mp * a.K / 3.8e12 + (depth > flops ? depth : flops) + 1.5e-6;
+    return t_block < t_rows;
 }
 
 // Length-sorted scheduling order: rank by (length descending, row id ascending).
@@ -195,7 +193,7 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
     }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     SpmmArgs a;
-    a.m_vec = m_vec; a.V = V; a.N = N; a.K = K;
+    a.m_vec = m_vec; a.V = V; a.N = N; a.n_out = N; a.K = K;
     a.row_indices = row_indices; a.row_offsets = row_offsets; a.column_indices = column_indices;
     a.values = static_cast<const __half*>(values); a.rhs = static_cast<const __half*>(rhs);
     a.out = out; a.out_f16 = out_f16; a.batch = batch;
@@ -203,74 +201,85 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
     a.stream = st;
 
     const int choice = g_kernel_choice.load();
-    const bool tc_ok = K > 0 && (N % 8 == 0) && aligned16(rhs) && aligned16(values) &&
-                       (values_stride * 2) % 16 == 0 && (batch == 1 || rhs_stride == (int64_t)K * N);
-    if (choice == 1 && !tc_ok) {
+    const bool values_ok = aligned16(values) && (values_stride * 2) % 16 == 0;
+    const bool rhs_ok = N % 8 == 0 && aligned16(rhs) && (batch == 1 || (rhs_stride * 2) % 16 == 0);
+    if (choice == 1 && !(K > 0 && values_ok && rhs_ok && (batch == 1 || rhs_stride == (int64_t)K * N))) {
         set_error("tensor-core kernel needs N %% 8 == 0, 16-byte aligned values/rhs and contiguous batches");
         return (int)cudaErrorInvalidValue;
     }
     cudaError_t e;
-    if (K == 0 || choice == 2 || !tc_ok) {
-        if (ex.query) return 0;
-        e = launch_sspmm_simt(a);
-        return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
-    }
-    const int64_t oes = out_f16 ? 2 : 4;
-    const bool block_ok = (batch == 1 || (values_stride == 0 && (rhs_stride * 2) % 16 == 0 && (out_stride * oes) % 16 == 0)) &&
-                          aligned16(out) && ((int64_t)N * oes) % 16 == 0 &&
-                          sspmm_block_scratch_bytes(a) <= ((size_t)2 << 30);
-    if (choice == 3 && !block_ok) {
-        set_error("block kernel needs 16-byte aligned output, a shared value array for batches and <= 2 GiB of scratch");
-        return (int)cudaErrorInvalidValue;
-    }
-    if (choice == 1) {                                     // TMA row-gather producers
-        if (ex.query) return 0;
-        e = launch_sspmm_gather(a);
-        return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
-    }
-    bool use_block = choice == 3;
-    long long nvec = ex.nvec;
-    if (nvec < 0 && !ex.query && (choice == 0 || choice == 4)) nvec = lookup_nvec(row_offsets, m_vec, st);
-    if (choice == 0 && block_ok) use_block = nvec >= 0 && block_kernel_is_faster(nvec, a);
-    if (!use_block) {                                      // gather kernel with load-instruction producers
-        int chunk = 0, cap = 0;
-        size_t bytes = 0;
-        sspmm_gather_lsu_plan(a, nvec, &chunk, &cap, &bytes);
-        if (ex.query) { *ex.query = bytes; return 0; }
-        void* scratch = nullptr;
-        if (ex.caller_workspace) {
-            if (bytes > ex.workspace_bytes) {          // too small: long rows are not split (slower, same result)
-                chunk = 0; cap = 0;
-                bytes = (ex.workspace && ex.workspace_bytes >= 16) ? 16 : 0;     // the work counter alone still fits
-            }
-            if (bytes) scratch = ex.workspace;
-        } else if (bytes) {
-            keep_pool_memory();
-            e = cudaMallocAsync(&scratch, bytes, st);
-            if (e != cudaSuccess) return fail(e, "scratch allocation for split rows");
+    // The other kernels read 16-byte pieces.  A dense operand that does not lie on 16-byte boundaries (any N) is copied
+    // once; without room for the copy, and for unaligned value vectors, the CUDA-core kernel takes the call.
+    const int64_t ld = ((int64_t)N + 7) & ~7LL;
+    const size_t copy_bytes = rhs_ok ? 0 : (((size_t)K * batch * ld * 2 + 255) & ~(size_t)255);
+    bool simt = K == 0 || choice == 2 || !values_ok || ld > 0x7fffffff || (!rhs_ok && (ex.query || ex.caller_workspace)) ||
+                copy_bytes > ((size_t)2 << 30);
+    if (!simt) {
+        if (choice == 1) {                                     // TMA row-gather producers
+            if (ex.query) return 0;
+            e = launch_sspmm_gather(a);
+            return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
         }
-        e = launch_sspmm_gather_lsu(a, chunk, cap, bytes ? scratch : nullptr);
-        if (scratch && !ex.caller_workspace) cudaFreeAsync(scratch, st);
-        return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
-    }
-    const size_t want = sspmm_block_scratch_bytes(a);
-    if (ex.query) { *ex.query = want; return 0; }
-    if (ex.caller_workspace) {
-        const size_t need = (size_t)K * m_vec * V * sizeof(__half);
-        if (ex.workspace_bytes < need || !ex.workspace) {
-            set_error("workspace of %zu bytes is too small: the block kernel needs at least %zu (sspmm_workspace_bytes reports %zu)",
-                      ex.workspace_bytes, need, want);
+        if (!rhs_ok) {
+            a.N = (int)ld;
+            a.rhs_stride = batch > 1 ? (int64_t)K * ld : 0;
+        }
+        const int64_t oes = out_f16 ? 2 : 4;
+        const bool out_ok = aligned16(out) && ((int64_t)N * oes) % 16 == 0;
+        // TMA reads whole batches with one stride; a copied operand is written out by the reduction, which has no batches
+        const bool block_ok = (batch == 1 || (values_stride == 0 && rhs_ok && rhs_stride == (int64_t)K * N && (out_stride * oes) % 16 == 0)) &&
+                              (a.n_out != a.N || out_ok) && sspmm_block_scratch_bytes(a) <= ((size_t)2 << 30);
+        if (choice == 3 && !block_ok && rhs_ok) {
+            set_error("block kernel needs 16-byte aligned output, a shared value array for batches and <= 2 GiB of scratch");
             return (int)cudaErrorInvalidValue;
         }
-        e = launch_sspmm_block(a, ex.workspace, ex.workspace_bytes);
-        return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
+        long long nvec = ex.nvec;
+        if (nvec < 0 && !ex.query && (choice == 0 || choice == 4)) nvec = lookup_nvec(row_offsets, m_vec, st);
+        const bool use_block = block_ok && (choice == 3 || (choice == 0 && nvec >= 0 && block_kernel_is_faster(nvec, a)));
+        const size_t want = use_block ? sspmm_block_scratch_bytes(a) : sspmm_rows_scratch_bytes(a, nvec);
+        if (ex.query) { *ex.query = want; return 0; }
+        void* scratch = nullptr;
+        size_t room = want;
+        if (ex.caller_workspace) {
+            room = ex.workspace_bytes;
+            if (use_block) {
+                const size_t need = (size_t)K * m_vec * V * sizeof(__half);
+                if (room < need || !ex.workspace) {
+                    set_error("workspace of %zu bytes is too small: the block kernel needs at least %zu (sspmm_workspace_bytes reports %zu)",
+                              room, need, want);
+                    return (int)cudaErrorInvalidValue;
+                }
+                scratch = ex.workspace;
+            } else if (want && room >= want) {
+                scratch = ex.workspace;                         // null or too small: long rows are not cut (slower)
+            }
+        } else if (copy_bytes + want) {
+            keep_pool_memory();
+            e = cudaMallocAsync(&scratch, copy_bytes + want, st);
+            if (e != cudaSuccess) {
+                if (rhs_ok) return fail(e, "scratch allocation for the SpMM");
+                cudaGetLastError();
+                simt = true;                                    // no room for the copy
+                a.N = N; a.rhs_stride = rhs_stride;
+            }
+        }
+        if (!simt) {
+            e = cudaSuccess;
+            uint8_t* rest = static_cast<uint8_t*>(scratch);
+            if (copy_bytes) {
+                SpmmArgs src = a;
+                src.N = N; src.rhs_stride = rhs_stride;
+                e = launch_align_rows(src, (int)ld, static_cast<__half*>(scratch));
+                a.rhs = static_cast<const __half*>(scratch);
+                rest += copy_bytes;
+            }
+            if (e == cudaSuccess) e = use_block ? launch_sspmm_block(a, rest, room) : launch_sspmm_rows(a, nvec, want ? rest : nullptr);
+            if (scratch && !ex.caller_workspace) cudaFreeAsync(scratch, st);
+            return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
+        }
     }
-    void* scratch = nullptr;
-    keep_pool_memory();
-    e = cudaMallocAsync(&scratch, want, st);
-    if (e != cudaSuccess) return fail(e, "scratch allocation for the block kernel");
-    e = launch_sspmm_block(a, scratch, want);
-    cudaFreeAsync(scratch, st);
+    if (ex.query) return 0;
+    e = launch_sspmm_simt(a);
     return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
 }
 
@@ -321,6 +330,16 @@ int sspmm_f16_f16_batched(int m_vec, int vec_length, int N, int K, int batch, co
                           int64_t out_stride, void* stream) {
     return spmm_entry(m_vec, vec_length, N, K, batch, row_indices, row_offsets, column_indices, values_f16,
                       values_stride, rhs_f16, rhs_stride, out_f16, out_stride, true, stream);
+}
+
+int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nvec, const int* row_indices, const int* row_offsets,
+                  const int* column_indices, const void* values_f16, int64_t values_stride, const void* rhs_f16, int64_t rhs_stride,
+                  void* out, int64_t out_stride, int out_is_f16, void* stream) {
+    if (nvec < 0) { g_err[0] = 0; set_error("nvec must be >= 0"); return (int)cudaErrorInvalidValue; }
+    SpmmExtra ex;
+    ex.nvec = nvec;
+    return spmm_entry(m_vec, vec_length, N, K, batch, row_indices, row_offsets, column_indices, values_f16, values_stride, rhs_f16,
+                      rhs_stride, out, out_stride, out_is_f16 != 0, stream, ex);
 }
 
 int sspmm_workspace_bytes(int m_vec, int vec_length, int N, int K, int64_t nvec, int out_is_f16, int64_t* bytes) {

@@ -11,7 +11,8 @@ namespace sspmm_b200 {
 struct SpmmArgs {
     int m_vec;                 // vector rows
     int V;                     // rows per vector (8 or 16)
-    int N;                     // columns of the dense operand / of the output
+    int N;                     // columns of the dense operand as it is read (its row pitch)
+    int n_out;                 // columns of the output (its row pitch); N unless the dense operand is an aligned copy
     int K;                     // rows of the dense operand
     const int* row_indices;    // optional scheduling order of vector rows (may be null)
     const int* row_offsets;    // [m_vec + 1]
@@ -30,10 +31,12 @@ struct SpmmArgs {
 
 // tcgen05 row-gather kernel.  Requires N % 8 == 0, 16-byte aligned rhs/values.
 cudaError_t launch_sspmm_gather(const SpmmArgs& a);
-// tcgen05 row-gather kernel with load-instruction producers and splitting of long rows.
-// sspmm_gather_lsu_plan sizes the optional scratch from the vector count (chunk = cap = 0: no splitting).
-void sspmm_gather_lsu_plan(const SpmmArgs& a, long long nvec, int* chunk, int* cap, size_t* scratch_bytes);
-cudaError_t launch_sspmm_gather_lsu(const SpmmArgs& a, int chunk, int cap, void* scratch);
+// Row-gather kernel: N % 8 == 0, rhs and values 16-byte aligned; any n_out <= N.
+// scratch: null, or sspmm_rows_scratch_bytes() bytes when that is not 0 (long rows are then cut); nvec < 0: unknown.
+size_t sspmm_rows_scratch_bytes(const SpmmArgs& a, long long nvec);
+cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch);
+// Copy of the dense operand with rows of `ld` columns (a multiple of 8, zeros in the columns added).
+cudaError_t launch_align_rows(const SpmmArgs& a, int ld, __half* dst);
 // tcgen05 block kernel on a dense transposed copy of A held in `scratch` (caller-owned, stream-ordered).
 // sspmm_block_scratch_bytes(a) is what the kernel would like (copy of A + split-K partial tiles); with less
 // (at least K * m_vec*V halfs) it runs without split-K.

@@ -1129,17 +1129,36 @@ int sspmm_planned(const sspmm_plan* plan, const void* values_f16, const void* rh
     if (plan->m_vec == 0 || N == 0) return 0;
     if (!plan->fused) {
         // sparse or irregular structure: the regular entry points (gather kernels) take it
-        if (out_is_f16)
-            return sspmm_f16_f16(plan->m_vec, plan->V, N, plan->K, nullptr, plan->row_offsets, plan->column_indices, values_f16,
-                                 rhs_f16, out, stream);
-        return sspmm_f16_f32(plan->m_vec, plan->V, N, plan->K, nullptr, plan->row_offsets, plan->column_indices, values_f16,
-                             rhs_f16, static_cast<float*>(out), stream);
+        return sspmm_counted(plan->m_vec, plan->V, N, plan->K, 1, plan->nvec > 0 ? plan->nvec : 0, nullptr, plan->row_offsets,
+                             plan->column_indices, values_f16, 0, rhs_f16, 0, out, 0, out_is_f16, stream);
     }
     const int sms = current_device_sm_count();
     if (sms <= 0) return (int)cudaErrorNoDevice;
     // widest tile that still gives every SM a tile
     int BN = 256;
     while (BN > 64 && (int64_t)plan->m_tiles * ((N + BN - 1) / BN) < sms) BN >>= 1;
+    // The tile kernel walks the whole K range of a tile on one SM (about 0.6 us per 64 columns, 4 us of start-up); with few
+    // tiles the row-gather kernel, which spreads a row's vectors over the chip, is done sooner (see block_kernel_is_faster for
+    // its rate).  512 x 2048, N = 200, V = 16: 22.9 against 9.3 us; 512 x 4608, N = 256, V = 8: 45.6 against 15.0 us.  Both
+    // are one launch without scratch.
+    {
+        const double rounds = (double)(((int64_t)plan->m_tiles * ((N + BN - 1) / BN) + sms - 1) / sms);
+        const double t_tiles = 4.0e-6 + rounds * (plan->k_steps * 0.6e-6 * (BN == 256 ? 1.0 : 0.9) + 1.5e-6);
+        const double t_rows = 3.7e-6 + 2.0 * (double)plan->nvec * N / 8.3e12;
+        if (t_rows < t_tiles && N % 8 == 0 && values_f16 && rhs_f16 && out && fused::aligned16(values_f16) &&
+            fused::aligned16(rhs_f16) && fused::aligned16(out)) {
+            SpmmArgs a;
+            a.m_vec = plan->m_vec; a.V = plan->V; a.N = N; a.n_out = N; a.K = plan->K;
+            a.row_indices = nullptr; a.row_offsets = plan->row_offsets; a.column_indices = plan->column_indices;
+            a.values = static_cast<const __half*>(values_f16); a.rhs = static_cast<const __half*>(rhs_f16);
+            a.out = out; a.out_f16 = out_is_f16 != 0; a.batch = 1;
+            a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
+            a.stream = static_cast<cudaStream_t>(stream);
+            const cudaError_t e = launch_sspmm_rows(a, plan->nvec, nullptr);
+            if (e != cudaSuccess) { set_error("SpMM launch: %s", cudaGetErrorString(e)); return (int)e; }
+            return 0;
+        }
+    }
     fused::Params p;
     p.probs = nullptr; p.items = nullptr; p.dynamic = 0; p.queue = nullptr; p.partials = nullptr; p.counters = nullptr;
     p.jobs = nullptr; p.n_jobs = 0; p.expand_blocks = 0; p.expand_state = nullptr;

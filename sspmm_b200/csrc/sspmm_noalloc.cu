@@ -80,7 +80,7 @@ extern "C" int sspmm_f16_f16_noalloc(int m_vec, int vec_length, int N, int K, co
         return (int)e;
     }
     SpmmArgs a;
-    a.m_vec = m_vec; a.V = vec_length; a.N = N; a.K = K;
+    a.m_vec = m_vec; a.V = vec_length; a.N = N; a.n_out = N; a.K = K;
     a.row_indices = row_indices; a.row_offsets = row_offsets; a.column_indices = column_indices;
     a.values = static_cast<const __half*>(values_f16); a.rhs = static_cast<const __half*>(rhs_f16);
     a.out = out_f16; a.out_f16 = true; a.batch = 1;

@@ -1,0 +1,675 @@
+// Vector-sparse SpMM by rows, for operands whose dense tiles would be mostly padding and for products so small that
+// start-up latency decides: every warp gathers the rows of B that a vector row names and multiplies them by itself.
+//
+// Same contract as the other SpMM kernels (reference entry: SSpMM/src/sspmm.cu:626-649).
+//
+// What bounds it: every vector moves a row of B from L2 to an SM for V output rows, so the work is 2 * nvec * N bytes
+// of L2 reads, and a warp that waits for each of its reads in turn sees their full latency.  The split follows from
+// that: sixteen independent warps per SM, each with two or three steps of sixteen gathered rows in flight.
+// The arithmetic is 16 gathered rows per instruction (mma.m16n8k16, the transposed product
+//   D[n][v] += B^T[n][k] * vals[k][v]);
+// a tcgen05.mma of that depth holds its issuing thread for longer (about 130 cycles measured, plus 100 per commit) than
+// this path needs for the whole 16-row step, and its accumulators would have to come back from tensor memory for every
+// row.  A warp keeps its own ring of steps in shared memory, filled by cp.async (16 bytes per lane, eight lanes per 128
+// bytes of a row of B) and read by ldmatrix, so that neither side has bank conflicts; loading the fragments straight
+// into registers was tried and is bound by the L1 data stage (four rows of B per quarter warp fall on the same banks:
+// 6.0 TB/s of gathers where the ring reaches 9 to 10).
+//
+// Measured (graph replays, against the former kernel that passed stages of 64 rows to tcgen05.mma): 512 x 512 at 70 %, N =
+// 256: 5.4 us (12.7); 2048 x 512 at 90 %, V = 16, N = 256: 8.0 (16.6); 512 x 4608 at 90 %, N = 64: 7.5 (26.3).
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <climits>
+
+#include "launch.h"
+#include "ptx.cuh"
+
+namespace sspmm_b200 {
+namespace rows {
+
+constexpr int kWarps = 8;                 // per CTA
+constexpr int kThreads = kWarps * 32;
+constexpr int kStep = 16;                 // vectors per step
+constexpr int kLightRow = 256;            // split launches: longest row that one warp does
+constexpr int kMaxCluster = 8;
+constexpr int kResident = 2;              // CTAs per SM: 16 warps with three or four steps in flight each
+
+struct Problem {
+    int m_vec, K, n_tiles;
+    int N;                                // columns of C (and its row pitch)
+    int ldb;                              // row pitch of B, a multiple of 8: columns [N, ldb) exist and are multiplied along
+    long long items;                      // m_vec * n_tiles * batch
+    const int* row_indices;
+    const int* row_offsets;
+    const int* col;
+    const __half* values;
+    const __half* rhs;
+    int64_t values_stride, rhs_stride, out_stride;
+    int out_pieces;                       // rows of C start on 16-byte boundaries
+    // split launches only (see sspmm_rows_split_kernel)
+    int chunk, cap;                       // vectors per part of a cut row, room for parts
+    int* header;                          // [0] parts, [1] next row item
+    int* arrivals;                        // [part][n_tile], at a row's part 0: its finished parts
+    int4* entries;                        // per part: vector row, first vector, vectors, parts of the row << 16 | number
+    float* partial;                       // [part][n_tile][V][NT] sums
+};
+
+// d += a * b of one instruction: 16 columns x 8 rows of C, 16 vectors deep.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                          uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
+    const uint32_t bytes = valid ? 16u : 0u;                       // 0: the destination is zero-filled, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t& r0, uint32_t& r1, uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr) : "memory");
+}
+
+struct Where { int row, j0, len, n0, batch; };      // row = -1: nothing to do
+
+__device__ __forceinline__ Where locate(const Problem& p, long long T, int NT) {
+    Where w;
+    w.row = -1; w.j0 = 0; w.len = 0; w.n0 = 0; w.batch = 0;
+    if (T >= p.items) return w;
+    const int sched = (int)(T % p.m_vec);
+    const int rest = (int)(T / p.m_vec);
+    const int i = p.row_indices ? __ldg(p.row_indices + sched) : sched;
+    if ((unsigned)i >= (unsigned)p.m_vec) return w;
+    w.row = i;
+    w.n0 = (rest % p.n_tiles) * NT;
+    w.batch = rest / p.n_tiles;
+    w.j0 = __ldg(p.row_offsets + i);
+    w.len = max(0, __ldg(p.row_offsets + i + 1) - w.j0);
+    return w;
+}
+
+// V rows per vector, H 64-column halves per tile.
+// ROUND: every step is summed from zero and added to the accumulator by an fp32 addition that rounds to nearest (the
+// instruction's own additions truncate, which adds up over a long row); fp32 results only, fp16 ones hide the difference.
+template <int V, int H, bool ROUND>
+struct Tile {
+    static constexpr int NT = 64 * H;
+    static constexpr int VB = V / 8;
+    static constexpr int kStages = H == 2 ? 3 : 4;                  // steps in flight per warp
+    static constexpr int kRowBytes = NT * 2;
+    static constexpr int kStageBytes = kStep * kRowBytes + kStep * V * 2;
+    static constexpr int kPitch = NT + 4;                           // floats per row of the tile of sums (conflict-free)
+    static constexpr int kSumBytes = V * kPitch * 4;
+    // shared memory of one warp: the ring of steps, later the warp's tile of sums
+    static constexpr int kWarpBytes = kStages * kStageBytes > kSumBytes ? kStages * kStageBytes : kSumBytes;
+    static constexpr int kPieces = NT / 8;                          // eight-column pieces of a row of C
+    static constexpr int kUnits = V * kPieces / 32;                 // a unit: one piece per lane
+    static constexpr int kFloats = V * NT;
+    float acc[VB][4 * H][4];                                        // [rows 8 vb ..][columns 16 x ..][one instruction's]
+
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int vb = 0; vb < VB; ++vb)
+#pragma unroll
+            for (int x = 0; x < 4 * H; ++x)
+#pragma unroll
+                for (int d = 0; d < 4; ++d) acc[vb][x][d] = 0.f;
+    }
+    __device__ __forceinline__ void mma(int x, const uint32_t (&a)[4], const uint32_t (&b)[VB][2]) {
+#pragma unroll
+        for (int vb = 0; vb < VB; ++vb) {
+            if constexpr (ROUND) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_16816(d, a[0], a[1], a[2], a[3], b[vb][0], b[vb][1]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[vb][x][e] += d[e];
+            } else {
+                mma_16816(acc[vb][x], a[0], a[1], a[2], a[3], b[vb][0], b[vb][1]);
+            }
+        }
+    }
+    // Column ids of two steps, one per lane (lanes 0-15 the first step, 16-31 the second); -1 past the end.
+    static __device__ __forceinline__ int load_cols(const int* __restrict__ col, int j0, int len, int step, int stride, int lane) {
+        const unsigned idx = (unsigned)(step + (lane >> 4) * stride) * kStep + (lane & 15);
+        return idx < (unsigned)len ? __ldg(col + j0 + idx) : -1;
+    }
+    // Rows of the step land as [16 vectors][NT] with their 16-byte pieces XOR-swizzled by the vector number, so that the
+    // copies (eight lanes per 128 bytes) and ldmatrix (eight rows per matrix) both touch every bank once.
+    static __device__ __forceinline__ void copy_step(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs,
+                                                     int n0, int j0, int len, int s, int cols, int half, int lane, uint32_t slot) {
+        constexpr int kLanes = kPieces;                     // lanes per row of B
+        constexpr int kRows = 32 / kLanes;
+        const int piece = lane % kLanes;
+        const bool in_n = n0 + piece * 8 < p.ldb;
+        const __half* base = rhs + n0 + piece * 8;
+#pragma unroll
+        for (int i = 0; i < kStep / kRows; ++i) {
+            const int r = i * kRows + lane / kLanes;
+            const int c = __shfl_sync(0xffffffffu, cols, half * 16 + r);
+            const bool ok = in_n && (unsigned)c < (unsigned)p.K;
+            cp_async_16(slot + r * kRowBytes + ((piece ^ (r & 7)) << 4), ok ? base + (int64_t)c * p.ldb : rhs, ok);
+        }
+        const int k = lane / VB, part = lane % VB;
+        if (lane < kStep * VB) {
+            const unsigned idx = (unsigned)s * kStep + k;
+            const bool ok = idx < (unsigned)len;
+            cp_async_16(slot + kStep * kRowBytes + k * (V * 2) + ((V == 16 ? part ^ ((k >> 2) & 1) : 0) << 4),
+                        ok ? values + ((int64_t)j0 + idx) * V + part * 8 : values, ok);
+        }
+    }
+    __device__ __forceinline__ void multiply_step(uint32_t slot, int lane) {
+        uint32_t b[VB][2];
+        const int k = lane & 15;
+        const uint32_t vrow = slot + kStep * kRowBytes + k * (V * 2);
+        if constexpr (V == 8) {
+            ldmatrix_x2_trans(b[0][0], b[0][1], vrow);
+        } else {
+            uint32_t r[4];
+            ldmatrix_x4_trans(r, vrow + (((lane >> 4) ^ ((k >> 2) & 1)) << 4));
+            b[0][0] = r[0]; b[0][1] = r[1]; b[VB - 1][0] = r[2]; b[VB - 1][1] = r[3];
+        }
+        const int kr = (lane >> 4) * 8 + (lane & 7), odd = (lane >> 3) & 1;
+        const uint32_t row = slot + kr * kRowBytes;
+#pragma unroll
+        for (int x = 0; x < 4 * H; ++x) {
+            uint32_t a[4];
+            ldmatrix_x4_trans(a, row + (((2 * x + odd) ^ (kr & 7)) << 4));
+            mma(x, a, b);
+        }
+    }
+    // Adds steps first, first + stride, ... of vectors [j0, j0 + len).  The whole warp takes part; `mem` is its shared memory.
+    __device__ __forceinline__ void accumulate(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs, int n0,
+                                               int j0, int len, int first, int stride, int lane, uint32_t mem) {
+        const int steps = (int)(((unsigned)len + kStep - 1) / kStep);
+        if (first >= steps) return;
+        const int mine = (steps - first + stride - 1) / stride;         // steps of this warp
+        int cols = load_cols(p.col, j0, len, first, stride, lane);
+        int next = load_cols(p.col, j0, len, first + 2 * stride, stride, lane);
+        int issued = 0;
+        uint32_t fill = 0, use = 0;                                     // ring slots
+        auto issue = [&]() {
+            if (issued < mine)
+                copy_step(p, values, rhs, n0, j0, len, first + issued * stride, cols, issued & 1, lane, mem + fill * kStageBytes);
+            cp_async_commit();
+            if (issued & 1) {
+                cols = next;
+                next = load_cols(p.col, j0, len, first + (issued + 3) * stride, stride, lane);
+            }
+            ++issued;
+            fill = fill + 1 == kStages ? 0 : fill + 1;
+        };
+#pragma unroll
+        for (int k = 0; k < kStages - 1; ++k) issue();
+        for (int k = 0; k < mine; ++k) {
+            cp_async_wait<kStages - 2>();
+            __syncwarp();                           // everyone's copies are in, and the slot refilled next has been read
+            issue();
+            multiply_step(mem + use * kStageBytes, lane);
+            use = use + 1 == kStages ? 0 : use + 1;
+        }
+        cp_async_wait<0>();
+        __syncwarp();                               // the ring may be used for something else
+    }
+    // This warp's accumulators to its tile of sums [V][kPitch].
+    __device__ __forceinline__ void spill(float* dst, int lane) const {
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int vb = 0; vb < VB; ++vb)
+#pragma unroll
+            for (int x = 0; x < 4 * H; ++x)
+#pragma unroll
+                for (int d = 0; d < 4; ++d)
+                    dst[(vb * 8 + 2 * t + (d & 1)) * kPitch + 16 * x + g + 8 * (d >> 1)] = acc[vb][x][d];
+    }
+    // This lane's piece of unit u in a tile of sums.
+    static __device__ __forceinline__ int piece_at(int u, int lane) {
+        const int id = u * 32 + lane;
+        return (id / kPieces) * kPitch + (id % kPieces) * 8;
+    }
+    static __device__ __forceinline__ void add_piece(const float* src, float (&o)[8]) {
+        const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+        o[0] += lo.x; o[1] += lo.y; o[2] += lo.z; o[3] += lo.w;
+        o[4] += hi.x; o[5] += hi.y; o[6] += hi.z; o[7] += hi.w;
+    }
+    // Writes this lane's piece of unit u to C (first_row: the first of the vector row's V rows).
+    template <typename OutT>
+    static __device__ __forceinline__ void store_unit(const Problem& p, OutT* __restrict__ out, int64_t first_row, int n0, int u, int lane,
+                                                      const float (&o)[8]) {
+        const int id = u * 32 + lane, n = n0 + (id % kPieces) * 8;
+        OutT* dst = out + (first_row + id / kPieces) * p.N + n;
+        if (p.out_pieces) {
+            if (n >= p.N) return;                                // rows of C are whole pieces: all eight or none
+            if constexpr (sizeof(OutT) == 2) {
+                const __half2 h0 = __floats2half2_rn(o[0], o[1]), h1 = __floats2half2_rn(o[2], o[3]);
+                const __half2 h2 = __floats2half2_rn(o[4], o[5]), h3 = __floats2half2_rn(o[6], o[7]);
+                uint4 w;
+                w.x = *reinterpret_cast<const uint32_t*>(&h0); w.y = *reinterpret_cast<const uint32_t*>(&h1);
+                w.z = *reinterpret_cast<const uint32_t*>(&h2); w.w = *reinterpret_cast<const uint32_t*>(&h3);
+                *reinterpret_cast<uint4*>(dst) = w;
+            } else {
+                *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
+                *reinterpret_cast<float4*>(dst + 4) = make_float4(o[4], o[5], o[6], o[7]);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (n + e < p.N) {
+                    if constexpr (sizeof(OutT) == 2) dst[e] = __float2half_rn(o[e]);
+                    else dst[e] = o[e];
+                }
+        }
+    }
+    // Four columns of one row to C.
+    template <typename OutT>
+    static __device__ __forceinline__ void store_four(const Problem& p, OutT* __restrict__ out, int64_t row, int n, const float4& o) {
+        OutT* dst = out + row * p.N + n;
+        if (p.out_pieces) {
+            if (n >= p.N) return;
+            if constexpr (sizeof(OutT) == 2) {
+                const __half2 h0 = __floats2half2_rn(o.x, o.y), h1 = __floats2half2_rn(o.z, o.w);
+                *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            } else {
+                *reinterpret_cast<float4*>(dst) = o;
+            }
+        } else {
+            const float v[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (n + e < p.N) {
+                    if constexpr (sizeof(OutT) == 2) dst[e] = __float2half_rn(v[e]);
+                    else dst[e] = v[e];
+                }
+        }
+    }
+    // A warp's own tile to C, eight rows at a time through one slot of its ring.
+    template <typename OutT>
+    __device__ __forceinline__ void store(const Problem& p, OutT* __restrict__ out, int64_t first_row, int n0, float* slot, int lane) const {
+        static_assert(8 * kPitch * 4 <= kWarpBytes, "eight rows of sums fit the ring");
+        const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+        for (int vb = 0; vb < VB; ++vb) {
+#pragma unroll
+            for (int x = 0; x < 4 * H; ++x)
+#pragma unroll
+                for (int d = 0; d < 4; ++d) slot[(2 * t + (d & 1)) * kPitch + 16 * x + g + 8 * (d >> 1)] = acc[vb][x][d];
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < kUnits / VB; ++u) {
+                float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                add_piece(slot + piece_at(u, lane), o);
+                store_unit(p, out, first_row + vb * 8, n0, u, lane, o);
+            }
+            __syncwarp();
+        }
+    }
+};
+
+// One launch, no scratch: an item (vector row, column tile, batch entry) is done by `team` warps of a CTA (1, 2, 4 or 8)
+// or, with clusters, by all warps of `cluster` CTAs; the warps take 16-vector steps in turn and their sums are added in
+// warp order through shared memory (of the cluster), so results do not depend on timing.
+template <int V, typename OutT, int H>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int team, int cluster) {
+    using T = Tile<V, H, sizeof(OutT) == 4>;
+    extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int per_cta = kWarps / team;
+    const int rank = cluster > 1 ? (int)cluster_cta_rank() : 0;
+    const long long cta_item = (long long)(blockIdx.x / cluster) * per_cta;
+    const int member = warp % team;
+    const Where w = locate(p, cta_item + warp / team, T::NT);
+    uint8_t* const mem = smem + warp * T::kWarpBytes;
+    T tile;
+    tile.clear();
+    if (w.row >= 0)
+        tile.accumulate(p, p.values + w.batch * p.values_stride, p.rhs + w.batch * p.rhs_stride, w.n0, w.j0, w.len, rank * team + member,
+                        team * cluster, lane, smem_u32(mem));
+    OutT* const cbase = out + w.batch * p.out_stride;
+    const int64_t first_row = (int64_t)w.row * V;
+    if (team == 1) {
+        if (w.row >= 0) tile.store(p, cbase, first_row, w.n0, reinterpret_cast<float*>(mem), lane);
+        return;
+    }
+    tile.spill(reinterpret_cast<float*>(mem), lane);
+    __syncthreads();
+    static_assert(T::kUnits <= kWarps && T::kFloats * 4 <= kWarps * T::kWarpBytes, "one unit per warp");
+    float kept[8];
+    for (int u = member; u < T::kUnits; u += team) {
+        float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int m = 0; m < team; ++m)
+            T::add_piece(reinterpret_cast<const float*>(smem + (warp - member + m) * T::kWarpBytes) + T::piece_at(u, lane), o);
+        if (cluster == 1) {
+            if (w.row >= 0) T::store_unit(p, cbase, first_row, w.n0, u, lane, o);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) kept[e] = o[e];
+        }
+    }
+    if (cluster == 1) return;
+    __syncthreads();                                      // the warps' tiles are read: the CTA's tile takes their place
+    float* const whole = reinterpret_cast<float*>(smem);
+    if (warp < T::kUnits)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) whole[(warp * 8 + e) * 32 + lane] = kept[e];
+    cluster_sync_all();                                   // every CTA's tile is complete and visible
+    for (int u = warp; u < T::kUnits; u += kWarps) {
+        if (u % cluster != rank) continue;                // the units are dealt over the CTAs
+        float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        const uint32_t at = smem_u32(whole + u * 256 + lane);
+        for (int c = 0; c < cluster; ++c) {
+            const uint32_t remote = cluster_map_shared(at, (uint32_t)c);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] += ld_cluster_f32(remote + e * 128);
+        }
+        if (w.row >= 0) T::store_unit(p, cbase, first_row, w.n0, u, lane, o);
+    }
+    cluster_sync_all();                                   // nobody leaves while its tile is being read
+}
+
+// Matrices whose rows differ in length by orders of magnitude (power-law matrices: half of the rows have fewer than 50
+// vectors, the longest tens of thousands; n = 51970, V = 8, N = 128: 46.8 us, with one CTA of tcgen05 stages per SM 67.8).
+// Rows longer than kLightRow are cut into parts of at most p.chunk vectors (listed by list_parts_kernel); a CTA does a
+// part with all its warps, the parts dealt out in turn since they are of one size, and whoever finishes the last part of
+// a row adds the parts up in order.  Then the warps, each on its own, take the remaining rows in the caller's order from
+// a counter.
+template <int V, typename OutT, int H>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_split_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
+    using T = Tile<V, H, sizeof(OutT) == 4>;
+    extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
+    __shared__ int seen;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint8_t* const mem = smem + warp * T::kWarpBytes;
+    // The list was sized from a vector count; if the matrix needs more parts than fit, nothing is cut.
+    const int listed = p.header[0];
+    const bool cut = listed <= p.cap;
+    const int parts_total = cut ? listed * p.n_tiles : 0;
+    const int none = INT_MAX;
+    int x = (int)blockIdx.x < parts_total ? (int)blockIdx.x : none;
+    int4 en = x < parts_total ? p.entries[x / p.n_tiles] : make_int4(0, 0, 0, 0);
+    while (x < parts_total) {
+        const int x2 = x < parts_total - (int)gridDim.x ? x + (int)gridDim.x : none;
+        int4 en2 = make_int4(0, 0, 0, 0);
+        if (x2 < parts_total) en2 = p.entries[x2 / p.n_tiles];
+        const int nt = x % p.n_tiles, part = en.w & 0xffff, parts = (int)((unsigned)en.w >> 16);
+        T tile;
+        tile.clear();
+        tile.accumulate(p, p.values, p.rhs, nt * T::NT, en.y, en.z, warp, kWarps, lane, smem_u32(mem));
+        tile.spill(reinterpret_cast<float*>(mem), lane);
+        __syncthreads();
+        const int first = x - part * p.n_tiles;                          // the row's part 0 for this column tile
+        for (int u = warp; u < T::kUnits; u += kWarps) {
+            float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int m = 0; m < kWarps; ++m)
+                T::add_piece(reinterpret_cast<const float*>(smem + m * T::kWarpBytes) + T::piece_at(u, lane), o);
+            if (parts == 1) {
+                T::store_unit(p, out, (int64_t)en.x * V, nt * T::NT, u, lane, o);
+            } else {
+                float4* dst = reinterpret_cast<float4*>(p.partial + (int64_t)x * T::kFloats) + u * 64 + lane * 2;
+                __stcg(dst, make_float4(o[0], o[1], o[2], o[3]));
+                __stcg(dst + 1, make_float4(o[4], o[5], o[6], o[7]));
+            }
+        }
+        if (parts > 1) {
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) seen = atomicAdd(p.arrivals + first, 1);
+            __syncthreads();
+            if (seen == parts - 1) {
+                // four columns per thread; sixteen parts' loads are under way together
+                __threadfence();
+                const int64_t step = (int64_t)p.n_tiles * (T::kFloats / 4);
+                for (int f = threadIdx.x; f < T::kFloats / 4; f += kThreads) {
+                    const float4* src = reinterpret_cast<const float4*>(p.partial + (int64_t)first * T::kFloats) + f;
+                    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int c0 = 0; c0 < parts; c0 += 16) {
+                        float4 v[16];
+#pragma unroll
+                        for (int c = 0; c < 16; ++c)
+                            v[c] = c0 + c < parts ? __ldcg(src + (c0 + c) * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) { o.x += v[c].x; o.y += v[c].y; o.z += v[c].z; o.w += v[c].w; }
+                    }
+                    T::store_four(p, out, (int64_t)en.x * V + f * 4 / T::NT, nt * T::NT + f * 4 % T::NT, o);
+                }
+            }
+        }
+        __syncthreads();                                  // the tiles of sums and `seen` are free again
+        x = x2; en = en2;
+    }
+    // row items, one warp each; the next item is looked up while the current one is in work
+    auto take = [&]() {
+        int T0 = 0;
+        if (lane == 0) T0 = atomicAdd(p.header + 1, 1);
+        return (long long)__shfl_sync(0xffffffffu, T0, 0);
+    };
+    long long at = take();
+    Where w = locate(p, at, T::NT);
+    while (at < p.items) {
+        const long long at2 = take();
+        const Where w2 = locate(p, at2, T::NT);
+        if (w.row >= 0 && !(cut && w.len > kLightRow)) {
+            T tile;
+            tile.clear();
+            tile.accumulate(p, p.values, p.rhs, w.n0, w.j0, w.len, 0, 1, lane, smem_u32(mem));
+            tile.store(p, out, (int64_t)w.row * V, w.n0, reinterpret_cast<float*>(mem), lane);
+        }
+        at = at2; w = w2;
+    }
+}
+
+// The list of parts (the parts of a row are consecutive, part 0 first), cleared arrival counters and, with one CTA, the
+// header; with several the header is zero at launch.
+__global__ void __launch_bounds__(1024)
+list_parts_kernel(const __grid_constant__ Problem p) {
+    __shared__ int count;
+    const bool alone = gridDim.x == 1;
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    const int stride = gridDim.x * 1024;
+    for (int x = blockIdx.x * 1024 + threadIdx.x; x < p.cap * p.n_tiles; x += stride) p.arrivals[x] = 0;
+    for (int64_t b = blockIdx.x * 1024 + threadIdx.x; b < p.m_vec; b += 4LL * stride) {
+        int j0[4], len[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t i = b + (int64_t)k * stride;
+            j0[k] = i < p.m_vec ? __ldg(p.row_offsets + i) : 0;
+            len[k] = i < p.m_vec ? __ldg(p.row_offsets + i + 1) - j0[k] : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (len[k] <= kLightRow) continue;
+            const int n = (len[k] + p.chunk - 1) / p.chunk;
+            const int first = alone ? atomicAdd(&count, n) : atomicAdd(p.header, n);
+            for (int c = 0; c < n && first + c < p.cap; ++c)
+                p.entries[first + c] = make_int4((int)(b + (int64_t)k * stride), j0[k] + c * p.chunk, min(p.chunk, len[k] - c * p.chunk), n << 16 | c);
+        }
+    }
+    __syncthreads();
+    if (alone && threadIdx.x == 0) { p.header[0] = count; p.header[1] = 0; }
+}
+
+template <typename Kern>
+cudaError_t allow_smem(Kern kern, DeviceOnce& once, int bytes) {
+    if (once.done()) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    if (bytes > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) once.mark();
+    return e;
+}
+
+template <int V, typename OutT, int H>
+cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, int team, int cluster) {
+    auto kern = sspmm_rows_kernel<V, OutT, H>;
+    using T = Tile<V, H, sizeof(OutT) == 4>;
+    static DeviceOnce once;
+    cudaError_t e = allow_smem(kern, once, kWarps * T::kWarpBytes);
+    if (e != cudaSuccess) return e;
+    const int per_cta = kWarps / team;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((p.items + per_cta - 1) / per_cta * cluster));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)kWarps * T::kWarpBytes; cfg.stream = a.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, p, static_cast<OutT*>(a.out), team, cluster);
+}
+
+template <int V, typename OutT, int H>
+cudaError_t launch_split(const SpmmArgs& a, const Problem& p, int sms) {
+    auto kern = sspmm_rows_split_kernel<V, OutT, H>;
+    constexpr int kBytes = kWarps * Tile<V, H, sizeof(OutT) == 4>::kWarpBytes;
+    static DeviceOnce once;
+    cudaError_t e = allow_smem(kern, once, kBytes);
+    if (e != cudaSuccess) return e;
+    const bool alone = a.m_vec <= 16384;                  // one CTA saves the launch that clears the header
+    if (!alone) {
+        e = cudaMemsetAsync(p.header, 0, 16, a.stream);
+        if (e != cudaSuccess) return e;
+    }
+    list_parts_kernel<<<alone ? 1 : sms, 1024, 0, a.stream>>>(p);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    kern<<<sms * kResident, kThreads, kBytes, a.stream>>>(p, static_cast<OutT*>(a.out));
+    return cudaGetLastError();
+}
+
+template <int V, typename OutT>
+cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, bool split, int team, int cluster, int sms) {
+    if (split) return H == 2 ? launch_split<V, OutT, 2>(a, p, sms) : launch_split<V, OutT, 1>(a, p, sms);
+    return H == 2 ? launch_plain<V, OutT, 2>(a, p, team, cluster) : launch_plain<V, OutT, 1>(a, p, team, cluster);
+}
+
+// Scratch of the variant that cuts rows: [16 B header][cap * n_tiles arrival counters][cap entries][partial tiles].
+struct Scratch {
+    int chunk = 0, cap = 0;                 // chunk = 0: not worth cutting
+    size_t entries_at = 0, partial_at = 0, bytes = 0;
+};
+// Rows are worth cutting when some row may be many times the mean: the columns bound a row's length, so K tells, and the
+// vector count tells the mean.
+Scratch plan_scratch(const SpmmArgs& a, long long nvec) {
+    Scratch r;
+    if (nvec <= 0 || a.batch != 1) return r;
+    const long long mean = nvec / a.m_vec + 1;
+    if (a.K < 2048 || a.K < 8 * mean) return r;
+    const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;
+    const long long nt = a.N <= 64 ? 64 : 128, n_tiles = (a.N + nt - 1) / nt;
+    // A part: a quarter of an SM's share of the vectors, at least four steps per warp.  n = 51970 (820 k vectors, V = 8,
+    // N = 128) takes 46.8 us with a quarter, 52.1 with an eighth and 78 with a sixteenth (every part drains the rings once).
+    long long c = nvec * n_tiles / ((long long)sms * 4) / 128 * 128;
+    if (c < 512) c = 512;
+    // every cut row has at most one part that is not full
+    const long long cap = nvec / c + nvec / kLightRow + 1;
+    const long long tiles = cap * n_tiles;
+    if (c > 0x3fffffff || a.K / c >= 32767 || tiles > 0x3fffffff || tiles * a.V * nt * 4 > (1LL << 30)) return r;
+    r.chunk = (int)c; r.cap = (int)cap;
+    r.entries_at = 16 + (((size_t)tiles * 4 + 15) & ~(size_t)15);
+    r.partial_at = r.entries_at + (size_t)cap * 16;
+    r.bytes = (r.partial_at + (size_t)tiles * a.V * nt * 4 + 255) & ~(size_t)255;
+    return r;
+}
+
+// Copies [rows][N] (any alignment) to [rows][ld], ld a multiple of 8, zeros in the columns added: one 16-byte piece of
+// the copy per thread.
+__global__ void __launch_bounds__(256)
+align_rows_kernel(const __half* __restrict__ src, __half* __restrict__ dst, int K, int N, int ld, int batch, int64_t src_stride) {
+    const int pieces = ld / 8;
+    const int64_t total = (int64_t)K * batch * pieces;
+    for (int64_t x = (int64_t)blockIdx.x * 256 + threadIdx.x; x < total; x += (int64_t)gridDim.x * 256) {
+        const int64_t r = x / pieces;
+        const int n = (int)(x - r * pieces) * 8;
+        const int64_t b = r / K;
+        const unsigned short* s = reinterpret_cast<const unsigned short*>(src + b * src_stride + (r - b * K) * N) + n;
+        unsigned short h[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) h[e] = n + e < N ? __ldg(s + e) : (unsigned short)0;
+        uint4 w;
+        w.x = h[0] | (uint32_t)h[1] << 16; w.y = h[2] | (uint32_t)h[3] << 16;
+        w.z = h[4] | (uint32_t)h[5] << 16; w.w = h[6] | (uint32_t)h[7] << 16;
+        *reinterpret_cast<uint4*>(dst + x * 8) = w;
+    }
+}
+
+}  // namespace rows
+
+size_t sspmm_rows_scratch_bytes(const SpmmArgs& a, long long nvec) { return rows::plan_scratch(a, nvec).bytes; }
+
+// scratch: null, or sspmm_rows_scratch_bytes() bytes (long rows are then cut); nvec < 0: unknown.
+cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    rows::Problem p;
+    p.m_vec = a.m_vec; p.N = a.n_out; p.ldb = a.N; p.K = a.K;
+    p.row_indices = a.row_indices; p.row_offsets = a.row_offsets; p.col = a.column_indices;
+    p.values = a.values; p.rhs = a.rhs;
+    p.values_stride = a.values_stride; p.rhs_stride = a.rhs_stride; p.out_stride = a.out_stride;
+    p.chunk = 0; p.cap = 0; p.header = nullptr; p.arrivals = nullptr; p.entries = nullptr; p.partial = nullptr;
+    const size_t es = a.out_f16 ? 2 : 4;
+    p.out_pieces = (a.n_out % 8 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 &&
+                    (a.batch == 1 || ((size_t)a.out_stride * es) % 16 == 0)) ? 1 : 0;
+    const bool split = scratch != nullptr;
+    // Tile width: 128 columns halve the work per gathered byte outside the loads; 64 when that is all there is or (one-launch
+    // kernel) when wide tiles, a CTA each, would leave SMs without one.
+    const long long rows_total = (long long)a.m_vec * a.batch;
+    const long long mean_steps = nvec > 0 ? (nvec / a.m_vec + rows::kStep) / rows::kStep : (a.K / 2 + rows::kStep) / rows::kStep;
+    const long long slots = (long long)sms * rows::kResident * rows::kWarps;
+    int H = a.N > 64 ? 2 : 1;
+    if (H == 2 && !split && rows_total * ((a.N + 127) / 128) * std::min<long long>(mean_steps, rows::kWarps) < slots) H = 1;
+    const int nt = 64 * H;
+    p.n_tiles = (a.N + nt - 1) / nt;
+    p.items = rows_total * p.n_tiles;
+    if (p.items + slots > 0x7fffffffLL / rows::kMaxCluster) {
+        set_error("problem too large for 32-bit tile ids");
+        return cudaErrorInvalidValue;
+    }
+    int team = 1, cluster = 1;
+    if (split) {
+        const rows::Scratch r = rows::plan_scratch(a, nvec);
+        uint8_t* s = static_cast<uint8_t*>(scratch);
+        p.chunk = r.chunk; p.cap = r.cap;
+        p.header = reinterpret_cast<int*>(s);
+        p.arrivals = reinterpret_cast<int*>(s + 16);
+        p.entries = reinterpret_cast<int4*>(s + r.entries_at);
+        p.partial = reinterpret_cast<float*>(s + r.partial_at);
+    } else {
+        // Warps per item: enough to fill the SMs, at least one step each; long rows get a whole CTA so that no single
+        // warp runs long after the others.
+        const long long want = std::min(slots / p.items, mean_steps);
+        while (team < rows::kWarps && (2 * team <= want || mean_steps > 32LL * team)) team *= 2;
+        if (team == rows::kWarps)
+            while (cluster < rows::kMaxCluster && (long long)cluster * 2 * team <= want && mean_steps >= 4LL * cluster * team) cluster *= 2;
+    }
+    if (a.V == 16)
+        return a.out_f16 ? rows::launch_typed<16, __half>(a, p, H, split, team, cluster, sms) : rows::launch_typed<16, float>(a, p, H, split, team, cluster, sms);
+    return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, split, team, cluster, sms) : rows::launch_typed<8, float>(a, p, H, split, team, cluster, sms);
+}
+
+// ---- dense operands whose rows do not start on 16-byte boundaries -------------------------------
+cudaError_t launch_align_rows(const SpmmArgs& a, int ld, __half* dst) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    const int64_t blocks = ((int64_t)a.K * a.batch * (ld / 8) + 255) / 256;
+    rows::align_rows_kernel<<<(unsigned)std::min<int64_t>(blocks, (int64_t)sms * 32), 256, 0, a.stream>>>(a.rhs, dst, a.K, a.N, ld, a.batch, a.rhs_stride);
+    return cudaGetLastError();
+}
+
+}  // namespace sspmm_b200

@@ -1,7 +1,6 @@
-// CUDA-core variant of the vector-sparse SpMM for operands the tensor-core path
-// cannot take: N not a multiple of 8, or pointers that are not 16-byte aligned.
-// Same contract as the reference entry (SSpMM/src/sspmm.cu:626-649); fp32
-// accumulation in the order of the column list.
+// CUDA-core variant of the vector-sparse SpMM for operands the tensor-core paths cannot take: K = 0, value vectors that
+// are not 16-byte aligned, or an unaligned dense operand (any N) when there is no room for an aligned copy of it.
+// Same contract as the reference entry (SSpMM/src/sspmm.cu:626-649); fp32 accumulation in the order of the column list.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 

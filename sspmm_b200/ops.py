@@ -53,9 +53,9 @@ def sspmm(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: torch
     K, N = rhs.shape
     if out is None:
         out = torch.empty((m_vec * vec_length, N), dtype=out_dtype, device=rhs.device)
-    fn = capi.lib().sspmm_f16_f16 if out.dtype == torch.float16 else capi.lib().sspmm_f16_f32
-    args = (m_vec, vec_length, N, K, _ptr(row_indices), row_offsets.data_ptr(), column_indices.data_ptr(),
-            values.data_ptr(), rhs.data_ptr(), out.data_ptr())
+    fn = capi.lib().sspmm_counted
+    args = (m_vec, vec_length, N, K, 1, column_indices.numel(), _ptr(row_indices), row_offsets.data_ptr(), column_indices.data_ptr(),
+            values.data_ptr(), 0, rhs.data_ptr(), 0, out.data_ptr(), 0, 1 if out.dtype == torch.float16 else 0)
     if torch.cuda.current_device() == rhs.device.index:
         rc = fn(*args, _stream_ptr())
     else:

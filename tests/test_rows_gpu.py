@@ -1,0 +1,112 @@
+"""GPU parity tests of the row-gather kernel and of the choice between it, the block kernel and the aligned copy of B, at
+the sizes where they can go wrong: one vector, one step and one more, rows of one CTA and of a cluster, partial column
+tiles, unaligned dense operands, row orders, rows that are cut.
+
+Tolerance: a sum of n products of fp16 numbers in fp32 in any order is within n * 2^-23 * sum|a||b| of the exact one (the
+tensor cores truncate, hence 2^-23 and not 2^-24); fp16 output adds half a unit of the result, 2^-11 |c|."""
+import numpy as np
+import pytest
+import torch
+
+from sspmm_b200 import ops
+from sspmm_b200.sptrans.spmm import bspmm
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def operands(lens, K, V, N, seed, offset=0):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(seed)
+    ptr = torch.zeros(len(lens) + 1, dtype=torch.int32, device=DEV)
+    ptr[1:] = torch.cumsum(torch.tensor(lens, device=DEV), 0)
+    nvec = int(ptr[-1])
+    col = torch.cat([torch.randperm(K, device=DEV, generator=g)[:n] for n in lens]).int()
+    val = (torch.rand(nvec * V, device=DEV, generator=g) * 2 - 1).half()
+    flat = torch.randn(K * N + offset, device=DEV, generator=g).half()
+    return ptr, col, val, flat[offset:].view(K, N)
+
+
+def exact(ptr, col, val, rhs, V):
+    """The product and the sums of magnitudes, in 64 bits."""
+    m = ptr.numel() - 1
+    rows = torch.repeat_interleave(torch.arange(m, device=DEV), (ptr[1:] - ptr[:-1]).long())
+    a = torch.zeros(m * V, rhs.shape[0], dtype=torch.float64, device=DEV)
+    v = val.double().view(-1, V)
+    for r in range(V):
+        a[rows * V + r, col.long()] = v[:, r]
+    return a @ rhs.double(), a.abs() @ rhs.double().abs()
+
+
+def check(got, ptr, col, val, rhs, V):
+    ref, mag = exact(ptr, col, val, rhs, V)
+    n = int((ptr[1:] - ptr[:-1]).max())
+    bound = max(n, 1) * 2.0 ** -23 * mag + 1e-30
+    if got.dtype == torch.float16:
+        bound = bound + 2.0 ** -11 * ref.abs() + 2.0 ** -24
+    assert (got.double() - ref).abs().le(bound).all()
+    assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("lens,K,N", [
+    ([1], 64, 8), ([16, 17, 0, 15, 33], 64, 72), ([300] * 3, 512, 64), ([2600, 1, 0], 4608, 136), ([700] * 300, 1024, 128),
+    ([40] * 3000, 300, 200)])
+@pytest.mark.parametrize("kernel", [ops.KERNEL_AUTO, ops.KERNEL_GATHER_LSU])
+def test_tile_edges_teams_and_clusters(lib, V, lens, K, N, kernel):
+    ptr, col, val, rhs = operands(lens, K, V, N, 3)
+    ops.set_kernel(kernel)
+    try:
+        for dt in (torch.float16, torch.float32):
+            check(ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt), ptr, col, val, rhs, V)
+    finally:
+        ops.set_kernel(ops.KERNEL_AUTO)
+
+
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("lens,K,N,offset", [([5, 0, 40], 64, 1, 0), ([900] * 4, 1000, 49, 0), ([40] * 20, 64, 50, 0), ([40] * 20, 64, 64, 3),
+                                             ([1000] * 64, 1024, 1001, 1)])
+def test_unaligned_dense_operand(lib, V, lens, K, N, offset):
+    """N not a multiple of 8, rhs off its 16-byte boundary; the last one runs the block kernel on the aligned copy."""
+    ptr, col, val, rhs = operands(lens, K, V, N, 4, offset)
+    for kernel in (ops.KERNEL_AUTO, ops.KERNEL_GATHER_LSU, ops.KERNEL_BLOCK, ops.KERNEL_SIMT):
+        ops.set_kernel(kernel)
+        try:
+            for dt in (torch.float16, torch.float32):
+                check(ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt), ptr, col, val, rhs, V)
+        finally:
+            ops.set_kernel(ops.KERNEL_AUTO)
+
+
+@pytest.mark.parametrize("V,N", [(8, 40), (8, 200), (16, 136)])
+def test_cut_rows_any_order(lib, V, N):
+    """One row of two parts, one of many, rows at both sides of what a warp does alone; any order gives the same numbers."""
+    lens = [257, 256, 0, 1, 600, 2900] + [20] * 200
+    ptr, col, val, rhs = operands(lens, 3000, V, N, 5)
+    base = ops.sspmm(ptr, col, val, rhs, V, out_dtype=torch.float32)
+    check(base, ptr, col, val, rhs, V)
+    order = torch.randperm(len(lens), device=DEV).int()
+    assert torch.equal(base, ops.sspmm(ptr, col, val, rhs, V, row_indices=order, out_dtype=torch.float32))
+    check(ops.sspmm(ptr, col, val, rhs, V), ptr, col, val, rhs, V)
+
+
+@pytest.mark.parametrize("V,N", [(8, 64), (16, 49)])
+def test_batches(lib, V, N):
+    lens = [51, 0, 70, 16]
+    ptr, col, val, _ = operands(lens, 80, V, 8, 6)
+    rhs = torch.randn(5, 80, N, device=DEV).half()
+    vals = torch.stack([val * s for s in (1.0, -1.0, 0.5, 2.0, 0.25)])
+    order = torch.arange(len(lens), dtype=torch.int32, device=DEV)
+    got = bspmm(order, ptr, col, vals, rhs, V)
+    for b in range(5):
+        check(got[b], ptr, col, vals[b], rhs[b], V)
+
+
+@pytest.mark.parametrize("V,M,K,N", [(8, 512, 2048, 200), (16, 64, 64, 8), (16, 1500, 3000, 72)])
+def test_planned_small_products(lib, V, M, K, N):
+    lens = [int(x) for x in np.random.default_rng(7).integers(K // 2, K, -(-M // V))]
+    ptr, col, val, rhs = operands(lens, K, V, N, 8)
+    plan = ops.Plan(ptr, col, V, K)
+    assert plan.one_launch
+    for dt in (torch.float16, torch.float32):
+        check(ops.sspmm_planned(plan, val, rhs, out_dtype=dt), ptr, col, val, rhs, V)
