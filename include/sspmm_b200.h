@@ -63,11 +63,12 @@ int sspmm_f16_f16_batched(int m_vec, int vec_length, int N, int K, int batch, co
  * The three calls above for a caller that knows the vector count nvec = row_offsets[m_vec] (the compression returns it):
  * nothing is read back or remembered and the call never synchronises.  nvec decides which kernel runs and how the work is
  * cut, never the result: a count that is only an upper bound (the length of column_indices) will do.  fp16 or fp32 output;
- * batch and strides as in sspmm_f16_f16_batched.
+ * batch and strides as in sspmm_f16_f16_batched.  bias_f16 (may be NULL): m_vec*V numbers, one per row of the output,
+ * added to the fp32 sums before the conversion.
  */
 int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nvec, const int* row_indices, const int* row_offsets,
                   const int* column_indices, const void* values_f16, int64_t values_stride, const void* rhs_f16, int64_t rhs_stride,
-                  void* out, int64_t out_stride, int out_is_f16, void* stream);
+                  const void* bias_f16, void* out, int64_t out_stride, int out_is_f16, void* stream);
 
 /*
  * Same product as sspmm_f16_f16, for callers that must not allocate device memory when they call:
@@ -225,6 +226,28 @@ int sspmm_device_status(int* status);
  * No counterpart in the reference (its kernels have no waits).
  */
 int sspmm_selftest_wait_expiry(long long limit_cycles, int* gave_up);
+
+/* ------------------------------------------------- encoder layer, feature-major --- */
+
+/*
+ * LayerNorm over the features of feature-major activations x[hidden][tokens] (fp16), statistics and normalisation in fp32:
+ * out[f][t] = (s[f][t] - mean_t) / sqrt(var_t + eps) * gamma[f] + beta[f], s = x + bias[f] + add[f][t] (either may be NULL;
+ * rounded to fp16 after each addition); with add, s is also written to sum_out.  tokens % 8 == 0, 16-byte aligned arrays, hidden <= 3072; 1 otherwise.
+ */
+int sspmm_layer_norm_fm(int hidden, int tokens, const void* x_f16, const void* bias_f16, const void* add_f16, void* sum_out_f16, const void* gamma_f16,
+                        const void* beta_f16, float eps, void* out_f16, void* stream);
+
+/* out = x + bias[f] + add on feature-major [rows][tokens] fp16, rounded after each addition; tokens % 8 == 0, 16-byte aligned. */
+int sspmm_add_bias_fm(int rows, int tokens, const void* x_f16, const void* bias_f16, const void* add_f16, void* out_f16, void* stream);
+
+/*
+ * Softmax attention on feature-major activations: q, k, v, out are [heads*64][batch*seq] fp16, token t of sequence b in
+ * column b*seq + t; scores scaled by 1/8, softmax in fp32, probabilities kept to 22 bits.
+ * bias_q, bias_v (may be NULL): fp16 per feature, added to q and v; one of k has no effect on the result.  Head width 64, seq % 8 == 0,
+ * 16-byte aligned arrays; 1 otherwise.
+ */
+int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* q_f16, const void* k_f16, const void* v_f16,
+                       const void* bias_q_f16, const void* bias_v_f16, void* out_f16, void* stream);
 
 /* ------------------------------------------------------------------- SVC --- */
 

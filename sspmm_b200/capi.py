@@ -18,7 +18,7 @@ SIGNATURES = {
     "sspmm_f16_f32": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_f16_f16": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_f16_f16_batched": (C.c_int, [C.c_int] * 5 + [_vp, _vp, _vp, _vp, C.c_int64, _vp, C.c_int64, _vp, C.c_int64, _vp]),
-    "sspmm_counted": (C.c_int, [C.c_int] * 5 + [C.c_int64, _vp, _vp, _vp, _vp, C.c_int64, _vp, C.c_int64, _vp, C.c_int64, C.c_int, _vp]),
+    "sspmm_counted": (C.c_int, [C.c_int] * 5 + [C.c_int64, _vp, _vp, _vp, _vp, C.c_int64, _vp, C.c_int64, _vp, _vp, C.c_int64, C.c_int, _vp]),
     "sspmm_f16_f16_noalloc": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_workspace_bytes": (C.c_int, [C.c_int] * 4 + [C.c_int64, C.c_int, C.POINTER(C.c_int64)]),
     "sspmm_f16_f16_ws": (C.c_int, [C.c_int] * 4 + [_vp] * 6 + [C.c_int64, _vp, C.c_int64, _vp]),
@@ -27,6 +27,9 @@ SIGNATURES = {
     "sspmm_plan_info": (C.c_int, [_vp, C.POINTER(C.c_int64), c_int_p, c_int_p, C.POINTER(C.c_int64)]),
     "sspmm_planned": (C.c_int, [_vp, _vp, _vp, _vp, C.c_int, C.c_int, _vp]),
     "sspmm_group_create": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, C.POINTER(_vp)]),
+    "sspmm_layer_norm_fm": (C.c_int, [C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, _vp, C.c_float, _vp, _vp]),
+    "sspmm_add_bias_fm": (C.c_int, [C.c_int] * 2 + [_vp] * 5),
+    "sspmm_attention_fm": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_group_run": (C.c_int, [_vp, _vp]),
     "sspmm_group_info": (C.c_int, [_vp, c_int_p, c_int_p, c_int_p, c_int_p, C.POINTER(C.c_int64)]),
     "sspmm_group_destroy": (C.c_int, [_vp]),

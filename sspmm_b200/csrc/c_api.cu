@@ -170,6 +170,7 @@ struct SpmmExtra {
     size_t workspace_bytes = 0;
     bool caller_workspace = false;
     size_t* query = nullptr;
+    const void* bias = nullptr;
 };
 
 static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_indices, const int* row_offsets,
@@ -196,11 +197,12 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
     a.m_vec = m_vec; a.V = V; a.N = N; a.n_out = N; a.K = K;
     a.row_indices = row_indices; a.row_offsets = row_offsets; a.column_indices = column_indices;
     a.values = static_cast<const __half*>(values); a.rhs = static_cast<const __half*>(rhs);
-    a.out = out; a.out_f16 = out_f16; a.batch = batch;
+    a.out = out; a.out_f16 = out_f16; a.bias = static_cast<const __half*>(ex.bias); a.batch = batch;
     a.values_stride = values_stride; a.rhs_stride = rhs_stride; a.out_stride = out_stride;
     a.stream = st;
 
-    const int choice = g_kernel_choice.load();
+    int choice = g_kernel_choice.load();
+    if (choice == 1 && a.bias) choice = 4;                     // the TMA gather kernel adds no bias
     const bool values_ok = aligned16(values) && (values_stride * 2) % 16 == 0;
     const bool rhs_ok = N % 8 == 0 && aligned16(rhs) && (batch == 1 || (rhs_stride * 2) % 16 == 0);
     if (choice == 1 && !(K > 0 && values_ok && rhs_ok && (batch == 1 || rhs_stride == (int64_t)K * N))) {
@@ -334,10 +336,10 @@ int sspmm_f16_f16_batched(int m_vec, int vec_length, int N, int K, int batch, co
 
 int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nvec, const int* row_indices, const int* row_offsets,
                   const int* column_indices, const void* values_f16, int64_t values_stride, const void* rhs_f16, int64_t rhs_stride,
-                  void* out, int64_t out_stride, int out_is_f16, void* stream) {
+                  const void* bias_f16, void* out, int64_t out_stride, int out_is_f16, void* stream) {
     if (nvec < 0) { g_err[0] = 0; set_error("nvec must be >= 0"); return (int)cudaErrorInvalidValue; }
     SpmmExtra ex;
-    ex.nvec = nvec;
+    ex.nvec = nvec; ex.bias = bias_f16;
     return spmm_entry(m_vec, vec_length, N, K, batch, row_indices, row_offsets, column_indices, values_f16, values_stride, rhs_f16,
                       rhs_stride, out, out_stride, out_is_f16 != 0, stream, ex);
 }

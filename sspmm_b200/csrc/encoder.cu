@@ -1,0 +1,393 @@
+// The parts of an encoder layer between its products, on feature-major activations x[features][tokens] (the layout the
+// SpMM reads and writes): LayerNorm with the residual sum before it, and softmax attention.  The reference runs both as
+// framework operations (end2end/sspmm_e2e/end_to_end.py:44-75).
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cmath>
+
+#include "../../include/sspmm_b200.h"
+#include "launch.h"
+#include "ptx.cuh"
+
+namespace sspmm_b200 {
+namespace enc {
+
+__device__ __forceinline__ void unpack8(const uint4& x, float (&f)[8]) {
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        f[2 * i] = v.x; f[2 * i + 1] = v.y;
+    }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 h = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// ---- LayerNorm ------------------------------------------------------------------------------------
+// Bound by memory: x (and add) read once, out (and the sum) written once.  A CTA takes TT tokens and keeps their features in
+// shared memory between the passes for the mean, the variance and the result, so nothing is read twice; a thread works on
+// eight tokens (16 bytes) of every (256 * 8 / TT)-th feature.  TT = 32 gives 64-byte runs; with few tokens TT = 8 spreads
+// them over more SMs.  768 x 16384: 300 us as eleven torch launches (fp32 copies, mean, variance, five broadcasts),
+// 20 us here.
+constexpr int kLnThreads = 256;
+template <int TT>
+__global__ void __launch_bounds__(kLnThreads)
+layer_norm_fm_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
+                     __half* __restrict__ sum_out,
+                     const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps, __half* __restrict__ out) {
+    constexpr int P = TT / 8, kRows = kLnThreads / P;      // pieces per feature, features per turn
+    extern __shared__ uint4 tile[];                         // [hidden][P]
+    __shared__ float red[kLnThreads / 32][TT];
+    const int piece = threadIdx.x % P, r0 = threadIdx.x / P, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * TT + piece * 8;
+    const bool in = t0 < tokens;
+    // sum over the features of eight numbers per token, the same in every thread of the piece
+    auto total = [&](float (&f)[8]) {
+#pragma unroll
+        for (int o = P; o < 32; o <<= 1)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] += __shfl_xor_sync(0xffffffffu, f[e], o);
+        if (lane < P)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) red[warp][piece * 8 + e] = f[e];
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            f[e] = 0.f;
+            for (int w = 0; w < kLnThreads / 32; ++w) f[e] += red[w][piece * 8 + e];
+        }
+        __syncthreads();
+    };
+    float mean[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int r = r0; r < hidden; r += kRows) {
+        uint4 v = make_uint4(0, 0, 0, 0);
+        const int64_t at = (int64_t)r * tokens + t0;
+        if (in) v = __ldg(reinterpret_cast<const uint4*>(x + at));
+        float f[8];
+        unpack8(v, f);
+        if (bias) {
+            const float b = __half2float(__ldg(bias + r));
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e] + b));
+            v = pack8(f);
+        }
+        if (add) {
+            float g[8];
+            unpack8(in ? __ldg(reinterpret_cast<const uint4*>(add + at)) : make_uint4(0, 0, 0, 0), g);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] += g[e];
+            v = pack8(f);
+            if (in) *reinterpret_cast<uint4*>(sum_out + at) = v;
+            unpack8(v, f);
+        }
+        tile[r * P + piece] = v;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) mean[e] += f[e];
+    }
+    total(mean);
+    const float inv = 1.f / (float)hidden;
+    float var[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mean[e] *= inv;
+#pragma unroll 4
+    for (int r = r0; r < hidden; r += kRows) {
+        float f[8];
+        unpack8(tile[r * P + piece], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { const float d = f[e] - mean[e]; var[e] = fmaf(d, d, var[e]); }
+    }
+    total(var);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) var[e] = rsqrtf(fmaf(var[e], inv, eps));
+#pragma unroll 4
+    for (int r = r0; r < hidden; r += kRows) {
+        float f[8];
+        unpack8(tile[r * P + piece], f);
+        const float g = __half2float(gamma[r]), b = __half2float(beta[r]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = (f[e] - mean[e]) * var[e] * g + b;
+        if (in) *reinterpret_cast<uint4*>(out + (int64_t)r * tokens + t0) = pack8(f);
+    }
+}
+
+// out = x + bias + add, rounded after each addition; one 16-byte piece per thread.
+__global__ void __launch_bounds__(256)
+add_bias_fm_kernel(int rows, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
+                   __half* __restrict__ out) {
+    const int64_t pieces = (int64_t)rows * (tokens / 8);
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < pieces; i += (int64_t)gridDim.x * 256) {
+        float f[8], g[8];
+        unpack8(__ldg(reinterpret_cast<const uint4*>(x) + i), f);
+        unpack8(__ldg(reinterpret_cast<const uint4*>(add) + i), g);
+        const float b = __half2float(__ldg(bias + i / (tokens / 8)));
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = __half2float(__float2half_rn(f[e] + b)) + g[e];
+        reinterpret_cast<uint4*>(out)[i] = pack8(f);
+    }
+}
+
+// ---- attention ------------------------------------------------------------------------------------
+// One CTA: 64 queries of one head of one sequence, four warps of 16 queries; keys and values pass through shared memory 64
+// tokens at a time (two buffers, cp.async), the running maximum, sum and output of a query stay in registers.  Head width
+// 64.  Everything is read as it lies, [feature][token]: q and k are fetched by transposing ldmatrix, v by the plain one.
+// Probabilities keep 22 bits: p = hi + lo, two fp16 numbers, two matrix instructions; the score path needs no such split,
+// its operands are fp16 already and their products exact in the fp32 accumulation.
+// Optional biases of q and v (per feature) are added here: q's to the fragments, v's to the result, since the probabilities
+// of a query sum to one; one of k would add the same number to all scores of a query, which the softmax does not see.
+// Bound by the matrix instructions (96 of m16n8k16 per warp and 64 keys) and the exponentials.  12 heads, 32 x 512 tokens:
+// 144 us, 1350 us as torch's unfused fp32 path (the strided views rule out its fused kernels), and as close to the exact result.
+constexpr int kHd = 64, kTile = 64, kAttnThreads = 128;
+constexpr int kTileBytes = kHd * kTile * 2;                 // 8 KB: [64 features][64 tokens], pieces swizzled by the feature
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
+    const uint32_t bytes = valid ? 16u : 0u;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// address of the 16-byte piece (feature row, piece) of a tile
+__device__ __forceinline__ uint32_t at(uint32_t tile, int row, int piece) { return tile + row * 128 + ((piece ^ (row & 7)) << 4); }
+
+__global__ void __launch_bounds__(kAttnThreads, 4)
+attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
+                    const __half* __restrict__ bias_q, const __half* __restrict__ bias_v, __half* __restrict__ out) {
+    __shared__ __align__(128) uint8_t smem[5 * kTileBytes];         // q (later the output), two buffers of k and v
+    const uint32_t s_q = smem_u32(smem), s_kv = s_q + kTileBytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int q0 = blockIdx.x * kTile, head = blockIdx.y;
+    const int64_t base = (int64_t)head * kHd * tokens + (int64_t)blockIdx.z * seq;
+    auto load = [&](uint32_t dst, const __half* src, int s0) {
+        for (int x = threadIdx.x; x < kHd * 8; x += kAttnThreads) {
+            const int row = x >> 3, piece = x & 7, s = s0 + piece * 8;
+            const bool ok = s < seq;                                // seq % 8 == 0: a piece is all in or all out
+            cp16(at(dst, row, piece), src + base + (int64_t)row * tokens + (ok ? s : 0), ok);
+        }
+    };
+    load(s_q, q, q0);
+    load(s_kv, k, 0);
+    load(s_kv + kTileBytes, v, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+
+    constexpr float kScale = 0.125f * 1.44269504088896340736f;      // 1 / sqrt(64), in powers of two
+    constexpr float kLift = 10.f;                                   // probabilities are carried times 2^10: their low halves stay normal numbers
+    float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+    uint32_t qf[4][4];                                              // [16 features][fragment]
+    const int rounds = (seq + kTile - 1) / kTile;
+    for (int it = 0; it < rounds; ++it) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                            // this round's tiles are in, the other buffer is free
+        if (it + 1 < rounds) {
+            const uint32_t next = s_kv + ((it + 1) & 1) * 2 * kTileBytes;
+            load(next, k, (it + 1) * kTile);
+            load(next + kTileBytes, v, (it + 1) * kTile);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const uint32_t s_k = s_kv + (it & 1) * 2 * kTileBytes, s_v = s_k + kTileBytes;
+        if (it == 0) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)                          // matrices (features lo, tokens lo), (lo, hi), (hi, lo), (hi, hi)
+                ldsm4_t(qf[kk], at(s_q, kk * 16 + (lane >> 4) * 8 + (lane & 7), warp * 2 + ((lane >> 3) & 1)));
+            if (bias_q) {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) {                   // features 2t, 2t + 1 of the fragment's half
+                        const __half* b = bias_q + head * kHd + kk * 16 + (f >> 1) * 8 + 2 * t;
+                        const __half2 s2 = __hadd2(*reinterpret_cast<const __half2*>(&qf[kk][f]), __halves2half2(b[0], b[1]));
+                        qf[kk][f] = *reinterpret_cast<const uint32_t*>(&s2);
+                    }
+            }
+        }
+        float s[8][4];
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int n2 = 0; n2 < 4; ++n2) {                        // two blocks of eight keys
+                uint32_t b[4];                                      // (features lo, keys a), (hi, a), (lo, b), (hi, b)
+                ldsm4_t(b, at(s_k, kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), n2 * 2 + (lane >> 4)));
+                mma(s[2 * n2], qf[kk], b[0], b[1]);
+                mma(s[2 * n2 + 1], qf[kk], b[2], b[3]);
+            }
+        const int left = seq - it * kTile;
+        if (left < kTile) {
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+                if (n * 8 >= left)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[n][e] = -INFINITY;
+        }
+        // rows g (elements 0, 1) and g + 8 (2, 3) of the warp's 16 queries
+        float shift[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float mx = m[h];
+#pragma unroll
+            for (int n = 0; n < 8; ++n) mx = fmaxf(mx, fmaxf(s[n][2 * h], s[n][2 * h + 1]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float keep = mx == -INFINITY ? 1.f : exp2f((m[h] - mx) * kScale);
+            m[h] = mx;
+            shift[h] = mx == -INFINITY ? 0.f : mx;
+            l[h] *= keep;
+#pragma unroll
+            for (int n = 0; n < 8; ++n) { o[n][2 * h] *= keep; o[n][2 * h + 1] *= keep; }
+        }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {                            // sixteen keys: score blocks 2 kk and 2 kk + 1 are the fragment
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {                           // (queries lo, keys lo), (hi, lo), (lo, hi), (hi, hi)
+                const int n = 2 * kk + (f >> 1), h = f & 1;
+                const float p0 = exp2f(fmaf(s[n][2 * h] - shift[h], kScale, kLift)), p1 = exp2f(fmaf(s[n][2 * h + 1] - shift[h], kScale, kLift));
+                l[h] += p0 + p1;
+                const __half2 ph = __floats2half2_rn(p0, p1);
+                const float2 back = __half22float2(ph);
+                const __half2 pl = __floats2half2_rn(p0 - back.x, p1 - back.y);
+                hi[f] = *reinterpret_cast<const uint32_t*>(&ph);
+                lo[f] = *reinterpret_cast<const uint32_t*>(&pl);
+            }
+#pragma unroll
+            for (int n2 = 0; n2 < 4; ++n2) {                        // two blocks of eight output features
+                uint32_t b[4];                                      // (features a, keys lo), (a, hi), (b, lo), (b, hi)
+                ldsm4(b, at(s_v, n2 * 16 + (lane >> 4) * 8 + (lane & 7), kk * 2 + ((lane >> 3) & 1)));
+                mma(o[2 * n2], lo, b[0], b[1]);
+                mma(o[2 * n2 + 1], lo, b[2], b[3]);
+                mma(o[2 * n2], hi, b[0], b[1]);
+                mma(o[2 * n2 + 1], hi, b[2], b[3]);
+            }
+        }
+    }
+    float inv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+        inv[h] = l[h] == 0.f ? 0.f : 1.f / l[h];
+    }
+    // the warp's 16 columns of the output tile [feature][query] take the place of its queries
+    __half* tile = reinterpret_cast<__half*>(smem);
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int row = n * 8 + 2 * t + (e & 1), piece = warp * 2 + (e >> 1);
+            const float b = bias_v ? __half2float(bias_v[head * kHd + row]) : 0.f;
+            tile[row * 64 + ((piece ^ (row & 7)) << 3) + g] = __float2half_rn(fmaf(o[n][e], inv[e >> 1], b));
+        }
+    __syncwarp();
+#pragma unroll
+    for (int x = lane; x < kHd * 2; x += 32) {
+        const int row = x >> 1, piece = warp * 2 + (x & 1), s = q0 + piece * 8;
+        if (s < seq)
+            *reinterpret_cast<uint4*>(out + base + (int64_t)row * tokens + s) = *reinterpret_cast<const uint4*>(tile + row * 64 + ((piece ^ (row & 7)) << 3));
+    }
+}
+
+bool piece_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }   // null passes
+
+}  // namespace enc
+}  // namespace sspmm_b200
+
+using namespace sspmm_b200;
+
+extern "C" {
+
+int sspmm_layer_norm_fm(int hidden, int tokens, const void* x, const void* bias, const void* add, void* sum_out, const void* gamma, const void* beta,
+                        float eps, void* out, void* stream) {
+    set_error("%s", "");
+    if (hidden <= 0 || hidden > 3072 || tokens < 0 || tokens % 8 != 0 || !x || !gamma || !beta || !out || (add && !sum_out) ||
+        !enc::piece_aligned(x) || !enc::piece_aligned(add) || !enc::piece_aligned(sum_out) || !enc::piece_aligned(out)) {
+        set_error("LayerNorm: bad argument (hidden=%d tokens=%d)", hidden, tokens);
+        return (int)cudaErrorInvalidValue;
+    }
+    if (tokens == 0) return 0;
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return (int)cudaErrorNoDevice;
+    // 32 tokens per CTA once that gives every SM one
+    const bool wide = tokens >= 32 * sms;
+    auto kern = wide ? enc::layer_norm_fm_kernel<32> : enc::layer_norm_fm_kernel<8>;
+    const int TT = wide ? 32 : 8;
+    const size_t smem = (size_t)hidden * TT * 2;
+    static DeviceOnce once_wide, once_narrow;
+    DeviceOnce& once = wide ? once_wide : once_narrow;
+    if (!once.done()) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * TT * 2);
+        if (e != cudaSuccess) { set_error("LayerNorm: %s", cudaGetErrorString(e)); return (int)e; }
+        once.mark();
+    }
+    kern<<<(tokens + TT - 1) / TT, enc::kLnThreads, smem, static_cast<cudaStream_t>(stream)>>>(
+        hidden, tokens, static_cast<const __half*>(x), static_cast<const __half*>(bias), static_cast<const __half*>(add), static_cast<__half*>(sum_out),
+        static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, static_cast<__half*>(out));
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("LayerNorm launch: %s", cudaGetErrorString(e)); return (int)e; }
+    return 0;
+}
+
+int sspmm_add_bias_fm(int rows, int tokens, const void* x, const void* bias, const void* add, void* out, void* stream) {
+    set_error("%s", "");
+    if (rows < 0 || tokens < 0 || tokens % 8 != 0 || !x || !bias || !add || !out || !enc::piece_aligned(x) || !enc::piece_aligned(add) ||
+        !enc::piece_aligned(out)) {
+        set_error("bias and residual: bad argument (rows=%d tokens=%d)", rows, tokens);
+        return (int)cudaErrorInvalidValue;
+    }
+    const int64_t pieces = (int64_t)rows * (tokens / 8);
+    if (pieces == 0) return 0;
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return (int)cudaErrorNoDevice;
+    const int64_t blocks = (pieces + 255) / 256, most = (int64_t)sms * 16;
+    enc::add_bias_fm_kernel<<<(unsigned)(blocks < most ? blocks : most), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        rows, tokens, static_cast<const __half*>(x), static_cast<const __half*>(bias), static_cast<const __half*>(add), static_cast<__half*>(out));
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("bias and residual launch: %s", cudaGetErrorString(e)); return (int)e; }
+    return 0;
+}
+
+int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* q, const void* k, const void* v, const void* bias_q,
+                       const void* bias_v, void* out, void* stream) {
+    set_error("%s", "");
+    if (heads < 0 || batch < 0 || seq < 0 || head_dim != enc::kHd || seq % 8 != 0 || heads > 65535 || batch > 65535 || !q || !k || !v || !out ||
+        !enc::piece_aligned(q) || !enc::piece_aligned(k) || !enc::piece_aligned(v) || !enc::piece_aligned(out)) {
+        set_error("attention: bad argument (heads=%d head_dim=%d batch=%d seq=%d)", heads, head_dim, batch, seq);
+        return (int)cudaErrorInvalidValue;
+    }
+    if (heads == 0 || batch == 0 || seq == 0) return 0;
+    const dim3 grid((seq + enc::kTile - 1) / enc::kTile, heads, batch);
+    enc::attention_fm_kernel<<<grid, enc::kAttnThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        seq, (int64_t)batch * seq, static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),
+        static_cast<const __half*>(bias_q), static_cast<const __half*>(bias_v), static_cast<__half*>(out));
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { set_error("attention launch: %s", cudaGetErrorString(e)); return (int)e; }
+    return 0;
+}
+
+}  // extern "C"

@@ -21,6 +21,7 @@ struct SpmmArgs {
     const __half* rhs;         // [K * N] row-major
     void* out;                 // [m_vec * V * N] row-major, fp32 or fp16
     bool out_f16;
+    const __half* bias;        // per row of the output, added before the conversion; may be null
     // batching (one launch, grid z-less: tiles enumerate the batch too)
     int batch;                 // >= 1
     int64_t values_stride;     // elements between batches (0 = shared)

@@ -118,7 +118,13 @@ struct BlockProblem {
     int wide;                // 1: the operand maps are chunked ({64, K, width/64[, batch]}), so ONE TMA instruction
                              // per operand and stage brings all 64-wide chunks; 0: one instruction per chunk
     int64_t out_stride;      // per batch, elements
+    const __half* bias;      // per row of C, added before the conversion; null: none (or added by the reduction)
 };
+
+__device__ __forceinline__ void add_bias(uint32_t (&w)[32], float bias) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) + bias);
+}
 
 template <int BN, int STAGES, typename OutT>
 __global__ void __launch_bounds__(kBlockThreads, 1)
@@ -248,6 +254,7 @@ sspmm_block_kernel(const __grid_constant__ CUtensorMap tmap_at, const __grid_con
             if (!named_barrier_and(2, 128, mbar_wait(bar_acc_full + 8 * buf, acc_phase, abort_flag, kStatusWaitBlock))) break;
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
+            const float bias = p.bias && m0 + row < p.Mp ? __half2float(p.bias[m0 + row]) : 0.f;
             uint32_t v[2][32];
             tmem_ld_x32(taddr, v[0]);
 #pragma unroll
@@ -260,7 +267,8 @@ sspmm_block_kernel(const __grid_constant__ CUtensorMap tmap_at, const __grid_con
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);        // accumulator drained
                 }
-                const uint32_t(&w)[32] = v[cc & 1];
+                uint32_t(&w)[32] = v[cc & 1];
+                if (p.bias) add_bias(w, bias);
 #pragma unroll
                 for (int h = 0; h < kStoresPerLoad; ++h) {
                     const uint32_t sb = st_it & 1u;
@@ -469,6 +477,7 @@ sspmm_block_pair_kernel(const __grid_constant__ CUtensorMap tmap_at, const __gri
             tc_fence_after_sync();
             const uint32_t drained = cluster_map_shared(bar_acc_empty + 8 * buf, 0);
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
+            const float bias = p.bias && m0 + row < p.Mp ? __half2float(p.bias[m0 + row]) : 0.f;
             uint32_t v[2][32];
             tmem_ld_x32(taddr, v[0]);
 #pragma unroll
@@ -481,7 +490,8 @@ sspmm_block_pair_kernel(const __grid_constant__ CUtensorMap tmap_at, const __gri
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(drained);
                 }
-                const uint32_t(&w)[32] = v[cc & 1];
+                uint32_t(&w)[32] = v[cc & 1];
+                if (p.bias) add_bias(w, bias);
 #pragma unroll
                 for (int h = 0; h < kStoresPerLoad; ++h) {
                     const uint32_t sb = st_it & 1u;
@@ -648,7 +658,8 @@ cudaError_t launch_block_pair(const SpmmArgs& a, const CUtensorMap& ta, const CU
 // C the first n_out of them.
 template <typename OutT>
 __global__ void __launch_bounds__(256)
-reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, int64_t elems, int splits, int N, int n_out) {
+reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, int64_t elems, int splits, int N, int n_out,
+                     const __half* __restrict__ bias) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= elems) return;                                      // elems is a multiple of 4 (N % 8 == 0)
     float4 acc = *reinterpret_cast<const float4*>(partial + i);
@@ -656,8 +667,12 @@ reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, 
         const float4 v = *reinterpret_cast<const float4*>(partial + (int64_t)s2 * elems + i);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
+    const int64_t row = n_out != N || bias ? i / N : 0;
+    if (bias) {
+        const float b = __half2float(bias[row]);
+        acc.x += b; acc.y += b; acc.z += b; acc.w += b;
+    }
     if (n_out != N) {
-        const int64_t row = i / N;
         const int n = (int)(i - row * N);
         const float v[4] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
@@ -780,6 +795,7 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     }
     p.total_tiles = (int)total;
     p.out_stride = a.out_stride;
+    p.bias = pl.splits > 1 || a.n_out != a.N ? nullptr : a.bias;
     CUtensorMap ta, tb, tc;
     const bool split = pl.splits > 1 || a.n_out != a.N;           // fp32 partial tiles, then the reduction
     if (split && pl.at_bytes + pl.partial_bytes > scratch_bytes) {
@@ -830,8 +846,8 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     if (e != cudaSuccess || !split) return e;
     const int64_t elems = (int64_t)Mp * a.N;
     const unsigned rgrid = (unsigned)((elems / 4 + 255) / 256);
-    if (a.out_f16) reduce_splits_kernel<__half><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<__half*>(a.out), elems, pl.splits, a.N, a.n_out);
-    else reduce_splits_kernel<float><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<float*>(a.out), elems, pl.splits, a.N, a.n_out);
+    if (a.out_f16) reduce_splits_kernel<__half><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<__half*>(a.out), elems, pl.splits, a.N, a.n_out, a.bias);
+    else reduce_splits_kernel<float><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<float*>(a.out), elems, pl.splits, a.N, a.n_out, a.bias);
     return cudaGetLastError();
 }
 

@@ -1130,7 +1130,7 @@ int sspmm_planned(const sspmm_plan* plan, const void* values_f16, const void* rh
     if (!plan->fused) {
         // sparse or irregular structure: the regular entry points (gather kernels) take it
         return sspmm_counted(plan->m_vec, plan->V, N, plan->K, 1, plan->nvec > 0 ? plan->nvec : 0, nullptr, plan->row_offsets,
-                             plan->column_indices, values_f16, 0, rhs_f16, 0, out, 0, out_is_f16, stream);
+                             plan->column_indices, values_f16, 0, rhs_f16, 0, nullptr, out, 0, out_is_f16, stream);
     }
     const int sms = current_device_sm_count();
     if (sms <= 0) return (int)cudaErrorNoDevice;
@@ -1151,7 +1151,7 @@ int sspmm_planned(const sspmm_plan* plan, const void* values_f16, const void* rh
             a.m_vec = plan->m_vec; a.V = plan->V; a.N = N; a.n_out = N; a.K = plan->K;
             a.row_indices = nullptr; a.row_offsets = plan->row_offsets; a.column_indices = plan->column_indices;
             a.values = static_cast<const __half*>(values_f16); a.rhs = static_cast<const __half*>(rhs_f16);
-            a.out = out; a.out_f16 = out_is_f16 != 0; a.batch = 1;
+            a.out = out; a.out_f16 = out_is_f16 != 0; a.bias = nullptr; a.batch = 1;
             a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
             a.stream = static_cast<cudaStream_t>(stream);
             const cudaError_t e = launch_sspmm_rows(a, plan->nvec, nullptr);

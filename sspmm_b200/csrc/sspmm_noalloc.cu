@@ -83,7 +83,7 @@ extern "C" int sspmm_f16_f16_noalloc(int m_vec, int vec_length, int N, int K, co
     a.m_vec = m_vec; a.V = vec_length; a.N = N; a.n_out = N; a.K = K;
     a.row_indices = row_indices; a.row_offsets = row_offsets; a.column_indices = column_indices;
     a.values = static_cast<const __half*>(values_f16); a.rhs = static_cast<const __half*>(rhs_f16);
-    a.out = out_f16; a.out_f16 = true; a.batch = 1;
+    a.out = out_f16; a.out_f16 = true; a.bias = nullptr; a.batch = 1;
     a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
     a.stream = static_cast<cudaStream_t>(stream);
     // The expansion kernel writes every element of the K x m_vec*V region it uses (zeros included),

@@ -46,6 +46,7 @@ struct Problem {
     const int* col;
     const __half* values;
     const __half* rhs;
+    const __half* bias;                   // per row of C, or null
     int64_t values_stride, rhs_stride, out_stride;
     int out_pieces;                       // rows of C start on 16-byte boundaries
     // split launches only (see sspmm_rows_split_kernel)
@@ -250,8 +251,13 @@ struct Tile {
     // Writes this lane's piece of unit u to C (first_row: the first of the vector row's V rows).
     template <typename OutT>
     static __device__ __forceinline__ void store_unit(const Problem& p, OutT* __restrict__ out, int64_t first_row, int n0, int u, int lane,
-                                                      const float (&o)[8]) {
+                                                      float (&o)[8]) {
         const int id = u * 32 + lane, n = n0 + (id % kPieces) * 8;
+        if (p.bias) {
+            const float b = __half2float(p.bias[first_row + id / kPieces]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] += b;
+        }
         OutT* dst = out + (first_row + id / kPieces) * p.N + n;
         if (p.out_pieces) {
             if (n >= p.N) return;                                // rows of C are whole pieces: all eight or none
@@ -277,8 +283,12 @@ struct Tile {
     }
     // Four columns of one row to C.
     template <typename OutT>
-    static __device__ __forceinline__ void store_four(const Problem& p, OutT* __restrict__ out, int64_t row, int n, const float4& o) {
+    static __device__ __forceinline__ void store_four(const Problem& p, OutT* __restrict__ out, int64_t row, int n, float4 o) {
         OutT* dst = out + row * p.N + n;
+        if (p.bias) {
+            const float b = __half2float(p.bias[row]);
+            o.x += b; o.y += b; o.z += b; o.w += b;
+        }
         if (p.out_pieces) {
             if (n >= p.N) return;
             if constexpr (sizeof(OutT) == 2) {
@@ -620,7 +630,7 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     rows::Problem p;
     p.m_vec = a.m_vec; p.N = a.n_out; p.ldb = a.N; p.K = a.K;
     p.row_indices = a.row_indices; p.row_offsets = a.row_offsets; p.col = a.column_indices;
-    p.values = a.values; p.rhs = a.rhs;
+    p.values = a.values; p.rhs = a.rhs; p.bias = a.bias;
     p.values_stride = a.values_stride; p.rhs_stride = a.rhs_stride; p.out_stride = a.out_stride;
     p.chunk = 0; p.cap = 0; p.header = nullptr; p.arrivals = nullptr; p.entries = nullptr; p.partial = nullptr;
     const size_t es = a.out_f16 ? 2 : 4;

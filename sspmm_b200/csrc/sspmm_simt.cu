@@ -13,7 +13,7 @@ template <int V, typename OutT>
 __global__ void __launch_bounds__(128)
 sspmm_simt_kernel(int m_vec, int N, const int* __restrict__ row_indices, const int* __restrict__ row_offsets,
                   const int* __restrict__ col, const __half* __restrict__ values, const __half* __restrict__ rhs,
-                  OutT* __restrict__ out, int64_t values_stride, int64_t rhs_stride, int64_t out_stride) {
+                  OutT* __restrict__ out, const __half* __restrict__ bias, int64_t values_stride, int64_t rhs_stride, int64_t out_stride) {
     const int sched = blockIdx.x;
     const int i = row_indices ? row_indices[sched] : sched;
     if ((unsigned)i >= (unsigned)m_vec) return;
@@ -36,6 +36,7 @@ sspmm_simt_kernel(int m_vec, int N, const int* __restrict__ row_indices, const i
 #pragma unroll
         for (int v = 0; v < V; ++v) {
             const int64_t o = ((int64_t)i * V + v) * N + n;
+            if (bias) acc[v] += __half2float(bias[i * V + v]);
             if constexpr (sizeof(OutT) == 2) out[o] = __float2half_rn(acc[v]);
             else out[o] = acc[v];
         }
@@ -46,7 +47,7 @@ template <int V, typename OutT>
 cudaError_t run(const SpmmArgs& a) {
     dim3 grid(a.m_vec, (a.N + 127) / 128, a.batch);
     sspmm_simt_kernel<V, OutT><<<grid, 128, 0, a.stream>>>(a.m_vec, a.N, a.row_indices, a.row_offsets, a.column_indices,
-                                                           a.values, a.rhs, static_cast<OutT*>(a.out), a.values_stride,
+                                                           a.values, a.rhs, static_cast<OutT*>(a.out), a.bias, a.values_stride,
                                                            a.rhs_stride, a.out_stride);
     return cudaGetLastError();
 }

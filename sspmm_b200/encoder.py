@@ -19,6 +19,12 @@ import torch.nn.functional as F
 from . import ops, synthetic
 
 
+def _plain(*tensors) -> bool:
+    """Tensors the kernels can take as they lie: contiguous fp16 on the GPU, 16-byte aligned, outside autograd."""
+    return all(t.is_cuda and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
+               and not (t.requires_grad and torch.is_grad_enabled()) for t in tensors)
+
+
 class SparseLinear:
     """y[out, tokens] = W_vs . x[in, tokens] + b, W pruned and held in the compressed format."""
 
@@ -33,7 +39,18 @@ class SparseLinear:
         self.bias = bias
         self.dense = torch.from_numpy(weight.dense()).to(device)          # only for the dense comparison
 
+    def bias_rows(self) -> Optional[torch.Tensor]:
+        """The bias as the product's epilogue takes it, one number per row of the padded output; None: not of that form."""
+        b = self.bias
+        if b is None or not _plain(b) or tuple(b.shape) != (self.out_features,):
+            return None
+        pad = -self.out_features % self.V
+        return F.pad(b, (0, pad)) if pad else b
+
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
+        rows = self.bias_rows()
+        if rows is not None:
+            return ops.sspmm_bias(self.row_offsets, self.col, self.values, x, self.V, rows, row_indices=self.row_indices)[: self.out_features]
         y = ops.sspmm(self.row_offsets, self.col, self.values, x, self.V, row_indices=self.row_indices)
         y = y[: self.out_features]
         return y if self.bias is None else y + self.bias[:, None]
@@ -70,15 +87,45 @@ class SparseEncoderLayer:
         o = F.scaled_dot_product_attention(split(q), split(k), split(v))
         return o.permute(1, 3, 0, 2).reshape(self.hidden, batch * seq)
 
+    def _norm(self, x, wb, add=None, bias=None, out=None, sum_out=None):
+        """LayerNorm of x + bias + add: (what was normalised, the result)."""
+        given = [t for t in (x, add, bias, *wb) if t is not None]
+        if _plain(*given) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
+                (add is None or add.shape == x.shape) and all(t.numel() == x.shape[0] for t in given if t is not x and t is not add):
+            out = torch.empty_like(x) if out is None else out
+            if add is not None and sum_out is None:
+                sum_out = torch.empty_like(x)
+            ops.layer_norm_fm(x, wb[0], wb[1], 1e-5, out, add, sum_out, bias)
+            return (x if add is None else sum_out), out
+        if bias is not None:
+            x = x + bias[:, None]
+        if add is not None:
+            x = x + add
+        y = self._layer_norm_fm(x, wb)
+        return x, (y if out is None else out.copy_(y))
+
+    def _attend(self, q, k, v, batch, seq, biases=(None, None, None), out=None):
+        tokens = (self.hidden, batch * seq)
+        given = [b for b in biases if b is not None]
+        if self.hidden == 64 * self.heads and seq % 8 == 0 and seq > 0 and 0 < batch <= 65535 and _plain(q, k, v, *given) and \
+                all(tuple(t.shape) == tokens for t in (q, k, v)) and all(tuple(b.shape) == (self.hidden,) for b in given):
+            out = torch.empty_like(q) if out is None else out
+            ops.attention_fm(q, k, v, self.heads, batch, seq, out, biases[0], biases[2])      # one of k changes nothing
+            return out
+        q, k, v = (t if b is None else t + b[:, None] for t, b in zip((q, k, v), biases))
+        att = self._attention(q, k, v, batch, seq)
+        return att.contiguous() if out is None else out.copy_(att)
+
     def _groups_for(self, tokens: int):
         """Activation buffers of fixed shape and, bound to them, one group per dependency level of the layer:
         {Q, K, V} share their input and run as one launch, then O, FFN1, FFN2."""
         if getattr(self, "_tokens", None) == tokens:
             return
+        L = self.linears
         z = lambda rows: torch.empty((rows, tokens), dtype=torch.float16, device=self.dev)
         b = self.buf = {"ln1": z(self.hidden), "q": z(self.hidden), "k": z(self.hidden), "v": z(self.hidden),
-                        "att": z(self.hidden), "o": z(self.hidden), "ln2": z(self.hidden), "h": z(self.ffn), "y": z(self.hidden)}
-        L = self.linears
+                        "att": z(self.hidden), "o": z(self.hidden), "sum": z(self.hidden), "ln2": z(self.hidden),
+                        "h": z(self.ffn), "y": z(self.hidden)}
         item = lambda l, src, dst: (l.plan, l.values, b[src], b[dst])
         self.groups = None
         if all(l.plan.one_launch and l.out_features % l.V == 0 for l in L):
@@ -88,30 +135,32 @@ class SparseEncoderLayer:
         self._tokens = tokens
 
     def forward_grouped(self, x: torch.Tensor, batch: int, seq: int) -> torch.Tensor:
-        """Same layer with the linears run as groups (sspmm_group_run) on preallocated activation buffers."""
+        """Same layer with the linears run as groups (sspmm_group_run) on preallocated activation buffers.  The biases of
+        Q and V go into the attention, the one of O into the LayerNorm, FFN2's into the last sum."""
         self._groups_for(batch * seq)
         if self.groups is None:
             return self.forward(x, batch, seq)
         b, L, g = self.buf, self.linears, self.groups
-        b["ln1"].copy_(self._layer_norm_fm(x, self.ln1))
+        self._norm(x, self.ln1, out=b["ln1"])
         g[0].run()
-        q, k, v = (b[n] + L[i].bias[:, None] for i, n in enumerate(("q", "k", "v")))
-        b["att"].copy_(self._attention(q, k, v, batch, seq))
+        self._attend(b["q"], b["k"], b["v"], batch, seq, [l.bias for l in L[:3]], out=b["att"])
         g[1].run()
-        out = b["o"] + L[3].bias[:, None] + x
-        b["ln2"].copy_(self._layer_norm_fm(out, self.ln2))
+        out, _ = self._norm(b["o"], self.ln2, add=x, bias=L[3].bias, out=b["ln2"], sum_out=b["sum"])
         g[2].run()
-        b["h"] += L[4].bias[:, None]
+        if L[4].bias is not None:
+            b["h"] += L[4].bias[:, None]
         g[3].run()
-        return b["y"] + L[5].bias[:, None] + out
+        bias = L[5].bias_rows()
+        if bias is not None and _plain(out) and out.shape[1] % 8 == 0:
+            return ops.add_bias_fm(b["y"], bias, out)
+        return (b["y"] if L[5].bias is None else b["y"] + L[5].bias[:, None]) + out
 
     def forward(self, x: torch.Tensor, batch: int, seq: int, dense: bool = False) -> torch.Tensor:
         """x: [hidden, batch*seq] fp16, feature-major (token t of sequence b is column b*seq + t)."""
         lin = [(l.dense_forward if dense else l) for l in self.linears]
-        out = self._layer_norm_fm(x, self.ln1)
+        _, out = self._norm(x, self.ln1)
         q, k, v = lin[0](out), lin[1](out), lin[2](out)
-        att = lin[3](self._attention(q, k, v, batch, seq).contiguous())
-        out = att + x
-        y = self._layer_norm_fm(out, self.ln2)
+        att = lin[3](self._attend(q, k, v, batch, seq))
+        out, y = self._norm(att, self.ln2, add=x)
         y = lin[5](lin[4](y))
         return y + out

@@ -43,6 +43,13 @@ def sspmm(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: torch
           vec_length: int, row_indices: Optional[torch.Tensor] = None, out_dtype=torch.float16,
           out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C[m_vec*V, N] = A_vs @ rhs[K, N] (the call made at SSpMM/sspmm_test.cpp:189)."""
+    return sspmm_bias(row_offsets, column_indices, values, rhs, vec_length, None, row_indices, out_dtype, out)
+
+
+def sspmm_bias(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: torch.Tensor, rhs: torch.Tensor,
+               vec_length: int, bias: Optional[torch.Tensor], row_indices: Optional[torch.Tensor] = None,
+               out_dtype=torch.float16, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``sspmm`` plus a number per output row (fp16, m_vec*V of them), added to the fp32 sums before the conversion."""
     _require(row_offsets, torch.int32, "row_offsets")
     _require(column_indices, torch.int32, "column_indices")
     _require(values, torch.float16, "values")
@@ -50,12 +57,16 @@ def sspmm(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: torch
     if row_indices is not None:
         _require(row_indices, torch.int32, "row_indices")
     m_vec = row_offsets.numel() - 1
+    if bias is not None:
+        _require(bias, torch.float16, "bias")
+        if bias.numel() != m_vec * vec_length:
+            raise ValueError(f"bias has {bias.numel()} numbers, the product {m_vec * vec_length} rows")
     K, N = rhs.shape
     if out is None:
         out = torch.empty((m_vec * vec_length, N), dtype=out_dtype, device=rhs.device)
     fn = capi.lib().sspmm_counted
     args = (m_vec, vec_length, N, K, 1, column_indices.numel(), _ptr(row_indices), row_offsets.data_ptr(), column_indices.data_ptr(),
-            values.data_ptr(), 0, rhs.data_ptr(), 0, out.data_ptr(), 0, 1 if out.dtype == torch.float16 else 0)
+            values.data_ptr(), 0, rhs.data_ptr(), 0, _ptr(bias), out.data_ptr(), 0, 1 if out.dtype == torch.float16 else 0)
     if torch.cuda.current_device() == rhs.device.index:
         rc = fn(*args, _stream_ptr())
     else:
@@ -158,6 +169,32 @@ def sorted_row_swizzle(row_offsets: torch.Tensor) -> torch.Tensor:
     with torch.cuda.device(row_offsets.device):
         capi.check(capi.lib().sspmm_sorted_row_swizzle(m_vec, row_offsets.data_ptr(), out.data_ptr(), _stream_ptr()))
     return out
+
+
+def layer_norm_fm(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, eps: float, out: torch.Tensor,
+                  add: Optional[torch.Tensor] = None, sum_out: Optional[torch.Tensor] = None,
+                  bias: Optional[torch.Tensor] = None) -> None:
+    """LayerNorm over dim 0 of x[hidden, tokens] + bias + add (that sum goes to ``sum_out``), ``sspmm_layer_norm_fm``."""
+    with torch.cuda.device(x.device):
+        capi.check(capi.lib().sspmm_layer_norm_fm(x.shape[0], x.shape[1], x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
+                                                  gamma.data_ptr(), beta.data_ptr(), eps, out.data_ptr(), _stream_ptr()))
+
+
+def add_bias_fm(x: torch.Tensor, bias: torch.Tensor, add: torch.Tensor) -> torch.Tensor:
+    """x[rows, tokens] + bias[:, None] + add, ``sspmm_add_bias_fm``."""
+    out = torch.empty_like(x)
+    with torch.cuda.device(x.device):
+        capi.check(capi.lib().sspmm_add_bias_fm(x.shape[0], x.shape[1], x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr(),
+                                                _stream_ptr()))
+    return out
+
+
+def attention_fm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, batch: int, seq: int, out: torch.Tensor,
+                 bias_q: Optional[torch.Tensor] = None, bias_v: Optional[torch.Tensor] = None) -> None:
+    """Softmax attention on feature-major q, k, v [hidden, batch * seq], ``sspmm_attention_fm``."""
+    with torch.cuda.device(q.device):
+        capi.check(capi.lib().sspmm_attention_fm(heads, q.shape[0] // heads, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                                 _ptr(bias_q), _ptr(bias_v), out.data_ptr(), _stream_ptr()))
 
 
 class Plan:

@@ -36,6 +36,6 @@ def bspmm(row_indices, row_offsets, column_indices, values, rhs_matrix, vec_leng
     with torch.cuda.device(rhs_matrix.device):
         capi.check(capi.lib().sspmm_counted(
             m_vec, vec_length, k, n, batch, column_indices.numel(), row_indices.data_ptr(), row_offsets.data_ptr(), column_indices.data_ptr(),
-            values.data_ptr(), 0 if shared_values else nnz, rhs_matrix.data_ptr(), n * k, out.data_ptr(),
+            values.data_ptr(), 0 if shared_values else nnz, rhs_matrix.data_ptr(), n * k, None, out.data_ptr(),
             m_vec * vec_length * k, 1, torch.cuda.current_stream().cuda_stream))
     return out

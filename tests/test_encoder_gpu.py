@@ -21,3 +21,70 @@ def test_sparse_encoder_layer_matches_dense_evaluation(lib):
     assert err <= 2e-2 * scale, (err, scale)
     rms = ((y_sparse.float() - y_dense.float()).pow(2).mean().sqrt() / y_dense.float().pow(2).mean().sqrt()).item()
     assert rms < 5e-3
+
+
+@pytest.mark.parametrize("hidden,tokens", [(64, 8), (3072, 40), (256, 4768), (100, 9600)])
+def test_layer_norm_feature_major(lib, hidden, tokens):
+    """Both tile widths, a partial tile, the largest and an odd number of features; the bound is the rounding of the result
+    (2^-11 of it) and of the fp32 statistics (a few 2^-22 of the spread)."""
+    from sspmm_b200 import ops
+    g = torch.Generator(device="cuda:0").manual_seed(hidden + tokens)
+    r = lambda *s: torch.randn(s, device="cuda:0", generator=g).half()
+    x, add, gamma, beta = r(hidden, tokens) * 3 + 1, r(hidden, tokens), r(hidden), r(hidden)
+    for a, bias in ((None, None), (add, None), (add, beta + 1), (None, gamma)):
+        out, total = torch.empty_like(x), torch.empty_like(x)
+        ops.layer_norm_fm(x, gamma, beta, 1e-5, out, a, total if a is not None else None, bias)
+        s = x if bias is None else x + bias[:, None]
+        s = s if a is None else s + a
+        if a is not None:
+            assert torch.equal(total, s)
+        d = s.double()
+        ref = (d - d.mean(0)) / torch.sqrt(d.var(0, unbiased=False) + 1e-5) * gamma.double()[:, None] + beta.double()[:, None]
+        assert ((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -19 * (1 + gamma.double().abs()[:, None] * 4)).all()
+
+
+@pytest.mark.parametrize("heads,batch,seq,scale", [(1, 1, 8, 1.0), (2, 3, 64, 1.0), (4, 2, 72, 3.0), (1, 2, 512, 6.0), (3, 1, 200, 0.1)])
+def test_attention_feature_major(lib, heads, batch, seq, scale):
+    """One key block and several, partial blocks, flat and peaked probabilities.  Bound: rounding of the fp16 result, and the
+    fp32 scores (2^-20 of their size, at most 64 * 8 * scale^2 / 8 times, enters a probability relatively)."""
+    from sspmm_b200 import ops
+    g = torch.Generator(device="cuda:0").manual_seed(seq)
+    r = lambda s: (torch.randn((heads * 64, batch * seq), device="cuda:0", generator=g) * s).half()
+    q, k, v = r(scale), r(scale), r(1.0)
+    bq, bk, bv = (torch.randn(heads * 64, device="cuda:0", generator=g).half() for _ in range(3))
+    out, with_bias = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    ops.attention_fm(q, k, v, heads, batch, seq, out)
+    ops.attention_fm(q, k, v, heads, batch, seq, with_bias, bq, bv)
+    split = lambda t: t.double().view(heads, 64, batch, seq).permute(2, 0, 3, 1)
+    # the bias of v is added to the finished sum, so |v| and |bias| enter the bound separately
+    for got, dq, dk, dv, mag in ((out, q.double(), k.double(), v.double(), v.double().abs()),
+                                 (with_bias, (q + bq[:, None]).double(), k.double() + bk.double()[:, None],
+                                  v.double() + bv.double()[:, None], v.double().abs() + bv.double().abs()[:, None])):
+        score = split(dq) @ split(dk).transpose(-1, -2) / 8
+        p = torch.softmax(score, -1)
+        ref = p @ split(dv)
+        slack = 2.0 ** -20 * (1 + score.abs().amax()) * (p @ split(mag))
+        assert ((split(got) - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -24 + slack).all()
+
+
+def test_bias_and_residual_feature_major(lib):
+    from sspmm_b200 import ops
+    x, add = (torch.randn(33, 72, device="cuda:0").half() for _ in range(2))
+    bias = torch.randn(33, device="cuda:0").half()
+    assert torch.equal(ops.add_bias_fm(x, bias, add), x + bias[:, None] + add)
+
+
+def test_grouped_layer_follows_replaced_bias_and_odd_shapes(lib):
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=256, ffn=1024, heads=4, sparsity=0.9, vec_length=16)
+    for batch, seq in ((2, 72), (3, 20), (1, 13)):                # the last two are outside what the fused parts take
+        x = torch.randn(256, batch * seq, device="cuda:0", dtype=torch.float16)
+        for _ in range(2):
+            if (batch * seq) % 8 == 0:
+                a, b = layer.forward(x, batch, seq), layer.forward_grouped(x, batch, seq)
+                assert (a.float() - b.float()).abs().max() <= 1e-2 * a.float().abs().max()
+            c, d = layer.forward(x, batch, seq), layer.forward(x, batch, seq, dense=True)
+            assert (c.float() - d.float()).abs().max() <= 2e-2 * d.float().abs().max()
+            layer.linears[0].bias = layer.linears[0].bias + 1.0
+            layer.linears[4].bias = layer.linears[4].bias + 0.5
+            layer.linears[5].bias = layer.linears[5].bias - 2.0

@@ -110,3 +110,24 @@ def test_planned_small_products(lib, V, M, K, N):
     assert plan.one_launch
     for dt in (torch.float16, torch.float32):
         check(ops.sspmm_planned(plan, val, rhs, out_dtype=dt), ptr, col, val, rhs, V)
+
+
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("lens,K,N", [([40, 0, 17], 64, 8), ([900] * 40, 1000, 49), ([700] * 40, 1024, 1024), ([400] * 80, 512, 8192),
+                                      ([600] + [5] * 300, 3000, 40)])
+def test_bias_in_every_epilogue(lib, V, lens, K, N):
+    """Per-row bias: row-gather (teams, cut rows, aligned copy), block kernel with and without split K, CTA pairs, CUDA cores."""
+    ptr, col, val, rhs = operands(lens, K, V, N, 9)
+    bias = torch.randn(len(lens) * V, device=DEV).half()
+    ref, mag = exact(ptr, col, val, rhs, V)
+    ref, mag = ref + bias.double()[:, None], mag + bias.double().abs()[:, None]
+    for kernel in (ops.KERNEL_AUTO, ops.KERNEL_GATHER_LSU, ops.KERNEL_BLOCK, ops.KERNEL_BLOCK_SINGLE, ops.KERNEL_SIMT):
+        ops.set_kernel(kernel)
+        try:
+            for dt in (torch.float16, torch.float32):
+                got = ops.sspmm_bias(ptr, col, val, rhs, V, bias, out_dtype=dt).double()
+                bound = (max(lens) + 1) * 2.0 ** -23 * mag + (2.0 ** -11 * ref.abs() + 2.0 ** -24 if dt == torch.float16 else 0)
+                assert (got - ref).abs().le(bound).all(), kernel
+        finally:
+            ops.set_kernel(ops.KERNEL_AUTO)
+    assert ops.device_status() == 0
