@@ -311,8 +311,11 @@ svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, 
 // ---------------------------------------------------------------- scans
 // Exclusive scans over the groups (vector row pointers from the counts, scratch offsets) and the lists of replayed
 // groups per class, in three small launches: per-block sums, a scan of the block sums by one CTA, and the final
-// positions.  A block covers kScanBlock groups; a block sum is kScanFields numbers: vectors, scratch ints, and
-// the groups of each replay class.
+// positions; matrices of one block (4096 groups) do it all in the last one.  A block covers kScanBlock groups; a block
+// sum is kScanFields numbers: vectors, scratch ints, and the groups of each list segment.
+// What bounds these kernels is their barriers: the segments are counted with shared-memory atomics and only the two sums
+// are reduced across the block.  (Reducing all twenty fields block-wide took 19 + 24 + 33 us whatever the size.)  Inside a
+// segment the groups are listed in no particular order; the lists only say who works on what.
 // totals: [0] nvec, [1] scratch ints, [2..2+kNumSegs) groups per list segment, then the bad-column flag
 constexpr int kScanThreads = 1024;
 constexpr int kScanPerThread = 4;
@@ -320,139 +323,152 @@ constexpr int kScanBlock = kScanThreads * kScanPerThread;
 constexpr int kScanFields = 2 + kNumSegs;
 static_assert(kScanFields == kSvcScanFields, "scan fields");
 
-// Sums `v` over the block; the result is valid in every thread.  sh: 32 long longs.
-__device__ __forceinline__ long long block_sum_ll(long long v, long long* sh) {
+// Exclusive prefixes of a and b over the threads of the block, in thread order, and their totals.  sh: 2 x 32 long longs.
+__device__ __forceinline__ void block_prefix_pair(long long& a, long long& b, long long& total_a, long long& total_b, long long (*sh)[32]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    long long t = 0;
-    for (int w = 0; w < kScanThreads / 32; ++w) t += sh[w];
-    __syncthreads();
-    return t;
-}
-// Exclusive prefix of `v` over the threads of the block, in thread order.  sh: 32 long longs.
-__device__ __forceinline__ long long block_prefix_ll(long long v, long long* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    long long inc = v;
+    long long ia = a, ib = b;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const long long t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
+        const long long ta = __shfl_up_sync(0xffffffffu, ia, o), tb = __shfl_up_sync(0xffffffffu, ib, o);
+        if (lane >= o) { ia += ta; ib += tb; }
     }
-    if (lane == 31) sh[warp] = inc;
+    if (lane == 31) { sh[0][warp] = ia; sh[1][warp] = ib; }
     __syncthreads();
-    long long before = 0;
-    for (int w = 0; w < warp; ++w) before += sh[w];
-    __syncthreads();
-    return before + inc - v;
+    // every warp scans the warp totals for itself
+    long long wa = sh[0][lane], wb = sh[1][lane];
+    const long long own_a = wa, own_b = wb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long ta = __shfl_up_sync(0xffffffffu, wa, o), tb = __shfl_up_sync(0xffffffffu, wb, o);
+        if (lane >= o) { wa += ta; wb += tb; }
+    }
+    total_a = __shfl_sync(0xffffffffu, wa, 31);
+    total_b = __shfl_sync(0xffffffffu, wb, 31);
+    a = ia - a + __shfl_sync(0xffffffffu, wa - own_a, warp);
+    b = ib - b + __shfl_sync(0xffffffffu, wb - own_b, warp);
 }
+
+// A thread's groups: counts, scratch and segments (-1 past the end).  Segments with list entries are counted into `seg`.
+struct ScanItems {
+    int u[kScanPerThread], cls[kScanPerThread], rank[kScanPerThread];
+    long long scr[kScanPerThread], vectors = 0, scratch = 0;
+    __device__ __forceinline__ void load(int m_vec, const int* counts, const int* tbl_len, int* seg) {
+        const int first = blockIdx.x * kScanBlock + threadIdx.x * kScanPerThread;
+        int len[kScanPerThread];
+#pragma unroll
+        for (int j = 0; j < kScanPerThread; ++j) {
+            u[j] = first + j < m_vec ? counts[first + j] : 0;
+            len[j] = first + j < m_vec ? tbl_len[first + j] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < kScanPerThread; ++j) {
+            cls[j] = -1; scr[j] = 0; rank[j] = 0;
+            if (first + j >= m_vec) continue;
+            scr[j] = group_scratch_ints(u[j], len[j]);
+            cls[j] = list_segment(u[j], len[j]);
+            vectors += u[j];
+            scratch += scr[j];
+        }
+        // one atomic per segment and warp: most groups of a matrix are in one or two segments
+#pragma unroll
+        for (int j = 0; j < kScanPerThread; ++j) {
+            const unsigned peers = __match_any_sync(0xffffffffu, cls[j]);
+            const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+            int base = 0;
+            if (lane == leader && cls[j] >= 0) base = atomicAdd(&seg[cls[j]], __popc(peers));
+            rank[j] = __shfl_sync(0xffffffffu, base, leader) + __popc(peers & ((1u << lane) - 1u));
+        }
+    }
+};
 
 __global__ void __launch_bounds__(kScanThreads)
 svc_scan_sums_kernel(int m_vec, const int* __restrict__ counts, const int* __restrict__ tbl_len,
                      long long* __restrict__ block_sums) {
-    __shared__ long long sh[32];
-    long long f[kScanFields];
-#pragma unroll
-    for (int k = 0; k < kScanFields; ++k) f[k] = 0;
-    const int first = blockIdx.x * kScanBlock + threadIdx.x * kScanPerThread;
-#pragma unroll
-    for (int j = 0; j < kScanPerThread; ++j) {
-        const int i = first + j;
-        if (i >= m_vec) break;
-        const int u = counts[i], len = tbl_len[i];
-        f[0] += u;
-        f[1] += group_scratch_ints(u, len);
-        const int c = list_segment(u, len);
-#pragma unroll
-        for (int k = 0; k < kNumSegs; ++k) f[2 + k] += (c == k) ? 1 : 0;
-    }
-#pragma unroll
-    for (int k = 0; k < kScanFields; ++k) {
-        const long long t = block_sum_ll(f[k], sh);
-        if (threadIdx.x == 0) block_sums[(size_t)blockIdx.x * kScanFields + k] = t;
-    }
+    __shared__ long long sh[2][32];
+    __shared__ int seg[kNumSegs];
+    if (threadIdx.x < kNumSegs) seg[threadIdx.x] = 0;
+    __syncthreads();
+    ScanItems it;
+    it.load(m_vec, counts, tbl_len, seg);
+    long long a = it.vectors, b = it.scratch, total_a, total_b;
+    block_prefix_pair(a, b, total_a, total_b, sh);          // its barrier also completes the segment counts
+    long long* mine = block_sums + (size_t)blockIdx.x * kScanFields;
+    if (threadIdx.x == 0) { mine[0] = total_a; mine[1] = total_b; }
+    if (threadIdx.x < kNumSegs) mine[2 + threadIdx.x] = seg[threadIdx.x];
 }
 
-// One CTA: block_sums -> exclusive prefixes in place, and the totals.
-__global__ void __launch_bounds__(kScanThreads)
+// One CTA: block_sums -> exclusive prefixes in place, and the totals; a warp per field.
+__global__ void __launch_bounds__(32 * kScanFields)
 svc_scan_blocks_kernel(int n_blocks, long long* __restrict__ block_sums, long long* __restrict__ totals) {
-    __shared__ long long sh[32];
-    __shared__ long long carry[kScanFields];
-    if (threadIdx.x < kScanFields) carry[threadIdx.x] = 0;
-    __syncthreads();
-    for (int b0 = 0; b0 < n_blocks; b0 += kScanThreads) {
-        const int b = b0 + threadIdx.x;
-        for (int k = 0; k < kScanFields; ++k) {
-            const long long v = (b < n_blocks) ? block_sums[(size_t)b * kScanFields + k] : 0;
-            const long long ex = block_prefix_ll(v, sh);
-            const long long c0 = carry[k];
-            if (b < n_blocks) block_sums[(size_t)b * kScanFields + k] = c0 + ex;
-            __syncthreads();
-            if (threadIdx.x == kScanThreads - 1) carry[k] = c0 + ex + v;
-            __syncthreads();
+    const int field = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    long long carry = 0;
+    for (int b0 = 0; b0 < n_blocks; b0 += 32) {
+        const int b = b0 + lane;
+        const long long v = b < n_blocks ? block_sums[(size_t)b * kScanFields + field] : 0;
+        long long inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
         }
+        if (b < n_blocks) block_sums[(size_t)b * kScanFields + field] = carry + inc - v;
+        carry += __shfl_sync(0xffffffffu, inc, 31);
     }
+    if (lane == 0) totals[field] = carry;
     if (threadIdx.x == 0) {
-        for (int k = 0; k < kScanFields; ++k) totals[k] = carry[k];
         totals[kScanFields] = g_svc_bad_column;          // reported with the totals, then cleared
         g_svc_bad_column = 0;
     }
 }
 
 // vec_ptr: counts in, exclusive scan out (and the total at [m_vec]); tbl_off: scratch offsets; class_list: the
-// replayed groups segment by segment (see list_segment), inside a segment in ascending order.
+// replayed groups segment by segment (see list_segment).  ALONE: the only block, which also writes the totals.
+template <bool ALONE>
 __global__ void __launch_bounds__(kScanThreads)
 svc_scan_place_kernel(int m_vec, int* __restrict__ vec_ptr, const int* __restrict__ tbl_len,
                       long long* __restrict__ tbl_off, const long long* __restrict__ block_sums,
-                      const long long* __restrict__ totals, int* __restrict__ class_list) {
-    __shared__ long long sh[32];
-    const int first = blockIdx.x * kScanBlock + threadIdx.x * kScanPerThread;
-    int u[kScanPerThread], cls[kScanPerThread];
-    long long scr[kScanPerThread];
-    long long f[kScanFields];
-#pragma unroll
-    for (int k = 0; k < kScanFields; ++k) f[k] = 0;
-#pragma unroll
-    for (int j = 0; j < kScanPerThread; ++j) {
-        const int i = first + j;
-        u[j] = 0; scr[j] = 0; cls[j] = -1;
-        if (i < m_vec) {
-            u[j] = vec_ptr[i];
-            const int len = tbl_len[i];
-            scr[j] = group_scratch_ints(u[j], len);
-            cls[j] = list_segment(u[j], len);
-            f[0] += u[j];
-            f[1] += scr[j];
-#pragma unroll
-            for (int k = 0; k < kNumSegs; ++k) f[2 + k] += (cls[j] == k) ? 1 : 0;
-        }
-    }
+                      long long* __restrict__ totals, int* __restrict__ class_list) {
+    __shared__ long long sh[2][32];
+    __shared__ int seg[kNumSegs], seg_at[kNumSegs];
+    if (threadIdx.x < kNumSegs) seg[threadIdx.x] = 0;
+    __syncthreads();
+    ScanItems it;
+    it.load(m_vec, vec_ptr, tbl_len, seg);
+    long long a = it.vectors, b = it.scratch, total_a, total_b;
+    block_prefix_pair(a, b, total_a, total_b, sh);          // its barrier also completes the segment counts
     // where segment k starts in the list: after all groups of the segments before it (segment 0 is not replayed)
-    long long at[kScanFields];
-#pragma unroll
-    for (int k = 0; k < kScanFields; ++k)
-        at[k] = block_sums[(size_t)blockIdx.x * kScanFields + k] + block_prefix_ll(f[k], sh);
-    long long class_base = 0;
-#pragma unroll
-    for (int k = 1; k < kNumSegs; ++k) {
-        at[2 + k] += class_base;
-        class_base += totals[2 + k];
+    if (threadIdx.x < 32) {
+        const int k = threadIdx.x;
+        const int groups = k >= 1 && k < kNumSegs ? (ALONE ? seg[k] : (int)totals[2 + k]) : 0;
+        const int start = warp_incl_scan(groups, k) - groups;
+        if (k < kNumSegs) seg_at[k] = start + (ALONE ? 0 : (int)block_sums[(size_t)blockIdx.x * kScanFields + 2 + k]);
     }
+    __syncthreads();
+    if (!ALONE) {
+        a += block_sums[(size_t)blockIdx.x * kScanFields];
+        b += block_sums[(size_t)blockIdx.x * kScanFields + 1];
+    }
+    const int first = blockIdx.x * kScanBlock + threadIdx.x * kScanPerThread;
 #pragma unroll
     for (int j = 0; j < kScanPerThread; ++j) {
         const int i = first + j;
         if (i >= m_vec) break;
-        vec_ptr[i] = (int)at[0];
-        tbl_off[i] = at[1];
-        at[0] += u[j];
-        at[1] += scr[j];
-#pragma unroll
-        for (int k = 1; k < kNumSegs; ++k)
-            if (cls[j] == k) class_list[at[2 + k]++] = i;
+        vec_ptr[i] = (int)a;
+        tbl_off[i] = b;
+        a += it.u[j];
+        b += it.scr[j];
+        if (it.cls[j] > 0) class_list[seg_at[it.cls[j]] + it.rank[j]] = i;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (ALONE) {
+        if (threadIdx.x < kNumSegs) totals[2 + threadIdx.x] = seg[threadIdx.x];
+        if (threadIdx.x == 0) {
+            totals[0] = total_a; totals[1] = total_b;
+            vec_ptr[m_vec] = (int)total_a;
+            tbl_off[m_vec] = total_b;
+            totals[kScanFields] = g_svc_bad_column;          // reported with the totals, then cleared
+            g_svc_bad_column = 0;
+        }
+    } else if (blockIdx.x == 0 && threadIdx.x == 0) {
         vec_ptr[m_vec] = (int)totals[0];
         tbl_off[m_vec] = totals[1];
     }
@@ -485,6 +501,8 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
             if ((unsigned)c < (unsigned)p.K) atomicOr(&bm[c >> 5], 1u << (c & 31));
         }
         Team::sync();
+        // columns by a lane per bit when the words are well filled (a thread per word would write up to 32 of them in turn)
+        const bool by_bit = Team::kSize >= 256 && (e1 - e0) >= 8 * words;
         int running = 0;
         for (int w0 = 0; w0 < words; w0 += Team::kSize) {
             const int w = w0 + tid;
@@ -512,15 +530,51 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
             int o = running + incl - pc;
             if (w < words) pre[w] = (unsigned)o;
             o += base;
-            while (word) {
+            while (word && !by_bit) {
                 const int b = __ffs(word) - 1;
                 out_col[o++] = w * 32 + b;
                 word &= word - 1;
             }
             running += chunk_total;
         }
+        if (by_bit) {
+            Team::sync();
+            const int lane = tid & 31;
+#pragma unroll 4
+            for (int w = tid >> 5; w < words; w += Team::kSize / 32) {
+                const unsigned word = bm[w];
+                if ((word >> lane) & 1u) out_col[base + (int)pre[w] + __popc(word & ((1u << lane) - 1u))] = w * 32 + lane;
+            }
+        }
         if (out_vals) {
             Team::sync();
+            int longest = 0;
+            if (Team::kSize >= 256)
+                for (int r = r0; r < r1; ++r) longest = max(longest, p.row_ptr[r + 1] - p.row_ptr[r]);
+            if (Team::kSize >= 256 && longest <= (e1 - e0) / 4 + 128) {
+                // a warp per matrix row: no search for the row of an entry, and four entries' look-ups in flight (rows of
+                // a power-law group differ too much for it: one warp would do nearly all of them)
+                const int lane = tid & 31;
+                for (int r = r0 + (tid >> 5); r < r1; r += Team::kSize / 32) {
+                    const int a0 = p.row_ptr[r], a1 = p.row_ptr[r + 1];
+                    __half* const col0 = out_vals + (int64_t)base * p.V + (r - i * p.V);
+                    for (int e = a0 + lane; e < a1; e += 128) {
+                        int c[4];
+                        __half v[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            c[k] = e + 32 * k < a1 ? p.col_idx[e + 32 * k] : -1;
+                            v[k] = e + 32 * k < a1 ? p.vals[e + 32 * k] : __half(0);
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if ((unsigned)c[k] < (unsigned)p.K) {
+                                const int pos = (int)pre[c[k] >> 5] + __popc(bm[c[k] >> 5] & ((1u << (c[k] & 31)) - 1u));
+                                col0[(int64_t)pos * p.V] = v[k];
+                            }
+                    }
+                }
+            } else {
             // all entries of the group, flat; the matrix row of entry e is found by walking the (at most V) row ends
             for (int e = e0 + tid; e < e1; e += Team::kSize) {
                 int r = r0;
@@ -530,6 +584,7 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
                     const int pos = (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
                     out_vals[((int64_t)base + pos) * p.V + (r - i * p.V)] = p.vals[e];
                 }
+            }
             }
         }
         Team::sync();
@@ -1026,9 +1081,13 @@ cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool /*
         if (e != cudaSuccess) return e;
     }
     const int n_blocks = p.m_vec > 0 ? (p.m_vec + kScanBlock - 1) / kScanBlock : 1;
+    if (n_blocks == 1) {
+        svc_scan_place_kernel<true><<<1, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, nullptr, s.totals, s.class_list);
+        return cudaGetLastError();
+    }
     svc_scan_sums_kernel<<<n_blocks, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.block_sums);
-    svc_scan_blocks_kernel<<<1, kScanThreads, 0, stream>>>(n_blocks, s.block_sums, s.totals);
-    svc_scan_place_kernel<<<n_blocks, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, s.block_sums, s.totals,
+    svc_scan_blocks_kernel<<<1, 32 * kScanFields, 0, stream>>>(n_blocks, s.block_sums, s.totals);
+    svc_scan_place_kernel<false><<<n_blocks, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, s.block_sums, s.totals,
                                                                  s.class_list);
     return cudaGetLastError();
 }
