@@ -832,39 +832,42 @@ __device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, i
             const int first_new = max(e_len, n_cur);
             bool dup_here = false;          // also raised when a bound is hit: the group is then redone sequentially
             volatile int* vtab = tab;
-            for (int q4 = tid; q4 < n_l && !dup_here; q4 += 4 * Team::kSize) {
-              int k4[4];
-#pragma unroll
-              for (int b = 0; b < 4; ++b) k4[b] = (q4 + b * Team::kSize < n_l) ? seq[q4 + b * Team::kSize] : 0;
-#pragma unroll
-              for (int b = 0; b < 4; ++b) {
-                const int q = q4 + b * Team::kSize;
-                if (q >= n_l || dup_here) break;
-                int e = q, key = k4[b];
-                Probe pr = probe_begin(key, mask);
-                for (unsigned tries = 0;; ++tries) {
-                    const int slot = (int)(pr.i + pr.w);
-                    // Slot values only ever decrease during a level, so a slot seen with an earlier element stays
-                    // out of reach; only a slot that looks free or later is worth the atomic.
-                    int cur = vtab[slot];
-                    if (cur > e) cur = atomicMin(&tab[slot], e);
-                    if (cur > e) {
-                        if (cur == kEmptyPrio) break;            // free slot taken: this chain ends
-                        // a later element sat here: the same thread carries it on, from the start of its own path
-                        // (every slot it passed before still holds an earlier element, so it walks to the same
-                        // place and beyond)
+            // One probe per turn of the loop, and a thread whose chain has ended goes on with its next element at once: a warp
+            // then takes as many turns as its slowest thread has probes in all, not the sum of the longest chains of its
+            // rounds (chains are 1.1 probes long on average, the longest of 32 several times that).
+            int q = tid;
+            int e = q, key = q < n_l ? seq[q] : 0;
+            int ahead = q + Team::kSize < n_l ? seq[q + Team::kSize] : 0;     // the next element's key, loaded early
+            Probe pr = probe_begin(key, mask);
+            unsigned tries = 0;
+            while (q < n_l) {
+                const int slot = (int)(pr.i + pr.w);
+                // Slot values only ever decrease during a level, so a slot seen with an earlier element stays
+                // out of reach; only a slot that looks free or later is worth the atomic.
+                int cur = vtab[slot];
+                if (cur > e) cur = atomicMin(&tab[slot], e);
+                if (cur > e) {
+                    // free slot taken: this chain ends.  Otherwise a later element sat here: the same thread carries it on,
+                    // from the start of its own path (every slot it passed before still holds an earlier element, so it
+                    // walks to the same place and beyond).
+                    if (cur == kEmptyPrio) {
+                        q += Team::kSize;
+                        e = q;
+                        key = ahead;
+                        ahead = q + Team::kSize < n_l ? seq[q + Team::kSize] : 0;
+                        tries = 0;
+                    } else {
                         e = cur;
                         key = seq[e];
-                        pr = probe_begin(key, mask);
-                        continue;
                     }
-                    if ((e >= first_new && seq[cur] == key) || tries > 16u * mask + 256u) {
-                        dup_here = true;
-                        break;
-                    }
-                    probe_advance(pr, mask);
+                    pr = probe_begin(key, mask);
+                    continue;
                 }
-              }
+                if ((e >= first_new && seq[cur] == key) || ++tries > 16u * mask + 256u) {
+                    dup_here = true;
+                    break;
+                }
+                probe_advance(pr, mask);
             }
             Team::sync();
             if (Team::any(dup_here, red)) { duplicate = true; break; }
