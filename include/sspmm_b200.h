@@ -207,7 +207,7 @@ int sspmm_group_destroy(sspmm_group* group);
 /* Kernel selection for the calls above: 0 = automatic (default), 1 = tensor-core
  * row-gather kernel fed by TMA gather requests (error if the operands do not qualify),
  * 2 = CUDA-core kernel only, 3 = tensor-core block kernel only, 4 = tensor-core
- * row-gather kernel fed by load instructions, 5 = block kernel only and without its
+ * row-gather kernel whose warps gather by themselves, 5 = block kernel only and without its
  * CTA-pair variant (one CTA per tile).  Process-wide; for tests and profiling. */
 int sspmm_set_kernel(int which);
 
