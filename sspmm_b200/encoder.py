@@ -90,8 +90,10 @@ class SparseEncoderLayer:
     def _norm(self, x, wb, add=None, bias=None, out=None, sum_out=None):
         """LayerNorm of x + bias + add: (what was normalised, the result)."""
         given = [t for t in (x, add, bias, *wb) if t is not None]
-        if _plain(*given) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
-                (add is None or add.shape == x.shape) and all(t.numel() == x.shape[0] for t in given if t is not x and t is not add):
+        whole = [t for t in (add, out, sum_out) if t is not None]           # the kernel takes these to lie as x does
+        if _plain(*given, *whole) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
+                all(t.shape == x.shape for t in whole) and (bias is None or add is not None) and \
+                all(t.numel() == x.shape[0] for t in given if t is not x and t is not add):
             out = torch.empty_like(x) if out is None else out
             if add is not None and sum_out is None:
                 sum_out = torch.empty_like(x)
