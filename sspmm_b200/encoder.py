@@ -20,8 +20,8 @@ from . import ops, synthetic
 
 
 def _plain(*tensors) -> bool:
-    """Tensors the kernels can take as they lie: contiguous fp16 on the GPU, 16-byte aligned, outside autograd."""
-    return all(t.is_cuda and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
+    """Tensors the kernels can take as they lie: contiguous fp16 on one GPU, 16-byte aligned, outside autograd."""
+    return all(t.is_cuda and t.device == tensors[0].device and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
                and not (t.requires_grad and torch.is_grad_enabled()) for t in tensors)
 
 
@@ -93,7 +93,7 @@ class SparseEncoderLayer:
         whole = [t for t in (add, out, sum_out) if t is not None]           # the kernel takes these to lie as x does
         if _plain(*given, *whole) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
                 all(t.shape == x.shape for t in whole) and (bias is None or add is not None) and \
-                all(t.numel() == x.shape[0] for t in given if t is not x and t is not add):
+                all(tuple(t.shape) == (x.shape[0],) for t in given if t is not x and t is not add):
             out = torch.empty_like(x) if out is None else out
             if add is not None and sum_out is None:
                 sum_out = torch.empty_like(x)

@@ -61,6 +61,8 @@ def sspmm_bias(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: 
         _require(bias, torch.float16, "bias")
         if bias.numel() != m_vec * vec_length:
             raise ValueError(f"bias has {bias.numel()} numbers, the product {m_vec * vec_length} rows")
+        if bias.device != rhs.device:
+            raise ValueError(f"bias is on {bias.device}, rhs on {rhs.device}")
     K, N = rhs.shape
     if out is None:
         out = torch.empty((m_vec * vec_length, N), dtype=out_dtype, device=rhs.device)
@@ -171,29 +173,53 @@ def sorted_row_swizzle(row_offsets: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def _require_fm(t: torch.Tensor, shape, like: torch.Tensor, name: str) -> None:
+    """An operand of the feature-major operators: the kernels see only its address."""
+    if tuple(t.shape) != tuple(shape):
+        raise ValueError(f"{name} has shape {tuple(t.shape)}, not {tuple(shape)}")
+    if t.device != like.device:
+        raise ValueError(f"{name} is on {t.device}, not {like.device}")
+    _require(t, torch.float16, name)
+
+
 def layer_norm_fm(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, eps: float, out: torch.Tensor,
                   add: Optional[torch.Tensor] = None, sum_out: Optional[torch.Tensor] = None,
                   bias: Optional[torch.Tensor] = None) -> None:
     """LayerNorm over dim 0 of x[hidden, tokens] + bias + add (that sum goes to ``sum_out``), ``sspmm_layer_norm_fm``."""
+    hidden, tokens = x.shape
+    if add is not None and sum_out is None:
+        raise ValueError("add needs sum_out")
+    for t, shape, name in ((x, x.shape, "x"), (gamma, (hidden,), "gamma"), (beta, (hidden,), "beta"), (bias, (hidden,), "bias"),
+                           (add, x.shape, "add"), (sum_out, x.shape, "sum_out"), (out, x.shape, "out")):
+        if t is not None:
+            _require_fm(t, shape, x, name)
     with torch.cuda.device(x.device):
-        capi.check(capi.lib().sspmm_layer_norm_fm(x.shape[0], x.shape[1], x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
+        capi.check(capi.lib().sspmm_layer_norm_fm(hidden, tokens, x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
                                                   gamma.data_ptr(), beta.data_ptr(), eps, out.data_ptr(), _stream_ptr()))
 
 
 def add_bias_fm(x: torch.Tensor, bias: torch.Tensor, add: torch.Tensor) -> torch.Tensor:
     """x[rows, tokens] + bias[:, None] + add, ``sspmm_add_bias_fm``."""
+    rows, tokens = x.shape
+    for t, shape, name in ((x, x.shape, "x"), (bias, (rows,), "bias"), (add, x.shape, "add")):
+        _require_fm(t, shape, x, name)
     out = torch.empty_like(x)
     with torch.cuda.device(x.device):
-        capi.check(capi.lib().sspmm_add_bias_fm(x.shape[0], x.shape[1], x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr(),
+        capi.check(capi.lib().sspmm_add_bias_fm(rows, tokens, x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr(),
                                                 _stream_ptr()))
     return out
 
 
 def attention_fm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, batch: int, seq: int, out: torch.Tensor,
                  bias_q: Optional[torch.Tensor] = None, bias_v: Optional[torch.Tensor] = None) -> None:
-    """Softmax attention on feature-major q, k, v [hidden, batch * seq], ``sspmm_attention_fm``."""
+    """Softmax attention of heads 64 wide on feature-major q, k, v [64 * heads, batch * seq], ``sspmm_attention_fm``."""
+    hidden = 64 * heads
+    for t, shape, name in ((q, (hidden, batch * seq), "q"), (k, (hidden, batch * seq), "k"), (v, (hidden, batch * seq), "v"),
+                           (out, (hidden, batch * seq), "out"), (bias_q, (hidden,), "bias_q"), (bias_v, (hidden,), "bias_v")):
+        if t is not None:
+            _require_fm(t, shape, q, name)
     with torch.cuda.device(q.device):
-        capi.check(capi.lib().sspmm_attention_fm(heads, q.shape[0] // heads, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+        capi.check(capi.lib().sspmm_attention_fm(heads, 64, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                                  _ptr(bias_q), _ptr(bias_v), out.data_ptr(), _stream_ptr()))
 
 

@@ -48,3 +48,56 @@ def test_norm_returns_what_was_normalised(launches):
     L, x, bias = layer(), torch.randn(8, 8).half(), torch.randn(8).half()
     was, _ = L._norm(x, L.ln1, bias=bias)
     assert torch.equal(was, x + bias[:, None])
+
+
+def fm(*shape, dtype=torch.float16):
+    return torch.zeros(shape, dtype=dtype)
+
+
+@pytest.mark.parametrize("change,message", [
+    ({"gamma": fm(7)}, "gamma has shape"), ({"beta": fm(8, 1)}, "beta has shape"), ({"out": fm(8, 8)}, "out has shape"),
+    ({"add": fm(8, 8), "sum_out": fm(8, 16)}, "add has shape"), ({"add": fm(8, 16)}, "add needs sum_out"),
+    ({"add": fm(8, 16), "sum_out": fm(16, 8)}, "sum_out has shape"), ({"bias": fm(9)}, "bias has shape"),
+    ({"gamma": torch.empty(8, device="meta").half()}, "gamma is on")])
+def test_layer_norm_rejects_operands_of_other_shapes(change, message):
+    args = {"x": fm(8, 16), "gamma": fm(8), "beta": fm(8), "eps": 1e-5, "out": fm(8, 16), **change}
+    # x itself is looked at first and is on the host here: give the others a chance
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(encoder.ops, "_require", lambda *a: None)
+        m.setattr(encoder.ops.capi, "lib", lambda: pytest.fail("launched"))
+        with pytest.raises(ValueError, match=message):
+            encoder.ops.layer_norm_fm(**args)
+
+
+@pytest.mark.parametrize("change,message", [
+    ({"q": fm(128, 24)}, "q has shape"), ({"k": fm(64, 24)}, "k has shape"), ({"v": fm(128, 16)}, "v has shape"),
+    ({"out": fm(128, 32)}, "out has shape"), ({"bias_q": fm(64)}, "bias_q has shape"), ({"bias_v": fm(128, 1)}, "bias_v has shape"),
+    ({"heads": 1}, "q has shape"), ({"seq": 8}, "q has shape")])
+def test_attention_rejects_operands_of_other_shapes(change, message):
+    args = {"q": fm(128, 48), "k": fm(128, 48), "v": fm(128, 48), "heads": 2, "batch": 3, "seq": 16, "out": fm(128, 48), **change}
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(encoder.ops, "_require", lambda *a: None)
+        m.setattr(encoder.ops.capi, "lib", lambda: pytest.fail("launched"))
+        with pytest.raises(ValueError, match=message):
+            encoder.ops.attention_fm(**args)
+
+
+def test_feature_major_operators_reject_types_and_layouts():
+    ops, x, w = encoder.ops, fm(8, 16), fm(8)
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(torch.Tensor, "is_cuda", True)
+        m.setattr(ops.capi, "lib", lambda: pytest.fail("launched"))
+        for bad, error in ((x.float(), TypeError), (fm(16, 8).t(), ValueError), (fm(8, 8), ValueError)):
+            with pytest.raises(error):
+                ops.add_bias_fm(x, w, bad)
+            with pytest.raises(error):
+                ops.layer_norm_fm(x, w, w, 1e-5, bad)
+        for bad, error in ((w.float(), TypeError), (fm(16)[::2], ValueError), (fm(7), ValueError)):
+            with pytest.raises(error):
+                ops.add_bias_fm(x, bad, x)
+            with pytest.raises(error):
+                ops.layer_norm_fm(x, w, bad, 1e-5, x)
+        q = fm(64, 16)
+        for bad in (q.float(), fm(16, 64).t()):
+            with pytest.raises((TypeError, ValueError)):
+                ops.attention_fm(q, q, bad, 1, 1, 16, q)
