@@ -15,12 +15,16 @@ from typing import Optional
 import numpy as np
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import ops, synthetic
 
 
 def _plain(*tensors) -> bool:
-    """Tensors the kernels can take as they lie: contiguous fp16 on one GPU, 16-byte aligned, outside autograd."""
+    """Tensors the kernels can take as they lie: contiguous fp16 on one GPU, 16-byte aligned, outside autograd, function
+    transforms and forward-mode differentiation (a dual tensor has an address too, and no requires_grad)."""
+    if torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0:
+        return False
     return all(t.is_cuda and t.device == tensors[0].device and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
                and not (t.requires_grad and torch.is_grad_enabled()) for t in tensors)
 

@@ -101,3 +101,29 @@ def test_feature_major_operators_reject_types_and_layouts():
         for bad in (q.float(), fm(16, 64).t()):
             with pytest.raises((TypeError, ValueError)):
                 ops.attention_fm(q, q, bad, 1, 1, 16, q)
+
+
+def test_transformed_tensors_take_the_general_path(monkeypatch):
+    """Products, LayerNorm and attention as framework operations carry tangents and batch dimensions; kernels drop them."""
+    monkeypatch.setattr(torch.Tensor, "is_cuda", True)
+    monkeypatch.setattr(encoder.ops, "layer_norm_fm", lambda *a, **k: pytest.fail("launched"))
+    monkeypatch.setattr(encoder.ops, "sspmm_bias", lambda *a, **k: pytest.fail("launched"))
+    monkeypatch.setattr(encoder.ops, "sspmm", lambda *a, **k: torch.zeros(8, 16).half())
+    L, x, t = layer(), torch.randn(8, 16).half(), torch.randn(8, 16).half()
+    assert encoder._plain(x, t)
+    general = lambda a: L._layer_norm_fm(a, L.ln1)
+    assert torch.equal(torch.func.jvp(lambda a: L._norm(a, L.ln1)[1], (x,), (t,))[1], torch.func.jvp(general, (x,), (t,))[1])
+    with torch.autograd.forward_ad.dual_level():
+        y = L._norm(torch.autograd.forward_ad.make_dual(x, t), L.ln1)[1]
+        assert torch.autograd.forward_ad.unpack_dual(y).tangent.any()
+    xs = torch.stack([x, t])
+    assert torch.equal(torch.vmap(lambda a: L._norm(a, L.ln1)[1])(xs), torch.vmap(general)(xs))
+    lin = encoder.SparseLinear.__new__(encoder.SparseLinear)
+    lin.out_features, lin.V = 8, 8
+    lin.row_offsets = lin.col = lin.values = lin.row_indices = None
+
+    def with_bias(b):
+        lin.bias = b
+        return lin(x)
+    b, db = torch.randn(8).half(), torch.randn(8).half()
+    assert torch.equal(torch.func.jvp(with_bias, (b,), (db,))[1], db[:, None].expand(8, 16))
