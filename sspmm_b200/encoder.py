@@ -162,11 +162,15 @@ class SparseEncoderLayer:
         return (b["y"] if L[5].bias is None else b["y"] + L[5].bias[:, None]) + out
 
     def forward(self, x: torch.Tensor, batch: int, seq: int, dense: bool = False) -> torch.Tensor:
-        """x: [hidden, batch*seq] fp16, feature-major (token t of sequence b is column b*seq + t)."""
-        lin = [(l.dense_forward if dense else l) for l in self.linears]
-        _, out = self._norm(x, self.ln1)
-        q, k, v = lin[0](out), lin[1](out), lin[2](out)
-        att = lin[3](self._attend(q, k, v, batch, seq))
+        """x: [hidden, batch*seq] fp16, feature-major (token t of sequence b is column b*seq + t).  ``dense``: the same layer
+        with dense products and framework operations only, nothing of this package's kernels."""
+        L = self.linears
+        if dense:
+            y = self._layer_norm_fm(x, self.ln1)
+            q, k, v = (l.dense_forward(y) for l in L[:3])
+            out = L[3].dense_forward(self._attention(q, k, v, batch, seq).contiguous()) + x
+            return L[5].dense_forward(L[4].dense_forward(self._layer_norm_fm(out, self.ln2))) + out
+        _, y = self._norm(x, self.ln1)
+        att = L[3](self._attend(L[0](y), L[1](y), L[2](y), batch, seq))
         out, y = self._norm(att, self.ln2, add=x)
-        y = lin[5](lin[4](y))
-        return y + out
+        return L[5](L[4](y)) + out

@@ -127,3 +127,26 @@ def test_transformed_tensors_take_the_general_path(monkeypatch):
         return lin(x)
     b, db = torch.randn(8).half(), torch.randn(8).half()
     assert torch.equal(torch.func.jvp(with_bias, (b,), (db,))[1], db[:, None].expand(8, 16))
+
+
+def test_dense_evaluation_uses_none_of_the_kernels(monkeypatch):
+    monkeypatch.setattr(encoder, "_plain", lambda *t: True)
+    for name in ("layer_norm_fm", "attention_fm", "add_bias_fm", "sspmm", "sspmm_bias"):
+        monkeypatch.setattr(encoder.ops, name, lambda *a, **k: pytest.fail("launched"))
+    L = layer(64)
+    for _ in range(6):
+        lin = encoder.SparseLinear.__new__(encoder.SparseLinear)
+        lin.dense, lin.bias = torch.randn(64, 64).half() / 8, torch.randn(64).half()
+        L.linears.append(lin)
+    x = torch.randn(64, 48).half().requires_grad_()
+    y = L.forward(x, 3, 16, dense=True)
+    d = [(l.dense.double(), l.bias.double()[:, None]) for l in L.linears]
+    norm = lambda t: (t - t.mean(0)) / torch.sqrt(t.var(0, unbiased=False) + 1e-5)
+    n = norm(x.double())
+    q, k, v = ((w @ n + b).view(64, 3, 16).permute(1, 2, 0) for w, b in d[:3])
+    att = (torch.softmax(q @ k.transpose(1, 2) / 8, -1) @ v).permute(2, 0, 1).reshape(64, 48)
+    out = d[3][0] @ att + d[3][1] + x.double()
+    ref = d[5][0] @ (d[4][0] @ norm(out) + d[4][1]) + d[5][1] + out
+    assert (y.double() - ref).norm() <= 4e-3 * ref.norm()            # eight roundings to fp16 of at most 2^-11 each
+    y.sum().backward()
+    assert x.grad is not None and x.grad.any()
