@@ -25,7 +25,8 @@ def _plain(*tensors) -> bool:
     transforms and forward-mode differentiation (a dual tensor has an address too, and no requires_grad)."""
     if torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0:
         return False
-    return all(t.is_cuda and t.device == tensors[0].device and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
+    gpu = tensors[0].get_device()
+    return gpu >= 0 and all(t.get_device() == gpu and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
                and not (t.requires_grad and torch.is_grad_enabled()) for t in tensors)
 
 
@@ -94,14 +95,14 @@ class SparseEncoderLayer:
     def _norm(self, x, wb, add=None, bias=None, out=None, sum_out=None):
         """LayerNorm of x + bias + add: (what was normalised, the result)."""
         given = [t for t in (x, add, bias, *wb) if t is not None]
-        whole = [t for t in (add, out, sum_out) if t is not None]           # the kernel takes these to lie as x does
-        if _plain(*given, *whole) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
-                all(t.shape == x.shape for t in whole) and (bias is None or add is not None) and \
-                all(tuple(t.shape) == (x.shape[0],) for t in given if t is not x and t is not add):
+        room = [t for t in (out, sum_out) if t is not None]
+        if _plain(*given, *room) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
+                (add is None or add.shape == x.shape) and all(t.shape == x.shape for t in room) and (bias is None or add is not None) and \
+                all(t.shape == (x.shape[0],) for t in given if t is not x and t is not add):
             out = torch.empty_like(x) if out is None else out
             if add is not None and sum_out is None:
                 sum_out = torch.empty_like(x)
-            ops.layer_norm_fm(x, wb[0], wb[1], 1e-5, out, add, sum_out, bias)
+            ops.launch_layer_norm_fm(x, wb[0], wb[1], 1e-5, out, add, sum_out, bias)
             return (x if add is None else sum_out), out
         if bias is not None:
             x = x + bias[:, None]
@@ -113,10 +114,11 @@ class SparseEncoderLayer:
     def _attend(self, q, k, v, batch, seq, biases=(None, None, None), out=None):
         tokens = (self.hidden, batch * seq)
         given = [b for b in biases if b is not None]
-        if self.hidden == 64 * self.heads and seq % 8 == 0 and seq > 0 and 0 < batch <= 65535 and _plain(q, k, v, *given) and \
-                all(tuple(t.shape) == tokens for t in (q, k, v)) and all(tuple(b.shape) == (self.hidden,) for b in given):
+        whole = [q, k, v] if out is None else [q, k, v, out]
+        if self.hidden == 64 * self.heads and seq % 8 == 0 and seq > 0 and 0 < batch <= 65535 and _plain(*whole, *given) and \
+                all(t.shape == tokens for t in whole) and all(b.shape == (self.hidden,) for b in given):
             out = torch.empty_like(q) if out is None else out
-            ops.attention_fm(q, k, v, self.heads, batch, seq, out, biases[0], biases[2])      # one of k changes nothing
+            ops.launch_attention_fm(q, k, v, self.heads, batch, seq, out, biases[0], biases[2])      # one of k changes nothing
             return out
         q, k, v = (t if b is None else t + b[:, None] for t, b in zip((q, k, v), biases))
         att = self._attention(q, k, v, batch, seq)
@@ -157,8 +159,8 @@ class SparseEncoderLayer:
             b["h"] += L[4].bias[:, None]
         g[3].run()
         bias = L[5].bias_rows()
-        if bias is not None and _plain(out) and out.shape[1] % 8 == 0:
-            return ops.add_bias_fm(b["y"], bias, out)
+        if bias is not None and _plain(b["y"], bias, out) and out.shape == b["y"].shape and out.shape[1] % 8 == 0:
+            return ops.launch_add_bias_fm(b["y"], bias, out)
         return (b["y"] if L[5].bias is None else b["y"] + L[5].bias[:, None]) + out
 
     def forward(self, x: torch.Tensor, batch: int, seq: int, dense: bool = False) -> torch.Tensor:

@@ -193,8 +193,13 @@ def layer_norm_fm(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, eps:
                            (add, x.shape, "add"), (sum_out, x.shape, "sum_out"), (out, x.shape, "out")):
         if t is not None:
             _require_fm(t, shape, x, name)
+    launch_layer_norm_fm(x, gamma, beta, eps, out, add, sum_out, bias)
+
+
+def launch_layer_norm_fm(x, gamma, beta, eps, out, add, sum_out, bias) -> None:
+    """``layer_norm_fm`` for a caller that has compared the operands itself."""
     with torch.cuda.device(x.device):
-        capi.check(capi.lib().sspmm_layer_norm_fm(hidden, tokens, x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
+        capi.check(capi.lib().sspmm_layer_norm_fm(x.shape[0], x.shape[1], x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
                                                   gamma.data_ptr(), beta.data_ptr(), eps, out.data_ptr(), _stream_ptr()))
 
 
@@ -203,9 +208,14 @@ def add_bias_fm(x: torch.Tensor, bias: torch.Tensor, add: torch.Tensor) -> torch
     rows, tokens = x.shape
     for t, shape, name in ((x, x.shape, "x"), (bias, (rows,), "bias"), (add, x.shape, "add")):
         _require_fm(t, shape, x, name)
+    return launch_add_bias_fm(x, bias, add)
+
+
+def launch_add_bias_fm(x, bias, add) -> torch.Tensor:
+    """``add_bias_fm`` for a caller that has compared the operands itself."""
     out = torch.empty_like(x)
     with torch.cuda.device(x.device):
-        capi.check(capi.lib().sspmm_add_bias_fm(rows, tokens, x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr(),
+        capi.check(capi.lib().sspmm_add_bias_fm(x.shape[0], x.shape[1], x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr(),
                                                 _stream_ptr()))
     return out
 
@@ -218,6 +228,11 @@ def attention_fm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, 
                            (out, (hidden, batch * seq), "out"), (bias_q, (hidden,), "bias_q"), (bias_v, (hidden,), "bias_v")):
         if t is not None:
             _require_fm(t, shape, q, name)
+    launch_attention_fm(q, k, v, heads, batch, seq, out, bias_q, bias_v)
+
+
+def launch_attention_fm(q, k, v, heads, batch, seq, out, bias_q, bias_v) -> None:
+    """``attention_fm`` for a caller that has compared the operands itself."""
     with torch.cuda.device(q.device):
         capi.check(capi.lib().sspmm_attention_fm(heads, 64, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(),
                                                  _ptr(bias_q), _ptr(bias_v), out.data_ptr(), _stream_ptr()))

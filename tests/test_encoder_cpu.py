@@ -10,7 +10,7 @@ def launches(monkeypatch):
     """Every tensor counts as one the kernels can take, and launches are only counted."""
     made = []
     monkeypatch.setattr(encoder, "_plain", lambda *t: True)
-    monkeypatch.setattr(encoder.ops, "layer_norm_fm", lambda *a, **k: made.append(a))
+    monkeypatch.setattr(encoder.ops, "launch_layer_norm_fm", lambda *a, **k: made.append(a))
     return made
 
 
@@ -105,8 +105,8 @@ def test_feature_major_operators_reject_types_and_layouts():
 
 def test_transformed_tensors_take_the_general_path(monkeypatch):
     """Products, LayerNorm and attention as framework operations carry tangents and batch dimensions; kernels drop them."""
-    monkeypatch.setattr(torch.Tensor, "is_cuda", True)
-    monkeypatch.setattr(encoder.ops, "layer_norm_fm", lambda *a, **k: pytest.fail("launched"))
+    monkeypatch.setattr(torch.Tensor, "get_device", lambda t: 0)
+    monkeypatch.setattr(encoder.ops, "launch_layer_norm_fm", lambda *a, **k: pytest.fail("launched"))
     monkeypatch.setattr(encoder.ops, "sspmm_bias", lambda *a, **k: pytest.fail("launched"))
     monkeypatch.setattr(encoder.ops, "sspmm", lambda *a, **k: torch.zeros(8, 16).half())
     L, x, t = layer(), torch.randn(8, 16).half(), torch.randn(8, 16).half()
@@ -131,7 +131,7 @@ def test_transformed_tensors_take_the_general_path(monkeypatch):
 
 def test_dense_evaluation_uses_none_of_the_kernels(monkeypatch):
     monkeypatch.setattr(encoder, "_plain", lambda *t: True)
-    for name in ("layer_norm_fm", "attention_fm", "add_bias_fm", "sspmm", "sspmm_bias"):
+    for name in ("launch_layer_norm_fm", "launch_attention_fm", "launch_add_bias_fm", "sspmm", "sspmm_bias"):
         monkeypatch.setattr(encoder.ops, name, lambda *a, **k: pytest.fail("launched"))
     L = layer(64)
     for _ in range(6):
