@@ -50,11 +50,12 @@ struct Problem {
     int64_t values_stride, rhs_stride, out_stride;
     int out_pieces;                       // rows of C start on 16-byte boundaries
     // split launches only (see sspmm_rows_split_kernel)
-    int chunk, cap;                       // vectors per part of a cut row, room for parts
-    int* header;                          // [0] parts, [1] next row item
+    int chunk;                            // vectors per part
+    int cap_cut, cap_whole;               // room for parts of rows with several, and for rows that are one part
+    int* header;                          // [0] parts of rows with several, [1] next row item, [2] rows that are one part
     int* arrivals;                        // [part][n_tile], at a row's part 0: its finished parts
-    int4* entries;                        // per part: vector row, first vector, vectors, parts of the row << 16 | number
-    float* partial;                       // [part][n_tile][V][NT] sums
+    int4* entries;                        // vector row, first vector, vectors, parts of the row << 16 | number: cap_cut parts, cap_whole rows
+    float* partial;                       // [part][n_tile][V][NT] sums, of rows with several parts only
 };
 
 // d += a * b of one instruction: 16 columns x 8 rows of C, 16 vectors deep.
@@ -396,8 +397,8 @@ sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int
 // vectors, the longest tens of thousands; n = 51970, V = 8, N = 128: 46.8 us, with one CTA of tcgen05 stages per SM 67.8).
 // Rows longer than kLightRow are cut into parts of at most p.chunk vectors (listed by list_parts_kernel); a CTA does a
 // part with all its warps, the parts dealt out in turn since they are of one size, and whoever finishes the last part of
-// a row adds the parts up in order.  Then the warps, each on its own, take the remaining rows in the caller's order from
-// a counter.
+// a row adds the parts up in order.  Rows of a single part follow those with several: they write C themselves and have no
+// partial sums.  Then the warps, each on its own, take the remaining rows in the caller's order from a counter.
 template <int V, typename OutT, int H>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_split_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
@@ -407,16 +408,20 @@ sspmm_rows_split_kernel(const __grid_constant__ Problem p, OutT* __restrict__ ou
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint8_t* const mem = smem + warp * T::kWarpBytes;
     // The list was sized from a vector count; if the matrix needs more parts than fit, nothing is cut.
-    const int listed = p.header[0];
-    const bool cut = listed <= p.cap;
-    const int parts_total = cut ? listed * p.n_tiles : 0;
+    const int several = p.header[0], whole = p.header[2];
+    const bool cut = several <= p.cap_cut && whole <= p.cap_whole;
+    const int parts_total = cut ? (several + whole) * p.n_tiles : 0;
     const int none = INT_MAX;
+    auto entry = [&](int at) {
+        const int i = at / p.n_tiles;
+        return p.entries[i < several ? i : p.cap_cut + (i - several)];
+    };
     int x = (int)blockIdx.x < parts_total ? (int)blockIdx.x : none;
-    int4 en = x < parts_total ? p.entries[x / p.n_tiles] : make_int4(0, 0, 0, 0);
+    int4 en = x < parts_total ? entry(x) : make_int4(0, 0, 0, 0);
     while (x < parts_total) {
         const int x2 = x < parts_total - (int)gridDim.x ? x + (int)gridDim.x : none;
         int4 en2 = make_int4(0, 0, 0, 0);
-        if (x2 < parts_total) en2 = p.entries[x2 / p.n_tiles];
+        if (x2 < parts_total) en2 = entry(x2);
         const int nt = x % p.n_tiles, part = en.w & 0xffff, parts = (int)((unsigned)en.w >> 16);
         T tile;
         tile.clear();
@@ -489,12 +494,14 @@ sspmm_rows_split_kernel(const __grid_constant__ Problem p, OutT* __restrict__ ou
 // header; with several the header is zero at launch.
 __global__ void __launch_bounds__(1024)
 list_parts_kernel(const __grid_constant__ Problem p) {
-    __shared__ int count;
+    __shared__ int count[2];
     const bool alone = gridDim.x == 1;
-    if (threadIdx.x == 0) count = 0;
+    if (threadIdx.x < 2) count[threadIdx.x] = 0;
     __syncthreads();
+    int* const several = alone ? &count[0] : p.header;
+    int* const whole = alone ? &count[1] : p.header + 2;
     const int stride = gridDim.x * 1024;
-    for (int x = blockIdx.x * 1024 + threadIdx.x; x < p.cap * p.n_tiles; x += stride) p.arrivals[x] = 0;
+    for (int x = blockIdx.x * 1024 + threadIdx.x; x < p.cap_cut * p.n_tiles; x += stride) p.arrivals[x] = 0;
     for (int64_t b = blockIdx.x * 1024 + threadIdx.x; b < p.m_vec; b += 4LL * stride) {
         int j0[4], len[4];
 #pragma unroll
@@ -506,14 +513,20 @@ list_parts_kernel(const __grid_constant__ Problem p) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             if (len[k] <= kLightRow) continue;
-            const int n = (len[k] + p.chunk - 1) / p.chunk;
-            const int first = alone ? atomicAdd(&count, n) : atomicAdd(p.header, n);
-            for (int c = 0; c < n && first + c < p.cap; ++c)
-                p.entries[first + c] = make_int4((int)(b + (int64_t)k * stride), j0[k] + c * p.chunk, min(p.chunk, len[k] - c * p.chunk), n << 16 | c);
+            const int row = (int)(b + (int64_t)k * stride);
+            if (len[k] <= p.chunk) {
+                const int at = atomicAdd(whole, 1);
+                if (at < p.cap_whole) p.entries[p.cap_cut + at] = make_int4(row, j0[k], len[k], 1 << 16);
+                continue;
+            }
+            const int n = (int)(((unsigned)len[k] + p.chunk - 1) / p.chunk);
+            const int first = atomicAdd(several, n);
+            for (int c = 0; c < n && first + c < p.cap_cut; ++c)
+                p.entries[first + c] = make_int4(row, j0[k] + c * p.chunk, min(p.chunk, len[k] - c * p.chunk), n << 16 | c);
         }
     }
     __syncthreads();
-    if (alone && threadIdx.x == 0) { p.header[0] = count; p.header[1] = 0; }
+    if (alone && threadIdx.x == 0) { p.header[0] = count[0]; p.header[1] = 0; p.header[2] = count[1]; }
 }
 
 template <typename Kern>
@@ -569,9 +582,10 @@ cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, bool split,
     return H == 2 ? launch_plain<V, OutT, 2>(a, p, team, cluster) : launch_plain<V, OutT, 1>(a, p, team, cluster);
 }
 
-// Scratch of the variant that cuts rows: [16 B header][cap * n_tiles arrival counters][cap entries][partial tiles].
+// Scratch of the variant that cuts rows: [16 B header][cap_cut * n_tiles arrival counters][cap_cut + cap_whole entries]
+// [cap_cut * n_tiles partial tiles].
 struct Scratch {
-    int chunk = 0, cap = 0;                 // chunk = 0: not worth cutting
+    int chunk = 0, cap_cut = 0, cap_whole = 0;      // chunk = 0: not worth cutting
     size_t entries_at = 0, partial_at = 0, bytes = 0;
 };
 // Rows are worth cutting when some row may be many times the mean: the columns bound a row's length, so K tells, and the
@@ -587,13 +601,14 @@ Scratch plan_scratch(const SpmmArgs& a, long long nvec) {
     // N = 128) takes 46.8 us with a quarter, 52.1 with an eighth and 78 with a sixteenth (every part drains the rings once).
     long long c = nvec * n_tiles / ((long long)sms * 4) / 128 * 128;
     if (c < 512) c = 512;
-    // every cut row has at most one part that is not full
-    const long long cap = nvec / c + nvec / kLightRow + 1;
-    const long long tiles = cap * n_tiles;
-    if (c > 0x3fffffff || a.K / c >= 32767 || tiles > 0x3fffffff || tiles * a.V * nt * 4 > (1LL << 30)) return r;
-    r.chunk = (int)c; r.cap = (int)cap;
+    // A row with several parts has at most one that is not full, so its parts are fewer than twice its vectors / c; their
+    // partial sums are a few MB at any N (two tiles for each of the sms * 4 shares).
+    const long long cap_cut = 2 * nvec / c + 1, cap_whole = nvec / kLightRow + 1;
+    const long long tiles = cap_cut * n_tiles, items = tiles + cap_whole * n_tiles;
+    if (c > 0x3fffffff || a.K / c >= 32767 || items > 0x3fffffff || tiles * a.V * nt * 4 > (1LL << 30)) return r;
+    r.chunk = (int)c; r.cap_cut = (int)cap_cut; r.cap_whole = (int)cap_whole;
     r.entries_at = 16 + (((size_t)tiles * 4 + 15) & ~(size_t)15);
-    r.partial_at = r.entries_at + (size_t)cap * 16;
+    r.partial_at = r.entries_at + (size_t)(cap_cut + cap_whole) * 16;
     r.bytes = (r.partial_at + (size_t)tiles * a.V * nt * 4 + 255) & ~(size_t)255;
     return r;
 }
@@ -632,7 +647,7 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     p.row_indices = a.row_indices; p.row_offsets = a.row_offsets; p.col = a.column_indices;
     p.values = a.values; p.rhs = a.rhs; p.bias = a.bias;
     p.values_stride = a.values_stride; p.rhs_stride = a.rhs_stride; p.out_stride = a.out_stride;
-    p.chunk = 0; p.cap = 0; p.header = nullptr; p.arrivals = nullptr; p.entries = nullptr; p.partial = nullptr;
+    p.chunk = 0; p.cap_cut = 0; p.cap_whole = 0; p.header = nullptr; p.arrivals = nullptr; p.entries = nullptr; p.partial = nullptr;
     const size_t es = a.out_f16 ? 2 : 4;
     p.out_pieces = (a.n_out % 8 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 &&
                     (a.batch == 1 || ((size_t)a.out_stride * es) % 16 == 0)) ? 1 : 0;
@@ -655,7 +670,7 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     if (split) {
         const rows::Scratch r = rows::plan_scratch(a, nvec);
         uint8_t* s = static_cast<uint8_t*>(scratch);
-        p.chunk = r.chunk; p.cap = r.cap;
+        p.chunk = r.chunk; p.cap_cut = r.cap_cut; p.cap_whole = r.cap_whole;
         p.header = reinterpret_cast<int*>(s);
         p.arrivals = reinterpret_cast<int*>(s + 16);
         p.entries = reinterpret_cast<int4*>(s + r.entries_at);

@@ -82,3 +82,12 @@ def test_python_ops_refuse_cpu_tensors():
     t = torch.zeros(3, dtype=torch.int32)
     with pytest.raises(ValueError):
         ops.sspmm(t, t, torch.zeros(8, dtype=torch.float16), torch.zeros(4, 8, dtype=torch.float16), 8)
+
+
+@pytest.mark.parametrize("n,V,N", [(51970, 8, 128), (65536, 16, 256), (65536, 8, 1024), (65536, 16, 4096), (655360, 8, 1024), (1000000, 16, 512)])
+def test_long_rows_are_cut_at_any_width(lib, n, V, N):
+    """Sixteen non-zeros per row, each a vector of its own: the cut rows' partial sums stay within a few MB (they were 9 to 15
+    for the first), so that no size goes without."""
+    from sspmm_b200 import ops
+    b = ops.workspace_bytes(-(-n // V), V, N, n, 16 * n)
+    assert 0 < b <= 20e6

@@ -131,3 +131,46 @@ def test_bias_in_every_epilogue(lib, V, lens, K, N):
         finally:
             ops.set_kernel(ops.KERNEL_AUTO)
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("V,N", [(8, 1000), (16, 4096)])
+def test_cut_rows_of_wide_products(lib, V, N):
+    """Parts grow with the number of column tiles: rows of several parts, of one, and short ones, over many tiles."""
+    lens = [2900, 513, 512, 257, 256, 0, 2900, 600] + [20] * 200
+    ptr, col, val, rhs = operands(lens, 3000, V, N, 10)
+    assert ops.workspace_bytes(len(lens), V, N, 3000, sum(lens)) > 0
+    for dt in (torch.float16, torch.float32):
+        check(ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt), ptr, col, val, rhs, V)
+
+
+@pytest.mark.parametrize("V,N", [(8, 136), (16, 64)])
+def test_cut_rows_listed_by_many_ctas(lib, V, N):
+    """More than 16384 vector rows: the list comes from several CTAs."""
+    lens = [3] * 9000 + [2500, 0, 300, 900] + [2] * 11000 + [1100]
+    ptr, col, val, rhs = operands(lens, 2600, V, N, 11)
+    assert ops.workspace_bytes(len(lens), V, N, 2600, sum(lens)) > 0
+    got = ops.sspmm(ptr, col, val, rhs, V, out_dtype=torch.float32)
+    for a, b in ((0, 40), (8990, 9020), (20000, len(lens))):
+        part = (ptr[a:b + 1] - ptr[a]).int()
+        s = slice(int(ptr[a]), int(ptr[b]))
+        check(got[a * V:b * V], part, col[s], val.view(-1, V)[s].reshape(-1), rhs, V)
+    assert torch.equal(got, ops.sspmm(ptr, col, val, rhs, V, row_indices=ops.sorted_row_swizzle(ptr), out_dtype=torch.float32))
+
+
+@pytest.mark.parametrize("stated", [300, 4000, 20000])
+def test_a_count_that_is_too_small_cuts_nothing(lib, stated):
+    """The list is sized from the count; when the matrix holds more long rows than that, the result is the same."""
+    from sspmm_b200 import capi
+    V, N, K = 8, 72, 3000
+    lens = [2800] * 40 + [300] * 300 + [10] * 60
+    ptr, col, val, rhs = operands(lens, K, V, N, 12)
+    assert ops.workspace_bytes(len(lens), V, N, K, stated) > 0
+    out = torch.full((len(lens) * V, N), float("nan"), device=DEV)
+    for kernel in (ops.KERNEL_AUTO, ops.KERNEL_GATHER_LSU):
+        ops.set_kernel(kernel)
+        try:
+            capi.check(capi.lib().sspmm_counted(len(lens), V, N, K, 1, stated, None, ptr.data_ptr(), col.data_ptr(), val.data_ptr(), 0,
+                                                rhs.data_ptr(), 0, None, out.data_ptr(), 0, 0, torch.cuda.current_stream().cuda_stream))
+            check(out, ptr, col, val, rhs, V)
+        finally:
+            ops.set_kernel(ops.KERNEL_AUTO)
