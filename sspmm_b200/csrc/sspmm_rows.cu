@@ -529,6 +529,23 @@ list_parts_kernel(const __grid_constant__ Problem p) {
     if (alone && threadIdx.x == 0) { p.header[0] = count[0]; p.header[1] = 0; p.header[2] = count[1]; }
 }
 
+// How the one-launch kernel divides a product by the mean row.  Tile width: 128 columns halve the work per gathered byte
+// outside the loads; 64 when that is all there is or when wide tiles, a CTA each, would leave SMs without one.  Warps per item:
+// enough to fill the SMs, at least one step each; long rows get a whole CTA so that no single warp runs long after the others.
+struct Division { int H, team, cluster; };
+Division divide(const SpmmArgs& a, long long nvec, int sms) {
+    const long long rows_total = (long long)a.m_vec * a.batch, slots = (long long)sms * kResident * kWarps;
+    const long long mean_steps = nvec > 0 ? (nvec / a.m_vec + kStep) / kStep : (a.K / 2 + kStep) / kStep;
+    Division d{a.N > 64 ? 2 : 1, 1, 1};
+    if (d.H == 2 && rows_total * ((a.N + 127) / 128) * std::min<long long>(mean_steps, kWarps) < slots) d.H = 1;
+    const long long items = rows_total * ((a.N + 64 * d.H - 1) / (64 * d.H));
+    const long long want = std::min(slots / items, mean_steps);
+    while (d.team < kWarps && (2 * d.team <= want || mean_steps > 32LL * d.team)) d.team *= 2;
+    if (d.team == kWarps)
+        while (d.cluster < kMaxCluster && (long long)d.cluster * 2 * d.team <= want && mean_steps >= 4LL * d.cluster * d.team) d.cluster *= 2;
+    return d;
+}
+
 template <typename Kern>
 cudaError_t allow_smem(Kern kern, DeviceOnce& once, int bytes) {
     if (once.done()) return cudaSuccess;
@@ -539,22 +556,22 @@ cudaError_t allow_smem(Kern kern, DeviceOnce& once, int bytes) {
 }
 
 template <int V, typename OutT, int H>
-cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, int team, int cluster) {
+cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d) {
     auto kern = sspmm_rows_kernel<V, OutT, H>;
     using T = Tile<V, H, sizeof(OutT) == 4>;
     static DeviceOnce once;
     cudaError_t e = allow_smem(kern, once, kWarps * T::kWarpBytes);
     if (e != cudaSuccess) return e;
-    const int per_cta = kWarps / team;
+    const int per_cta = kWarps / d.team;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((p.items + per_cta - 1) / per_cta * cluster));
+    cfg.gridDim = dim3((unsigned)((p.items + per_cta - 1) / per_cta * d.cluster));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = (size_t)kWarps * T::kWarpBytes; cfg.stream = a.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, p, static_cast<OutT*>(a.out), team, cluster);
+    attr[0].val.clusterDim.x = (unsigned)d.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = d.cluster > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, p, static_cast<OutT*>(a.out), d.team, d.cluster);
 }
 
 template <int V, typename OutT, int H>
@@ -577,9 +594,9 @@ cudaError_t launch_split(const SpmmArgs& a, const Problem& p, int sms) {
 }
 
 template <int V, typename OutT>
-cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, bool split, int team, int cluster, int sms) {
+cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, bool split, const Division& d, int sms) {
     if (split) return H == 2 ? launch_split<V, OutT, 2>(a, p, sms) : launch_split<V, OutT, 1>(a, p, sms);
-    return H == 2 ? launch_plain<V, OutT, 2>(a, p, team, cluster) : launch_plain<V, OutT, 1>(a, p, team, cluster);
+    return H == 2 ? launch_plain<V, OutT, 2>(a, p, d) : launch_plain<V, OutT, 1>(a, p, d);
 }
 
 // Scratch of the variant that cuts rows: [16 B header][cap_cut * n_tiles arrival counters][cap_cut + cap_whole entries]
@@ -589,13 +606,18 @@ struct Scratch {
     size_t entries_at = 0, partial_at = 0, bytes = 0;
 };
 // Rows are worth cutting when some row may be many times the mean: the columns bound a row's length, so K tells, and the
-// vector count tells the mean.
+// vector count tells the mean.  Below 2048 columns that is so only where the one-launch kernel leaves a warp more than 48 steps of
+// such a row (a step takes about 0.65 us, the list of parts 5): eight rows of 2000 vectors among 1024 of 40, V = 16, N = 128,
+// 41 to 46 us, cut 14; 512 rows of 36 of 1200, V = 8, N = 1024, 11 us, listed in vain 15.
 Scratch plan_scratch(const SpmmArgs& a, long long nvec) {
     Scratch r;
     if (nvec <= 0 || a.batch != 1) return r;
-    const long long mean = nvec / a.m_vec + 1;
-    if (a.K < 2048 || a.K < 8 * mean) return r;
     const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;
+    if (a.K < 8 * (nvec / a.m_vec + 1)) return r;
+    if (a.K < 2048) {
+        const Division d = divide(a, nvec, sms);
+        if (a.K <= 48LL * kStep * d.team * d.cluster) return r;
+    }
     const long long nt = a.N <= 64 ? 64 : 128, n_tiles = (a.N + nt - 1) / nt;
     // A part: a quarter of an SM's share of the vectors, at least four steps per warp.  n = 51970 (820 k vectors, V = 8,
     // N = 128) takes 46.8 us with a quarter, 52.1 with an eighth and 78 with a sixteenth (every part drains the rings once).
@@ -652,21 +674,16 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     p.out_pieces = (a.n_out % 8 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 &&
                     (a.batch == 1 || ((size_t)a.out_stride * es) % 16 == 0)) ? 1 : 0;
     const bool split = scratch != nullptr;
-    // Tile width: 128 columns halve the work per gathered byte outside the loads; 64 when that is all there is or (one-launch
-    // kernel) when wide tiles, a CTA each, would leave SMs without one.
-    const long long rows_total = (long long)a.m_vec * a.batch;
-    const long long mean_steps = nvec > 0 ? (nvec / a.m_vec + rows::kStep) / rows::kStep : (a.K / 2 + rows::kStep) / rows::kStep;
+    const rows::Division d = rows::divide(a, nvec, sms);
+    const int H = split ? (a.N > 64 ? 2 : 1) : d.H;
     const long long slots = (long long)sms * rows::kResident * rows::kWarps;
-    int H = a.N > 64 ? 2 : 1;
-    if (H == 2 && !split && rows_total * ((a.N + 127) / 128) * std::min<long long>(mean_steps, rows::kWarps) < slots) H = 1;
     const int nt = 64 * H;
     p.n_tiles = (a.N + nt - 1) / nt;
-    p.items = rows_total * p.n_tiles;
+    p.items = (long long)a.m_vec * a.batch * p.n_tiles;
     if (p.items + slots > 0x7fffffffLL / rows::kMaxCluster) {
         set_error("problem too large for 32-bit tile ids");
         return cudaErrorInvalidValue;
     }
-    int team = 1, cluster = 1;
     if (split) {
         const rows::Scratch r = rows::plan_scratch(a, nvec);
         uint8_t* s = static_cast<uint8_t*>(scratch);
@@ -675,17 +692,10 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
         p.arrivals = reinterpret_cast<int*>(s + 16);
         p.entries = reinterpret_cast<int4*>(s + r.entries_at);
         p.partial = reinterpret_cast<float*>(s + r.partial_at);
-    } else {
-        // Warps per item: enough to fill the SMs, at least one step each; long rows get a whole CTA so that no single
-        // warp runs long after the others.
-        const long long want = std::min(slots / p.items, mean_steps);
-        while (team < rows::kWarps && (2 * team <= want || mean_steps > 32LL * team)) team *= 2;
-        if (team == rows::kWarps)
-            while (cluster < rows::kMaxCluster && (long long)cluster * 2 * team <= want && mean_steps >= 4LL * cluster * team) cluster *= 2;
     }
     if (a.V == 16)
-        return a.out_f16 ? rows::launch_typed<16, __half>(a, p, H, split, team, cluster, sms) : rows::launch_typed<16, float>(a, p, H, split, team, cluster, sms);
-    return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, split, team, cluster, sms) : rows::launch_typed<8, float>(a, p, H, split, team, cluster, sms);
+        return a.out_f16 ? rows::launch_typed<16, __half>(a, p, H, split, d, sms) : rows::launch_typed<16, float>(a, p, H, split, d, sms);
+    return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, split, d, sms) : rows::launch_typed<8, float>(a, p, H, split, d, sms);
 }
 
 // ---- dense operands whose rows do not start on 16-byte boundaries -------------------------------

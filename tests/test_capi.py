@@ -91,3 +91,11 @@ def test_long_rows_are_cut_at_any_width(lib, n, V, N):
     from sspmm_b200 import ops
     b = ops.workspace_bytes(-(-n // V), V, N, n, 16 * n)
     assert 0 < b <= 20e6
+
+
+@pytest.mark.parametrize("m_vec,K,mean,V,N,cut", [
+    (1024, 2000, 40, 16, 128, True), (4096, 2000, 20, 8, 64, True), (256, 1000, 20, 8, 1024, True),
+    (64, 600, 20, 8, 1024, False), (512, 700, 20, 16, 256, False), (512, 2000, 300, 16, 256, False), (256, 1000, 20, 8, 64, False)])
+def test_rows_are_cut_where_a_warp_would_be_left_with_a_long_one(lib, m_vec, K, mean, V, N, cut):
+    from sspmm_b200 import ops
+    assert (ops.workspace_bytes(m_vec, V, N, K, m_vec * mean) > 0) == cut

@@ -174,3 +174,31 @@ def test_a_count_that_is_too_small_cuts_nothing(lib, stated):
             check(out, ptr, col, val, rhs, V)
         finally:
             ops.set_kernel(ops.KERNEL_AUTO)
+
+
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("lens,K,N", [
+    ([1500] + [30] * 4000, 1600, 128), ([20] * 2403 + [257, 256, 700, 1, 1600], 1600, 136), ([1600] * 9 + [0] * 700 + [512, 513], 1600, 64),
+    ([30] * 300 + [1025, 1024, 1600], 1600, 200), ([300] * 600 + [2000] * 3, 2000, 1000)])
+def test_long_rows_below_2048_columns(lib, V, lens, K, N):
+    """Long rows among short ones, cut (all but the last) and not; any order gives the same numbers."""
+    ptr, col, val, rhs = operands(lens, K, V, N, 15)
+    ops.set_kernel(ops.KERNEL_GATHER_LSU)
+    try:
+        base = ops.sspmm(ptr, col, val, rhs, V, out_dtype=torch.float32)
+        check(base, ptr, col, val, rhs, V)
+        for order in (ops.sorted_row_swizzle(ptr), torch.randperm(len(lens), device=DEV).int()):
+            assert torch.equal(base, ops.sspmm(ptr, col, val, rhs, V, row_indices=order, out_dtype=torch.float32))
+        check(ops.sspmm(ptr, col, val, rhs, V), ptr, col, val, rhs, V)
+    finally:
+        ops.set_kernel(ops.KERNEL_AUTO)
+
+
+def test_long_rows_of_a_batch(lib):
+    V, K, N, lens = 8, 1024, 72, [1024, 1024] + [40] * 70 + [600]
+    ptr, col, val, _ = operands(lens, K, V, 8, 16)
+    rhs = torch.randn(30, K, N, device=DEV).half()
+    vals = torch.stack([val * (1 - b / 64) for b in range(30)])
+    got = bspmm(ops.sorted_row_swizzle(ptr), ptr, col, vals, rhs, V)
+    for b in (0, 1, 17, 29):
+        check(got[b], ptr, col, vals[b], rhs[b], V)
