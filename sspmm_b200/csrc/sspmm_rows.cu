@@ -680,7 +680,7 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     const int nt = 64 * H;
     p.n_tiles = (a.N + nt - 1) / nt;
     p.items = (long long)a.m_vec * a.batch * p.n_tiles;
-    if (p.items + slots > 0x7fffffffLL / rows::kMaxCluster) {
+    if (p.items + slots > 0x7fffffffLL) {                  // the work counter, and CTAs (clusters only where items are few)
         set_error("problem too large for 32-bit tile ids");
         return cudaErrorInvalidValue;
     }

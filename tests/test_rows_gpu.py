@@ -202,3 +202,25 @@ def test_long_rows_of_a_batch(lib):
     got = bspmm(ops.sorted_row_swizzle(ptr), ptr, col, vals, rhs, V)
     for b in (0, 1, 17, 29):
         check(got[b], ptr, col, vals[b], rhs[b], V)
+
+
+def test_more_than_two_to_the_28_items(lib):
+    """Vector rows times column tiles are counted in 32 bits: up to 2^31 - 1 of them, less what the counter may run over."""
+    V, N, K, m_vec = 8, 8, 64, (1 << 28) + 3
+    if torch.cuda.mem_get_info()[0] < 60 << 30:
+        pytest.skip("needs 36 GB")
+    ptr = torch.zeros(m_vec + 1, dtype=torch.int32, device=DEV)
+    ptr[5:] = 2
+    ptr[m_vec] = 5
+    col = torch.tensor([3, 60, 1, 2, 63], dtype=torch.int32, device=DEV)
+    val = torch.randn(5 * V, device=DEV).half()
+    rhs = torch.randn(K, N, device=DEV).half()
+    out = torch.full((m_vec * V, N), float("nan"), dtype=torch.float16, device=DEV)
+    ops.sspmm(ptr, col, val, rhs, V, out=out)
+    v = val.double().view(5, V, 1)
+    for row, s in ((4, slice(0, 2)), (m_vec - 1, slice(2, 5))):
+        ref = (v[s] * rhs[col[s].long()].double()[:, None, :]).sum(0)
+        assert (out[row * V:row * V + V].double() - ref).abs().max() <= 2.0 ** -9 * ref.abs().max()
+    # everything else was written, with zeros
+    assert sum(int(torch.count_nonzero(part)) for part in out.view(-1).split(1 << 30)) == 2 * V * N
+    assert ops.device_status() == 0
