@@ -654,11 +654,10 @@ cudaError_t launch_block_pair(const SpmmArgs& a, const CUtensorMap& ta, const CU
     return cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, p);
 }
 
-// out[i] = sum over splits of partial[s][i], converted once.  Rows of `partial` have N columns (a multiple of 8), rows of
-// C the first n_out of them.
+// out[i] = sum over splits of partial[s][i] (and the row's bias), converted once.
 template <typename OutT>
 __global__ void __launch_bounds__(256)
-reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, int64_t elems, int splits, int N, int n_out,
+reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, int64_t elems, int splits, int N,
                      const __half* __restrict__ bias) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= elems) return;                                      // elems is a multiple of 4 (N % 8 == 0)
@@ -667,21 +666,11 @@ reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, 
         const float4 v = *reinterpret_cast<const float4*>(partial + (int64_t)s2 * elems + i);
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
-    const int64_t row = n_out != N || bias ? i / N : 0;
     if (bias) {
-        const float b = __half2float(bias[row]);
+        const float b = __half2float(bias[i / N]);
         acc.x += b; acc.y += b; acc.z += b; acc.w += b;
     }
-    if (n_out != N) {
-        const int n = (int)(i - row * N);
-        const float v[4] = {acc.x, acc.y, acc.z, acc.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (n + e < n_out) {
-                if constexpr (sizeof(OutT) == 2) out[row * n_out + n + e] = __float2half_rn(v[e]);
-                else out[row * n_out + n + e] = v[e];
-            }
-    } else if constexpr (sizeof(OutT) == 2) {
+    if constexpr (sizeof(OutT) == 2) {
         __half2 lo = __floats2half2_rn(acc.x, acc.y), hi = __floats2half2_rn(acc.z, acc.w);
         uint2 w;
         w.x = *reinterpret_cast<uint32_t*>(&lo); w.y = *reinterpret_cast<uint32_t*>(&hi);
@@ -722,8 +711,7 @@ BlockPlan plan_block(const SpmmArgs& a, int sms, size_t budget) {
     const int k_steps = (a.K + kBK - 1) / kBK;
     pl.steps_per_split = k_steps;
     pl.at_bytes = (((size_t)a.K * Mp * sizeof(__half)) + 255) & ~(size_t)255;
-    // rows of C that are not whole 16-byte pieces are written by the reduction, whatever the number of splits
-    pl.partial_bytes = a.n_out != a.N ? (size_t)Mp * a.N * sizeof(float) : 0;
+    pl.partial_bytes = 0;
     if (pl.pair || a.batch != 1 || tiles256 >= units || k_steps < 8) return pl;
     // Fewer 256-column tiles than SMs: pick tile width and split-K factor by a small time model
     // (microseconds, constants measured on B200): a work item costs 2 + steps * 0.40 (128 columns) or
@@ -738,7 +726,7 @@ BlockPlan plan_block(const SpmmArgs& a, int sms, size_t budget) {
             if (want > 1 && sps < 4) break;
             const int splits = (k_steps + sps - 1) / sps;                // every split gets at least one step
             if (splits != want) continue;
-            const size_t bytes = splits > 1 || a.n_out != a.N ? (size_t)splits * Mp * a.N * sizeof(float) : 0;
+            const size_t bytes = splits > 1 ? (size_t)splits * Mp * a.N * sizeof(float) : 0;
             if (pl.at_bytes + bytes > budget) continue;
             const int64_t waves = (tiles * splits + units - 1) / units;
             double t = (double)waves * (2.0 + sps * (bn == 256 ? 0.45 : 0.40));
@@ -795,9 +783,9 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     }
     p.total_tiles = (int)total;
     p.out_stride = a.out_stride;
-    p.bias = pl.splits > 1 || a.n_out != a.N ? nullptr : a.bias;
+    p.bias = pl.splits > 1 ? nullptr : a.bias;
     CUtensorMap ta, tb, tc;
-    const bool split = pl.splits > 1 || a.n_out != a.N;           // fp32 partial tiles, then the reduction
+    const bool split = pl.splits > 1;
     if (split && pl.at_bytes + pl.partial_bytes > scratch_bytes) {
         set_error("scratch too small for the split-K partial tiles");
         return cudaErrorInvalidValue;
@@ -846,8 +834,8 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     if (e != cudaSuccess || !split) return e;
     const int64_t elems = (int64_t)Mp * a.N;
     const unsigned rgrid = (unsigned)((elems / 4 + 255) / 256);
-    if (a.out_f16) reduce_splits_kernel<__half><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<__half*>(a.out), elems, pl.splits, a.N, a.n_out, a.bias);
-    else reduce_splits_kernel<float><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<float*>(a.out), elems, pl.splits, a.N, a.n_out, a.bias);
+    if (a.out_f16) reduce_splits_kernel<__half><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<__half*>(a.out), elems, pl.splits, a.N, a.bias);
+    else reduce_splits_kernel<float><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<float*>(a.out), elems, pl.splits, a.N, a.bias);
     return cudaGetLastError();
 }
 

@@ -224,3 +224,36 @@ def test_more_than_two_to_the_28_items(lib):
     # everything else was written, with zeros
     assert sum(int(torch.count_nonzero(part)) for part in out.view(-1).split(1 << 30)) == 2 * V * N
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("V,M,K,N,offset", [(8, 64, 1024, 1001, 0), (16, 128, 4608, 601, 0), (8, 128, 2048, 1024, 4)])
+def test_unaligned_dense_operand_keeps_fp32_sums(lib, V, M, K, N, offset):
+    """Products that the dense-tile path would take if they were aligned: fp32 results are no further from 64 bits than those of
+    the CUDA-core kernel, which adds in round-to-nearest."""
+    ptr, col, val, rhs = operands([K - 24] * M, K, V, N, 13, offset)
+    ref, _ = exact(ptr, col, val, rhs, V)
+    error = {}
+    for kernel in (ops.KERNEL_AUTO, ops.KERNEL_BLOCK, ops.KERNEL_SIMT):
+        ops.set_kernel(kernel)
+        try:
+            error[kernel] = (ops.sspmm(ptr, col, val, rhs, V, out_dtype=torch.float32).double() - ref).norm()
+        finally:
+            ops.set_kernel(ops.KERNEL_AUTO)
+    assert error[ops.KERNEL_AUTO] <= error[ops.KERNEL_SIMT] and error[ops.KERNEL_BLOCK] <= error[ops.KERNEL_SIMT]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("N,offset", [(1001, 0), (1024, 3)])
+def test_unaligned_dense_operand_with_infinities(lib, N, offset, dtype):
+    """An infinity or NaN of B reaches the vector rows that name its row, and no others."""
+    K, V, lens = 1024, 8, [900] * 64
+    ptr, col, val, rhs = operands(lens, K, V, N, 14, offset)
+    rhs[5, 7], rhs[900, N - 1], rhs[17, 30] = float("inf"), float("-inf"), float("nan")
+    got = ops.sspmm(ptr, col, val, rhs, V, out_dtype=dtype)
+    names = lambda k: torch.stack([(col[a:b] == k).any() for a, b in zip(ptr[:-1].tolist(), ptr[1:].tolist())])
+    want = torch.zeros(len(lens) * V, N, dtype=torch.bool, device=DEV)
+    for k, n in ((5, 7), (900, N - 1), (17, 30)):
+        hit = names(k).repeat_interleave(V)
+        assert hit.any() and not hit.all()
+        want[:, n] = hit
+    assert torch.equal(~got.isfinite(), want)
