@@ -169,14 +169,21 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
 // address of the 16-byte piece (feature row, piece) of a tile
 __device__ __forceinline__ uint32_t at(uint32_t tile, int row, int piece) { return tile + row * 128 + ((piece ^ (row & 7)) << 4); }
 
-__global__ void __launch_bounds__(kAttnThreads, 4)
-attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
-                    const __half* __restrict__ bias_q, const __half* __restrict__ bias_v, __half* __restrict__ out) {
-    __shared__ __align__(128) uint8_t smem[5 * kTileBytes];         // q (later the output), two buffers of k and v
-    const uint32_t s_q = smem_u32(smem), s_kv = s_q + kTileBytes;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int q0 = blockIdx.x * kTile, head = blockIdx.y;
-    const int64_t base = (int64_t)head * kHd * tokens + (int64_t)blockIdx.z * seq;
+// Which elements of two fp16 numbers are infinite or NaN, as a mask of their bits.
+__device__ __forceinline__ uint32_t nonfinite(uint32_t x) {
+    return ((x & 0x7c00u) == 0x7c00u ? 0xffffu : 0u) | ((x & 0x7c000000u) == 0x7c000000u ? 0xffff0000u : 0u);
+}
+
+// Sums over all keys for the 16 queries of a warp: o[block of 8 features][query g: 0, 1; g + 8: 2, 3], and 1 / sum of
+// probabilities.  The whole CTA takes part.
+// SPECIAL: infinities and NaNs of v are multiplied by whether a probability is zero and not by its two terms, of which the
+// low one may be zero or negative (which would make NaN of an infinite result).
+template <bool SPECIAL>
+__device__ __forceinline__ void attend(int seq, int64_t tokens, int64_t base, int q0, const __half* __restrict__ q, const __half* __restrict__ k,
+                                       const __half* __restrict__ v, const __half* __restrict__ bias_q, uint32_t s_q, float (&o)[8][4],
+                                       float (&inv)[2]) {
+    const uint32_t s_kv = s_q + kTileBytes;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
     auto load = [&](uint32_t dst, const __half* src, int s0) {
         for (int x = threadIdx.x; x < kHd * 8; x += kAttnThreads) {
             const int row = x >> 3, piece = x & 7, s = s0 + piece * 8;
@@ -191,7 +198,7 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
 
     constexpr float kScale = 0.125f * 1.44269504088896340736f;      // 1 / sqrt(64), in powers of two
     constexpr float kLift = 10.f;                                   // probabilities are carried times 2^10: their low halves stay normal numbers
-    float o[8][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
@@ -217,7 +224,7 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
                 for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
                     for (int f = 0; f < 4; ++f) {                   // features 2t, 2t + 1 of the fragment's half
-                        const __half* b = bias_q + head * kHd + kk * 16 + (f >> 1) * 8 + 2 * t;
+                        const __half* b = bias_q + kk * 16 + (f >> 1) * 8 + 2 * t;
                         const __half2 s2 = __hadd2(*reinterpret_cast<const __half2*>(&qf[kk][f]), __halves2half2(b[0], b[1]));
                         qf[kk][f] = *reinterpret_cast<const uint32_t*>(&s2);
                     }
@@ -263,7 +270,7 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
         }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {                            // sixteen keys: score blocks 2 kk and 2 kk + 1 are the fragment
-            uint32_t hi[4], lo[4];
+            uint32_t hi[4], lo[4], some[4];
 #pragma unroll
             for (int f = 0; f < 4; ++f) {                           // (queries lo, keys lo), (hi, lo), (lo, hi), (hi, hi)
                 const int n = 2 * kk + (f >> 1), h = f & 1;
@@ -274,11 +281,19 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
                 const __half2 pl = __floats2half2_rn(p0 - back.x, p1 - back.y);
                 hi[f] = *reinterpret_cast<const uint32_t*>(&ph);
                 lo[f] = *reinterpret_cast<const uint32_t*>(&pl);
+                if constexpr (SPECIAL) some[f] = (p0 > 0.f ? 0x3c00u : 0u) | (p1 > 0.f ? 0x3c000000u : 0u);
             }
 #pragma unroll
             for (int n2 = 0; n2 < 4; ++n2) {                        // two blocks of eight output features
                 uint32_t b[4];                                      // (features a, keys lo), (a, hi), (b, lo), (b, hi)
                 ldsm4(b, at(s_v, n2 * 16 + (lane >> 4) * 8 + (lane & 7), kk * 2 + ((lane >> 3) & 1)));
+                if constexpr (SPECIAL) {
+                    uint32_t x[4];
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) { x[f] = b[f] & nonfinite(b[f]); b[f] ^= x[f]; }
+                    mma(o[2 * n2], some, x[0], x[1]);
+                    mma(o[2 * n2 + 1], some, x[2], x[3]);
+                }
                 mma(o[2 * n2], lo, b[0], b[1]);
                 mma(o[2 * n2 + 1], lo, b[2], b[3]);
                 mma(o[2 * n2], hi, b[0], b[1]);
@@ -286,13 +301,31 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
             }
         }
     }
-    float inv[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
         l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
-        inv[h] = l[h] == 0.f ? 0.f : 1.f / l[h];
+        inv[h] = 1.f / l[h];                                       // no score above -inf: 0 * inf, NaN
     }
+}
+
+__global__ void __launch_bounds__(kAttnThreads, 4)
+attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
+                    const __half* __restrict__ bias_q, const __half* __restrict__ bias_v, __half* __restrict__ out) {
+    __shared__ __align__(128) uint8_t smem[5 * kTileBytes];         // q (later the output), two buffers of k and v
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int q0 = blockIdx.x * kTile, head = blockIdx.y;
+    const int64_t base = (int64_t)head * kHd * tokens + (int64_t)blockIdx.z * seq;
+    if (bias_q) bias_q += head * kHd;
+    float o[8][4], inv[2];
+    attend<false>(seq, tokens, base, q0, q, k, v, bias_q, smem_u32(smem), o, inv);
+    bool nan = false;
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) nan |= isnan(o[n][e]);
+    // something infinite or NaN went in (the barrier also frees the buffers)
+    if (__syncthreads_or(nan)) attend<true>(seq, tokens, base, q0, q, k, v, bias_q, smem_u32(smem), o, inv);
     // the warp's 16 columns of the output tile [feature][query] take the place of its queries
     __half* tile = reinterpret_cast<__half*>(smem);
     __syncwarp();

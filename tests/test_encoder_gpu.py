@@ -88,3 +88,32 @@ def test_grouped_layer_follows_replaced_bias_and_odd_shapes(lib):
             layer.linears[0].bias = layer.linears[0].bias + 1.0
             layer.linears[4].bias = layer.linears[4].bias + 0.5
             layer.linears[5].bias = layer.linears[5].bias - 2.0
+
+
+@pytest.mark.parametrize("seq,scale", [(64, 0.0), (64, 1.0), (136, 1.0), (200, 0.5)])
+def test_attention_infinities_and_nans(lib, seq, scale):
+    """An infinite value times any probability is infinite (all of these are above 2^-60), two of opposite sign and a NaN give
+    NaN, other features and sequences keep their numbers; a query whose scores are all -inf has no softmax.  scale 0: every
+    probability is a power of two and its low term zero.  Bound of the numbers: see test_attention_feature_major."""
+    from sspmm_b200 import ops
+    heads, batch = 2, 2
+    g = torch.Generator(device="cuda:0").manual_seed(seq)
+    r = lambda s: (torch.randn((heads * 64, batch * seq), device="cuda:0", generator=g) * s).half()
+    q, k, v = r(scale), r(scale), r(1.0)
+    inf = float("inf")
+    v[3, 5], v[10, seq - 1], v[70, 0], v[90, 1], v[90, seq - 2], v[127, seq + 7] = inf, -inf, inf, inf, -inf, float("nan")
+    q[64, seq + 9], k[64, seq:] = inf, -1.0            # sequence 1, head 1, query 9: every score is -inf
+    if scale == 0:
+        k[64:, seq:] = -1.0                             # equal scores for the other queries as well
+    out = torch.full_like(q, float("nan"))
+    ops.attention_fm(q, k, v, heads, batch, seq, out)
+    split = lambda t: t.double().view(heads, 64, batch, seq).permute(2, 0, 3, 1)
+    score = split(q) @ split(k).transpose(-1, -2) / 8
+    p = torch.softmax(score, -1)
+    ref, got = p @ split(v), split(out)
+    assert torch.equal(ref.isnan(), got.isnan()) and torch.equal(ref.isposinf(), got.isposinf()) and torch.equal(ref.isneginf(), got.isneginf())
+    assert ref.isinf().any() and ref.isnan().any()
+    fin = ref.isfinite()
+    top = score[score.isfinite()].abs().amax()
+    slack = 2.0 ** -20 * (1 + top) * (p @ split(v).abs())
+    assert ((got - ref).abs()[fin] <= (2.0 ** -11 * ref.abs() + 2.0 ** -24 + slack)[fin]).all()
