@@ -242,7 +242,7 @@ int sspmm_add_bias_fm(int rows, int tokens, const void* x_f16, const void* bias_
 
 /*
  * Softmax attention on feature-major activations: q, k, v, out are [heads*64][batch*seq] fp16, token t of sequence b in
- * column b*seq + t; scores scaled by 1/8, softmax in fp32, probabilities kept to 22 bits.
+ * column b*seq + t; scores scaled by 1/8, softmax in fp32, probabilities kept to 22 bits (or to 2^-35 of the largest of a query).
  * bias_q, bias_v (may be NULL): fp16 per feature, added to q and v; one of k has no effect on the result.  Head width 64, seq % 8 == 0,
  * 16-byte aligned arrays; 1 otherwise.
  */

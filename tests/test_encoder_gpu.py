@@ -117,3 +117,20 @@ def test_attention_infinities_and_nans(lib, seq, scale):
     top = score[score.isfinite()].abs().amax()
     slack = 2.0 ** -20 * (1 + top) * (p @ split(v).abs())
     assert ((got - ref).abs()[fin] <= (2.0 ** -11 * ref.abs() + 2.0 ** -24 + slack)[fin]).all()
+
+
+def test_attention_sums_have_no_drift(lib):
+    """Values of one sign: truncated additions would pull every result the same way.  A block of 64 keys adds eight times to
+    a sum that starts at zero, each time losing at most 2^-23 of it; over half a million results the rounding to fp16
+    (2^-11 / sqrt(12) of a result at most) averages out to 2^-11 / sqrt(12 n), four of which are allowed."""
+    from sspmm_b200 import ops
+    heads, batch, seq = 2, 2, 2048
+    g = torch.Generator(device="cuda:0").manual_seed(0)
+    q, k = ((torch.randn(heads * 64, batch * seq, device="cuda:0", generator=g) * 0.5).half() for _ in range(2))
+    v = (torch.rand(heads * 64, batch * seq, device="cuda:0", generator=g) + 1).half()
+    out = torch.empty_like(q)
+    ops.attention_fm(q, k, v, heads, batch, seq, out)
+    split = lambda t: t.double().view(heads, 64, batch, seq).permute(2, 0, 3, 1)
+    ref = torch.softmax(split(q) @ split(k).transpose(-1, -2) / 8, -1) @ split(v)
+    drift = (split(out) / ref - 1).mean().abs().item()
+    assert drift <= 8 * 2.0 ** -23 + 4 * 2.0 ** -11 / (12 * out.numel()) ** 0.5
