@@ -19,6 +19,15 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
+def _launch(fn, like: torch.Tensor, *args) -> None:
+    """fn(*args, stream) on the device of ``like``; switching devices costs more than asking for the current one."""
+    if torch.cuda.current_device() == like.get_device():
+        capi.check(fn(*args, _stream_ptr()))
+    else:
+        with torch.cuda.device(like.device):
+            capi.check(fn(*args, _stream_ptr()))
+
+
 def _require(t: torch.Tensor, dtype, name: str) -> None:
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
@@ -198,9 +207,8 @@ def layer_norm_fm(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, eps:
 
 def launch_layer_norm_fm(x, gamma, beta, eps, out, add, sum_out, bias) -> None:
     """``layer_norm_fm`` for a caller that has compared the operands itself."""
-    with torch.cuda.device(x.device):
-        capi.check(capi.lib().sspmm_layer_norm_fm(x.shape[0], x.shape[1], x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
-                                                  gamma.data_ptr(), beta.data_ptr(), eps, out.data_ptr(), _stream_ptr()))
+    _launch(capi.lib().sspmm_layer_norm_fm, x, x.shape[0], x.shape[1], x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
+            gamma.data_ptr(), beta.data_ptr(), eps, out.data_ptr())
 
 
 def add_bias_fm(x: torch.Tensor, bias: torch.Tensor, add: torch.Tensor) -> torch.Tensor:
@@ -214,9 +222,7 @@ def add_bias_fm(x: torch.Tensor, bias: torch.Tensor, add: torch.Tensor) -> torch
 def launch_add_bias_fm(x, bias, add) -> torch.Tensor:
     """``add_bias_fm`` for a caller that has compared the operands itself."""
     out = torch.empty_like(x)
-    with torch.cuda.device(x.device):
-        capi.check(capi.lib().sspmm_add_bias_fm(x.shape[0], x.shape[1], x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr(),
-                                                _stream_ptr()))
+    _launch(capi.lib().sspmm_add_bias_fm, x, x.shape[0], x.shape[1], x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr())
     return out
 
 
@@ -233,9 +239,8 @@ def attention_fm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, 
 
 def launch_attention_fm(q, k, v, heads, batch, seq, out, bias_q, bias_v) -> None:
     """``attention_fm`` for a caller that has compared the operands itself."""
-    with torch.cuda.device(q.device):
-        capi.check(capi.lib().sspmm_attention_fm(heads, 64, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(),
-                                                 _ptr(bias_q), _ptr(bias_v), out.data_ptr(), _stream_ptr()))
+    _launch(capi.lib().sspmm_attention_fm, q, heads, 64, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(bias_q), _ptr(bias_v),
+            out.data_ptr())
 
 
 class Plan:
