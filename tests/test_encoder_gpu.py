@@ -134,3 +134,72 @@ def test_attention_sums_have_no_drift(lib):
     ref = torch.softmax(split(q) @ split(k).transpose(-1, -2) / 8, -1) @ split(v)
     drift = (split(out) / ref - 1).mean().abs().item()
     assert drift <= 8 * 2.0 ** -23 + 4 * 2.0 ** -11 / (12 * out.numel()) ** 0.5
+
+
+def exact_layer(layer, x, batch, seq):
+    """The layer in 64 bits, from its dense weights."""
+    lin = [(l.dense.double(), 0 if l.bias is None else l.bias.double()[:, None]) for l in layer.linears]
+
+    def norm(t, wb):
+        return (t - t.mean(0)) / torch.sqrt(t.var(0, unbiased=False) + 1e-5) * wb[0].double()[:, None] + wb[1].double()[:, None]
+    x = x.double()
+    n = norm(x, layer.ln1)
+    q, k, v = ((w @ n + b).view(layer.heads, -1, batch, seq).permute(2, 0, 3, 1) for w, b in lin[:3])
+    att = torch.softmax(q @ k.transpose(-1, -2) / q.shape[-1] ** 0.5, -1) @ v
+    out = lin[3][0] @ att.permute(1, 3, 0, 2).reshape(x.shape) + lin[3][1] + x
+    return lin[5][0] @ (lin[4][0] @ norm(out, layer.ln2) + lin[4][1]) + lin[5][1] + out
+
+
+@pytest.mark.parametrize("hidden,heads,batch,seq", [(256, 4, 3, 72), (128, 2, 1, 200), (128, 4, 2, 64), (256, 4, 2, 20)])
+def test_layer_against_64_bits(lib, hidden, heads, batch, seq):
+    """Heads, sequences, residuals and biases end up where they belong (head width 32 and sequences that are not a multiple of
+    eight take the framework's attention).  An activation is rounded to fp16 at most a dozen times on the way, each time by at
+    most 2^-11 of its norm, and the layer's parts pass a relative error on without raising it."""
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=hidden, ffn=4 * hidden, heads=heads, sparsity=0.9, vec_length=16)
+    g = torch.Generator(device="cuda:0").manual_seed(hidden + seq)
+    r = lambda *s: torch.randn(s, device="cuda:0", generator=g)
+    layer.ln1, layer.ln2 = ((r(hidden) * 0.3 + 1).half(), r(hidden).half()), ((r(hidden) * 0.3 - 1).half(), r(hidden).half())
+    for l in layer.linears:
+        l.bias = r(l.out_features).half()
+    x = (r(hidden, batch * seq) * 2 + 0.5).half()
+    ref = exact_layer(layer, x, batch, seq)
+    for got in (layer.forward(x, batch, seq), layer.forward_grouped(x, batch, seq), layer.forward(x, batch, seq, dense=True)):
+        assert got.shape == x.shape and (got.double() - ref).norm() <= 12 * 2.0 ** -11 * ref.norm()
+
+
+def test_layer_under_autograd_takes_framework_operations(lib):
+    """With a bias that wants a gradient the sums, LayerNorm and attention are recorded, and the numbers are the same."""
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=128, ffn=512, heads=2, sparsity=0.9, vec_length=16)
+    x = torch.randn(128, 144, device="cuda:0", dtype=torch.float16)
+    plain = layer.forward(x, 2, 72)
+    layer.linears[5].bias.requires_grad_()
+    y = layer.forward(x, 2, 72)
+    assert (y - plain).norm() <= 12 * 2.0 ** -11 * plain.norm()
+    y.sum().backward()
+    assert torch.equal(layer.linears[5].bias.grad, torch.full((128,), 144.0, device="cuda:0").half())
+
+
+def test_grouped_layer_refuses_other_token_counts(lib):
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=128, ffn=512, heads=2, sparsity=0.9, vec_length=16)
+    x = torch.randn(128, 144, device="cuda:0", dtype=torch.float16)
+    y = layer.forward_grouped(x, 2, 72).clone()
+    before = {n: t.clone() for n, t in layer.buf.items()}
+    for other in (x[:, :136].contiguous(), torch.cat([x, x], 1)):
+        with pytest.raises(RuntimeError):
+            layer.forward_grouped(other, 2, 72)
+    assert all(torch.equal(before[n].view(torch.int16), t.view(torch.int16)) for n, t in layer.buf.items())
+    assert torch.equal(y, layer.forward_grouped(x, 2, 72))
+
+
+def test_layer_norm_wide_tile_with_most_features(lib):
+    """32 tokens per CTA and 3072 features: all of the shared memory it may ask for; bound as in test_layer_norm_feature_major."""
+    from sspmm_b200 import ops
+    x = torch.randn(3072, 32 * 148 + 8, device="cuda:0").half()
+    w, b, out = torch.randn(3072, device="cuda:0").half(), torch.randn(3072, device="cuda:0").half(), torch.empty_like(x)
+    ops.layer_norm_fm(x, w, b, 1e-5, out)
+    d = x.double()
+    ref = (d - d.mean(0)) / torch.sqrt(d.var(0, unbiased=False) + 1e-5) * w.double()[:, None] + b.double()[:, None]
+    assert ((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -19 * (1 + w.double().abs()[:, None] * 4)).all()
