@@ -498,8 +498,6 @@ list_parts_kernel(const __grid_constant__ Problem p) {
     const bool alone = gridDim.x == 1;
     if (threadIdx.x < 2) count[threadIdx.x] = 0;
     __syncthreads();
-    int* const several = alone ? &count[0] : p.header;
-    int* const whole = alone ? &count[1] : p.header + 2;
     const int stride = gridDim.x * 1024;
     for (int x = blockIdx.x * 1024 + threadIdx.x; x < p.cap_cut * p.n_tiles; x += stride) p.arrivals[x] = 0;
     for (int64_t b = blockIdx.x * 1024 + threadIdx.x; b < p.m_vec; b += 4LL * stride) {
@@ -515,12 +513,12 @@ list_parts_kernel(const __grid_constant__ Problem p) {
             if (len[k] <= kLightRow) continue;
             const int row = (int)(b + (int64_t)k * stride);
             if (len[k] <= p.chunk) {
-                const int at = atomicAdd(whole, 1);
+                const int at = alone ? atomicAdd(&count[1], 1) : atomicAdd(p.header + 2, 1);
                 if (at < p.cap_whole) p.entries[p.cap_cut + at] = make_int4(row, j0[k], len[k], 1 << 16);
                 continue;
             }
             const int n = (int)(((unsigned)len[k] + p.chunk - 1) / p.chunk);
-            const int first = atomicAdd(several, n);
+            const int first = alone ? atomicAdd(&count[0], n) : atomicAdd(p.header, n);
             for (int c = 0; c < n && first + c < p.cap_cut; ++c)
                 p.entries[first + c] = make_int4(row, j0[k] + c * p.chunk, min(p.chunk, len[k] - c * p.chunk), n << 16 | c);
         }
