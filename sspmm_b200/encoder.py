@@ -94,11 +94,11 @@ class SparseEncoderLayer:
 
     def _norm(self, x, wb, add=None, bias=None, out=None, sum_out=None):
         """LayerNorm of x + bias + add: (what was normalised, the result)."""
-        given = [t for t in (x, add, bias, *wb) if t is not None]
-        room = [t for t in (out, sum_out) if t is not None]
-        if _plain(*given, *room) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and \
-                (add is None or add.shape == x.shape) and all(t.shape == x.shape for t in room) and (bias is None or add is not None) and \
-                all(t.shape == (x.shape[0],) for t in given if t is not x and t is not add):
+        whole = [t for t in (x, add, out, sum_out) if t is not None]
+        rows = [t for t in (bias, *wb) if t is not None]
+        shape = x.shape
+        if _plain(*whole, *rows) and len(shape) == 2 and shape[1] % 8 == 0 and 0 < shape[0] <= 3072 and \
+                (bias is None or add is not None) and all(t.shape == shape for t in whole) and all(t.shape == shape[:1] for t in rows):
             out = torch.empty_like(x) if out is None else out
             if add is not None and sum_out is None:
                 sum_out = torch.empty_like(x)
@@ -159,7 +159,7 @@ class SparseEncoderLayer:
             b["h"] += L[4].bias[:, None]
         g[3].run()
         bias = L[5].bias_rows()
-        if bias is not None and _plain(b["y"], bias, out) and out.shape == b["y"].shape and out.shape[1] % 8 == 0:
+        if bias is not None and out is b["sum"] and bias.get_device() == out.get_device():       # as LayerNorm's kernel left it
             return ops.launch_add_bias_fm(b["y"], bias, out)
         return (b["y"] if L[5].bias is None else b["y"] + L[5].bias[:, None]) + out
 
