@@ -8,7 +8,7 @@ C = A_vs * B with B = K x 25088 fp16 N(0,1), B and C sharded along N over the
 ranks (strong scaling, no collective on the data path).  One step = all 32
 products once.  The weights are compressed by the GPU SVC before timing.
 
-One JSON line on stdout (rank 0).  `value` = useful TFLOP/s = 2*nnz*N_total summed
+One JSON line on stdout (rank 0; the per-product and per-case lists follow on stderr).  `value` = useful TFLOP/s = 2*nnz*N_total summed
 over the 32 products / device time of a step, operands resident in HBM; `e2e` =
 the same with B coming from pinned host memory and C going back every step.
 `--impl reference` times the reference's CPU path (restated in oracle/) on the
@@ -598,9 +598,23 @@ def run_ours(args):
                 "gpu_launches": args.steps * launches_per_step, "clocks": clocks, "device_status": status,
                 "wall_s_timed_region": wall}
         line.update(extras)
+        line, detail = split_line(line)
+        sys.stderr.write(json.dumps({"detail": detail}) + "\n")
         print(json.dumps(line))
     if world > 1:
         dist.destroy_process_group()
+
+
+def split_line(line):
+    """(the result line, the per-case lists): a line of all of it is 21 KB, more than what reads it may keep of the output, so
+    the lists go to stderr."""
+    short = {k: v for k, v in line.items() if k not in ("per_product", "per_product_note", "svc", "ffn")}
+    detail = {k: v for k, v in line.items() if k not in short}
+    comp = short.get("comparators") or {}
+    if "per_product" in comp.get("reference_gpu_kernel", {}):
+        detail["reference_gpu_kernel_per_product"] = comp["reference_gpu_kernel"]["per_product"]
+        short["comparators"] = {**comp, "reference_gpu_kernel": {k: v for k, v in comp["reference_gpu_kernel"].items() if k != "per_product"}}
+    return short, detail
 
 
 class L2Flush:
