@@ -34,7 +34,7 @@ constexpr int kThreads = kWarps * 32;
 constexpr int kStep = 16;                 // vectors per step
 constexpr int kLightRow = 256;            // split launches: longest row that one warp does
 constexpr int kMaxCluster = 8;
-constexpr int kResident = 2;              // CTAs per SM: 16 warps with three or four steps in flight each
+constexpr int kResident = 2;              // CTAs per SM: 16 warps with two or three steps in flight each
 
 struct Problem {
     int m_vec, K, n_tiles;
@@ -113,7 +113,7 @@ template <int V, int H, bool ROUND>
 struct Tile {
     static constexpr int NT = 64 * H;
     static constexpr int VB = V / 8;
-    static constexpr int kStages = H == 2 ? 3 : 4;                  // steps in flight per warp
+    static constexpr int kStages = H == 2 ? 3 : 4;                  // steps in the ring: one in work, the others in flight
     static constexpr int kRowBytes = NT * 2;
     static constexpr int kStageBytes = kStep * kRowBytes + kStep * V * 2;
     static constexpr int kPitch = NT + 4;                           // floats per row of the tile of sums (conflict-free)

@@ -1,6 +1,7 @@
 """Transformer encoder layer whose six weight matrices (Q, K, V, O, FFN1, FFN2) are magnitude-pruned,
-compressed by the GPU SVC and applied with the vector-sparse SpMM; attention itself and LayerNorm
-stay dense PyTorch ops.
+compressed by the GPU SVC and applied with the vector-sparse SpMM.  LayerNorm, attention and the last residual sum
+are kernels of this package for contiguous fp16 activations with heads 64 wide and whole multiples of eight
+tokens, and PyTorch operations otherwise, as in the dense evaluation.
 
 Block structure follows the reference's end-to-end script (end2end/sspmm_e2e/end_to_end.py:44-75:
 LayerNorm -> attention -> residual -> LayerNorm -> linear1 -> linear2 -> residual, no activation

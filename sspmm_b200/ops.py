@@ -8,6 +8,7 @@ import torch
 
 from . import capi
 
+# KERNEL_GATHER: TMA row gather; KERNEL_GATHER_LSU: the row-gather kernel whose warps gather by themselves
 KERNEL_AUTO, KERNEL_GATHER, KERNEL_SIMT, KERNEL_BLOCK, KERNEL_GATHER_LSU, KERNEL_BLOCK_SINGLE = 0, 1, 2, 3, 4, 5
 
 
