@@ -27,17 +27,26 @@
 //                      fixed length is "first come, first served" along each key's
 //                      probe path, which has a unique fixed point: slot = the first
 //                      one on my path not held by an earlier element.  The team finds
-//                      it in parallel with atomicMin on the element's sequence number (an
-//                      element pushed out of a slot by an earlier one starts its path again);
-//                      table growth steps are replayed level by level (8, 32, 128, ...).
+//                      it in parallel with atomicMin on words that hold the element's
+//                      sequence number and its column; table growth steps are replayed
+//                      level by level (8, 32, 128, ...).  What bounds it is the longest
+//                      chain of elements that push one another on, one after another
+//                      (rows are ascending and so come to sit in runs), so the tables
+//                      of a rebuild are kept and the next one starts from them.
+//                      Stack of 16 power-law matrices (n 4096 to 65536, V = 8), whole
+//                      call: 3450 us with every rebuild from free tables and sequences
+//                      apart from the tables, 1310 now; per launch, classes L, M2, M1, S, XS
+//                      776, 576, 392, 276, 284 us one after another.
 // The replay kernels take their groups from per-class lists (written by the scan kernel)
 // through a work counter, so a CTA never walks over groups of other classes and the
 // groups of a class, whose cost differs by an order of magnitude, balance themselves.
 #include "svc.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 #include "launch.h"
+#include "ptx.cuh"
 
 namespace sspmm_b200 {
 
@@ -48,7 +57,6 @@ namespace {
 constexpr int kMinTable = 8;
 constexpr int kLinearProbes = 9;
 constexpr int kPerturbShift = 5;
-constexpr int kEmptyPrio = 0x7fffffff;
 
 // Replay classes by number of distinct columns u (and final table length):
 constexpr int kClassSorted = 0;   // no replay
@@ -67,8 +75,6 @@ constexpr int kM1CapU = 1228, kM1CapT = 2048;
 constexpr int kM2CapU = 4914, kM2CapT = 8192;
 constexpr int kLCapT = 32768;
 constexpr int kLCapU = 19660;   // most keys a table of kLCapT slots holds
-constexpr int kLSeqInts = 19664;    // a table of kLCapT slots holds fewer than 19661 keys; class L keeps the level's sequence in shared memory
-constexpr int kListsPerGroup = 4;   // X2, NEW, P, Q (the fifth list is the output slice)
 
 __host__ __device__ inline void next_level(int size, long long& trig, int& next_size) {
     const long long mask = size - 1;
@@ -140,11 +146,11 @@ __host__ inline void class_segments(int c, int& s0, int& s1) {
     }
 }
 
-// Global scratch ints of one replayed group.
+// Global scratch ints of one replayed group: a list of class L, class XL's table and two lists.
 __host__ __device__ inline long long group_scratch_ints(int u, int tbl_len) {
     const int c = replay_class(u, tbl_len);
-    if (c == kClassL) return (long long)kListsPerGroup * u;
-    if (c == kClassXL) return (long long)kListsPerGroup * u + tbl_len;
+    if (c == kClassL) return ((long long)u + 3) & ~3ll;
+    if (c == kClassXL) return ((2ll * u + 3) & ~3ll) + tbl_len;
     return 0;
 }
 
@@ -178,12 +184,6 @@ struct WarpTeam {
     __device__ static int sum(int v, int*) { return warp_sum(v); }
     __device__ static int max_of(int v, int*) { return warp_max(v); }
     __device__ static int broadcast(int v, int*) { return __shfl_sync(0xffffffffu, v, 0); }   // value of thread 0
-    // rank of this thread among the flagged threads of the team, in thread order
-    __device__ static int rank(bool flag, int& total, int*) {
-        const unsigned b = __ballot_sync(0xffffffffu, flag);
-        total = __popc(b);
-        return __popc(b & ((1u << (threadIdx.x & 31)) - 1u));
-    }
 };
 
 template <int THREADS>
@@ -219,36 +219,15 @@ struct BlockTeam {
         __syncthreads();
         return r;
     }
-    // exclusive prefix sum of v over the threads of the block, in thread order
-    __device__ static int scan_exclusive(int v, int& total, int* scratch) {
+    // sum of the warps' numbers (the same in every lane) before this warp, and of all; scratch: 32 ints, free until the next barrier
+    __device__ static int before(int count, int& total, int* scratch) {
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int inc = warp_incl_scan(v, lane);
-        if (lane == 31) scratch[warp] = inc;
+        if (lane == 0) scratch[warp] = count;
         __syncthreads();
-        int before = 0, all = 0;
-        for (int w = 0; w < THREADS / 32; ++w) {
-            const int c = scratch[w];
-            if (w < warp) before += c;
-            all += c;
-        }
-        __syncthreads();
-        total = all;
-        return before + inc - v;
-    }
-    __device__ static int rank(bool flag, int& total, int* scratch) {
-        const unsigned b = __ballot_sync(0xffffffffu, flag);
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        if (lane == 0) scratch[warp] = __popc(b);
-        __syncthreads();
-        int before = 0, all = 0;
-        for (int w = 0; w < THREADS / 32; ++w) {
-            const int c = scratch[w];
-            if (w < warp) before += c;
-            all += c;
-        }
-        __syncthreads();
-        total = all;
-        return before + __popc(b & ((1u << lane) - 1u));
+        const int v = lane < THREADS / 32 ? scratch[lane] : 0;
+        const int incl = warp_incl_scan(v, lane);
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        return __shfl_sync(0xffffffffu, incl - v, warp);
     }
 };
 
@@ -597,350 +576,507 @@ struct Probe {            // position on a key's probe path
     unsigned w;           // offset inside the window
     unsigned perturb;
 };
-__device__ __forceinline__ Probe probe_begin(int key, unsigned mask) {
+__device__ __forceinline__ Probe probe_begin(unsigned key, unsigned mask) {
     Probe p;
-    p.i = (unsigned)key & mask; p.w = 0; p.perturb = (unsigned)key;
+    p.i = key & mask; p.w = 0; p.perturb = key;
     return p;
 }
-// Returns true when the step was a jump to a new window.
-__device__ __forceinline__ bool probe_advance(Probe& p, unsigned mask) {
+__device__ __forceinline__ void probe_advance(Probe& p, unsigned mask) {
     const unsigned window = (p.i + kLinearProbes <= mask) ? kLinearProbes : 0;
     if (p.w < window) {
         ++p.w;
-        return false;
+        return;
     }
     p.perturb >>= kPerturbShift;
     p.i = (p.i * 5u + 1u + p.perturb) & mask;
     p.w = 0;
-    return true;
 }
-// Table of KEYS (-1 = free): slot holding `key`, or -1 when the path reaches a free slot first.
-// Every probe loop is bounded (a table is never more than 60 % full, so a free slot is near).
-__device__ __forceinline__ int find_key(const int* tab, unsigned mask, int key) {
+// Growth of a set's table (next_level in closed form for the lengths that occur, at most 2^19).
+__device__ __forceinline__ int level_trigger(int size) { return (3 * (size - 1) + 4) / 5; }       // the fill that makes it grow
+__device__ __forceinline__ int level_next(int size) { return size > 65536 ? size * 2 : size * 4; }
+
+// Position of a slot on a key's probe path.
+__device__ __forceinline__ Probe probe_at(unsigned key, unsigned mask, unsigned slot) {
     Probe p = probe_begin(key, mask);
-    for (unsigned n = 0; n <= 8u * mask + 64u; ++n) {
-        const int e = tab[p.i + p.w];
-        if (e == key) return (int)(p.i + p.w);
-        if (e == -1) return -1;
-        probe_advance(p, mask);
-    }
-    return -1;
-}
-// Same, returning the first free slot when the key is absent (sequential insertion).
-__device__ __forceinline__ int find_slot(const int* tab, unsigned mask, int key) {
-    Probe p = probe_begin(key, mask);
-    for (unsigned n = 0; n <= 8u * mask + 64u; ++n) {
-        const int e = tab[p.i + p.w];
-        if (e == key || e == -1) return (int)(p.i + p.w);
-        probe_advance(p, mask);
-    }
-    return (int)(p.i + p.w);
+    for (unsigned n = 0; p.i + p.w != slot && n <= 8u * mask + 64u; ++n) probe_advance(p, mask);
+    return p;
 }
 
-struct ReplayBuffers {
-    int* table;      // cap ints
-    int* lists[4];   // lists of u ints: X2 (alternates with the output slice as the ordered list), NEW, P, Q
-    int* seq_local;  // non-null: u ints of shared memory that hold the insertion sequence of the current level
-                     // (the lists are then in global memory and are only streamed through)
+constexpr unsigned kFree = 0xffffffffu;          // word of a free slot
+
+struct SharedWords {
+    uint32_t at;
+    __device__ __forceinline__ SharedWords part(unsigned i) const { return SharedWords{at + 4u * i}; }
+    __device__ __forceinline__ unsigned ld(unsigned i) const {
+        unsigned v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at + 4u * i) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void st(unsigned i, unsigned v) const { asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + 4u * i), "r"(v) : "memory"); }
+    __device__ __forceinline__ void free4(unsigned i) const {
+        asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at + 4u * i), "r"(kFree) : "memory");
+    }
+    __device__ __forceinline__ unsigned take(unsigned i, unsigned v) const {       // atomic minimum, the word before
+        unsigned old;
+        asm volatile("atom.shared.min.u32 %0, [%1], %2;" : "=r"(old) : "r"(at + 4u * i), "r"(v) : "memory");
+        return old;
+    }
+    __device__ __forceinline__ bool give_up(unsigned i, unsigned v) const {        // frees the slot if it still holds v
+        unsigned old;
+        asm volatile("atom.shared.cas.b32 %0, [%1], %2, %3;" : "=r"(old) : "r"(at + 4u * i), "r"(v), "r"(kFree) : "memory");
+        return old == v;
+    }
+};
+struct GlobalWords {
+    unsigned* at;
+    __device__ __forceinline__ GlobalWords part(unsigned i) const { return GlobalWords{at + i}; }
+    __device__ __forceinline__ unsigned ld(unsigned i) const { return __ldcg(at + i); }
+    __device__ __forceinline__ void st(unsigned i, unsigned v) const { __stcg(at + i, v); }
+    __device__ __forceinline__ void free4(unsigned i) const { __stcg(reinterpret_cast<uint4*>(at + i), make_uint4(kFree, kFree, kFree, kFree)); }
+    __device__ __forceinline__ unsigned take(unsigned i, unsigned v) const { return atomicMin(at + i, v); }
+    __device__ __forceinline__ bool give_up(unsigned i, unsigned v) const { return atomicCAS(at + i, v, kFree) == v; }
 };
 
-// Ordered extraction: keys of `tab` in slot order into dst; returns how many.  With seq != null the
-// table holds sequence numbers (kEmptyPrio = free) and is rewritten in place to hold keys (-1 = free).
-template <class Team>
-__device__ int extract_ordered(int* tab, int size, const int* seq, int* dst, int* red) {
-    const int tid = Team::tid();
-    if constexpr (Team::kSize >= 256) {
-        // Large table, CTA team: every warp owns a contiguous run of size / warps slots and walks it 32
-        // slots at a time (one ballot gives the occupancy of a row), so the whole table needs one prefix sum
-        // over warp totals instead of a block-wide one per kSize slots, and the key lookups of four rows
-        // are in flight together.
-        if (size >= Team::kSize) {
-            const int lane = tid & 31, warp = tid >> 5;
-            const int rows = size / Team::kSize;                    // rows of 32 slots per warp
-            const int first = warp * rows * 32 + lane;
-            int cnt = 0;
-            for (int j = 0; j < rows; ++j) {
-                const int e = tab[first + j * 32];
-                cnt += __popc(__ballot_sync(0xffffffffu, seq ? (e != kEmptyPrio) : (e != -1)));
-            }
-            if (lane == 0) red[warp] = cnt;
-            Team::sync();
-            int pos = 0, total = 0;
-            for (int w = 0; w < Team::kSize / 32; ++w) {
-                const int c = red[w];
-                if (w < warp) pos += c;
-                total += c;
-            }
-            Team::sync();
-            for (int j0 = 0; j0 < rows; j0 += 4) {
-                int e4[4], k4[4];
-                bool f4[4];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    e4[b] = (j0 + b < rows) ? tab[first + (j0 + b) * 32] : (seq ? kEmptyPrio : -1);
-                    f4[b] = seq ? (e4[b] != kEmptyPrio) : (e4[b] != -1);
-                }
-#pragma unroll
-                for (int b = 0; b < 4; ++b) k4[b] = f4[b] ? (seq ? seq[e4[b]] : e4[b]) : -1;
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    if (j0 + b < rows) {
-                        const unsigned m = __ballot_sync(0xffffffffu, f4[b]);
-                        if (f4[b]) dst[pos + __popc(m & ((1u << lane) - 1u))] = k4[b];
-                        if (seq) tab[first + (j0 + b) * 32] = k4[b];
-                        pos += __popc(m);
-                    }
-                }
-            }
-            Team::sync();
-            return total;
-        }
-    }
-    int n = 0;
-    for (int s0 = 0; s0 < size; s0 += Team::kSize) {
-        const int s = s0 + tid;
-        int key = -1;
-        if (s < size) {
-            const int e = tab[s];
-            if (seq) {
-                key = (e == kEmptyPrio) ? -1 : seq[e];
-                tab[s] = key;
-            } else {
-                key = e;
-            }
-        }
-        int total;
-        const int rk = Team::rank(key != -1, total, red);
-        if (key != -1) dst[n + rk] = key;
-        n += total;
-    }
-    Team::sync();
-    return n;
-}
+constexpr int kWarpLevels = 128;      // tables up to this length are done by one warp also in a CTA team
 
-// Sequential replay by one thread (used when a matrix row lists a column twice; rare).  tab holds keys.
-__device__ int replay_sequential(const SvcProblem& p, int r0, int r1, int* tab, int cap, int* xa, int* xb, int* tmp) {
+// A set being rebuilt.  `list` is the insertion sequence: what the set held, in its order, then the row's new columns; a level's
+// extraction writes the order of its table over the part that the level inserted.  A slot's word is the number of its
+// element in the list and, packed (SHIFT bits), its column; unpacked the column is looked up in the list.  After the last level
+// of the last rebuild the number is the position in the ordered set, so a word also answers where a column went.
+// Packed, every level above kWarpLevels has a table of its own, which stays for the next rebuild: between two rebuilds its words
+// have the number kVacant (later than every element's), which a new element takes like a free slot.
+enum class After { kFreed, kVacated, kNumbered };     // what becomes of a level's words when its order has been read
+template <class Words, class List, int SHIFT>
+struct HashSet {
+    Words tab;
+    List list;
+    GlobalWords ext;          // unpacked only: extraction goes here first, since words refer to the list
+    static constexpr bool kPacked = SHIFT > 0;
+    static constexpr unsigned kVacant = kPacked ? ((1u << (32 - SHIFT)) - 2u) << SHIFT : kFree;      // words from here on name no element
+    // where the table of a level starts (lengths above kWarpLevels grow by four as long as words are packed)
+    __device__ __forceinline__ static unsigned start(int size) { return kPacked && size > kWarpLevels ? (unsigned)(size - kWarpLevels) / 3u : 0u; }
+    __device__ __forceinline__ HashSet level(int size) const { return HashSet{tab.part(start(size)), list, ext}; }
+    __device__ __forceinline__ unsigned word(unsigned number, unsigned key) const { return kPacked ? number << SHIFT | key : number; }
+    __device__ __forceinline__ unsigned key_of(unsigned w) const { return kPacked ? w & ((1u << SHIFT) - 1u) : list.ld(w); }
+    __device__ __forceinline__ static unsigned number_of(unsigned w) { return w >> SHIFT; }
+    // slot of a column, or of the free slot at which its path ends (the loop is bounded; a table is never more than 60 % full)
+    __device__ __forceinline__ unsigned find(unsigned mask, unsigned key, unsigned& word) const {
+        Probe p = probe_begin(key, mask);
+        word = kFree;
+        for (unsigned n = 0; n <= 8u * mask + 64u; ++n) {
+            word = tab.ld(p.i + p.w);
+            if (word == kFree || key_of(word) == key) break;
+            probe_advance(p, mask);
+        }
+        return p.i + p.w;
+    }
+    __device__ __forceinline__ bool contains(unsigned mask, unsigned key) const {
+        unsigned w;
+        find(mask, key, w);
+        return w != kFree;
+    }
+    // Insertion is first come, first served: an element takes a slot by an atomic minimum; whoever loses one (the element
+    // itself, or a later one that had come to sit there) goes on along its path from there.  In a table that was free before, slots
+    // only ever get earlier owners, so what was lost stays lost and the result does not depend on timing.
+    // walk: from path position p on, until a slot was free.  True: a column occurs twice (or a bound was hit).
+    __device__ __forceinline__ bool walk(unsigned me, unsigned mine, Probe p, unsigned mask) const {
+        for (unsigned steps = 0; steps <= 64u * mask + 4096u; ++steps) {
+            const unsigned slot = p.i + p.w;
+            const unsigned cur = tab.take(slot, me);
+            if (cur >= kVacant) return false;
+            const unsigned other = key_of(cur);
+            if (other == mine) return true;
+            if (cur > me) {
+                me = cur;
+                mine = other;
+                p = probe_at(mine, mask, slot);
+            }
+            probe_advance(p, mask);
+        }
+        return true;
+    }
+    // Elements first, first + stride, ... below n into a free table.  All are first tried at their home slots, four at a time and
+    // without a branch; only losers walk.
+    __device__ __forceinline__ bool insert(int n, unsigned mask, int first, int stride) const {
+        constexpr int kTry = 4;
+        for (int q0 = first; q0 < n; q0 += kTry * stride) {
+            unsigned key[kTry], old[kTry];
+#pragma unroll
+            for (int b = 0; b < kTry; ++b) key[b] = q0 + b * stride < n ? list.ld(q0 + b * stride) : 0u;
+#pragma unroll
+            for (int b = 0; b < kTry; ++b)
+                old[b] = q0 + b * stride < n ? tab.take(key[b] & mask, word(q0 + b * stride, key[b])) : kFree;
+            bool again = false;
+            unsigned lost[kTry];
+            int losers = 0;
+#pragma unroll
+            for (int b = 0; b < kTry; ++b)
+                if (old[b] < kVacant) {
+                    again |= key_of(old[b]) == key[b];
+#pragma unroll
+                    for (int x = kTry - 1; x > 0; --x) lost[x] = lost[x - 1];
+                    lost[0] = max(old[b], word(q0 + b * stride, key[b]));
+                    ++losers;
+                }
+            bool walking = false;
+            unsigned me = 0, mine = 0, steps = 0;
+            Probe p = probe_begin(0, mask);
+            while (!again && (walking || losers > 0)) {
+                if (!walking) {                                   // the next loser; its home slot is out of reach
+                    me = lost[0];
+                    mine = key_of(me);
+#pragma unroll
+                    for (int x = 0; x + 1 < kTry; ++x) lost[x] = lost[x + 1];
+                    --losers;
+                    p = probe_begin(mine, mask);
+                    probe_advance(p, mask);
+                    walking = true;
+                }
+                const unsigned slot = p.i + p.w;
+                const unsigned cur = tab.take(slot, me);
+                if (cur >= kVacant) {
+                    walking = false;
+                } else {
+                    const unsigned other = key_of(cur);
+                    again = other == mine;
+                    if (cur > me) {
+                        me = cur;
+                        mine = other;
+                        p = probe_at(mine, mask, slot);
+                    }
+                    probe_advance(p, mask);
+                    again |= ++steps > 64u * mask + 4096u;
+                }
+            }
+            if (again) return true;
+        }
+        return false;
+    }
+    // Whether every slot on the path of the element in `slot` before that one has an earlier element.
+    __device__ __forceinline__ bool in_place(unsigned w, unsigned slot, unsigned mask) const {
+        Probe p = probe_begin(key_of(w), mask);
+        for (unsigned n = 0; p.i + p.w != slot && n <= 8u * mask + 64u; ++n) {
+            if (tab.ld(p.i + p.w) > w) return false;
+            probe_advance(p, mask);
+        }
+        return true;
+    }
+    // One warp: the table's columns in slot order to the list.
+    template <After AFTER>
+    __device__ __forceinline__ void extract_warp(int size) const {
+        const int lane = threadIdx.x & 31;
+        int n = 0;
+        for (int s0 = 0; s0 < size; s0 += 128) {
+            unsigned w[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) w[b] = s0 + b * 32 + lane < size ? tab.ld(s0 + b * 32 + lane) : kFree;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                if (s0 + b * 32 >= size) break;
+                const unsigned m = __ballot_sync(0xffffffffu, w[b] != kFree);
+                if (w[b] != kFree) {
+                    const int pos = n + __popc(m & ((1u << lane) - 1u));
+                    const unsigned key = key_of(w[b]);
+                    if (kPacked) list.st(pos, key); else ext.st(pos, key);
+                    tab.st(s0 + b * 32 + lane, AFTER == After::kNumbered ? word(pos, key) : kFree);
+                }
+                n += __popc(m);
+            }
+        }
+        __syncwarp();
+        if (!kPacked) {
+            for (int q = lane; q < n; q += 32) list.st(q, ext.ld(q));
+            __syncwarp();
+        }
+    }
+    // One warp: levels from length 8 up to `last`, each in the same free table; the level of length `final` is kept.
+    __device__ __forceinline__ bool levels_warp(int n_total, int last, int final) const {
+        for (int size = kMinTable; size <= last; size = level_next(size)) {
+            const bool again = insert(min(level_trigger(size), n_total), (unsigned)size - 1u, threadIdx.x & 31, 32);
+            if (__any_sync(0xffffffffu, again)) return true;
+            __syncwarp();
+            if (size == final) extract_warp<After::kNumbered>(size); else extract_warp<After::kFreed>(size);
+        }
+        return false;
+    }
+};
+
+// Sequential replay by one thread (a matrix row lists a column twice; rare).  The table holds columns until the end; the list is
+// overwritten in place: when a growing table is emptied into its head, that part of the sequence has been inserted.
+template <class Set>
+__device__ int replay_sequential(const SvcProblem& p, const int* rows, int n_rows, const Set& t, int cap, unsigned& mask_out) {
     int n_cur = 0;
-    int* x = xa;
-    int* xn = xb;
     unsigned mask = kMinTable - 1;
-    for (int r = r0; r < r1; ++r) {
-        const int rs = p.row_ptr[r], rlen = p.row_ptr[r + 1] - rs;
+    auto slot_of = [&](unsigned m, unsigned key) {
+        Probe pr = probe_begin(key, m);
+        for (unsigned n = 0; n <= 8u * m + 64u; ++n) {
+            const unsigned e = t.tab.ld(pr.i + pr.w);
+            if (e == key || e == kFree) break;
+            probe_advance(pr, m);
+        }
+        return pr.i + pr.w;
+    };
+    for (int r = 0; r < n_rows; ++r) {
+        const int rs = rows[r], rlen = rows[r + 1] - rs;
         int size = kMinTable, used = 0;
         mask = kMinTable - 1;
-        for (int s = 0; s < size; ++s) tab[s] = -1;
-        for (int t = 0; t < n_cur + rlen; ++t) {
-            const int key = (t < n_cur) ? x[t] : p.col_idx[rs + t - n_cur];
-            if ((unsigned)key >= (unsigned)p.K) continue;
-            const int s = find_slot(tab, mask, key);
-            if (tab[s] == key) continue;
-            tab[s] = key;
-            ++used;
-            if ((long long)used * 5 >= (long long)mask * 3) {
-                long long trig; int nsize;
-                next_level(size, trig, nsize);
-                if (nsize > cap) nsize = cap;
+        for (int s = 0; s < size; ++s) t.tab.st(s, kFree);
+        for (int x = 0; x < n_cur + rlen; ++x) {
+            const unsigned key = x < n_cur ? t.list.ld(x) : (unsigned)p.col_idx[rs + x - n_cur];
+            if (key >= (unsigned)p.K) continue;
+            const unsigned s = slot_of(mask, key);
+            if (t.tab.ld(s) == key) continue;
+            t.tab.st(s, key);
+            if (++used >= level_trigger(size)) {
+                const int next = min(level_next(size), cap);
                 int cnt = 0;
-                for (int q = 0; q < size; ++q) if (tab[q] != -1) tmp[cnt++] = tab[q];
-                for (int q = 0; q < nsize; ++q) tab[q] = -1;
-                const unsigned nmask = (unsigned)nsize - 1u;
-                for (int q = 0; q < cnt; ++q) tab[find_slot(tab, nmask, tmp[q])] = tmp[q];
-                size = nsize; mask = nmask;
+                for (int q = 0; q < size; ++q) if (t.tab.ld(q) != kFree) t.list.st(cnt++, t.tab.ld(q));
+                for (int q = 0; q < next; ++q) t.tab.st(q, kFree);
+                mask = (unsigned)next - 1u;
+                for (int q = 0; q < cnt; ++q) { const unsigned k = t.list.ld(q); t.tab.st(slot_of(mask, k), k); }
+                size = next;
             }
         }
-        int cnt = 0;
-        for (int q = 0; q < size; ++q) if (tab[q] != -1) xn[cnt++] = tab[q];
-        n_cur = cnt;
-        int* t2 = x; x = xn; xn = t2;
+        n_cur = 0;
+        for (int q = 0; q < size; ++q) if (t.tab.ld(q) != kFree) t.list.st(n_cur++, t.tab.ld(q));
     }
-    return (int)mask;      // the ordered list is in `x` = xa if (r1-r0) is even else xb; caller arranges parity
+    int n = 0;
+    for (unsigned s = 0; s <= mask; ++s)
+        if (t.tab.ld(s) != kFree) { const unsigned key = t.tab.ld(s); t.tab.st(s, t.word(n++, key)); }
+    mask_out = mask;
+    return n_cur;
 }
 
-template <class Team>
-__device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, int base, ReplayBuffers bufs,
-                             int* __restrict__ out_col, __half* __restrict__ out_vals, int* red) {
-    const int tid = Team::tid();
-    const int r0 = min(i * p.V, p.M), r1 = min(i * p.V + p.V, p.M);
-    const int n_rebuilds = r1 - r0;
-    int* const tab = bufs.table;
-    // the ordered list alternates between two buffers; arrange that the last rebuild writes the output slice
-    int* const out_slice = out_col + base;
-    int* x = (n_rebuilds & 1) ? bufs.lists[0] : out_slice;      // list before the first rebuild (empty)
-    int* xn = (n_rebuilds & 1) ? out_slice : bufs.lists[0];     // written by the first rebuild
-    int* const fresh = bufs.lists[1];                           // NEW: columns of the row not yet in the set
-    // insertion sequence of the current level, and the list the next level's head is extracted into: two lists
-    // that swap roles, or (seq_local) a fixed shared-memory sequence refilled from one extraction list
-    int* seq = bufs.seq_local ? bufs.seq_local : bufs.lists[2];
-    int* ext = bufs.seq_local ? bufs.lists[2] : bufs.lists[3];
-
-    int n_cur = 0;
-    unsigned mask_prev = kMinTable - 1;
-    if (tid < kMinTable) tab[tid] = -1;
+// CTA team: the table's columns in slot order to the list.  Every warp owns a run of rows of 32 slots.
+template <class Team, class Set>
+__device__ __forceinline__ void extract_cta(const Set& t, int size, After after, int* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rows = max(1, size / Team::kSize);
+    const int first = warp * rows * 32 + lane;
+    const bool in = warp * rows * 32 < size;
+    int cnt = 0;
+    if (in)
+#pragma unroll 4
+        for (int j = 0; j < rows; ++j) cnt += __popc(__ballot_sync(0xffffffffu, t.tab.ld(first + j * 32) < Set::kVacant));
+    int total;
+    int pos = Team::before(cnt, total, red);
+    if (in)
+        for (int j0 = 0; j0 < rows; j0 += 4) {
+            unsigned w[4], key[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) w[b] = j0 + b < rows ? t.tab.ld(first + (j0 + b) * 32) : kFree;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) key[b] = w[b] < Set::kVacant ? t.key_of(w[b]) : 0u;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const unsigned m = __ballot_sync(0xffffffffu, w[b] < Set::kVacant);
+                if (w[b] < Set::kVacant) {
+                    const int x = pos + __popc(m & ((1u << lane) - 1u));
+                    if (Set::kPacked) t.list.st(x, key[b]); else t.ext.st(x, key[b]);
+                    t.tab.st(first + (j0 + b) * 32, after == After::kNumbered ? t.word(x, key[b]) : after == After::kVacated ? Set::kVacant | key[b] : kFree);
+                } else if (w[b] != kFree) {
+                    t.tab.st(first + (j0 + b) * 32, kFree);         // an element that left this level
+                }
+                pos += __popc(m);
+            }
+        }
     Team::sync();
-    bool duplicate = false;
+    if (!Set::kPacked) {
+        for (int q = threadIdx.x; q < total; q += Team::kSize) t.list.st(q, t.ext.ld(q));
+        Team::sync();
+    }
+}
 
-    for (int r = r0; r < r1 && !duplicate; ++r) {
-        const int rs = p.row_ptr[r], rlen = p.row_ptr[r + 1] - rs;
-        // ---- columns of this row that are not in the current set, in row order
+// A level whose table still has the columns of the rebuild before, vacated.  Most elements end where they ended then (a row adds
+// a few columns to the set, and few elements change their order), and inserting them one after another into a free table is what
+// costs: an element that comes to sit in an earlier one's place is pushed on, pushes the next one, and so on, up to 200 links one
+// after another for 18 k columns.  So elements start from their old slots, the others are inserted, and then every element is
+// checked: the one assignment in which each element has the first slot of its path that no earlier element holds is the result
+// of inserting them in turn, whatever it was reached from.  Elements that are not in place are inserted again, until
+// all are (the first wrong one in insertion order is final after a round, so there is an end; few rounds do in practice).
+// Links on the critical path, 33903 columns, one row of 17.8 k: 12243 over all rebuilds from free tables, of which 600 are left.
+template <class Team, class Set>
+__device__ __forceinline__ bool relevel(const Set& t, int n, int size, int* red) {
+    const int tid = threadIdx.x;
+    const unsigned mask = (unsigned)size - 1u;
+    unsigned todo = 0;                                     // a bit per element of this thread: not in the table
+    for (int k0 = 0; k0 * Team::kSize < n; k0 += 4) {
+        unsigned key[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) key[b] = (k0 + b) * Team::kSize + tid < n ? t.list.ld((k0 + b) * Team::kSize + tid) : 0u;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int q = (k0 + b) * Team::kSize + tid;
+            if (q >= n) break;
+            unsigned w;
+            const unsigned slot = t.find(mask, key[b], w);
+            if (w == kFree) todo |= 1u << (k0 + b);
+            else t.tab.st(slot, t.word(q, key[b]));        // same column: other searches see no difference
+        }
+    }
+    Team::sync();
+    bool again = false;
+    for (; todo && !again; todo &= todo - 1u) {
+        const int q = (__ffs(todo) - 1) * Team::kSize + tid;
+        const unsigned key = t.list.ld(q);
+        again = t.walk(t.word(q, key), key, probe_begin(key, mask), mask);
+    }
+    Team::sync();
+    constexpr int kRounds = 64;
+    for (int round = 0; round <= kRounds; ++round) {
+        for (int j = 0; j * Team::kSize + tid < size; ++j) {
+            const unsigned s = j * Team::kSize + tid, w = t.tab.ld(s);
+            if (w < Set::kVacant && (t.key_of(w) & mask) != s && !t.in_place(w, s, mask)) todo |= 1u << j;
+        }
+        if (!Team::any(again || todo != 0, red)) return false;
+        if (Team::any(again, red)) return true;
+        for (; todo && !again; todo &= todo - 1u) {
+            const unsigned s = (__ffs(todo) - 1) * Team::kSize + tid, w = t.tab.ld(s);
+            // (not there any more: someone has pushed it on)
+            if (w < Set::kVacant && t.tab.give_up(s, w)) again = t.walk(w, t.key_of(w), probe_begin(t.key_of(w), mask), mask);
+        }
+        todo = 0;
+        Team::sync();
+    }
+    for (int s = tid * 4; s < size; s += Team::kSize * 4) t.tab.free4(s);
+    Team::sync();
+    return Team::any(t.insert(n, mask, tid, Team::kSize), red);
+}
+
+// One group.  rows: kRowInts ints of shared memory; red: 96.
+template <class Team, class Set>
+__device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, int base, const Set& t, int* rows, int* red,
+                             int* __restrict__ out_col, __half* __restrict__ out_vals) {
+    constexpr bool kWarp = Team::kSize == 32, kKeep = !kWarp && Set::kPacked;
+    const int tid = Team::tid(), lane = threadIdx.x & 31;
+    const int r0 = min(i * p.V, p.M), n_rows = min(i * p.V + p.V, p.M) - r0;
+    if (tid <= n_rows) rows[tid] = p.row_ptr[r0 + tid];
+    for (int s = tid * 4; s < (int)(kKeep ? Set::start(cap) : 0u) + cap; s += Team::kSize * 4) t.tab.free4(s);
+    Team::sync();
+    // a warp team does all levels in one table
+    auto table = [&](int size) { return kKeep ? t.level(size) : t; };
+
+    int n_cur = 0, size = 0;                   // length of the table of the last rebuild (0: none yet, all slots free)
+    bool again = false;
+    int turn = 0;                              // which of two sets of warp counts is in use
+    int next_key = tid < rows[1] - rows[0] ? p.col_idx[rows[0] + tid] : -1;          // the next row's columns are under way early
+    for (int r = 0; r < n_rows; ++r) {
+        const int rs = rows[r], rlen = rows[r + 1] - rs;
+        int key = next_key;
+        if (r + 1 < n_rows) next_key = tid < rows[r + 2] - rows[r + 1] ? p.col_idx[rows[r + 1] + tid] : -1;
+        // ---- columns of this row that are not in the set yet, in row order
+        const Set held = table(size);
         int n_new = 0;
         for (int t0 = 0; t0 < rlen; t0 += Team::kSize) {
-            const int t = t0 + tid;
-            const int key = (t < rlen) ? p.col_idx[rs + t] : -1;
-            const bool isnew = (t < rlen) && (unsigned)key < (unsigned)p.K && find_key(tab, mask_prev, key) < 0;
-            int total;
-            const int rk = Team::rank(isnew, total, red);
-            if (isnew && n_cur + n_new + rk < u_final) fresh[n_new + rk] = key;
-            n_new += total;
-        }
-        Team::sync();
-        const int n_total = n_cur + n_new;
-        if (n_total > u_final) { duplicate = true; break; }     // only possible when the row repeats a column
-
-        // ---- replay  set(list)  for the sequence  D = x[0..n_cur) ++ fresh[0..n_new), level by level.
-        // Inside a level the table length is fixed and insertion is first come, first served: an element
-        // takes a slot with atomicMin on its sequence number; if that displaces a later element, the same
-        // thread carries the displaced element on from the slot it had recorded, so one pass settles all.
-        int size = kMinTable, e_len = 0;
-        unsigned mask = kMinTable - 1;
-        for (;;) {
-            long long trig_ll; int next_size;
-            next_level(size, trig_ll, next_size);
-            const int trig = (int)(trig_ll > 0x7fffffff ? 0x7fffffff : trig_ll);
-            const int n_l = min(trig, n_total);
-            mask = (unsigned)size - 1u;
-            if (size >= 4 * Team::kSize) {
-                const int4 fill = make_int4(kEmptyPrio, kEmptyPrio, kEmptyPrio, kEmptyPrio);
-                int4* t4 = reinterpret_cast<int4*>(tab);
-                for (int s = tid; s < size / 4; s += Team::kSize) t4[s] = fill;
+            if (t0 > 0) key = t0 + tid < rlen ? p.col_idx[rs + t0 + tid] : -1;
+            const bool fresh = (unsigned)key < (unsigned)p.K && (n_cur == 0 || !held.contains((unsigned)size - 1u, (unsigned)key));
+            const unsigned b = __ballot_sync(0xffffffffu, fresh);
+            int at = n_cur + n_new + __popc(b & ((1u << lane) - 1u));
+            if constexpr (kWarp) {
+                n_new += __popc(b);
             } else {
-                for (int s = tid; s < size; s += Team::kSize) tab[s] = kEmptyPrio;
+                int total;
+                at += Team::before(__popc(b), total, red + 32 + 32 * turn);
+                n_new += total;
+                turn ^= 1;
             }
-            if (bufs.seq_local)                                                  // head of the sequence: last level's table order
-                for (int q = tid; q < e_len; q += Team::kSize) seq[q] = ext[q];
-            for (int q = e_len + tid; q < n_l; q += 4 * Team::kSize) {          // four loads in flight
-                int v4[4];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    const int qq = q + b * Team::kSize;
-                    v4[b] = (qq < n_l) ? ((qq < n_cur) ? x[qq] : fresh[qq - n_cur]) : 0;
-                }
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-                    if (q + b * Team::kSize < n_l) seq[q + b * Team::kSize] = v4[b];
-            }
-            Team::sync();
-            const int first_new = max(e_len, n_cur);
-            bool dup_here = false;          // also raised when a bound is hit: the group is then redone sequentially
-            volatile int* vtab = tab;
-            // One probe per turn of the loop, and a thread whose chain has ended goes on with its next element at once: a warp
-            // then takes as many turns as its slowest thread has probes in all, not the sum of the longest chains of its
-            // rounds (chains are 1.1 probes long on average, the longest of 32 several times that).
-            int q = tid;
-            int e = q, key = q < n_l ? seq[q] : 0;
-            int ahead = q + Team::kSize < n_l ? seq[q + Team::kSize] : 0;     // the next element's key, loaded early
-            Probe pr = probe_begin(key, mask);
-            unsigned tries = 0;
-            while (q < n_l) {
-                const int slot = (int)(pr.i + pr.w);
-                // Slot values only ever decrease during a level, so a slot seen with an earlier element stays
-                // out of reach; only a slot that looks free or later is worth the atomic.
-                int cur = vtab[slot];
-                if (cur > e) cur = atomicMin(&tab[slot], e);
-                if (cur > e) {
-                    // free slot taken: this chain ends.  Otherwise a later element sat here: the same thread carries it on,
-                    // from the start of its own path (every slot it passed before still holds an earlier element, so it
-                    // walks to the same place and beyond).
-                    if (cur == kEmptyPrio) {
-                        q += Team::kSize;
-                        e = q;
-                        key = ahead;
-                        ahead = q + Team::kSize < n_l ? seq[q + Team::kSize] : 0;
-                        tries = 0;
-                    } else {
-                        e = cur;
-                        key = seq[e];
-                    }
-                    pr = probe_begin(key, mask);
-                    continue;
-                }
-                if ((e >= first_new && seq[cur] == key) || ++tries > 16u * mask + 256u) {
-                    dup_here = true;
-                    break;
-                }
-                probe_advance(pr, mask);
-            }
-            Team::sync();
-            if (Team::any(dup_here, red)) { duplicate = true; break; }
-            if (n_total < trig) {
-                // no further growth: this table is final; keys in place, ordered list out
-                n_cur = extract_ordered<Team>(tab, size, seq, xn, red);
-                break;
-            }
-            e_len = extract_ordered<Team>(tab, size, seq, ext, red);
-            if (!bufs.seq_local) { int* t3 = seq; seq = ext; ext = t3; }
-            size = (next_size > cap) ? cap : next_size;
+            if (fresh && at < u_final) t.list.st(at, (unsigned)key);
         }
-        if (duplicate) break;
-        int* t2 = x; x = xn; xn = t2;
-        mask_prev = mask;
-    }
-
-    if (duplicate) {
-        // rare: fall back to the sequential replay of the whole group by one thread
-        int* xa = (n_rebuilds & 1) ? bufs.lists[0] : out_slice;
-        int* xb = (n_rebuilds & 1) ? out_slice : bufs.lists[0];
-        int m = 0;
-        if (tid == 0) m = replay_sequential(p, r0, r1, tab, cap, xa, xb, bufs.lists[2]);
-        Team::sync();
-        mask_prev = (unsigned)Team::max_of(m, red);
-        n_cur = u_final;
-    }
-    // here: out_slice holds the ordered list, tab holds its keys at their slots
-    if (out_vals && n_cur > 0) {
-        const int size = (int)mask_prev + 1;
-        // a list that is free by now (the group is finished with its sequences)
-        unsigned* const state = reinterpret_cast<unsigned*>(bufs.seq_local ? bufs.seq_local : bufs.lists[1]);
-        int n = 0;
-        for (int s0 = 0; s0 < size; s0 += Team::kSize) {        // slot -> position
-            const int s = s0 + tid;
-            const int key = (s < size) ? tab[s] : -1;
-            int total;
-            const int rk = Team::rank(key != -1, total, red);
-            if (key != -1) state[n + rk] = (unsigned)s;          // position -> slot (ascending), searched below
-            n += total;
+        const int n_total = n_cur + n_new;
+        if (n_total > u_final) { again = true; break; }     // only possible when the row repeats a column
+        if (n_total == 0) continue;
+        int final = kMinTable;
+        while (n_total >= level_trigger(final)) final = level_next(final);
+        // ---- set(list), level by level
+        if constexpr (kWarp) {
+            __syncwarp();
+            for (int s = lane * 4; s < size; s += 128) t.tab.free4(s);
+            __syncwarp();
+            again = t.levels_warp(n_total, final, final);
+        } else {
+            Team::sync();                                   // the list is complete, the table has been read
+            const int used = kKeep && size > kWarpLevels ? 0 : size;          // tables of their own stay
+            if (threadIdx.x < 32) {
+                for (int s = lane * 4; s < min(used, kWarpLevels); s += 128) t.tab.free4(s);
+                __syncwarp();
+                again = t.levels_warp(n_total, min(final, kWarpLevels), final);
+            } else {
+                for (int s = kWarpLevels + (tid - 32) * 4; s < used; s += (Team::kSize - 32) * 4) t.tab.free4(s);
+            }
+            again = Team::any(again, red);
+            for (int level = level_next(kWarpLevels); level <= final && !again; level = level_next(level)) {
+                const Set l = table(level);
+                const int n = min(level_trigger(level), n_total);
+                if (kKeep && level <= size) again = relevel<Team>(l, n, level, red);
+                else again = Team::any(l.insert(n, (unsigned)level - 1u, tid, Team::kSize), red);
+                if (!again)
+                    extract_cta<Team>(l, level, level == final && (!kKeep || r + 1 == n_rows) ? After::kNumbered : kKeep ? After::kVacated : After::kFreed, red);
+            }
         }
+        if (again) break;
+        n_cur = n_total;
+        size = final;
+    }
+    if (again) {
+        unsigned mask = 0;
         Team::sync();
-        const int e0 = p.row_ptr[r0], e1 = p.row_ptr[r1];
+        if (tid == 0) { n_cur = replay_sequential(p, rows, n_rows, table(cap), cap, mask); size = (int)mask + 1; }
+        n_cur = Team::broadcast(n_cur, red);
+        size = Team::broadcast(size, red);
+    }
+    // the list is the ordered set, the words of the table name positions in it
+    const Set held = table(size);
+    for (int q = tid; q < n_cur; q += Team::kSize) out_col[base + q] = (int)t.list.ld(q);
+    if (out_vals) {
+        const int e0 = rows[0], e1 = rows[n_rows];
         for (int e = e0 + tid; e < e1; e += Team::kSize) {
-            int r = r0;
-            while (r + 1 < r1 && e >= p.row_ptr[r + 1]) ++r;
-            const int c = p.col_idx[e];
-            if ((unsigned)c >= (unsigned)p.K) continue;
-            const int s = find_key(tab, mask_prev, c);
-            if (s < 0) continue;
-            // position of slot s = number of occupied slots before it: binary search in the slot list
-            int lo = 0, hi = n - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if ((int)state[mid] < s) lo = mid + 1; else hi = mid;
-            }
-            out_vals[((int64_t)base + lo) * p.V + (r - i * p.V)] = p.vals[e];
+            const unsigned c = (unsigned)p.col_idx[e];
+            int r = 0;                                       // the row of entry e
+#pragma unroll
+            for (int step = 8; step > 0; step >>= 1)
+                if (r + step < n_rows && e >= rows[r + step]) r += step;
+            if (c >= (unsigned)p.K) continue;
+            unsigned w;
+            held.find((unsigned)size - 1u, c, w);
+            if (w != kFree) out_vals[((int64_t)base + Set::number_of(w)) * p.V + r] = p.vals[e];
         }
     }
     Team::sync();
 }
 
-template <class Team, int CLASS>
-__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock,
-                                  ((CLASS == kClassM1 || CLASS == kClassXS) ? 1536 : 1024) / (Team::kSize * Team::kPerBlock))
+// What a team of a class has in shared memory: its tables, a list and the row ends of its group.  Class L with a table per level
+// leaves no room for the list, and class XL has everything, in global scratch.
+// SHIFT: bits of a column in a word; numbers of a list and two more fit the others (0: unpacked).
+constexpr int kRowInts = 20;
+template <int CLASS, int SHIFT>
+struct ClassShape {
+    static constexpr int kTeam = CLASS == kClassM1 ? 256 : CLASS == kClassM2 ? 512 : CLASS == kClassL || CLASS == kClassXL ? 1024 : 32;
+    static constexpr int kCapU = CLASS == kClassXS ? kXSCapU : CLASS == kClassS ? kSCapU : CLASS == kClassM1 ? kM1CapU : CLASS == kClassM2 ? kM2CapU : kLCapU;
+    static constexpr int kCapT = CLASS == kClassXS ? kXSCapT : CLASS == kClassS ? kSCapT : CLASS == kClassM1 ? kM1CapT : CLASS == kClassM2 ? kM2CapT : kLCapT;
+    static constexpr bool kListInSmem = CLASS != kClassXL && !(CLASS == kClassL && SHIFT > 0);
+    static constexpr int kTable = CLASS == kClassXL ? 0 : kTeam > 32 && SHIFT > 0 ? kCapT + (kCapT - kWarpLevels) / 3 : kCapT;
+    static constexpr int kList = kListInSmem ? (kCapU + 3) & ~3 : 0;
+    static constexpr int kInts = kTable + kList + kRowInts;          // of a team, in shared memory
+    static constexpr int kThreads = kTeam == 32 ? 256 : kTeam;       // of a block
+    static constexpr int kBlocks = (kTeam == 1024 ? 1024 : 1536) / kThreads;      // per SM
+    using Team = std::conditional_t<kTeam == 32, WarpTeam, BlockTeam<kTeam>>;
+    using Words = std::conditional_t<CLASS == kClassXL, GlobalWords, SharedWords>;
+    using List = std::conditional_t<kListInSmem, SharedWords, GlobalWords>;
+    static_assert(SHIFT == 0 || kCapU < (1ll << (32 - SHIFT)) - 2, "numbers of a list fit the words");
+    static_assert(SHIFT == 0 || (kCapU <= 32 * kTeam && kCapT <= 32 * kTeam), "relevel: a bit per element and slot of a thread");
+};
+
+template <int CLASS, int SHIFT>
+__global__ void __launch_bounds__(ClassShape<CLASS, SHIFT>::kThreads, ClassShape<CLASS, SHIFT>::kBlocks)
 svc_emit_replay_kernel(SvcProblem p, const int* __restrict__ vec_ptr, const int* __restrict__ tbl_len,
                        const long long* __restrict__ tbl_off, int* __restrict__ scratch, int* __restrict__ out_col,
-                       __half* __restrict__ out_vals, int smem_table_ints, int smem_list_ints,
-                       const int* __restrict__ groups, int n_groups, int* __restrict__ queue) {
-    extern __shared__ int sm_ints[];
-    __shared__ int red[34];
-    const int per_team = smem_table_ints + kListsPerGroup * smem_list_ints;
-    int* mine = sm_ints + (size_t)Team::index_in_block() * per_team;
+                       __half* __restrict__ out_vals, const int* __restrict__ groups, int n_groups, int* __restrict__ queue) {
+    using Shape = ClassShape<CLASS, SHIFT>;
+    using Team = typename Shape::Team;
+    static_assert(Shape::kInts % 4 == 0, "tables start on 16-byte boundaries");
+    extern __shared__ __align__(16) int sm_ints[];
+    __shared__ int red[96];
+    int* mine = sm_ints + (size_t)Team::index_in_block() * Shape::kInts;
     for (;;) {
         int k = 0;
         if (Team::tid() == 0) k = atomicAdd(queue, 1);
@@ -950,18 +1086,14 @@ svc_emit_replay_kernel(SvcProblem p, const int* __restrict__ vec_ptr, const int*
         const int base = vec_ptr[i];
         const int u = vec_ptr[i + 1] - base;
         const int cap = tbl_len[i];
-        ReplayBuffers b;
-        b.seq_local = nullptr;
-        if (CLASS == kClassXS || CLASS == kClassS || CLASS == kClassM1 || CLASS == kClassM2) {
-            b.table = mine;
-            for (int l = 0; l < kListsPerGroup; ++l) b.lists[l] = mine + smem_table_ints + l * smem_list_ints;
-        } else {
-            int* g = scratch + tbl_off[i];
-            for (int l = 0; l < kListsPerGroup; ++l) b.lists[l] = g + (size_t)l * u;
-            b.table = (CLASS == kClassL) ? mine : g + (size_t)kListsPerGroup * u;
-            if (CLASS == kClassL) b.seq_local = mine + smem_table_ints;
-        }
-        replay_group<Team>(p, i, u, cap, base, b, out_col, out_vals, red);
+        unsigned* g = reinterpret_cast<unsigned*>(scratch) + (CLASS == kClassL || CLASS == kClassXL ? tbl_off[i] : 0);
+        HashSet<typename Shape::Words, typename Shape::List, SHIFT> t;
+        if constexpr (CLASS == kClassXL) { t.tab.at = g; g += cap; }
+        else t.tab.at = smem_u32(mine);
+        if constexpr (Shape::kListInSmem) t.list.at = smem_u32(mine + Shape::kTable);
+        else { t.list.at = g; g += u; }
+        t.ext.at = g;
+        replay_group<Team>(p, i, u, cap, base, t, mine + Shape::kTable + Shape::kList, red, out_col, out_vals);
     }
 }
 
@@ -1017,13 +1149,14 @@ struct Fork {
     }
 };
 
-template <class Team, int CLASS>
+template <int CLASS, int SHIFT>
 cudaError_t launch_replay(const SvcProblem& p, const SvcScratch& s, int* out_col, __half* out_vals, long long groups,
-                          long long first, int table_ints, int list_ints, cudaStream_t stream) {
+                          long long first, cudaStream_t stream) {
     if (groups <= 0) return cudaSuccess;
-    auto kern = svc_emit_replay_kernel<Team, CLASS>;
-    const size_t smem = ((size_t)Team::kPerBlock * (table_ints + (size_t)kListsPerGroup * list_ints) +
-                         (CLASS == kClassL ? kLSeqInts : 0)) * sizeof(int);
+    using Shape = ClassShape<CLASS, SHIFT>;
+    using Team = typename Shape::Team;
+    auto kern = svc_emit_replay_kernel<CLASS, SHIFT>;
+    const size_t smem = (size_t)Team::kPerBlock * Shape::kInts * sizeof(int);
     static DeviceOnce once;
     if (!once.done()) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1033,15 +1166,11 @@ cudaError_t launch_replay(const SvcProblem& p, const SvcScratch& s, int* out_col
         if (e != cudaSuccess) return e;
         once.mark();
     }
-    const int sms = device_sm_count();
-    long long want = (groups + Team::kPerBlock - 1) / Team::kPerBlock;
     // as many blocks as can be resident: the groups are handed out through the class's work counter
-    const long long cap_blocks = (long long)sms * (smem > 113 * 1024 ? 1 : (smem > 75 * 1024 ? 2 : (smem > 56 * 1024 ? 3 : (smem > 45 * 1024 ? 4 : (smem > 28 * 1024 ? 6 : 8)))));
-    int grid = (int)(want < cap_blocks ? want : cap_blocks);
-    if (grid < 1) grid = 1;
-    kern<<<grid, Team::kSize * Team::kPerBlock, smem, stream>>>(p, s.vec_ptr, s.tbl_len, s.tbl_off, s.tables, out_col,
-                                                                 out_vals, table_ints, list_ints, s.class_list + first,
-                                                                 (int)groups, s.queue + CLASS);
+    const long long want = (groups + Team::kPerBlock - 1) / Team::kPerBlock;
+    const long long most = (long long)device_sm_count() * Shape::kBlocks;
+    kern<<<(unsigned)(want < most ? want : most), Shape::kThreads, smem, stream>>>(p, s.vec_ptr, s.tbl_len, s.tbl_off, s.tables, out_col, out_vals,
+                                                                            s.class_list + first, (int)groups, s.queue + CLASS);
     return cudaGetLastError();
 }
 
@@ -1142,19 +1271,16 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    // where each class starts in the list of replayed groups (the order svc_scan_place_kernel writes them in)
     // the largest groups first: they are the critical path
-    e = launch_replay<BlockTeam<1024>, kClassXL>(p, s, out_col, out_vals, class_groups[kClassXL], first[kClassXL], 0, 0, f.next());
-    if (e == cudaSuccess)
-        e = launch_replay<BlockTeam<1024>, kClassL>(p, s, out_col, out_vals, class_groups[kClassL], first[kClassL], kLCapT, 0, f.next());
-    if (e == cudaSuccess)
-        e = launch_replay<BlockTeam<512>, kClassM2>(p, s, out_col, out_vals, class_groups[kClassM2], first[kClassM2], kM2CapT, kM2CapU + 2, f.next());
-    if (e == cudaSuccess)
-        e = launch_replay<BlockTeam<256>, kClassM1>(p, s, out_col, out_vals, class_groups[kClassM1], first[kClassM1], kM1CapT, kM1CapU + 4, f.next());
-    if (e == cudaSuccess)
-        e = launch_replay<WarpTeam, kClassS>(p, s, out_col, out_vals, class_groups[kClassS], first[kClassS], kSCapT, kSCapU + 2, f.next());
-    if (e == cudaSuccess)
-        e = launch_replay<WarpTeam, kClassXS>(p, s, out_col, out_vals, class_groups[kClassXS], first[kClassXS], kXSCapT, kXSCapU + 2, stream);
+    auto replay = [&](auto kernel, int c, cudaStream_t st) {
+        if (e == cudaSuccess) e = kernel(p, s, out_col, out_vals, class_groups[c], first[c], st);
+    };
+    replay(launch_replay<kClassXL, 0>, kClassXL, f.next());
+    replay(p.K <= 1 << 17 ? launch_replay<kClassL, 17> : launch_replay<kClassL, 0>, kClassL, f.next());
+    replay(launch_replay<kClassM2, 18>, kClassM2, f.next());
+    replay(launch_replay<kClassM1, 18>, kClassM1, f.next());
+    replay(launch_replay<kClassS, 18>, kClassS, f.next());
+    replay(launch_replay<kClassXS, 18>, kClassXS, stream);
     if (e != cudaSuccess) return e;
     return f.join();
 }

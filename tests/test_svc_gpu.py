@@ -225,3 +225,40 @@ def test_reader_rows_take_the_array_path_through_the_python_entry_point(lib, tmp
     assert fast.vec_colInd_list == slow.vec_colInd_list == r.vec_colInd_list
     assert fast.tile_num == r.tile_num and fast.vec_colInd_list_array == r.vec_colInd_list_array
     assert fast.return_TCF_storage() == r.return_TCF_storage() and fast.return_SRBCSR_storage() == r.return_SRBCSR_storage()
+
+
+def _one_group(K, lens, seed, repeat=0, order="ascending"):
+    """A matrix of one vector row whose matrix rows have these lengths; `repeat`: so many columns of the longest row twice."""
+    rng = np.random.default_rng(seed)
+    rows = [rng.permutation(K)[:n] for n in lens]
+    if order == "ascending":
+        rows = [np.sort(r) for r in rows]
+    if repeat:
+        at = int(np.argmax(lens))
+        rows[at] = rng.permutation(np.concatenate([rows[at], rows[at][:repeat]]))
+    ptr = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+    col = np.concatenate(rows).astype(np.int32)
+    val = rng.uniform(-1, 1, K).astype(np.float16)[col]        # by column: which of two equal entries is kept makes no difference
+    return synthetic.CSR(len(lens), K, ptr, col, val)
+
+
+@pytest.mark.parametrize("order", ["ascending", "any"])
+@pytest.mark.parametrize("K,big", [
+    (140, 70), (600, 150), (600, 300), (2100, 400), (2100, 1220), (8300, 1300), (9000, 4900),            # tables of 128 to 8192 slots, wrapped a little
+    (33000, 5000), (33903, 17900), (32900, 19600), (65536, 15000), (131072, 19650),                      # 32768 slots
+    (131073, 19600), (140000, 9000), (262144, 19655),                                                    # 32768 slots, columns of 18 bits
+    (140000, 21000), (200000, 78600)])                                                                   # tables in global memory
+def test_replay_of_every_table_length(lib, K, big, order):
+    """The long row first, in the middle and last: the sets of the rows after it are rebuilt from nearly the same sequence, and
+    later rows bring nothing, few and many new columns."""
+    for at, others in ((0, [1, 0, 3, 9, 2, 40, 5]), (3, [2, 7, 1, 60, 0, 2, 5]), (7, [3] * 7), (2, [30, big // 3, 8, big // 2, 0, 1, 4])):
+        lens = others[:at] + [big] + others[at:]
+        check_against_oracle(_one_group(K, lens, K + at, order=order), 8)
+    check_against_oracle(_one_group(K, [big // 20] * 16, K + 1, order=order), 16)
+
+
+@pytest.mark.parametrize("K,big", [(140, 60), (2100, 300), (2100, 1100), (9000, 4800), (33000, 17000), (140000, 18000), (140000, 21000)])
+def test_replay_of_rows_that_repeat_columns(lib, K, big):
+    for repeat in (1, 5):
+        check_against_oracle(_one_group(K, [4, big, 3, 0, 6, 1, 2, 9], K + repeat, repeat=repeat), 8)
+        check_against_oracle(_one_group(K, [4, 9, 3, big, 6], K + repeat, repeat=repeat), 8)
