@@ -6,6 +6,7 @@ this module raises if the shared object is missing (build it with
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libsspmm_b200.so")
@@ -78,6 +79,21 @@ def load(path: str = _LIB_PATH) -> C.CDLL:
 
 
 _lib = None
+_native = None
+
+
+def native():
+    """The extension module of csrc/binding.cpp: the calls made once per product, without the interpreter's share."""
+    global _native
+    if _native is None:
+        path = os.path.join(os.path.dirname(_LIB_PATH), "_sspmm_native.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: build it with `python -m sspmm_b200.build`")
+        lib()
+        spec = importlib.util.spec_from_file_location("_sspmm_native", path)
+        _native = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(_native)
+    return _native
 
 
 def lib() -> C.CDLL:

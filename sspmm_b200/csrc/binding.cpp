@@ -1,0 +1,270 @@
+// The calls of ops.py that a program makes once per product, without the interpreter's share of them: checking four to six
+// tensors, allocating the result, asking for device and stream and marshalling eighteen arguments took ops.sspmm 14.5 us a call,
+// for a kernel of 5.2 (512 x 512, N = 256); with one extension call it is 6.6, launch included.
+//
+// Each function takes the ordinary case and nothing else.  None means that the operands are not plain (other types or layouts, host
+// tensors, subclasses, wrapped tensors of a function transform, an active torch mode, ...); the caller then goes through the checks
+// in Python, which accept or refuse as they always have.  An int is an error code of the library.
+#define PY_SSIZE_T_CLEAN
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/cuda/CUDAContextLight.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/sspmm_b200.h"
+
+namespace {
+
+bool modes_active() {
+    return at::impl::PythonTorchFunctionTLS::stack_len() > 0 || c10::impl::TorchDispatchModeTLS::any_modes_set();
+}
+
+// A dense CUDA tensor of this type with nothing on it but autograd's keys, contiguous; null: not one.
+const at::Tensor* plain(PyObject* o, at::ScalarType type) {
+    static const c10::DispatchKeySet allowed =
+        c10::DispatchKeySet(c10::DispatchKey::CUDA) | c10::DispatchKeySet(c10::DispatchKey::AutogradCUDA) |
+        c10::DispatchKeySet(c10::DispatchKey::ADInplaceOrView) | c10::DispatchKeySet(c10::DispatchKey::AutocastCUDA);
+    if (!THPVariable_CheckExact(o)) return nullptr;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (!t.defined() || !t.is_cuda() || t.scalar_type() != type || !t.has_storage() || !allowed.isSupersetOf(t.key_set()) || !t.is_contiguous())
+        return nullptr;
+    return &t;
+}
+
+bool small_int(PyObject* o, long lo, long hi, long* v) {
+    if (!PyLong_CheckExact(o)) return false;
+    int over = 0;
+    *v = PyLong_AsLongAndOverflow(o, &over);
+    return over == 0 && *v >= lo && *v <= hi;
+}
+
+void* stream_of(c10::DeviceIndex device) { return static_cast<void*>(at::cuda::getCurrentCUDAStream(device).stream()); }
+
+// f(stream) on the device and its current stream, without the interpreter lock.
+template <typename F>
+int launch(c10::DeviceIndex device, F&& f) {
+    int rc;
+    const c10::cuda::OptionalCUDAGuard guard(device);
+    void* const stream = stream_of(device);
+    Py_BEGIN_ALLOW_THREADS
+    rc = f(stream);
+    Py_END_ALLOW_THREADS
+    return rc;
+}
+
+PyObject* result(int rc, const at::Tensor& out) {
+    if (rc != 0) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(out);
+}
+
+// Runs a body that may throw (allocation, device guard): the exception becomes the Python one torch would raise.
+template <typename F>
+PyObject* guarded(F&& f) {
+    HANDLE_TH_ERRORS
+    return f();
+    END_HANDLE_TH_ERRORS
+}
+
+// sspmm(row_offsets, column_indices, values, rhs, vec_length, bias, row_indices, out_dtype)
+PyObject* py_sspmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long V;
+        if (n != 8 || modes_active() || !small_int(a[4], 1, 1 << 20, &V) || !THPDtype_Check(a[7])) Py_RETURN_NONE;
+        const at::ScalarType type = reinterpret_cast<THPDtype*>(a[7])->scalar_type;
+        if (type != at::kHalf && type != at::kFloat) Py_RETURN_NONE;
+        const at::Tensor *ptr = plain(a[0], at::kInt), *col = plain(a[1], at::kInt), *val = plain(a[2], at::kHalf), *rhs = plain(a[3], at::kHalf);
+        const at::Tensor* bias = a[5] == Py_None ? nullptr : plain(a[5], at::kHalf);
+        const at::Tensor* order = a[6] == Py_None ? nullptr : plain(a[6], at::kInt);
+        if (!ptr || !col || !val || !rhs || (a[5] != Py_None && !bias) || (a[6] != Py_None && !order) || rhs->dim() != 2) Py_RETURN_NONE;
+        const int64_t m_vec = ptr->numel() - 1, K = rhs->size(0), N = rhs->size(1), most = 0x7fffffff;
+        if (m_vec < 0 || m_vec > most / V || K > most || N > most) Py_RETURN_NONE;
+        if (bias && (bias->numel() != m_vec * V || bias->device() != rhs->device())) Py_RETURN_NONE;
+        at::Tensor out = at::empty({m_vec * V, N}, rhs->options().dtype(type).requires_grad(false));
+        return result(launch(rhs->get_device(), [&](void* st) {
+            return sspmm_counted((int)m_vec, (int)V, (int)N, (int)K, 1, col->numel(), order ? static_cast<const int*>(order->data_ptr()) : nullptr,
+                                 static_cast<const int*>(ptr->data_ptr()), static_cast<const int*>(col->data_ptr()), val->data_ptr(), 0,
+                                 rhs->data_ptr(), 0, bias ? bias->data_ptr() : nullptr, out.data_ptr(), 0, type == at::kHalf, st);
+        }), out);
+    });
+}
+
+// bspmm(row_indices, row_offsets, column_indices, values, rhs_matrix, vec_length)
+PyObject* py_bspmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long V;
+        if (n != 6 || modes_active() || !small_int(a[5], 1, 1 << 20, &V)) Py_RETURN_NONE;
+        const at::Tensor *order = plain(a[0], at::kInt), *ptr = plain(a[1], at::kInt), *col = plain(a[2], at::kInt), *val = plain(a[3], at::kHalf),
+                         *rhs = plain(a[4], at::kHalf);
+        if (!order || !ptr || !col || !val || !rhs || rhs->dim() < 2) Py_RETURN_NONE;
+        const int64_t m_vec = ptr->numel() - 1, K = rhs->size(-2), N = rhs->size(-1), most = 0x7fffffff;
+        if (m_vec < 0 || m_vec > most / V || K > most || N > most || K * N == 0) Py_RETURN_NONE;
+        const int64_t batch = rhs->numel() / (K * N), nnz = col->numel() * V;
+        if (batch > most) Py_RETURN_NONE;
+        const bool shared = val->numel() == nnz && batch != 1;
+        at::Tensor out = at::empty({batch, m_vec * V, N}, rhs->options().requires_grad(false));
+        return result(launch(rhs->get_device(), [&](void* st) {
+            return sspmm_counted((int)m_vec, (int)V, (int)N, (int)K, (int)batch, col->numel(), static_cast<const int*>(order->data_ptr()),
+                                 static_cast<const int*>(ptr->data_ptr()), static_cast<const int*>(col->data_ptr()), val->data_ptr(), shared ? 0 : nnz,
+                                 rhs->data_ptr(), K * N, nullptr, out.data_ptr(), m_vec * V * N, 1, st);
+        }), out);
+    });
+}
+
+// planned(handle, rows of the output, K, values, rhs, out_dtype)
+PyObject* py_planned(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long rows, K;
+        if (n != 6 || modes_active() || !PyLong_CheckExact(a[0]) || !small_int(a[1], 0, 0x7fffffff, &rows) || !small_int(a[2], 0, 0x7fffffff, &K) ||
+            !THPDtype_Check(a[5]))
+            Py_RETURN_NONE;
+        const at::ScalarType type = reinterpret_cast<THPDtype*>(a[5])->scalar_type;
+        if (type != at::kHalf && type != at::kFloat) Py_RETURN_NONE;
+        const at::Tensor *val = plain(a[3], at::kHalf), *rhs = plain(a[4], at::kHalf);
+        if (!val || !rhs || rhs->dim() != 2 || rhs->size(0) != K || rhs->size(1) > 0x7fffffff) Py_RETURN_NONE;
+        const sspmm_plan* plan = static_cast<const sspmm_plan*>(PyLong_AsVoidPtr(a[0]));
+        if (!plan) Py_RETURN_NONE;
+        at::Tensor out = at::empty({rows, rhs->size(1)}, rhs->options().dtype(type).requires_grad(false));
+        return result(launch(rhs->get_device(), [&](void* st) {
+            return sspmm_planned(plan, val->data_ptr(), rhs->data_ptr(), out.data_ptr(), (int)rhs->size(1), type == at::kHalf, st);
+        }), out);
+    });
+}
+
+// group_run(handle, device index) -> error code
+PyObject* py_group_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long device;
+        if (n != 2 || !PyLong_CheckExact(a[0]) || !small_int(a[1], 0, 127, &device)) {
+            PyErr_SetString(PyExc_TypeError, "group_run(handle, device index)");
+            return nullptr;
+        }
+        sspmm_group* group = static_cast<sspmm_group*>(PyLong_AsVoidPtr(a[0]));
+        return PyLong_FromLong(launch((c10::DeviceIndex)device, [&](void* st) { return sspmm_group_run(group, st); }));
+    });
+}
+
+// same_plain(tensors...): contiguous fp16 tensors on one GPU, 16-byte aligned, outside autograd (see encoder._plain)
+PyObject* py_same_plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    const at::Tensor* first = nullptr;
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        const at::Tensor* t = plain(a[i], at::kHalf);
+        if (!t || (first && t->get_device() != first->get_device()) || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0 ||
+            (t->requires_grad() && c10::GradMode::is_enabled()))
+            Py_RETURN_FALSE;
+        if (!first) first = t;
+    }
+    if (!first) Py_RETURN_FALSE;
+    Py_RETURN_TRUE;
+}
+
+void* address(PyObject* o) { return o == Py_None ? nullptr : THPVariable_Unpack(o).data_ptr(); }
+bool on_gpu(PyObject* o) { return THPVariable_Check(o) && THPVariable_Unpack(o).is_cuda(); }
+bool tensors_or_none(PyObject* const* a, Py_ssize_t n) {
+    for (Py_ssize_t i = 0; i < n; ++i)
+        if (a[i] != Py_None && !THPVariable_Check(a[i])) return false;
+    return true;
+}
+
+// layer_norm_fm(x, gamma, beta, eps, out, add, sum_out, bias), attention_fm(q, k, v, heads, batch, seq, out, bias_q, bias_v) and
+// add_bias_fm(x, bias, add, out): for a caller that has compared the operands; -> error code
+PyObject* py_layer_norm_fm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        if (n != 8 || !PyFloat_Check(a[3]) || !on_gpu(a[0]) || !tensors_or_none(a + 1, 2) || !tensors_or_none(a + 4, 4)) Py_RETURN_NONE;
+        const at::Tensor& x = THPVariable_Unpack(a[0]);
+        return PyLong_FromLong(launch(x.get_device(), [&](void* st) {
+            return sspmm_layer_norm_fm((int)x.size(0), (int)x.size(1), x.data_ptr(), address(a[7]), address(a[5]), address(a[6]), address(a[1]),
+                                       address(a[2]), (float)PyFloat_AS_DOUBLE(a[3]), address(a[4]), st);
+        }));
+    });
+}
+PyObject* py_attention_fm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long heads, batch, seq;
+        if (n != 9 || !on_gpu(a[0]) || !tensors_or_none(a + 1, 2) || !tensors_or_none(a + 6, 3) || !small_int(a[3], 0, 0x7fffffff, &heads) ||
+            !small_int(a[4], 0, 0x7fffffff, &batch) || !small_int(a[5], 0, 0x7fffffff, &seq))
+            Py_RETURN_NONE;
+        const at::Tensor& q = THPVariable_Unpack(a[0]);
+        return PyLong_FromLong(launch(q.get_device(), [&](void* st) {
+            return sspmm_attention_fm((int)heads, 64, (int)batch, (int)seq, q.data_ptr(), address(a[1]), address(a[2]), address(a[7]), address(a[8]),
+                                      address(a[6]), st);
+        }));
+    });
+}
+PyObject* py_add_bias_fm(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        if (n != 4 || !on_gpu(a[0]) || !tensors_or_none(a + 1, 3)) Py_RETURN_NONE;
+        const at::Tensor& x = THPVariable_Unpack(a[0]);
+        return PyLong_FromLong(launch(x.get_device(), [&](void* st) {
+            return sspmm_add_bias_fm((int)x.size(0), (int)x.size(1), x.data_ptr(), address(a[1]), address(a[2]), address(a[3]), st);
+        }));
+    });
+}
+
+// svc(row_ptr, col_idx, values or None, M, K, vec_length) -> (vec_ptr, vec_col, vec_values or None, replayed rows)
+PyObject* py_svc(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long M, K, V;
+        if (n != 6 || modes_active() || !small_int(a[3], 0, 0x7ffffff0, &M) || !small_int(a[4], 0, 0x7fffffff, &K) || !small_int(a[5], 1, 1 << 20, &V))
+            Py_RETURN_NONE;
+        const at::Tensor *ptr = plain(a[0], at::kInt), *col = plain(a[1], at::kInt), *val = a[2] == Py_None ? nullptr : plain(a[2], at::kHalf);
+        if (!ptr || !col || (a[2] != Py_None && !val)) Py_RETURN_NONE;
+        const c10::cuda::CUDAGuard guard(ptr->device());
+        struct Job {
+            svc_job* job = nullptr;
+            ~Job() { svc_free(job); }
+        } j;
+        int64_t nvec = 0, replayed = 0;
+        int rc = launch(ptr->get_device(), [&](void* st) {
+            return svc_begin((int)M, (int)K, (int)V, static_cast<const int*>(ptr->data_ptr()), static_cast<const int*>(col->data_ptr()),
+                             val ? val->data_ptr() : nullptr, st, &j.job, &nvec);
+        });
+        if (rc != 0) return PyLong_FromLong(rc);
+        const auto ints = ptr->options().requires_grad(false);
+        at::Tensor out_ptr = at::empty({(M + V - 1) / V + 1}, ints), out_col = at::empty({nvec}, ints), out_val;
+        if (val) out_val = at::empty({nvec * V}, ints.dtype(at::kHalf));
+        rc = launch(ptr->get_device(), [&](void* st) {
+            const int e = svc_replayed_rows(j.job, &replayed);
+            return e != 0 ? e : svc_finish(j.job, static_cast<int*>(out_ptr.data_ptr()), static_cast<int*>(out_col.data_ptr()),
+                                           val ? out_val.data_ptr() : nullptr, st);
+        });
+        if (rc != 0) return PyLong_FromLong(rc);
+        PyObject* values = Py_None;
+        if (val) values = THPVariable_Wrap(out_val); else Py_INCREF(Py_None);
+        return Py_BuildValue("(NNNL)", THPVariable_Wrap(out_ptr), THPVariable_Wrap(out_col), values, (long long)replayed);
+    });
+}
+
+// sorted_row_swizzle(row_offsets)
+PyObject* py_sorted_row_swizzle(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        const at::Tensor* ptr = n == 1 && !modes_active() ? plain(a[0], at::kInt) : nullptr;
+        if (!ptr || ptr->numel() < 1 || ptr->numel() > 0x7fffffff) Py_RETURN_NONE;
+        const int m_vec = (int)(ptr->numel() - 1);
+        at::Tensor out = at::empty({m_vec}, ptr->options().requires_grad(false));
+        return result(launch(ptr->get_device(), [&](void* st) {
+            return sspmm_sorted_row_swizzle(m_vec, static_cast<const int*>(ptr->data_ptr()), static_cast<int*>(out.data_ptr()), st);
+        }), out);
+    });
+}
+
+PyMethodDef methods[] = {
+    {"svc", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_svc)), METH_FASTCALL, nullptr},
+    {"sorted_row_swizzle", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sorted_row_swizzle)), METH_FASTCALL, nullptr},
+    {"sspmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sspmm)), METH_FASTCALL, nullptr},
+    {"bspmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bspmm)), METH_FASTCALL, nullptr},
+    {"planned", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_planned)), METH_FASTCALL, nullptr},
+    {"group_run", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_group_run)), METH_FASTCALL, nullptr},
+    {"same_plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_same_plain)), METH_FASTCALL, nullptr},
+    {"layer_norm_fm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer_norm_fm)), METH_FASTCALL, nullptr},
+    {"attention_fm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention_fm)), METH_FASTCALL, nullptr},
+    {"add_bias_fm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_add_bias_fm)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_sspmm_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__sspmm_native(void) { return PyModule_Create(&module); }

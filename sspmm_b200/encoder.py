@@ -18,7 +18,7 @@ import torch
 import torch.nn.functional as F
 from torch.autograd import forward_ad
 
-from . import ops, synthetic
+from . import capi, ops, synthetic
 
 
 def _plain(*tensors) -> bool:
@@ -26,6 +26,8 @@ def _plain(*tensors) -> bool:
     transforms and forward-mode differentiation (a dual tensor has an address too, and no requires_grad)."""
     if torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0:
         return False
+    if capi.native().same_plain(*tensors):
+        return True
     gpu = tensors[0].get_device()
     return gpu >= 0 and all(t.get_device() == gpu and t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0
                and not (t.requires_grad and torch.is_grad_enabled()) for t in tensors)

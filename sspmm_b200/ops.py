@@ -56,10 +56,21 @@ def sspmm(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: torch
     return sspmm_bias(row_offsets, column_indices, values, rhs, vec_length, None, row_indices, out_dtype, out)
 
 
+def _made(got):
+    """What an extension call returned: a tensor, or an error code of the library."""
+    if type(got) is int:
+        capi.check(got)
+    return got
+
+
 def sspmm_bias(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: torch.Tensor, rhs: torch.Tensor,
                vec_length: int, bias: Optional[torch.Tensor], row_indices: Optional[torch.Tensor] = None,
                out_dtype=torch.float16, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``sspmm`` plus a number per output row (fp16, m_vec*V of them), added to the fp32 sums before the conversion."""
+    if out is None:
+        got = capi.native().sspmm(row_offsets, column_indices, values, rhs, vec_length, bias, row_indices, out_dtype)
+        if got is not None:
+            return _made(got)
     _require(row_offsets, torch.int32, "row_offsets")
     _require(column_indices, torch.int32, "column_indices")
     _require(values, torch.float16, "values")
@@ -94,6 +105,9 @@ def svc(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: Optional[torch.Ten
     """Sparse vector compression of a CSR matrix held on the GPU.
     Returns (vec_row_ptr[m_vec+1], vec_col[nvec], vec_values[nvec*V] or None, replayed_rows)."""
     import ctypes as C
+    got = capi.native().svc(row_ptr, col_idx, values, M, K, vec_length)
+    if got is not None:
+        return _made(got)
     _require(row_ptr, torch.int32, "row_ptr")
     _require(col_idx, torch.int32, "col_idx")
     if values is not None:
@@ -175,6 +189,9 @@ def svc_batch(mats, vec_length: int, nnz=None):
 
 
 def sorted_row_swizzle(row_offsets: torch.Tensor) -> torch.Tensor:
+    got = capi.native().sorted_row_swizzle(row_offsets)
+    if got is not None:
+        return _made(got)
     _require(row_offsets, torch.int32, "row_offsets")
     m_vec = row_offsets.numel() - 1
     out = torch.empty(m_vec, dtype=torch.int32, device=row_offsets.device)
@@ -208,6 +225,9 @@ def layer_norm_fm(x: torch.Tensor, gamma: torch.Tensor, beta: torch.Tensor, eps:
 
 def launch_layer_norm_fm(x, gamma, beta, eps, out, add, sum_out, bias) -> None:
     """``layer_norm_fm`` for a caller that has compared the operands itself."""
+    rc = capi.native().layer_norm_fm(x, gamma, beta, eps, out, add, sum_out, bias)
+    if rc is not None:
+        return capi.check(rc)
     _launch(capi.lib().sspmm_layer_norm_fm, x, x.shape[0], x.shape[1], x.data_ptr(), _ptr(bias), _ptr(add), _ptr(sum_out),
             gamma.data_ptr(), beta.data_ptr(), eps, out.data_ptr())
 
@@ -223,6 +243,10 @@ def add_bias_fm(x: torch.Tensor, bias: torch.Tensor, add: torch.Tensor) -> torch
 def launch_add_bias_fm(x, bias, add) -> torch.Tensor:
     """``add_bias_fm`` for a caller that has compared the operands itself."""
     out = torch.empty_like(x)
+    rc = capi.native().add_bias_fm(x, bias, add, out)
+    if rc is not None:
+        capi.check(rc)
+        return out
     _launch(capi.lib().sspmm_add_bias_fm, x, x.shape[0], x.shape[1], x.data_ptr(), bias.data_ptr(), add.data_ptr(), out.data_ptr())
     return out
 
@@ -240,6 +264,9 @@ def attention_fm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, heads: int, 
 
 def launch_attention_fm(q, k, v, heads, batch, seq, out, bias_q, bias_v) -> None:
     """``attention_fm`` for a caller that has compared the operands itself."""
+    rc = capi.native().attention_fm(q, k, v, heads, batch, seq, out, bias_q, bias_v)
+    if rc is not None:
+        return capi.check(rc)
     _launch(capi.lib().sspmm_attention_fm, q, heads, 64, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(), _ptr(bias_q), _ptr(bias_v),
             out.data_ptr())
 
@@ -284,6 +311,10 @@ class Plan:
 def sspmm_planned(plan: Plan, values: torch.Tensor, rhs: torch.Tensor, out_dtype=torch.float16,
                   out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """C = A_vs @ rhs through ``sspmm_planned``: one launch, nothing allocated by the library."""
+    if out is None and plan.handle:
+        got = capi.native().planned(plan.handle.value, plan.m_vec * plan.V, plan.K, values, rhs, out_dtype)
+        if got is not None:
+            return _made(got)
     _require(values, torch.float16, "values")
     _require(rhs, torch.float16, "rhs")
     K, N = rhs.shape
@@ -333,12 +364,8 @@ class Group:
         self.launches = launches.value
 
     def run(self) -> None:
-        if torch.cuda.current_device() == self.device.index:
-            rc = capi.lib().sspmm_group_run(self._h, _stream_ptr())
-        else:
-            with torch.cuda.device(self.device):
-                rc = capi.lib().sspmm_group_run(self._h, _stream_ptr())
-        if rc != 0:
+        rc = capi.native().group_run(self._h.value if self._h else 0, self.device.index)
+        if rc:
             capi.check(rc)
 
     def close(self) -> None:

@@ -23,6 +23,9 @@ def spmm(row_indices, row_offsets, column_indices, values, rhs_matrix, vec_lengt
 
 
 def bspmm(row_indices, row_offsets, column_indices, values, rhs_matrix, vec_length):
+    got = capi.native().bspmm(row_indices, row_offsets, column_indices, values, rhs_matrix, vec_length)
+    if got is not None:
+        return ops._made(got)
     for t, dt, name in ((row_indices, torch.int32, "row_indices"), (row_offsets, torch.int32, "row_offsets"),
                         (column_indices, torch.int32, "column_indices"), (values, torch.float16, "values"),
                         (rhs_matrix, torch.float16, "rhs_matrix")):
