@@ -922,6 +922,8 @@ struct sspmm_plan {
 
 struct sspmm_group {
     int device, count, BN;
+    std::vector<SpmmArgs> rows;        // not empty: the row-gather kernel does the products, in one launch (nothing below is set)
+    long long rows_nvec;
     bool out_f16;
     bool pair;                 // CTA-pair kernel (tiles of 256 x 256); always expanded
     bool expanded;             // A tiles by TMA from dense transposed copies that the kernel's loader warps write at every run
@@ -963,7 +965,6 @@ cudaError_t launch_bn(const Params& p, int BN, int grid, cudaStream_t st, bool s
 
 // CTA-pair kernel (sspmm_fused_pair.cu)
 cudaError_t launch_pair(const Params& p, bool out_f16, int pairs, cudaStream_t st, bool setup_only);
-constexpr bool kAutoPairs = false;
 
 cudaError_t launch(const Params& p, int BN, bool out_f16, bool a_tma, int grid, cudaStream_t st, bool setup_only = false) {
     if (a_tma) return out_f16 ? launch_bn<__half, true>(p, BN, grid, st, setup_only) : launch_bn<float, true>(p, BN, grid, st, setup_only);
@@ -998,6 +999,45 @@ bool fill_problem(Problem* P, const sspmm_plan* plan, const void* values, const 
     P->Mp = Mp; P->N = N; P->K = plan->K; P->V = plan->V;
     P->k_steps = plan->k_steps; P->m_tiles = pair ? (plan->m_tiles + 1) / 2 : plan->m_tiles; P->n_tiles = (N + BN - 1) / BN; P->expand_blocks = 0;
     return true;
+}
+
+// ---- how a group is divided -----------------------------------------------------------------
+struct Shape { int m_tiles, k_steps, N; };
+struct GroupChoice { int BN, cut; double us; };      // tile width, K steps above which a tile's range is cut (0: never), modelled time
+
+int parts_of(int k_steps, int cut) { return cut > 0 && k_steps > cut ? std::min(16, (k_steps + cut - 1) / cut) : 1; }
+
+// Modelled time of the tile kernel with A tiles from the loader warps, in microseconds.  Fitted to groups of the conv layers at
+// N = 64 to 5000 and of encoder products (256 to 768 wide, 256 to 8192 columns), every width with and without cuts: a K
+// step takes 0.515 us whatever the width (the loaders set the pace), an item 1.2 more, the launch 6 to 7.  A cut tile's
+// parts are added by the CTA that finishes last, 0.85 us per part and 64 columns, and that is what cuts cost.
+// So tiles are as wide as leaves the rounds of items few, and only ranges much longer than an SM's share are cut: conv layers
+// at N = 800 take 67 us with 608 whole tiles of 256 columns, 133 with 1976 of 64 (as many tiles as give every SM two, the rule before);
+// N = 64: 47 with whole tiles, 29 cut; 768 x 3072 at N = 4096: 33 with 96 tiles of 256, 90 with 384 of 64.
+GroupChoice choose_tiles(const std::vector<Shape>& shapes, int units, bool only_256) {
+    GroupChoice best{256, 0, -1.0};
+    for (int BN = 256; BN >= (only_256 ? 256 : 64); BN /= 2)
+        for (int cut : {0, 36, 24, 16, 12, 8}) {
+            double longest = 0, total = 0, last_sum = 0, first_item = -1;
+            int64_t n = 0;
+            bool uniform = true;
+            for (const Shape& s : shapes) {
+                const int parts = parts_of(s.k_steps, cut), steps = (s.k_steps + parts - 1) / parts;
+                const int64_t tiles = (int64_t)s.m_tiles * ((s.N + BN - 1) / BN);
+                const double item = 0.515 * steps + 1.2;
+                const double sum = parts > 1 ? ((std::min(BN, s.N) + 63) / 64) * (1.1 + 0.85 * parts) : 0.0;
+                longest = std::max(longest, item + sum);
+                last_sum = std::max(last_sum, sum);
+                total += tiles * (parts * item + sum);
+                n += tiles * parts;
+                uniform = uniform && (first_item < 0 || first_item == item);
+                first_item = item;
+            }
+            const double spread = uniform ? (double)((n + units - 1) / units) * first_item + last_sum : total / units;
+            const double us = (BN == 256 ? 7.2 : BN == 128 ? 6.3 : 6.0) + std::max(longest, spread);
+            if (best.us < 0 || us < best.us) best = GroupChoice{BN, cut, us};
+        }
+    return best;
 }
 
 }  // namespace fused
@@ -1189,41 +1229,58 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
         if (pl->device != dev) { set_error("product %d: plan was built on device %d, current device is %d", i, pl->device, dev); return (int)cudaErrorInvalidValue; }
         if (items[i].N <= 0) { set_error("product %d: N must be positive", i); return (int)cudaErrorInvalidValue; }
     }
-    // tile width: the widest that gives the grid at least two tiles per SM
-    int BN = 256;
-    for (;; BN >>= 1) {
-        int64_t tiles = 0;
-        for (int i = 0; i < count; ++i) tiles += (int64_t)items[i].plan->m_tiles * ((items[i].N + BN - 1) / BN);
-        if (tiles >= 2 * sms || BN == 64) break;
-    }
-    // CTA pairs (tiles of 256 x 256, see sspmm_fused_pair.cu) when asked for, or when the group is large enough for
-    // 256-column tiles and for the expanded mode
-    bool pair = mode == 3;
-    if (mode == 0 && BN == 256 && fused::kAutoPairs) {
-        double est = 0;
-        for (int i = 0; i < count; ++i)
-            est += (double)items[i].plan->m_tiles * ((items[i].N + 255) / 256) * (items[i].plan->k_steps + 2);
-        pair = est / sms >= 48.0;
-    }
-    if (pair) BN = 256;
+    // CTA pairs (tiles of 256 x 256, see sspmm_fused_pair.cu) only when asked for
+    const bool pair = mode == 3;
     const int units = pair ? sms / 2 : sms;            // what holds one tile: an SM, or a pair of SMs
+    std::vector<fused::Shape> shapes((size_t)count);
+    for (int i = 0; i < count; ++i)
+        shapes[i] = fused::Shape{pair ? (items[i].plan->m_tiles + 1) / 2 : items[i].plan->m_tiles, items[i].plan->k_steps, items[i].N};
+    const fused::GroupChoice choice = fused::choose_tiles(shapes, units, pair);
+    const int BN = choice.BN;
+    // Small groups go to the row-gather kernel, which spreads every vector row over the chip instead of walking a tile's K range
+    // (launch and look-ups, then 2 * nvec * N bytes of gathers at 6 TB/s: 768 x 3072 at N = 128 10 us against 24, three 256 x 256 at 128
+    // 4 against 9; they meet at 13 to 15 us).
+    if (mode == 0 && count <= kRowsMaxSet) {
+        double gathers = 0;
+        long long nvec = 0;
+        bool ok = true;
+        std::vector<SpmmArgs> args((size_t)count);
+        for (int i = 0; i < count; ++i) {
+            const sspmm_plan* pl = items[i].plan;
+            SpmmArgs& a = args[i];
+            a.m_vec = pl->m_vec; a.V = pl->V; a.N = items[i].N; a.n_out = items[i].N; a.K = pl->K;
+            a.row_indices = nullptr; a.row_offsets = pl->row_offsets; a.column_indices = pl->column_indices;
+            a.values = static_cast<const __half*>(items[i].values_f16); a.rhs = static_cast<const __half*>(items[i].rhs_f16);
+            a.out = items[i].out; a.out_f16 = out_is_f16 != 0; a.bias = nullptr; a.batch = 1;
+            a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0; a.stream = nullptr;
+            gathers += 2.0 * (double)pl->nvec * items[i].N;
+            nvec += pl->nvec;
+            ok = ok && pl->V == items[0].plan->V && items[i].N % 8 == 0 && a.values && a.rhs && a.out && fused::aligned16(a.values) &&
+                 fused::aligned16(a.rhs) && fused::aligned16(a.out);
+        }
+        if (ok && 4.0 + gathers / 6.0e6 < choice.us) {
+            sspmm_group* g = new (std::nothrow) sspmm_group();
+            if (!g) return (int)cudaErrorMemoryAllocation;
+            g->device = dev; g->count = count; g->out_f16 = out_is_f16 != 0; g->rows_nvec = nvec;
+            g->BN = 64; g->n_items = 0;
+            for (const SpmmArgs& a : args) g->n_items += a.m_vec * ((a.N + 63) / 64);
+            g->grid = std::min(g->n_items, sms);
+            g->rows = std::move(args);
+            *group = g;
+            return 0;
+        }
+    }
     std::vector<fused::Problem> probs((size_t)count);
     int64_t tiles = 0;
-    double work = 0;                                   // K steps, with a fixed cost of two steps per tile
     for (int i = 0; i < count; ++i) {
         if (!fused::fill_problem(&probs[i], items[i].plan, items[i].values_f16, items[i].rhs_f16, items[i].out, items[i].N,
                                  out_is_f16 != 0, BN, pair))
             return (int)cudaErrorInvalidValue;
-        const int64_t t = (int64_t)probs[i].m_tiles * probs[i].n_tiles;
-        tiles += t;
-        work += (double)t * (probs[i].k_steps + 2);
+        tiles += (int64_t)probs[i].m_tiles * probs[i].n_tiles;
     }
     if (tiles > (1 << 26)) { set_error("group too large (%lld tiles)", (long long)tiles); return (int)cudaErrorInvalidValue; }
-    // Tiles longer than `cut` K steps are cut into parts so that no single item is a large share of an
-    // SM's work; the parts' fp32 partial tiles are summed by whichever part finishes last.
-    const double per_sm = work / units;
-    int cut = (int)(per_sm / 3.0);
-    if (cut < 8) cut = 8;
+    // Tiles longer than choice.cut K steps are cut into parts; the parts' fp32 partial tiles are summed by whichever part
+    // finishes last.
     std::vector<fused::Item> list;
     list.reserve((size_t)tiles + 1024);
     int pslots = 0, cslots = 0;
@@ -1254,21 +1311,7 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
             }
         }
         const fused::Problem& L = probs[lead];
-        int parts = (tiles < 8 * (int64_t)units && L.k_steps > cut) ? (L.k_steps + cut - 1) / cut : 1;
-        if (parts > 16) parts = 16;
-        if (count == 1) {
-            // One product: the number of parts that gives the shortest critical path.  An item costs its K steps
-            // plus two for the hand-over, and a cut tile pays for its fp32 partial tiles (written once, read once:
-            // measured about 17 K steps' worth per part for a 128 x 256 tile when every SM does it at once).
-            const int64_t t = (int64_t)L.m_tiles * L.n_tiles;
-            const int64_t extra = 17 * BN / 256 + 1;
-            int64_t best = -1;
-            for (int q = 1; q <= 16 && q <= L.k_steps; ++q) {
-                const int64_t rounds = (t * q + units - 1) / units;
-                const int64_t cost = rounds * ((L.k_steps + q - 1) / q + 2 + (q > 1 ? extra : 0));
-                if (best < 0 || cost < best) { best = cost; parts = q; }
-            }
-        }
+        int parts = fused::parts_of(L.k_steps, choice.cut);
         const int sps = (L.k_steps + parts - 1) / parts;
         parts = (L.k_steps + sps - 1) / sps;
         for (int nt = 0; nt < L.n_tiles; ++nt)
@@ -1295,10 +1338,18 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
     g->n_items = (int)list.size();
     g->grid = g->n_items < units ? g->n_items : units;  // CTAs, or CTA pairs
     g->pair = pair;
-    // Measured on B200: with the A tiles built by the loader warps a K step takes about 1150 cycles, with A tiles
-    // fetched by TMA from a dense copy about 700-750; writing the copies costs one more launch and a few tens of
-    // microseconds.  So groups with much work per SM expand, small ones (latency matters) do not.
-    g->expanded = pair || mode == 2 || (mode == 0 && per_sm >= 48.0);
+    // With A tiles by TMA from a dense copy a K step of a loaded chip takes about 0.3 us less per SM than when the loader warps
+    // build them; against that stands the writing of the copies: 10 us, and 4.5 for every further round of blocks (the
+    // first items wait for theirs).  Conv layers, 15 steps per SM and 256 columns: N = 1200 74 us built, 92 copied; 1600 97 and 92;
+    // 3136 163 and 138.  768 x 768 at 8192: 43 and 38; 3072 x 768 at 4096: 30 and 34.
+    int64_t copy_blocks = 0, steps = 0;
+    for (int i = 0; i < count; ++i) {
+        copy_blocks += ((int64_t)items[i].plan->m_vec * 8 * items[i].plan->k_steps + 255) / 256;
+        steps += (int64_t)probs[i].m_tiles * probs[i].n_tiles * probs[i].k_steps;
+    }
+    const double rounds_of_copies = (double)copy_blocks / g->grid;
+    g->expanded = pair || mode == 2 || (mode == 0 && BN == 256 && choice.cut == 0 &&
+                                        0.3 * (double)steps / sms > 10.0 + 4.5 * std::max(0.0, rounds_of_copies - 1.0));
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     std::vector<fused::ExpandJob> jobs;
     std::vector<size_t> at_off((size_t)count, 0);
@@ -1390,6 +1441,13 @@ int sspmm_group_run(sspmm_group* group, void* stream) {
     set_error("%s", "");
     if (!group) { set_error("null group"); return (int)cudaErrorInvalidValue; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (!group->rows.empty()) {
+        SpmmArgs args[kRowsMaxSet];
+        for (int i = 0; i < group->count; ++i) { args[i] = group->rows[i]; args[i].stream = st; }
+        const cudaError_t e = launch_sspmm_rows_set(args, group->count, group->rows_nvec);
+        if (e != cudaSuccess) { set_error("group launch: %s", cudaGetErrorString(e)); return (int)e; }
+        return 0;
+    }
     cudaError_t e = group->pair ? fused::launch_pair(group->params, group->out_f16, group->grid, st, false)
                                 : fused::launch(group->params, group->BN, group->out_f16, group->expanded, group->grid, st);
     if (e != cudaSuccess) { set_error("group launch: %s", cudaGetErrorString(e)); return (int)e; }

@@ -334,17 +334,15 @@ struct Tile {
 // One launch, no scratch: an item (vector row, column tile, batch entry) is done by `team` warps of a CTA (1, 2, 4 or 8)
 // or, with clusters, by all warps of `cluster` CTAs; the warps take 16-vector steps in turn and their sums are added in
 // warp order through shared memory (of the cluster), so results do not depend on timing.
+// item: this warp's, of problem p.
 template <int V, typename OutT, int H>
-__global__ void __launch_bounds__(kThreads, kResident)
-sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int team, int cluster) {
+__device__ __forceinline__ void do_item(const Problem& p, OutT* __restrict__ out, long long item, int team, int cluster) {
     using T = Tile<V, H, sizeof(OutT) == 4>;
     extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int per_cta = kWarps / team;
     const int rank = cluster > 1 ? (int)cluster_cta_rank() : 0;
-    const long long cta_item = (long long)(blockIdx.x / cluster) * per_cta;
     const int member = warp % team;
-    const Where w = locate(p, cta_item + warp / team, T::NT);
+    const Where w = locate(p, item, T::NT);
     uint8_t* const mem = smem + warp * T::kWarpBytes;
     T tile;
     tile.clear();
@@ -391,6 +389,30 @@ sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int
         if (w.row >= 0) T::store_unit(p, cbase, first_row, w.n0, u, lane, o);
     }
     cluster_sync_all();                                   // nobody leaves while its tile is being read
+}
+
+template <int V, typename OutT, int H>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int team, int cluster) {
+    const int per_cta = kWarps / team, warp = threadIdx.x >> 5;
+    do_item<V, OutT, H>(p, out, (long long)(blockIdx.x / cluster) * per_cta + warp / team, team, cluster);
+}
+
+// Several products in one launch: the items of one after those of the other.
+struct ProblemSet {
+    int count;
+    int first[kRowsMaxSet + 1];           // first item of each product, and the end
+    void* out[kRowsMaxSet];
+    Problem p[kRowsMaxSet];
+};
+template <int V, typename OutT, int H>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_set_kernel(const __grid_constant__ ProblemSet s, int team, int cluster) {
+    const int per_cta = kWarps / team, warp = threadIdx.x >> 5;
+    const long long item = (long long)(blockIdx.x / cluster) * per_cta + warp / team;
+    int k = 0;
+    while (k + 1 < s.count && item >= s.first[k + 1]) ++k;
+    do_item<V, OutT, H>(s.p[k], static_cast<OutT*>(s.out[k]), item - s.first[k], team, cluster);
 }
 
 // Matrices whose rows differ in length by orders of magnitude (power-law matrices: half of the rows have fewer than 50
@@ -531,13 +553,21 @@ list_parts_kernel(const __grid_constant__ Problem p) {
 // outside the loads; 64 when that is all there is or when wide tiles, a CTA each, would leave SMs without one.  Warps per item:
 // enough to fill the SMs, at least one step each; long rows get a whole CTA so that no single warp runs long after the others.
 struct Division { int H, team, cluster; };
-Division divide(const SpmmArgs& a, long long nvec, int sms) {
-    const long long rows_total = (long long)a.m_vec * a.batch, slots = (long long)sms * kResident * kWarps;
-    const long long mean_steps = nvec > 0 ? (nvec / a.m_vec + kStep) / kStep : (a.K / 2 + kStep) / kStep;
-    Division d{a.N > 64 ? 2 : 1, 1, 1};
-    if (d.H == 2 && rows_total * ((a.N + 127) / 128) * std::min<long long>(mean_steps, kWarps) < slots) d.H = 1;
-    const long long items = rows_total * ((a.N + 64 * d.H - 1) / (64 * d.H));
-    const long long want = std::min(slots / items, mean_steps);
+long long count_items(const SpmmArgs* a, int count, int H) {
+    long long n = 0;
+    for (int k = 0; k < count; ++k) n += (long long)a[k].m_vec * a[k].batch * ((a[k].N + 64 * H - 1) / (64 * H));
+    return n;
+}
+// nvec: vectors of all products (<= 0: unknown)
+Division divide(const SpmmArgs* a, int count, long long nvec, int sms) {
+    const long long slots = (long long)sms * kResident * kWarps;
+    long long rows = 0;
+    int widest = 0;
+    for (int k = 0; k < count; ++k) { rows += a[k].m_vec; widest = std::max(widest, a[k].N); }
+    const long long mean_steps = nvec > 0 ? (nvec / rows + kStep) / kStep : (a->K / 2 + kStep) / kStep;
+    Division d{widest > 64 ? 2 : 1, 1, 1};
+    if (d.H == 2 && count_items(a, count, 2) * std::min<long long>(mean_steps, kWarps) < slots) d.H = 1;
+    const long long want = std::min(slots / count_items(a, count, d.H), mean_steps);
     while (d.team < kWarps && (2 * d.team <= want || mean_steps > 32LL * d.team)) d.team *= 2;
     if (d.team == kWarps)
         while (d.cluster < kMaxCluster && (long long)d.cluster * 2 * d.team <= want && mean_steps >= 4LL * d.cluster * d.team) d.cluster *= 2;
@@ -553,23 +583,34 @@ cudaError_t allow_smem(Kern kern, DeviceOnce& once, int bytes) {
     return e;
 }
 
-template <int V, typename OutT, int H>
-cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d) {
-    auto kern = sspmm_rows_kernel<V, OutT, H>;
-    using T = Tile<V, H, sizeof(OutT) == 4>;
-    static DeviceOnce once;
-    cudaError_t e = allow_smem(kern, once, kWarps * T::kWarpBytes);
+template <int V, typename OutT, int H, typename Kern, typename... Args>
+cudaError_t launch_items(Kern kern, DeviceOnce& once, long long items, const Division& d, cudaStream_t stream, Args... args) {
+    constexpr int kBytes = kWarps * Tile<V, H, sizeof(OutT) == 4>::kWarpBytes;
+    cudaError_t e = allow_smem(kern, once, kBytes);
     if (e != cudaSuccess) return e;
     const int per_cta = kWarps / d.team;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((p.items + per_cta - 1) / per_cta * d.cluster));
+    cfg.gridDim = dim3((unsigned)((items + per_cta - 1) / per_cta * d.cluster));
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = (size_t)kWarps * T::kWarpBytes; cfg.stream = a.stream;
+    cfg.dynamicSmemBytes = (size_t)kBytes; cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)d.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = d.cluster > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, p, static_cast<OutT*>(a.out), d.team, d.cluster);
+    return cudaLaunchKernelEx(&cfg, kern, args..., d.team, d.cluster);
+}
+
+template <int V, typename OutT, int H>
+cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d) {
+    static DeviceOnce once;
+    return launch_items<V, OutT, H>(sspmm_rows_kernel<V, OutT, H>, once, p.items, d, a.stream, p, static_cast<OutT*>(a.out));
+}
+
+template <int V, typename OutT>
+cudaError_t launch_set(const ProblemSet& s, const Division& d, cudaStream_t stream) {
+    static DeviceOnce once_wide, once_narrow;
+    if (d.H == 2) return launch_items<V, OutT, 2>(sspmm_rows_set_kernel<V, OutT, 2>, once_wide, s.first[s.count], d, stream, s);
+    return launch_items<V, OutT, 1>(sspmm_rows_set_kernel<V, OutT, 1>, once_narrow, s.first[s.count], d, stream, s);
 }
 
 template <int V, typename OutT, int H>
@@ -613,7 +654,7 @@ Scratch plan_scratch(const SpmmArgs& a, long long nvec) {
     const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;
     if (a.K < 8 * (nvec / a.m_vec + 1)) return r;
     if (a.K < 2048) {
-        const Division d = divide(a, nvec, sms);
+        const Division d = divide(&a, 1, nvec, sms);
         if (a.K <= 48LL * kStep * d.team * d.cluster) return r;
     }
     const long long nt = a.N <= 64 ? 64 : 128, n_tiles = (a.N + nt - 1) / nt;
@@ -658,30 +699,37 @@ align_rows_kernel(const __half* __restrict__ src, __half* __restrict__ dst, int 
 
 size_t sspmm_rows_scratch_bytes(const SpmmArgs& a, long long nvec) { return rows::plan_scratch(a, nvec).bytes; }
 
-// scratch: null, or sspmm_rows_scratch_bytes() bytes (long rows are then cut); nvec < 0: unknown.
-cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) {
-    const int sms = current_device_sm_count();
-    if (sms <= 0) return cudaErrorNoDevice;
-    rows::Problem p;
+namespace rows {
+Problem problem_of(const SpmmArgs& a, int H) {
+    Problem p = {};
     p.m_vec = a.m_vec; p.N = a.n_out; p.ldb = a.N; p.K = a.K;
     p.row_indices = a.row_indices; p.row_offsets = a.row_offsets; p.col = a.column_indices;
     p.values = a.values; p.rhs = a.rhs; p.bias = a.bias;
     p.values_stride = a.values_stride; p.rhs_stride = a.rhs_stride; p.out_stride = a.out_stride;
-    p.chunk = 0; p.cap_cut = 0; p.cap_whole = 0; p.header = nullptr; p.arrivals = nullptr; p.entries = nullptr; p.partial = nullptr;
     const size_t es = a.out_f16 ? 2 : 4;
     p.out_pieces = (a.n_out % 8 == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 &&
                     (a.batch == 1 || ((size_t)a.out_stride * es) % 16 == 0)) ? 1 : 0;
-    const bool split = scratch != nullptr;
-    const rows::Division d = rows::divide(a, nvec, sms);
-    const int H = split ? (a.N > 64 ? 2 : 1) : d.H;
-    const long long slots = (long long)sms * rows::kResident * rows::kWarps;
-    const int nt = 64 * H;
-    p.n_tiles = (a.N + nt - 1) / nt;
+    p.n_tiles = (a.N + 64 * H - 1) / (64 * H);
     p.items = (long long)a.m_vec * a.batch * p.n_tiles;
-    if (p.items + slots > 0x7fffffffLL) {                  // the work counter, and CTAs (clusters only where items are few)
-        set_error("problem too large for 32-bit tile ids");
-        return cudaErrorInvalidValue;
-    }
+    return p;
+}
+// the work counter, and CTAs (clusters only where items are few)
+bool too_many(long long items, int sms) {
+    if (items + (long long)sms * kResident * kWarps <= 0x7fffffffLL) return false;
+    set_error("problem too large for 32-bit tile ids");
+    return true;
+}
+}  // namespace rows
+
+// scratch: null, or sspmm_rows_scratch_bytes() bytes (long rows are then cut); nvec < 0: unknown.
+cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    const bool split = scratch != nullptr;
+    const rows::Division d = rows::divide(&a, 1, nvec, sms);
+    const int H = split ? (a.N > 64 ? 2 : 1) : d.H;
+    rows::Problem p = rows::problem_of(a, H);
+    if (rows::too_many(p.items, sms)) return cudaErrorInvalidValue;
     if (split) {
         const rows::Scratch r = rows::plan_scratch(a, nvec);
         uint8_t* s = static_cast<uint8_t*>(scratch);
@@ -694,6 +742,23 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     if (a.V == 16)
         return a.out_f16 ? rows::launch_typed<16, __half>(a, p, H, split, d, sms) : rows::launch_typed<16, float>(a, p, H, split, d, sms);
     return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, split, d, sms) : rows::launch_typed<8, float>(a, p, H, split, d, sms);
+}
+
+cudaError_t launch_sspmm_rows_set(const SpmmArgs* a, int count, long long nvec) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    const rows::Division d = rows::divide(a, count, nvec, sms);
+    if (count > kRowsMaxSet || rows::too_many(rows::count_items(a, count, d.H), sms)) return cudaErrorInvalidValue;
+    rows::ProblemSet s;
+    s.count = count;
+    s.first[0] = 0;
+    for (int k = 0; k < count; ++k) {
+        s.p[k] = rows::problem_of(a[k], d.H);
+        s.out[k] = a[k].out;
+        s.first[k + 1] = s.first[k] + (int)s.p[k].items;
+    }
+    if (a->V == 16) return a->out_f16 ? rows::launch_set<16, __half>(s, d, a->stream) : rows::launch_set<16, float>(s, d, a->stream);
+    return a->out_f16 ? rows::launch_set<8, __half>(s, d, a->stream) : rows::launch_set<8, float>(s, d, a->stream);
 }
 
 // ---- dense operands whose rows do not start on 16-byte boundaries -------------------------------

@@ -164,3 +164,50 @@ def test_conv_layer_planned_wide(lib, N):
         ref = spmm_oracle.sspmm_host(V, ptr, col, vals, rhs, rows=rows, threads=8)
         assert_close(a_np[rows[0] * V: rows[1] * V], ref)
         assert_close(b_np[rows[0] * V: rows[1] * V], ref)
+
+
+@pytest.mark.parametrize("out_dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("shapes,rows", [
+    ([(24, 64, 8)], True), ([(256, 256, 128)] * 3, True), ([(256, 1024, 128)], True), ([(8, 100, 72), (1000, 300, 8), (64, 64, 200)], True),
+    ([(40, 130, 64)] * 8, True),                                                # as many products as one launch takes
+    ([(40, 130, 64)] * 9, False),
+    ([(128, 4608, 1000), (64, 576, 512)], False),                              # deep tiles are cut, shallow ones are not
+    ([(768, 3072, 1000)], False), ([(384, 2048, 2048)], False), ([(1024, 768, 4104)], False)])      # few wide tiles, many, copies of A
+def test_automatic_group(lib, shapes, rows, out_dtype):
+    """Automatic groups on both sides of the lines between the row-gather kernel, cut tiles, whole tiles and dense copies."""
+    rng = np.random.default_rng(len(shapes))
+    prods, refs = [], []
+    for (M, K, N) in shapes:
+        a = synthetic.magnitude_pruned(M, K, 0.8, rng)
+        ptr, col, vals = compress(a, 8)
+        rhs = rng.normal(0, 1, (K, N)).astype(np.float16)
+        d_ptr, d_col, d_val, d_rhs = dev(ptr, col, vals, rhs)
+        plan = ops.Plan(d_ptr, d_col, 8, K)
+        prods.append((plan, d_val, d_rhs, torch.full((plan.m_vec * 8, N), float("nan"), dtype=out_dtype, device=DEV)))
+        refs.append((spmm_oracle.sspmm_host(8, ptr, col, vals, rhs, threads=8)))
+    g = ops.Group(prods)
+    assert g.launches == 1 and (g.work_items == sum((p[0].m_vec * -(-p[2].shape[1] // 64)) for p in prods)) == rows
+    for _ in range(2):
+        for p in prods:
+            p[3].fill_(float("nan"))
+        g.run()
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        for p, ref in zip(prods, refs):
+            assert_close(p[3].float().cpu().numpy(), ref, fp32=out_dtype == torch.float32)
+
+
+def test_automatic_group_of_both_vector_lengths(lib):
+    rng = np.random.default_rng(3)
+    prods, refs = [], []
+    for V in (8, 16):
+        ptr, col, vals = compress(synthetic.magnitude_pruned(64, 200, 0.7, rng), V)
+        rhs = rng.normal(0, 1, (200, 72)).astype(np.float16)
+        d_ptr, d_col, d_val, d_rhs = dev(ptr, col, vals, rhs)
+        prods.append((ops.Plan(d_ptr, d_col, V, 200), d_val, d_rhs, torch.empty((64, 72), dtype=torch.float16, device=DEV)))
+        refs.append(spmm_oracle.sspmm_host(V, ptr, col, vals, rhs))
+    g = ops.Group(prods)
+    g.run()
+    g.run()
+    for p, ref in zip(prods, refs):
+        assert_close(p[3].float().cpu().numpy(), ref)
