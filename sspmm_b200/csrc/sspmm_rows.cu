@@ -198,10 +198,15 @@ struct Tile {
     // Adds steps first, first + stride, ... of vectors [j0, j0 + len).  The whole warp takes part; `mem` is its shared memory.
     __device__ __forceinline__ void accumulate(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs, int n0,
                                                int j0, int len, int first, int stride, int lane, uint32_t mem) {
+        accumulate(p, values, rhs, n0, j0, len, first, stride, lane, mem, load_cols(p.col, j0, len, first, stride, lane), [] {});
+    }
+    // cols: load_cols of the first two steps.  meanwhile() is called once, when the first steps are under way.
+    template <class F>
+    __device__ __forceinline__ void accumulate(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs, int n0,
+                                               int j0, int len, int first, int stride, int lane, uint32_t mem, int cols, F&& meanwhile) {
         const int steps = (int)(((unsigned)len + kStep - 1) / kStep);
-        if (first >= steps) return;
+        if (first >= steps) { meanwhile(); return; }
         const int mine = (steps - first + stride - 1) / stride;         // steps of this warp
-        int cols = load_cols(p.col, j0, len, first, stride, lane);
         int next = load_cols(p.col, j0, len, first + 2 * stride, stride, lane);
         int issued = 0;
         uint32_t fill = 0, use = 0;                                     // ring slots
@@ -218,6 +223,7 @@ struct Tile {
         };
 #pragma unroll
         for (int k = 0; k < kStages - 1; ++k) issue();
+        meanwhile();
         for (int k = 0; k < mine; ++k) {
             cp_async_wait<kStages - 2>();
             __syncwarp();                           // everyone's copies are in, and the slot refilled next has been read
@@ -396,6 +402,38 @@ __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int team, int cluster) {
     const int per_cta = kWarps / team, warp = threadIdx.x >> 5;
     do_item<V, OutT, H>(p, out, (long long)(blockIdx.x / cluster) * per_cta + warp / team, team, cluster);
+}
+
+// More items than warps, one warp each: every warp walks over its items, and looks up the columns of the next one and the place of
+// the one after that while the first steps of its item are under way.  (With a CTA for every eight items the look-ups, four
+// dependent loads, were paid for by every round of CTAs: 96 products of 512 x 512 at 90 %, N = 64, 12.6 us, now 10.6.)
+// Neighbouring items go to different SMs: rows are often ordered by length.
+template <typename OutT, int H>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_walk_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
+    constexpr int V = 8;
+    using T = Tile<V, H, sizeof(OutT) == 4>;
+    extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint8_t* const mem = smem + warp * T::kWarpBytes;
+    const long long stride = (long long)gridDim.x * kWarps;
+    long long item = (long long)warp * gridDim.x + blockIdx.x;
+    Where w = locate(p, item, T::NT);
+    int cols = T::load_cols(p.col, w.j0, w.len, 0, 1, lane);
+    Where w1 = locate(p, item + stride, T::NT);
+    for (; item < p.items; item += stride) {
+        Where w2;
+        int cols1;
+        T tile;
+        tile.clear();
+        tile.accumulate(p, p.values + w.batch * p.values_stride, p.rhs + w.batch * p.rhs_stride, w.n0, w.j0, w.len, 0, 1, lane, smem_u32(mem), cols,
+                        [&] {
+                            cols1 = T::load_cols(p.col, w1.j0, w1.len, 0, 1, lane);
+                            w2 = locate(p, item + 2 * stride, T::NT);
+                        });
+        if (w.row >= 0) tile.store(p, out + w.batch * p.out_stride, (int64_t)w.row * V, w.n0, reinterpret_cast<float*>(mem), lane);
+        w = w1; cols = cols1; w1 = w2;
+    }
 }
 
 // Several products in one launch: the items of one after those of the other.
@@ -601,7 +639,19 @@ cudaError_t launch_items(Kern kern, DeviceOnce& once, long long items, const Div
 }
 
 template <int V, typename OutT, int H>
-cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d) {
+cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d, int sms) {
+    // (vectors of 16 rows leave no registers for the look-ahead: 2048 x 512 at 98 %, N = 8192 46 us, walking 48)
+    if constexpr (V == 8) {
+        static DeviceOnce once_walk;
+        if (d.team == 1 && p.items > (long long)sms * kResident * kWarps) {
+            auto kern = sspmm_rows_walk_kernel<OutT, H>;
+            constexpr int kBytes = kWarps * Tile<V, H, sizeof(OutT) == 4>::kWarpBytes;
+            const cudaError_t e = allow_smem(kern, once_walk, kBytes);
+            if (e != cudaSuccess) return e;
+            kern<<<sms * kResident, kThreads, kBytes, a.stream>>>(p, static_cast<OutT*>(a.out));
+            return cudaGetLastError();
+        }
+    }
     static DeviceOnce once;
     return launch_items<V, OutT, H>(sspmm_rows_kernel<V, OutT, H>, once, p.items, d, a.stream, p, static_cast<OutT*>(a.out));
 }
@@ -635,7 +685,7 @@ cudaError_t launch_split(const SpmmArgs& a, const Problem& p, int sms) {
 template <int V, typename OutT>
 cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, bool split, const Division& d, int sms) {
     if (split) return H == 2 ? launch_split<V, OutT, 2>(a, p, sms) : launch_split<V, OutT, 1>(a, p, sms);
-    return H == 2 ? launch_plain<V, OutT, 2>(a, p, d) : launch_plain<V, OutT, 1>(a, p, d);
+    return H == 2 ? launch_plain<V, OutT, 2>(a, p, d, sms) : launch_plain<V, OutT, 1>(a, p, d, sms);
 }
 
 // Scratch of the variant that cuts rows: [16 B header][cap_cut * n_tiles arrival counters][cap_cut + cap_whole entries]
