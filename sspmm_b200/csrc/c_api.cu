@@ -494,7 +494,8 @@ int svc_finish(svc_job* j, int* d_vec_row_ptr, int* d_vec_col, void* d_vec_value
     if (e != cudaSuccess) return fail(e, "row pointer copy");
     if (j->nvec == 0) return 0;
     __half* ov = j->with_values ? static_cast<__half*>(d_vec_values_f16) : nullptr;
-    if (ov) {
+    j->p.zero_values = aligned16(ov);
+    if (ov && !j->p.zero_values) {
         e = cudaMemsetAsync(ov, 0, (size_t)j->nvec * j->p.V * sizeof(__half), st);
         if (e != cudaSuccess) return fail(e, "value clear");
     }
@@ -615,7 +616,8 @@ int svc_batch_finish(svc_batch_job* b, int* d_vec_row_ptr, int* d_vec_col, void*
     if (j->nvec == 0) return 0;
     if (!d_vec_col) { set_error("null pointer"); return (int)cudaErrorInvalidValue; }
     __half* ov = j->with_values ? static_cast<__half*>(d_vec_values_f16) : nullptr;
-    if (ov) {
+    j->p.zero_values = aligned16(ov);
+    if (ov && !j->p.zero_values) {
         e = cudaMemsetAsync(ov, 0, (size_t)j->nvec * j->p.V * sizeof(__half), st);
         if (e != cudaSuccess) return fail(e, "value clear");
     }

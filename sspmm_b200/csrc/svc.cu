@@ -234,13 +234,14 @@ struct BlockTeam {
 // Groups with many entries get a whole CTA, the others a warp: two launches of the same kernel,
 // each taking the groups that pass its filter (0 = all, 1 = at most kBigGroup entries, 2 = more).
 constexpr int kBigGroup = 1024;
+constexpr int kBigTeam = 1024;             // threads of such a CTA
 __device__ __forceinline__ bool group_passes(int filter, int entries) {
     return filter == 0 || (filter == 1) == (entries <= kBigGroup);
 }
 
 // ---------------------------------------------------------------- pass 1: count
 template <class Team>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock)
 svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, int* __restrict__ mode,
                  int* __restrict__ tbl_len) {
     extern __shared__ unsigned int sm_words[];
@@ -261,15 +262,21 @@ svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, 
         }
         Team::sync();
         int cnt = 0, mx = -1, bad = 0;
-        for (int e = e0 + tid; e < e1; e += Team::kSize) {
-            const int c = p.col_idx[e];
-            if ((unsigned)c < (unsigned)p.K) {
-                const unsigned bit = 1u << (c & 31);
-                const unsigned old = atomicOr(&bm[c >> 5], bit);
-                cnt += (old & bit) ? 0 : 1;
-                mx = max(mx, c);
-            } else {
-                bad = 1;
+        for (int e = e0 + tid; e < e1; e += 4 * Team::kSize) {             // four loads in flight
+            int c4[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) c4[b] = e + b * Team::kSize < e1 ? p.col_idx[e + b * Team::kSize] : -1;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int c = c4[b];
+                if ((unsigned)c < (unsigned)p.K) {
+                    const unsigned bit = 1u << (c & 31);
+                    const unsigned old = atomicOr(&bm[c >> 5], bit);
+                    cnt += (old & bit) ? 0 : 1;
+                    mx = max(mx, c);
+                } else if (e + b * Team::kSize < e1) {
+                    bad = 1;
+                }
             }
         }
         cnt = Team::sum(cnt, red);
@@ -454,30 +461,74 @@ svc_scan_place_kernel(int m_vec, int* __restrict__ vec_ptr, const int* __restric
 }
 
 // ---------------------------------------------------------------- pass 2a: ascending order
+// Zeroes the value vectors of a group; the team's barrier before the values are put in.
 template <class Team>
-__global__ void __launch_bounds__(256)
+__device__ __forceinline__ void zero_values(__half* out_vals, int64_t base, int n, int V) {
+    uint4* dst = reinterpret_cast<uint4*>(out_vals + base * V);
+    for (int x = Team::tid(); x < n * (V / 8); x += Team::kSize) dst[x] = make_uint4(0, 0, 0, 0);
+}
+// Row ends of a group in shared memory: rows[0 .. n_rows].
+constexpr int kRowInts = 20;
+// The matrix row (inside the group) of entry e.
+__device__ __forceinline__ int row_of_entry(const int* rows, int n_rows, int e) {
+    int r = 0;
+#pragma unroll
+    for (int step = 8; step > 0; step >>= 1)
+        if (r + step < n_rows && e >= rows[r + step]) r += step;
+    return r;
+}
+// Calls f(row, column, value) for the group's entries, four in flight per thread.
+template <class Team, class F>
+__device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* rows, int n_rows, F&& f) {
+    const int e1 = rows[n_rows];
+    for (int e = rows[0] + Team::tid(); e < e1; e += 4 * Team::kSize) {
+        int c[4];
+        __half v[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int x = e + b * Team::kSize;
+            c[b] = x < e1 ? p.col_idx[x] : -1;
+            v[b] = x < e1 ? p.vals[x] : __half(0);
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if ((unsigned)c[b] < (unsigned)p.K) f(row_of_entry(rows, n_rows, e + b * Team::kSize), c[b], v[b]);
+    }
+}
+
+// Bound by the latency of its look-ups, so the large groups get 1024 threads and every thread four entries at a time (conv weight of
+// 512 x 4608, 64 groups: 14.7 us with 256 threads and an entry each, 10.6 now, zeroing included).
+template <class Team>
+__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock)
 svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restrict__ vec_ptr,
                        const int* __restrict__ mode, int* __restrict__ out_col, __half* __restrict__ out_vals,
                        const int* __restrict__ list, int n_list) {
     extern __shared__ unsigned int sm_words[];
-    __shared__ int red[33];
+    __shared__ int red[33], all_rows[Team::kPerBlock * kRowInts];
     unsigned int* bm = sm_words + (size_t)Team::index_in_block() * words * 2;
     unsigned int* pre = bm + words;
-    const int tid = Team::tid();
+    int* const rows = all_rows + Team::index_in_block() * kRowInts;
+    const int tid = Team::tid(), lane = tid & 31;
     // with a list: only the groups it names; else every group
     const int n_loop = list ? n_list : p.m_vec;
     for (int k = blockIdx.x * Team::kPerBlock + Team::index_in_block(); k < n_loop; k += gridDim.x * Team::kPerBlock) {
         const int i = list ? list[k] : k;
         if (mode[i] != 0) continue;
-        const int r0 = min(i * p.V, p.M), r1 = min(i * p.V + p.V, p.M);
-        const int e0 = p.row_ptr[r0], e1 = p.row_ptr[r1];
+        const int r0 = min(i * p.V, p.M), n_rows = min(i * p.V + p.V, p.M) - r0;
+        const int e0 = p.row_ptr[r0], e1 = p.row_ptr[r0 + n_rows];
         const int base = vec_ptr[i];
         if (e1 == e0 || !group_passes(filter, e1 - e0)) continue;
+        if (tid <= n_rows) rows[tid] = p.row_ptr[r0 + tid];
         for (int w = tid; w < words; w += Team::kSize) bm[w] = 0u;
+        if (out_vals && p.zero_values) zero_values<Team>(out_vals, base, vec_ptr[i + 1] - base, p.V);
         Team::sync();
-        for (int e = e0 + tid; e < e1; e += Team::kSize) {
-            const int c = p.col_idx[e];
-            if ((unsigned)c < (unsigned)p.K) atomicOr(&bm[c >> 5], 1u << (c & 31));
+        for (int e = e0 + tid; e < e1; e += 4 * Team::kSize) {
+            int c[4];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) c[b] = e + b * Team::kSize < e1 ? p.col_idx[e + b * Team::kSize] : -1;
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if ((unsigned)c[b] < (unsigned)p.K) atomicOr(&bm[c[b] >> 5], 1u << (c[b] & 31));
         }
         Team::sync();
         // columns by a lane per bit when the words are well filled (a thread per word would write up to 32 of them in turn)
@@ -488,23 +539,13 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
             unsigned word = (w < words) ? bm[w] : 0u;
             const int pc = __popc(word);
             // exclusive prefix of pc over the team, in thread order
-            int incl = warp_incl_scan(pc, tid & 31);
+            int incl = warp_incl_scan(pc, lane);
             int chunk_total;
             if constexpr (Team::kSize == 32) {
                 chunk_total = __shfl_sync(0xffffffffu, incl, 31);
             } else {
-                const int wp = tid >> 5;
-                if ((tid & 31) == 31) red[wp] = incl;
-                __syncthreads();
-                int before = 0, all = 0;
-                for (int x = 0; x < Team::kSize / 32; ++x) {
-                    const int c = red[x];
-                    if (x < wp) before += c;
-                    all += c;
-                }
-                __syncthreads();
-                incl += before;
-                chunk_total = all;
+                incl += Team::before(__shfl_sync(0xffffffffu, incl, 31), chunk_total, red);
+                Team::sync();
             }
             int o = running + incl - pc;
             if (w < words) pre[w] = (unsigned)o;
@@ -516,56 +557,19 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
             }
             running += chunk_total;
         }
+        Team::sync();
         if (by_bit) {
-            Team::sync();
-            const int lane = tid & 31;
 #pragma unroll 4
             for (int w = tid >> 5; w < words; w += Team::kSize / 32) {
                 const unsigned word = bm[w];
                 if ((word >> lane) & 1u) out_col[base + (int)pre[w] + __popc(word & ((1u << lane) - 1u))] = w * 32 + lane;
             }
         }
-        if (out_vals) {
-            Team::sync();
-            int longest = 0;
-            if (Team::kSize >= 256)
-                for (int r = r0; r < r1; ++r) longest = max(longest, p.row_ptr[r + 1] - p.row_ptr[r]);
-            if (Team::kSize >= 256 && longest <= (e1 - e0) / 4 + 128) {
-                // a warp per matrix row: no search for the row of an entry, and four entries' look-ups in flight (rows of
-                // a power-law group differ too much for it: one warp would do nearly all of them)
-                const int lane = tid & 31;
-                for (int r = r0 + (tid >> 5); r < r1; r += Team::kSize / 32) {
-                    const int a0 = p.row_ptr[r], a1 = p.row_ptr[r + 1];
-                    __half* const col0 = out_vals + (int64_t)base * p.V + (r - i * p.V);
-                    for (int e = a0 + lane; e < a1; e += 128) {
-                        int c[4];
-                        __half v[4];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            c[k] = e + 32 * k < a1 ? p.col_idx[e + 32 * k] : -1;
-                            v[k] = e + 32 * k < a1 ? p.vals[e + 32 * k] : __half(0);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if ((unsigned)c[k] < (unsigned)p.K) {
-                                const int pos = (int)pre[c[k] >> 5] + __popc(bm[c[k] >> 5] & ((1u << (c[k] & 31)) - 1u));
-                                col0[(int64_t)pos * p.V] = v[k];
-                            }
-                    }
-                }
-            } else {
-            // all entries of the group, flat; the matrix row of entry e is found by walking the (at most V) row ends
-            for (int e = e0 + tid; e < e1; e += Team::kSize) {
-                int r = r0;
-                while (r + 1 < r1 && e >= p.row_ptr[r + 1]) ++r;
-                const int c = p.col_idx[e];
-                if ((unsigned)c < (unsigned)p.K) {
-                    const int pos = (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
-                    out_vals[((int64_t)base + pos) * p.V + (r - i * p.V)] = p.vals[e];
-                }
-            }
-            }
-        }
+        if (out_vals)
+            for_each_value<Team>(p, rows, n_rows, [&](int r, int c, __half v) {
+                const int pos = (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
+                out_vals[((int64_t)base + pos) * p.V + r] = v;
+            });
         Team::sync();
     }
 }
@@ -952,6 +956,7 @@ __device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, i
     const int r0 = min(i * p.V, p.M), n_rows = min(i * p.V + p.V, p.M) - r0;
     if (tid <= n_rows) rows[tid] = p.row_ptr[r0 + tid];
     for (int s = tid * 4; s < (int)(kKeep ? Set::start(cap) : 0u) + cap; s += Team::kSize * 4) t.tab.free4(s);
+    if (out_vals && p.zero_values) zero_values<Team>(out_vals, base, u_final, p.V);
     Team::sync();
     // a warp team does all levels in one table
     auto table = [&](int size) { return kKeep ? t.level(size) : t; };
@@ -1027,27 +1032,18 @@ __device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, i
     // the list is the ordered set, the words of the table name positions in it
     const Set held = table(size);
     for (int q = tid; q < n_cur; q += Team::kSize) out_col[base + q] = (int)t.list.ld(q);
-    if (out_vals) {
-        const int e0 = rows[0], e1 = rows[n_rows];
-        for (int e = e0 + tid; e < e1; e += Team::kSize) {
-            const unsigned c = (unsigned)p.col_idx[e];
-            int r = 0;                                       // the row of entry e
-#pragma unroll
-            for (int step = 8; step > 0; step >>= 1)
-                if (r + step < n_rows && e >= rows[r + step]) r += step;
-            if (c >= (unsigned)p.K) continue;
+    if (out_vals)
+        for_each_value<Team>(p, rows, n_rows, [&](int r, int c, __half v) {
             unsigned w;
-            held.find((unsigned)size - 1u, c, w);
-            if (w != kFree) out_vals[((int64_t)base + Set::number_of(w)) * p.V + r] = p.vals[e];
-        }
-    }
+            held.find((unsigned)size - 1u, (unsigned)c, w);
+            if (w != kFree) out_vals[((int64_t)base + Set::number_of(w)) * p.V + r] = v;
+        });
     Team::sync();
 }
 
 // What a team of a class has in shared memory: its tables, a list and the row ends of its group.  Class L with a table per level
 // leaves no room for the list, and class XL has everything, in global scratch.
 // SHIFT: bits of a column in a word; numbers of a list and two more fit the others (0: unpacked).
-constexpr int kRowInts = 20;
 template <int CLASS, int SHIFT>
 struct ClassShape {
     static constexpr int kTeam = CLASS == kClassM1 ? 256 : CLASS == kClassM2 ? 512 : CLASS == kClassL || CLASS == kClassXL ? 1024 : 32;
@@ -1191,14 +1187,14 @@ cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool /*
         const int words = (p.K + 31) / 32;
         const int sms = device_sm_count();
         static DeviceOnce once_block, once_warp;
-        cudaError_t e = allow_big_smem(svc_count_kernel<BlockTeam<256>>, once_block, 200 * 1024);
+        cudaError_t e = allow_big_smem(svc_count_kernel<BlockTeam<kBigTeam>>, once_block, 200 * 1024);
         if (e == cudaSuccess) e = allow_big_smem(svc_count_kernel<WarpTeam>, once_warp, 200 * 1024);
         if (e != cudaSuccess) return e;
         const size_t warp_smem = (size_t)WarpTeam::kPerBlock * words * 4;
         if (p.m_vec <= 16 * sms || warp_smem > 200 * 1024) {
             // few groups (or bitmaps too large for eight per block): one CTA per group
             const int grid = p.m_vec < sms * 16 ? p.m_vec : sms * 16;
-            svc_count_kernel<BlockTeam<256>><<<grid, 256, (size_t)words * 4, stream>>>(p, words, 0, s.vec_ptr, s.mode, s.tbl_len);
+            svc_count_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 4, stream>>>(p, words, 0, s.vec_ptr, s.mode, s.tbl_len);
             e = cudaGetLastError();
         } else {
             std::lock_guard<std::mutex> lk(g_aux_mu);
@@ -1206,7 +1202,7 @@ cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool /*
             int grid = (p.m_vec + WarpTeam::kPerBlock - 1) / WarpTeam::kPerBlock;
             if (grid > sms * 8) grid = sms * 8;
             svc_count_kernel<WarpTeam><<<grid, 256, warp_smem, f.next()>>>(p, words, 1, s.vec_ptr, s.mode, s.tbl_len);
-            svc_count_kernel<BlockTeam<256>><<<sms * 4, 256, (size_t)words * 4, f.next()>>>(p, words, 2, s.vec_ptr, s.mode, s.tbl_len);
+            svc_count_kernel<BlockTeam<kBigTeam>><<<sms * 2, kBigTeam, (size_t)words * 4, f.next()>>>(p, words, 2, s.vec_ptr, s.mode, s.tbl_len);
             e = cudaGetLastError();
             if (e == cudaSuccess) e = f.join();
         }
@@ -1230,7 +1226,7 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
     const int sms = device_sm_count();
     const int words = (p.K + 31) / 32;
     static DeviceOnce once_block, once_warp;
-    cudaError_t e = allow_big_smem(svc_emit_sorted_kernel<BlockTeam<256>>, once_block, 208 * 1024);
+    cudaError_t e = allow_big_smem(svc_emit_sorted_kernel<BlockTeam<kBigTeam>>, once_block, 208 * 1024);
     if (e == cudaSuccess) e = allow_big_smem(svc_emit_sorted_kernel<WarpTeam>, once_warp, 208 * 1024);
     if (e != cudaSuccess) return e;
 
@@ -1256,7 +1252,7 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
         const size_t warp_smem = (size_t)WarpTeam::kPerBlock * words * 8;
         if (p.m_vec <= 16 * sms || warp_smem > 200 * 1024) {
             const int grid = p.m_vec < sms * 16 ? p.m_vec : sms * 16;
-            svc_emit_sorted_kernel<BlockTeam<256>><<<grid, 256, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals,
+            svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals,
                                                                                              nullptr, 0);
         } else {
             int grid = (p.m_vec + WarpTeam::kPerBlock - 1) / WarpTeam::kPerBlock;
@@ -1264,7 +1260,7 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
             svc_emit_sorted_kernel<WarpTeam><<<grid, 256, warp_smem, stream>>>(p, words, 1, s.vec_ptr, s.mode, out_col, out_vals, nullptr, 0);
             if (n_big > 0) {
                 const int big_grid = n_big < sms * 2 ? n_big : sms * 2;
-                svc_emit_sorted_kernel<BlockTeam<256>><<<big_grid, 256, (size_t)words * 8, f.next()>>>(p, words, 2, s.vec_ptr, s.mode, out_col,
+                svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<big_grid, kBigTeam, (size_t)words * 8, f.next()>>>(p, words, 2, s.vec_ptr, s.mode, out_col,
                                                                                                      out_vals, big_list, n_big);
             }
         }

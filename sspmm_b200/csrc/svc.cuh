@@ -20,6 +20,7 @@ struct SvcProblem {
     const int* row_ptr;   // [M+1]
     const int* col_idx;   // [nnz]
     const __half* vals;   // [nnz] or null
+    bool zero_values;     // pass 2: every group zeroes its own value vectors (which then start on 16-byte boundaries)
 };
 
 // Scratch owned by one compression.  Sizes in elements.
@@ -45,7 +46,7 @@ constexpr int kSvcScanFields = 2 + kSvcSegs;   // numbers per block of the scans
 
 // Pass 1: per-group distinct counts, mode decision, scans.  Asynchronous on `stream`.
 cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool with_values, cudaStream_t stream);
-// Pass 2: emits column lists (and value vectors when out_vals != null; out_vals must be zero-filled).
+// Pass 2: emits column lists (and value vectors when out_vals != null, which must be zero-filled unless p.zero_values).
 // seg_groups = totals[2..2+kSvcSegs) read back by the host (launches are skipped for empty classes).
 cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* seg_groups, int* out_col,
                      __half* out_vals, cudaStream_t stream);

@@ -262,3 +262,20 @@ def test_replay_of_rows_that_repeat_columns(lib, K, big):
     for repeat in (1, 5):
         check_against_oracle(_one_group(K, [4, big, 3, 0, 6, 1, 2, 9], K + repeat, repeat=repeat), 8)
         check_against_oracle(_one_group(K, [4, 9, 3, big, 6], K + repeat, repeat=repeat), 8)
+
+
+def test_value_vectors_off_their_boundary(lib):
+    """The caller's value array need not start on a 16-byte boundary; nothing before or after it is written."""
+    import ctypes as C
+    a = _one_group(9000, [4, 2000, 3, 0, 60, 1, 2, 9] * 3, 5)
+    dev = torch.device("cuda:0")
+    d = [torch.from_numpy(x).to(dev) for x in (a.row_ptr, a.col_idx, a.values)]
+    want = ops.svc(*d, a.M, a.K, 8)
+    job, nvec, st = C.c_void_p(), C.c_int64(), torch.cuda.current_stream().cuda_stream
+    assert lib.svc_begin(a.M, a.K, 8, d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), st, C.byref(job), C.byref(nvec)) == 0
+    ptr, col = torch.empty(4, dtype=torch.int32, device=dev), torch.empty(nvec.value, dtype=torch.int32, device=dev)
+    room = torch.full((nvec.value * 8 + 16,), 7.0, dtype=torch.float16, device=dev)
+    assert lib.svc_finish(job, ptr.data_ptr(), col.data_ptr(), room.data_ptr() + 6, st) == 0
+    lib.svc_free(job)
+    assert torch.equal(ptr, want[0]) and torch.equal(col, want[1]) and torch.equal(room[3: 3 + want[2].numel()], want[2])
+    assert (room[:3] == 7).all() and (room[3 + want[2].numel():] == 7).all()
