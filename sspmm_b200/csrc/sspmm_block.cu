@@ -40,22 +40,24 @@ std::atomic<bool> g_block_pairs{true};
 
 // ---- expansion of the compressed operand ------------------------------------
 // At[k][i*V .. i*V+V) = values of the vector of row i at column k, or zeros.
-// One CTA per (vector row i, chunk of kExpandChunk columns): the row's column
+// One CTA per (vector row i, chunk of columns): the row's column
 // list is turned into a column -> vector map in shared memory, then every
 // column of the chunk is written (value vector or zeros), so no separate zero
-// fill of At is needed.
-constexpr int kExpandChunk = 1024;
+// fill of At is needed.  Bound by its chain of look-ups, and every CTA reads its
+// row's whole list, so chunks are as long as leaves every SM two CTAs (768 x 768,
+// V = 16: 6.3 us in 48 CTAs, 5.1 in 144).
+constexpr int kExpandChunk = 1024;           // longest
 
 template <int V>
 __global__ void __launch_bounds__(256)
-expand_transposed_kernel(int m_vec, int K, const int* __restrict__ row_offsets, const int* __restrict__ col,
+expand_transposed_kernel(int m_vec, int K, int chunk, const int* __restrict__ row_offsets, const int* __restrict__ col,
                          const __half* __restrict__ values, __half* __restrict__ at) {
     __shared__ int slot[kExpandChunk];
     const int64_t mp = (int64_t)m_vec * V;
-    const int k_begin = blockIdx.x * kExpandChunk;
-    const int k_end = min(K, k_begin + kExpandChunk);
+    const int k_begin = blockIdx.x * chunk;
+    const int k_end = min(K, k_begin + chunk);
     for (int i = blockIdx.y; i < m_vec; i += gridDim.y) {
-        for (int k = threadIdx.x; k < kExpandChunk; k += blockDim.x) slot[k] = -1;
+        for (int k = threadIdx.x; k < chunk; k += blockDim.x) slot[k] = -1;
         __syncthreads();
         const int j0 = row_offsets[i], j1 = row_offsets[i + 1];
         // four independent loads in flight per thread: the kernel is a chain of dependent reads otherwise
@@ -824,9 +826,11 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     if (e != cudaSuccess) return e;
     {
         const int by = a.m_vec < 32768 ? a.m_vec : 32768;
-        const dim3 grid((a.K + kExpandChunk - 1) / kExpandChunk, by);
-        if (a.V == 16) expand_transposed_kernel<16><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, a.row_offsets, a.column_indices, a.values, at);
-        else expand_transposed_kernel<8><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, a.row_offsets, a.column_indices, a.values, at);
+        int chunk = kExpandChunk;
+        while (chunk > 256 && (int64_t)by * ((a.K + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
+        const dim3 grid((a.K + chunk - 1) / chunk, by);
+        if (a.V == 16) expand_transposed_kernel<16><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, a.row_offsets, a.column_indices, a.values, at);
+        else expand_transposed_kernel<8><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, a.row_offsets, a.column_indices, a.values, at);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -203,3 +203,35 @@ def test_layer_norm_wide_tile_with_most_features(lib):
     d = x.double()
     ref = (d - d.mean(0)) / torch.sqrt(d.var(0, unbiased=False) + 1e-5) * w.double()[:, None] + b.double()[:, None]
     assert ((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -19 * (1 + w.double().abs()[:, None] * 4)).all()
+
+
+def test_stacked_linears_follow_their_tensors(lib):
+    """Q, K and V as one product: values and biases changed in place count, and so do tensors put in their place."""
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=128, ffn=512, heads=2, sparsity=0.9, vec_length=16)
+    x = torch.randn(128, 144, device="cuda:0", dtype=torch.float16)
+    L = layer.linears[:3]
+
+    def check(taken):
+        got = layer.qkv(L, x)
+        assert (got is not None) == taken
+        for y, l in zip(got or [], L):
+            assert (y.double() - l(x).double()).norm() <= 2 * 2.0 ** -11 * y.double().norm() and y.is_contiguous()
+        y = layer.forward(x, 2, 72)
+        qkv, layer.qkv = layer.qkv, None
+        want = layer.forward(x, 2, 72)
+        layer.qkv = qkv
+        assert (y.double() - want.double()).norm() <= 12 * 2.0 ** -11 * want.double().norm()
+    check(True)
+    L[1].values.mul_(2.0)
+    L[2].bias.add_(1.0)
+    check(True)
+    L[0].bias = L[0].bias + 1.0
+    check(False)
+    L[0].bias = layer.qkv.bias[:128]
+    check(True)
+    L[2].values = L[2].values * 0.5
+    check(False)
+    L[2].values = layer.qkv.values[-L[2].values.numel():]
+    L[1].bias.requires_grad_()
+    check(False)
