@@ -1,6 +1,7 @@
 // The parts of an encoder layer between its products, on feature-major activations x[features][tokens] (the layout the
 // SpMM reads and writes): LayerNorm with the residual sum before it, and softmax attention.  The reference runs both as
 // framework operations (end2end/sspmm_e2e/end_to_end.py:44-75).
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -210,7 +211,7 @@ __device__ __forceinline__ void attend(int seq, int64_t tokens, int64_t base, in
     const int rounds = (seq + kTile - 1) / kTile;
     for (int it = 0; it < rounds; ++it) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                                            // this round's tiles are in, the other buffer is free
+        named_barrier_sync(1, kAttnThreads);                        // this round's tiles are in, the other buffer is free
         if (it + 1 < rounds) {
             const uint32_t next = s_kv + ((it + 1) & 1) * 2 * kTileBytes;
             load(next, k, (it + 1) * kTile);
@@ -321,24 +322,10 @@ __device__ __forceinline__ void attend(int seq, int64_t tokens, int64_t base, in
     }
 }
 
-__global__ void __launch_bounds__(kAttnThreads, 4)
-attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
-                    const __half* __restrict__ bias_q, const __half* __restrict__ bias_v, __half* __restrict__ out) {
-    __shared__ __align__(128) uint8_t smem[5 * kTileBytes];         // q (later the output), two buffers of k and v
+// The warp's 16 columns of the output tile [feature][query] take the place of its queries, and go out.
+__device__ __forceinline__ void store_queries(int seq, int64_t tokens, int64_t base, int q0, int head, const __half* __restrict__ bias_v,
+                                              uint8_t* smem, const float (&o)[8][4], const float (&inv)[2], __half* __restrict__ out) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int q0 = blockIdx.x * kTile, head = blockIdx.y;
-    const int64_t base = (int64_t)head * kHd * tokens + (int64_t)blockIdx.z * seq;
-    if (bias_q) bias_q += head * kHd;
-    float o[8][4], inv[2];
-    attend<false>(seq, tokens, base, q0, q, k, v, bias_q, smem_u32(smem), o, inv);
-    bool nan = false;
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) nan |= isnan(o[n][e]);
-    // something infinite or NaN went in (the barrier also frees the buffers)
-    if (__syncthreads_or(nan)) attend<true>(seq, tokens, base, q0, q, k, v, bias_q, smem_u32(smem), o, inv);
-    // the warp's 16 columns of the output tile [feature][query] take the place of its queries
     __half* tile = reinterpret_cast<__half*>(smem);
     __syncwarp();
 #pragma unroll
@@ -356,6 +343,296 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
         if (s < seq)
             *reinterpret_cast<uint4*>(out + base + (int64_t)row * tokens + s) = *reinterpret_cast<const uint4*>(tile + row * 64 + ((piece ^ (row & 7)) << 3));
     }
+}
+
+__global__ void __launch_bounds__(kAttnThreads, 4)
+attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
+                    const __half* __restrict__ bias_q, const __half* __restrict__ bias_v, __half* __restrict__ out) {
+    __shared__ __align__(128) uint8_t smem[5 * kTileBytes];         // q (later the output), two buffers of k and v
+    const int q0 = blockIdx.x * kTile, head = blockIdx.y;
+    const int64_t base = (int64_t)head * kHd * tokens + (int64_t)blockIdx.z * seq;
+    if (bias_q) bias_q += head * kHd;
+    float o[8][4], inv[2];
+    attend<false>(seq, tokens, base, q0, q, k, v, bias_q, smem_u32(smem), o, inv);
+    bool nan = false;
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) nan |= isnan(o[n][e]);
+    // something infinite or NaN went in (the barrier also frees the buffers)
+    if (__syncthreads_or(nan)) attend<true>(seq, tokens, base, q0, q, k, v, bias_q, smem_u32(smem), o, inv);
+    store_queries(seq, tokens, base, q0, head, bias_v, smem, o, inv, out);
+}
+
+// ---- attention on tcgen05 ---------------------------------------------------------------------------
+// One CTA: 128 queries of one head of one sequence.  Four warps hold a query per thread: they read its 64 scores of a block of keys
+// from tensor memory, keep the running maximum, sum and output in registers and put the probabilities (two fp16 numbers
+// each) back in place of the scores; a fifth warp requests tiles by TMA and issues the products.  Keys and values pass through
+// three stages of 64 tokens; scores and partial outputs have two buffers each in tensor memory, so the scores of the
+// next block are computed while this block's probabilities are, and a partial output is taken one block later.
+// The arithmetic is attend's: blocks of 64 keys, sums of a block from zero, joined in round-to-nearest.
+// Bound by the softmax warps: about ten instructions per score, and the waits between them and the products, which two CTAs per SM
+// do not fill.  12 heads, 32 x 512 tokens: 85 us (attention_fm_kernel 146); 16 x 512 45 (79), 1 x 2048 47 (86).  Distance from 64
+// bits as there: 2.075754e-4 against 2.075754e-4 (scores of size 1) and 2.073792e-4 against 2.073791e-4 (size 5), of which rounding the
+// result is 2.075753e-4 and 2.073788e-4.  A CTA that walks over tiles with the next one's operands on their way takes 96 us.
+constexpr int kTcQueries = 128, kTcStages = 3, kTcThreads = 160;
+struct TcSmem {
+    static constexpr int kQ = 0;                                     // two chunks of [64 features][64 queries]
+    static constexpr int kKv = 2 * kTileBytes;                       // [stage][k, v][64 features][64 keys]
+    static constexpr int kBar = kKv + kTcStages * 2 * kTileBytes;
+    static constexpr int kBars = kTcStages + 1 + 8;
+    static constexpr int kTmem = kBar + kBars * 8;
+    static constexpr int kAbort = kTmem + 8;
+    static constexpr int kBytes = kAbort + 8;
+    static constexpr int kDynamic = kBytes + 1024;
+    static_assert(5 * kTileBytes <= kBar, "attend's tiles fit in place of the stages");
+};
+constexpr uint32_t kTcTmemCols = 256;                                // scores / probabilities 2 x 64, partial outputs 2 x 64
+
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__global__ void __launch_bounds__(kTcThreads, 2)
+attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                    const __grid_constant__ CUtensorMap tmap_v, const __half* __restrict__ q, const __half* __restrict__ k,
+                    const __half* __restrict__ v, const __half* __restrict__ bias_q, const __half* __restrict__ bias_v,
+                    __half* __restrict__ out) {
+    using L = TcSmem;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const uint32_t sbase = smem_u32(smem);
+    const uint32_t bar_kv_full = sbase + L::kBar, bar_q = bar_kv_full + 8 * kTcStages;
+    const uint32_t bar_s_full = bar_q + 8, bar_p_full = bar_s_full + 16, bar_o_full = bar_p_full + 16, bar_o_free = bar_o_full + 16;
+    volatile uint32_t* tmem_at = reinterpret_cast<volatile uint32_t*>(smem + L::kTmem);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kAbort);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q0 = blockIdx.x * kTcQueries, head = blockIdx.y, b = blockIdx.z;
+    const int rounds = (seq + kTile - 1) / kTile;
+    auto tile = [&](int stage, int which) { return sbase + L::kKv + (stage * 2 + which) * kTileBytes; };
+    int loaded = 0;
+    auto request = [&]() {                                           // the next block's tiles; their stage is free
+        const int s = loaded % kTcStages;
+        mbar_arrive_expect_tx(bar_kv_full + 8 * s, 2 * kTileBytes);
+        tma_load_3d(tile(s, 0), &tmap_k, loaded * kTile, head * kHd, b, bar_kv_full + 8 * s);
+        tma_load_3d(tile(s, 1), &tmap_v, loaded * kTile, head * kHd, b, bar_kv_full + 8 * s);
+        ++loaded;
+    };
+
+    if (warp == 4) {
+        if (lane == 0) {
+            for (int s = 0; s < kTcStages; ++s) mbar_init(bar_kv_full + 8 * s, 1);
+            mbar_init(bar_q, 1);
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(bar_s_full + 8 * i, 1);
+                mbar_init(bar_p_full + 8 * i, 4);
+                mbar_init(bar_o_full + 8 * i, 1);
+                mbar_init(bar_o_free + 8 * i, 4);
+            }
+            *abort_flag = 0;
+            mbar_fence_init();
+            // on their way while the others start
+            mbar_arrive_expect_tx(bar_q, 2 * kTileBytes);
+            tma_load_3d(sbase + L::kQ, &tmap_q, q0, head * kHd, b, bar_q);
+            tma_load_3d(sbase + L::kQ + kTileBytes, &tmap_q, q0 + 64, head * kHd, b, bar_q);
+            while (loaded < min(rounds, kTcStages)) request();
+        }
+        __syncwarp();
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_at)), kTcTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = *tmem_at;
+
+    bool nan = false;
+    if (warp == 4) {
+        if (lane == 0) {
+            // queries are in when the softmax warps say so (they add the bias first): their arrival is the first phase of o_free[0]
+            bool ok = mbar_wait(bar_o_free, 0, abort_flag, kStatusWaitAttention);
+            constexpr uint32_t idesc_s = make_idesc_f16_f32(kTcQueries, kTile, true, true);
+            constexpr uint32_t idesc_o = make_idesc_f16_f32(kTcQueries, kHd, false, false);
+            auto scores = [&](int it) -> bool {
+                const int s = it % kTcStages;
+                if (!mbar_wait(bar_kv_full + 8 * s, (it / kTcStages) & 1, abort_flag, kStatusWaitAttention)) return false;
+                tc_fence_after_sync();
+                for (int kk = 0; kk < 4; ++kk)
+                    tc_mma_f16(tmem + (it & 1) * kTile, make_smem_desc(sbase + L::kQ + kk * 2048, kTileBytes, 1024, 2),
+                               make_smem_desc(tile(s, 0) + kk * 2048, kTileBytes, 1024, 2), idesc_s, kk > 0 ? 1u : 0u);
+                tc_commit(bar_s_full + 8 * (it & 1));
+                return true;
+            };
+            ok = ok && scores(0);
+            for (int it = 0; ok && it < rounds; ++it) {
+                const int buf = it & 1, s = it % kTcStages;
+                if (it > 0) {
+                    // the block before is done: its stage is free, and so is the buffer that the next scores go to
+                    if (!mbar_wait(bar_o_full + 8 * (buf ^ 1), ((it - 1) >> 1) & 1, abort_flag, kStatusWaitAttention)) break;
+                    tc_fence_after_sync();
+                    if (loaded < rounds) request();
+                }
+                if (it + 1 < rounds && !scores(it + 1)) break;
+                if (!mbar_wait(bar_p_full + 8 * buf, (it >> 1) & 1, abort_flag, kStatusWaitAttention)) break;
+                // the partial output two blocks ago has been taken (buffer 0 is one phase ahead, see above)
+                if (it >= 2 && !mbar_wait(bar_o_free + 8 * buf, (((it - 2) >> 1) + (buf == 0 ? 1 : 0)) & 1, abort_flag, kStatusWaitAttention)) break;
+                tc_fence_after_sync();
+                const uint32_t p = tmem + buf * kTile, o = tmem + 2 * kTile + buf * kHd;
+                for (int part = 0; part < 2; ++part)                // low halves first
+                    for (int kk = 0; kk < 4; ++kk)
+                        tc_mma_f16_ts(o, p + (part == 0 ? 32 : 0) + kk * 8, make_smem_desc(tile(s, 1) + kk * 32, 16, 1024, 2), idesc_o,
+                                      part + kk > 0 ? 1u : 0u);
+                tc_commit(bar_o_full + 8 * buf);
+            }
+        }
+    } else {
+        const int row = threadIdx.x;                                // query of the tile
+        const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+        constexpr float kScale = 0.125f * 1.44269504088896340736f;
+        constexpr float kLift = 10.f;
+        bool ok = mbar_wait(bar_q, 0, abort_flag, kStatusWaitAttention);
+        if (ok && bias_q) {
+            for (int x = threadIdx.x; x < kHd * 16; x += 128) {     // 64 features x 16 pieces of eight queries
+                const int f = x >> 4, piece = x & 15;
+                uint4* at16 = reinterpret_cast<uint4*>(smem + L::kQ + (piece >> 3) * kTileBytes + f * 128 + (((piece & 7) ^ (f & 7)) << 4));
+                uint4 w = *at16;
+                const __half2 bb = __half2half2(bias_q[head * kHd + f]);
+                uint32_t* h = reinterpret_cast<uint32_t*>(&w);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const __half2 sum = __hadd2(*reinterpret_cast<const __half2*>(&h[e]), bb);
+                    h[e] = *reinterpret_cast<const uint32_t*>(&sum);
+                }
+                *at16 = w;
+            }
+            fence_proxy_async_smem();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_o_free);
+        float o[kHd], m = -INFINITY, l[4] = {0.f, 0.f, 0.f, 0.f}, keep = 1.f;
+#pragma unroll
+        for (int f = 0; f < kHd; ++f) o[f] = 0.f;
+        // adds the partial output of block it: o = o * factor + partial
+        auto join = [&](int it, float factor) -> bool {
+            const int buf = it & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_o_full + 8 * buf, (it >> 1) & 1, abort_flag, kStatusWaitAttention))) return false;
+            tc_fence_after_sync();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t d[32];
+                tmem_ld_x32(tmem + lanes + 2 * kTile + buf * kHd + h * 32, d);
+                tc_wait_ld();
+#pragma unroll
+                for (int f = 0; f < 32; ++f) o[h * 32 + f] = fmaf(o[h * 32 + f], factor, __uint_as_float(d[f]));
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_o_free + 8 * buf);
+            return true;
+        };
+        for (int it = 0; it < rounds; ++it) {
+            const int buf = it & 1;
+            if (!__all_sync(0xffffffffu, ok && mbar_wait(bar_s_full + 8 * buf, (it >> 1) & 1, abort_flag, kStatusWaitAttention))) { ok = false; break; }
+            tc_fence_after_sync();
+            uint32_t s[2][32];
+            tmem_ld_x32(tmem + lanes + buf * kTile, s[0]);
+            tmem_ld_x32(tmem + lanes + buf * kTile + 32, s[1]);
+            tc_wait_ld();
+            const int left = seq - it * kTile;
+            if (left < kTile) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int n = 0; n < 32; ++n)
+                        if (h * 32 + n >= left) s[h][n] = 0xff800000u;       // -inf
+            }
+            float mx[4] = {m, m, m, m};
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int n = 0; n < 32; ++n) mx[n & 3] = fmaxf(mx[n & 3], __uint_as_float(s[h][n]));
+            mx[0] = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            const float last = keep;
+            keep = mx[0] == -INFINITY ? 1.f : exp2f((m - mx[0]) * kScale);
+            m = mx[0];
+            const float shift = m == -INFINITY ? 0.f : m;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) l[e] *= keep;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint32_t hi[16], lo[16];
+#pragma unroll
+                for (int n = 0; n < 16; ++n) {
+                    const float p0 = ex2(fmaf(__uint_as_float(s[h][2 * n]) - shift, kScale, kLift));
+                    const float p1 = ex2(fmaf(__uint_as_float(s[h][2 * n + 1]) - shift, kScale, kLift));
+                    l[(2 * n) & 3] += p0;
+                    l[(2 * n + 1) & 3] += p1;
+                    const __half2 ph = __floats2half2_rn(p0, p1);
+                    const float2 back = __half22float2(ph);
+                    const __half2 pl = __floats2half2_rn(p0 - back.x, p1 - back.y);
+                    hi[n] = *reinterpret_cast<const uint32_t*>(&ph);
+                    lo[n] = *reinterpret_cast<const uint32_t*>(&pl);
+                }
+                tmem_st_x16(tmem + lanes + buf * kTile + h * 16, hi);
+                tmem_st_x16(tmem + lanes + buf * kTile + 32 + h * 16, lo);
+            }
+            tc_wait_st();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_p_full + 8 * buf);
+            if (it > 0 && !join(it - 1, last)) { ok = false; break; }
+        }
+        ok = ok && join(rounds - 1, keep);
+        if (ok && q0 + row < seq) {
+            const float inv = 1.f / ((l[0] + l[1]) + (l[2] + l[3]));
+#pragma unroll
+            for (int f = 0; f < kHd; ++f) nan |= isnan(o[f]);
+            __half* dst = out + (int64_t)head * kHd * tokens + (int64_t)b * seq + q0 + row;
+#pragma unroll
+            for (int f = 0; f < kHd; ++f)
+                dst[f * tokens] = __float2half_rn(fmaf(o[f], inv, bias_v ? __half2float(bias_v[head * kHd + f]) : 0.f));
+        }
+    }
+    tc_fence_before_sync();
+    nan = __syncthreads_or(nan);
+    if (warp == 4) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, kTcTmemCols);
+    }
+    // something infinite or NaN went in: again, with infinities and NaNs of v apart, 64 queries at a time
+    if (nan && warp < 4) {
+        const int64_t base = (int64_t)head * kHd * tokens + (int64_t)b * seq;
+        for (int at = q0; at < min(seq, q0 + kTcQueries); at += kTile) {
+            float o[8][4], inv[2];
+            attend<true>(seq, tokens, base, at, q, k, v, bias_q ? bias_q + head * kHd : nullptr, sbase, o, inv);
+            store_queries(seq, tokens, base, at, head, bias_v, smem, o, inv, out);
+            named_barrier_sync(1, kAttnThreads);
+        }
+    }
+}
+
+using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeFn encode_fn() {
+    static EncodeFn cached = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess)
+            fn = nullptr;
+        return reinterpret_cast<EncodeFn>(fn);
+    }();
+    return cached;
+}
+// {token of a sequence, feature, sequence}, boxes of 64 tokens x 64 features; tokens past a sequence read as zeros
+bool encode_tokens(EncodeFn enc, CUtensorMap* m, const void* x, int hidden, int batch, int seq) {
+    const cuuint64_t dim[3] = {(cuuint64_t)seq, (cuuint64_t)hidden, (cuuint64_t)batch};
+    const cuuint64_t stride[2] = {(cuuint64_t)batch * seq * 2, (cuuint64_t)seq * 2};
+    const cuuint32_t box[3] = {kTile, kHd, 1}, step[3] = {1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dim, stride, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool piece_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }   // null passes
@@ -426,10 +703,31 @@ int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* 
         return (int)cudaErrorInvalidValue;
     }
     if (heads == 0 || batch == 0 || seq == 0) return 0;
-    const dim3 grid((seq + enc::kTile - 1) / enc::kTile, heads, batch);
-    enc::attention_fm_kernel<<<grid, enc::kAttnThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        seq, (int64_t)batch * seq, static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),
-        static_cast<const __half*>(bias_q), static_cast<const __half*>(bias_v), static_cast<__half*>(out));
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return (int)cudaErrorNoDevice;
+    const __half *hq = static_cast<const __half*>(q), *hk = static_cast<const __half*>(k), *hv = static_cast<const __half*>(v);
+    const __half *bq = static_cast<const __half*>(bias_q), *bv = static_cast<const __half*>(bias_v);
+    const int64_t tokens = (int64_t)batch * seq;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // tiles of 128 queries once that gives every SM one; below, 64 queries per CTA use more of the chip
+    const dim3 wide((seq + enc::kTcQueries - 1) / enc::kTcQueries, heads, batch);
+    const int64_t tiles = (int64_t)wide.x * heads * batch;
+    CUtensorMap tq, tk, tv;
+    enc::EncodeFn encode = tiles >= sms ? enc::encode_fn() : nullptr;
+    if (encode && enc::encode_tokens(encode, &tq, q, heads * head_dim, batch, seq) &&
+        enc::encode_tokens(encode, &tk, k, heads * head_dim, batch, seq) && enc::encode_tokens(encode, &tv, v, heads * head_dim, batch, seq)) {
+        static DeviceOnce once;
+        if (!once.done()) {
+            const cudaError_t e = cudaFuncSetAttribute(enc::attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, enc::TcSmem::kDynamic);
+            if (e != cudaSuccess) { set_error("attention: %s", cudaGetErrorString(e)); return (int)e; }
+            once.mark();
+        }
+        enc::attention_tc_kernel<<<wide, enc::kTcThreads, enc::TcSmem::kDynamic, st>>>(seq, tokens, tq, tk, tv, hq, hk, hv, bq, bv,
+                                                                                        static_cast<__half*>(out));
+    } else {
+        const dim3 grid((seq + enc::kTile - 1) / enc::kTile, heads, batch);
+        enc::attention_fm_kernel<<<grid, enc::kAttnThreads, 0, st>>>(seq, tokens, hq, hk, hv, bq, bv, static_cast<__half*>(out));
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("attention launch: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;

@@ -235,3 +235,34 @@ def test_stacked_linears_follow_their_tensors(lib):
     L[2].values = layer.qkv.values[-L[2].values.numel():]
     L[1].bias.requires_grad_()
     check(False)
+
+
+@pytest.mark.parametrize("heads,batch,seq,scale", [(2, 74, 8, 1.0), (4, 37, 64, 1.0), (3, 50, 72, 3.0), (2, 80, 120, 1.0), (4, 40, 128, 1.0),
+                                                   (2, 40, 136, 0.1), (1, 80, 200, 1.0), (3, 13, 512, 6.0), (1, 10, 1928, 1.0)])
+def test_attention_with_a_tile_for_every_sm(lib, heads, batch, seq, scale):
+    """Enough tiles of 128 queries for the tcgen05 kernel: one block of keys, two, three stages and more, half tiles, sequences that
+    end inside a block."""
+    test_attention_feature_major(lib, heads, batch, seq, scale)
+
+
+@pytest.mark.parametrize("seq,scale", [(64, 0.0), (136, 1.0), (200, 0.5)])
+def test_attention_infinities_and_nans_with_a_tile_for_every_sm(lib, seq, scale):
+    """As test_attention_infinities_and_nans, in some of the tiles of the tcgen05 kernel."""
+    from sspmm_b200 import ops
+    heads, batch, inf = 2, 75, float("inf")
+    g = torch.Generator(device="cuda:0").manual_seed(seq)
+    r = lambda s: (torch.randn((heads * 64, batch * seq), device="cuda:0", generator=g) * s).half()
+    q, k, v = r(scale), r(scale), r(1.0)
+    v[3, 5], v[10, seq - 1], v[70, 0], v[90, 1], v[90, seq - 2], v[127, seq + 7] = inf, -inf, inf, inf, -inf, float("nan")
+    q[64, seq + 9], k[64, seq: 2 * seq] = inf, -1.0
+    out = torch.full_like(q, float("nan"))
+    ops.attention_fm(q, k, v, heads, batch, seq, out)
+    split = lambda t: t.double().view(heads, 64, batch, seq).permute(2, 0, 3, 1)
+    score = split(q) @ split(k).transpose(-1, -2) / 8
+    p = torch.softmax(score, -1)
+    ref, got = p @ split(v), split(out)
+    assert torch.equal(ref.isnan(), got.isnan()) and torch.equal(ref.isposinf(), got.isposinf()) and torch.equal(ref.isneginf(), got.isneginf())
+    assert ref.isinf().any() and ref.isnan().any()
+    fin = ref.isfinite()
+    slack = 2.0 ** -20 * (1 + score[score.isfinite()].abs().amax()) * (p @ split(v).abs())
+    assert ((got - ref).abs()[fin] <= (2.0 ** -11 * ref.abs() + 2.0 ** -24 + slack)[fin]).all()
