@@ -372,9 +372,9 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
 // next block are computed while this block's probabilities are, and a partial output is taken one block later.
 // The arithmetic is attend's: blocks of 64 keys, sums of a block from zero, joined in round-to-nearest.
 // Bound by the softmax warps: about ten instructions per score, and the waits between them and the products, which two CTAs per SM
-// do not fill.  12 heads, 32 x 512 tokens: 85 us (attention_fm_kernel 146); 16 x 512 45 (79), 1 x 2048 47 (86).  Distance from 64
-// bits as there: 2.075754e-4 against 2.075754e-4 (scores of size 1) and 2.073792e-4 against 2.073791e-4 (size 5), of which rounding the
-// result is 2.075753e-4 and 2.073788e-4.  A CTA that walks over tiles with the next one's operands on their way takes 96 us.
+// do not fill.  12 heads, 32 x 512 tokens: 75 us (attention_fm_kernel 141; 85 with the first requests after the set-up); 16 x 512 40 (75),
+// 1 x 2048 44 (83).  Distance from 64 bits as there: 2.074969e-4 against 2.074970e-4 (scores of size 1), 2.073688e-4 against 2.073688e-4
+// (size 5).  A CTA that walks over tiles with the next one's operands on their way takes 96 us.
 constexpr int kTcQueries = 128, kTcStages = 3, kTcThreads = 160;
 struct TcSmem {
     static constexpr int kQ = 0;                                     // two chunks of [64 features][64 queries]
@@ -561,12 +561,12 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
 #pragma unroll
             for (int e = 0; e < 4; ++e) l[e] *= keep;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t hi[16], lo[16];
+            for (int h = 0; h < 4; ++h) {
+                uint32_t hi[8], lo[8];
 #pragma unroll
-                for (int n = 0; n < 16; ++n) {
-                    const float p0 = ex2(fmaf(__uint_as_float(s[h][2 * n]) - shift, kScale, kLift));
-                    const float p1 = ex2(fmaf(__uint_as_float(s[h][2 * n + 1]) - shift, kScale, kLift));
+                for (int n = 0; n < 8; ++n) {
+                    const float p0 = ex2(fmaf(__uint_as_float(s[h >> 1][(h & 1) * 16 + 2 * n]) - shift, kScale, kLift));
+                    const float p1 = ex2(fmaf(__uint_as_float(s[h >> 1][(h & 1) * 16 + 2 * n + 1]) - shift, kScale, kLift));
                     l[(2 * n) & 3] += p0;
                     l[(2 * n + 1) & 3] += p1;
                     const __half2 ph = __floats2half2_rn(p0, p1);
@@ -575,8 +575,8 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
                     hi[n] = *reinterpret_cast<const uint32_t*>(&ph);
                     lo[n] = *reinterpret_cast<const uint32_t*>(&pl);
                 }
-                tmem_st_x16(tmem + lanes + buf * kTile + h * 16, hi);
-                tmem_st_x16(tmem + lanes + buf * kTile + 32 + h * 16, lo);
+                tmem_st_x8(tmem + lanes + buf * kTile + h * 8, hi);
+                tmem_st_x8(tmem + lanes + buf * kTile + 32 + h * 8, lo);
             }
             tc_wait_st();
             tc_fence_before_sync();
@@ -709,11 +709,12 @@ int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* 
     const __half *bq = static_cast<const __half*>(bias_q), *bv = static_cast<const __half*>(bias_v);
     const int64_t tokens = (int64_t)batch * seq;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // tiles of 128 queries once that gives every SM one; below, 64 queries per CTA use more of the chip
+    // Tiles of 128 queries need blocks of keys to pay for their start-up (about 3 us) and are half as many: at 8 heads of 64 tokens 152
+    // tiles take 5.8 us against 4.6, at 256 tokens 64 tiles 8.2 (7.8), 128 8.5 (10.2), at 512 tokens 48 tiles 11.9 (13.2).
     const dim3 wide((seq + enc::kTcQueries - 1) / enc::kTcQueries, heads, batch);
     const int64_t tiles = (int64_t)wide.x * heads * batch;
     CUtensorMap tq, tk, tv;
-    enc::EncodeFn encode = tiles >= sms ? enc::encode_fn() : nullptr;
+    enc::EncodeFn encode = 2 * tiles * ((seq - 1) / enc::kTile) >= 3 * sms ? enc::encode_fn() : nullptr;
     if (encode && enc::encode_tokens(encode, &tq, q, heads * head_dim, batch, seq) &&
         enc::encode_tokens(encode, &tk, k, heads * head_dim, batch, seq) && enc::encode_tokens(encode, &tv, v, heads * head_dim, batch, seq)) {
         static DeviceOnce once;
