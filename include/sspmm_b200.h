@@ -199,6 +199,9 @@ typedef struct sspmm_group_item {
 } sspmm_group_item;
 int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16, int mode, sspmm_group** group);
 int sspmm_group_run(sspmm_group* group, void* stream);
+/* A number per output row of product `item` (fp16, m_vec*V of them; NULL: none), added to the fp32 sums before the conversion in
+ * the runs that follow.  taken = 0: this group's kernel adds no biases (groups of the tile kernels), nothing has changed. */
+int sspmm_group_bias(sspmm_group* group, int item, const void* bias_f16, int* taken);
 /* Any output pointer may be NULL.  launches = kernels per run (always 1). */
 int sspmm_group_info(const sspmm_group* group, int* tile_columns, int* work_items, int* ctas, int* launches,
                      int64_t* scratch_bytes);

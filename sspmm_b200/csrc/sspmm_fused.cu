@@ -1239,7 +1239,8 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
     const int BN = choice.BN;
     // Small groups go to the row-gather kernel, which spreads every vector row over the chip instead of walking a tile's K range
     // (launch and look-ups, then 2 * nvec * N bytes of gathers at 6 TB/s: 768 x 3072 at N = 128 10 us against 24, three 256 x 256 at 128
-    // 4 against 9; they meet at 13 to 15 us).
+    // 4 against 9; they meet at 13 to 15 us).  Its warps share the rows by the mean, so matrices with rows far longer than
+    // that stay with the tiles, which do not see them.
     if (mode == 0 && count <= kRowsMaxSet) {
         double gathers = 0;
         long long nvec = 0;
@@ -1255,7 +1256,7 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
             a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0; a.stream = nullptr;
             gathers += 2.0 * (double)pl->nvec * items[i].N;
             nvec += pl->nvec;
-            ok = ok && pl->V == items[0].plan->V && items[i].N % 8 == 0 && a.values && a.rhs && a.out && fused::aligned16(a.values) &&
+            ok = ok && pl->max_len <= 4 * (pl->nvec / pl->m_vec) + 64 && pl->V == items[0].plan->V && items[i].N % 8 == 0 && a.values && a.rhs && a.out && fused::aligned16(a.values) &&
                  fused::aligned16(a.rhs) && fused::aligned16(a.out);
         }
         if (ok && 4.0 + gathers / 6.0e6 < choice.us) {
@@ -1451,6 +1452,14 @@ int sspmm_group_run(sspmm_group* group, void* stream) {
     cudaError_t e = group->pair ? fused::launch_pair(group->params, group->out_f16, group->grid, st, false)
                                 : fused::launch(group->params, group->BN, group->out_f16, group->expanded, group->grid, st);
     if (e != cudaSuccess) { set_error("group launch: %s", cudaGetErrorString(e)); return (int)e; }
+    return 0;
+}
+
+int sspmm_group_bias(sspmm_group* group, int item, const void* bias_f16, int* taken) {
+    set_error("%s", "");
+    if (!group || !taken || item < 0 || item >= group->count) { set_error("bad group, item or output pointer"); return (int)cudaErrorInvalidValue; }
+    *taken = group->rows.empty() ? 0 : 1;
+    if (*taken) group->rows[(size_t)item].bias = static_cast<const __half*>(bias_f16);
     return 0;
 }
 

@@ -203,8 +203,10 @@ class SparseEncoderLayer:
         self._attend(b["q"], b["k"], b["v"], batch, seq, [l.bias for l in L[:3]], out=b["att"])
         g[1].run()
         out, _ = self._norm(b["o"], self.ln2, add=x, bias=L[3].bias, out=b["ln2"], sum_out=b["sum"])
+        bias = L[4].bias_rows()
+        added = g[2].bias(0, bias) and bias is not None
         g[2].run()
-        if L[4].bias is not None:
+        if L[4].bias is not None and not added:
             b["h"] += L[4].bias[:, None]
         g[3].run()
         bias = L[5].bias_rows()

@@ -344,7 +344,7 @@ class Group:
         import ctypes as C
         if not products:
             raise ValueError("a group needs at least one product")
-        self._keep = list(products)
+        self._keep, self._biases = list(products), {}
         out_dtype = products[0][3].dtype
         arr = (capi.GroupItem * len(products))()
         for i, (plan, values, rhs, out) in enumerate(products):
@@ -362,6 +362,21 @@ class Group:
         capi.check(capi.lib().sspmm_group_info(self._h, C.byref(bn), C.byref(items), C.byref(ctas), C.byref(launches), C.byref(nbytes)))
         self.tile_columns, self.work_items, self.ctas, self.scratch_bytes = bn.value, items.value, ctas.value, nbytes.value
         self.launches = launches.value
+
+    def bias(self, item: int, bias: Optional[torch.Tensor]) -> bool:
+        """Adds a number per output row (fp16) of a product before its results are rounded, from the next run on; False: this
+        group's kernel does not, and nothing has changed."""
+        import ctypes as C
+        if bias is not None:
+            _require(bias, torch.float16, "bias")
+            out = self._keep[item][3]
+            if bias.numel() != out.shape[0] or bias.device != out.device:
+                raise ValueError(f"bias has {bias.numel()} numbers on {bias.device}, the product {out.shape[0]} rows on {out.device}")
+        taken = C.c_int(0)
+        capi.check(capi.lib().sspmm_group_bias(self._h, item, _ptr(bias), C.byref(taken)))
+        if taken.value:
+            self._biases[item] = bias
+        return bool(taken.value)
 
     def run(self) -> None:
         rc = capi.native().group_run(self._h.value if self._h else 0, self.device.index)

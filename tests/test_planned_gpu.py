@@ -211,3 +211,41 @@ def test_automatic_group_of_both_vector_lengths(lib):
     g.run()
     for p, ref in zip(prods, refs):
         assert_close(p[3].float().cpu().numpy(), ref)
+
+
+def test_group_biases(lib):
+    """A group of the row-gather kernel adds biases from the run after they were given, a tile group says that it does not."""
+    rng = np.random.default_rng(12)
+    ptr, col, vals = compress(synthetic.magnitude_pruned(100, 200, 0.7, rng), 8)
+    for N, taken in ((72, True), (20000, False)):
+        rhs = rng.normal(0, 1, (200, N)).astype(np.float16)
+        d_ptr, d_col, d_val, d_rhs = dev(ptr, col, vals, rhs)
+        out = torch.empty((104, N), dtype=torch.float32, device=DEV)
+        g = ops.Group([(ops.Plan(d_ptr, d_col, 8, 200), d_val, d_rhs, out)])
+        g.run()
+        plain = out.clone()
+        bias = torch.randn(104, device=DEV).half()
+        assert g.bias(0, bias) == taken
+        g.run()
+        assert torch.equal(out, plain + bias.float()[:, None] if taken else plain)
+        assert g.bias(0, None) == taken
+        g.run()
+        assert torch.equal(out, plain)
+        with pytest.raises(ValueError):
+            g.bias(0, bias[:100])
+        with pytest.raises(IndexError):
+            g.bias(1, bias)
+
+
+@pytest.mark.parametrize("longest,rows", [(300, True), (2000, False)])
+def test_automatic_group_with_a_long_row(lib, longest, rows):
+    rng = np.random.default_rng(longest)
+    ptr, col, vals = random_cvse(rng, 40, 2048, 8, [140] * 39 + [longest])
+    rhs = rng.normal(0, 1, (2048, 64)).astype(np.float16)
+    d_ptr, d_col, d_val, d_rhs = dev(ptr, col, vals, rhs)
+    out = torch.empty((320, 64), dtype=torch.float32, device=DEV)
+    plan = ops.Plan(d_ptr, d_col, 8, 2048)
+    g = ops.Group([(plan, d_val, d_rhs, out)])
+    assert plan.one_launch and (g.work_items == 40) == rows
+    g.run()
+    assert_close(out.cpu().numpy(), spmm_oracle.sspmm_host(8, ptr, col, vals, rhs), fp32=True)
