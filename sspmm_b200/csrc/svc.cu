@@ -34,9 +34,9 @@
 //                      (rows are ascending and so come to sit in runs), so the tables
 //                      of a rebuild are kept and the next one starts from them.
 //                      Stack of 16 power-law matrices (n 4096 to 65536, V = 8), whole
-//                      call: 3450 us with every rebuild from free tables and sequences
-//                      apart from the tables, 1310 now; per launch, classes L, M2, M1, S, XS
-//                      776, 576, 392, 276, 284 us one after another.
+//                      call: 3080 to 3450 us with every rebuild from free tables and
+//                      sequences apart from the tables, 1141 now; per launch, classes L,
+//                      M2, M1, S, XS 680, 573, 367, 235, 295 us one after another.
 // The replay kernels take their groups from per-class lists (written by the scan kernel)
 // through a work counter, so a CTA never walks over groups of other classes and the
 // groups of a class, whose cost differs by an order of magnitude, balance themselves.

@@ -335,8 +335,8 @@ class Group:
     ``sspmm_group_run``).  ``products`` is a list of (plan, values, rhs, out); all outputs share one dtype.
     ``mode``: COMPRESSED builds the A tiles inside the kernel from the compressed operand (no scratch for A),
     EXPANDED lets the kernel's loader warps write dense copies of A while the first tiles are multiplied (faster per
-    K step), PAIRS is EXPANDED with 256 x 256 tiles on CTA pairs, AUTO picks COMPRESSED or EXPANDED by the work per
-    SM.  Every mode is one launch per run."""
+    K step), PAIRS is EXPANDED with 256 x 256 tiles on CTA pairs, AUTO picks COMPRESSED or EXPANDED by a model of their
+    times, or the row-gather kernel for small groups.  Every mode is one launch per run."""
 
     AUTO, COMPRESSED, EXPANDED, PAIRS = 0, 1, 2, 3
 
