@@ -71,6 +71,17 @@ int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nv
                   const void* bias_f16, void* out, int64_t out_stride, int out_is_f16, void* stream);
 
 /*
+ * sspmm_counted for several operands of one height and width that multiply the same rhs: `pieces` of m_vec vector rows each, results
+ * one below the other in out [pieces * m_vec*V][N], as one product.  column_indices, values and bias hold the pieces one after
+ * another (nvec[i] vectors, m_vec*V biases); each keeps its own row pointers, which start at 0, and row order (either pointer of
+ * row_indices, or the array, may be NULL).  taken = 0: not a call for one product (more than four pieces, unaligned operands, rows
+ * long enough to be cut, no room for the scratch); nothing was launched, and sspmm_counted takes the pieces one by one.
+ */
+int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int64_t* nvec, const int* const* row_indices,
+                  const int* const* row_offsets, const int* column_indices, const void* values_f16, const void* rhs_f16,
+                  const void* bias_f16, void* out, int out_is_f16, void* stream, int* taken);
+
+/*
  * Same product as sspmm_f16_f16, for callers that must not allocate device memory when they call:
  * a server that gave all device memory to its own arena at start-up, or a latency-critical loop
  * in which an allocation could fail or stall other streams.  No counterpart in the reference (its

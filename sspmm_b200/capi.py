@@ -19,6 +19,7 @@ SIGNATURES = {
     "sspmm_f16_f32": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_f16_f16": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_f16_f16_batched": (C.c_int, [C.c_int] * 5 + [_vp, _vp, _vp, _vp, C.c_int64, _vp, C.c_int64, _vp, C.c_int64, _vp]),
+    "sspmm_stacked": (C.c_int, [C.c_int] * 5 + [C.POINTER(C.c_int64)] + [_vp] * 7 + [C.c_int, _vp, c_int_p]),
     "sspmm_counted": (C.c_int, [C.c_int] * 5 + [C.c_int64, _vp, _vp, _vp, _vp, C.c_int64, _vp, C.c_int64, _vp, _vp, C.c_int64, C.c_int, _vp]),
     "sspmm_f16_f16_noalloc": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
     "sspmm_workspace_bytes": (C.c_int, [C.c_int] * 4 + [C.c_int64, C.c_int, C.POINTER(C.c_int64)]),

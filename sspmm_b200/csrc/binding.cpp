@@ -92,6 +92,49 @@ PyObject* py_sspmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// stacked(row_offsets of each piece, row_indices of each, where the pieces' vectors end, column_indices, values, rhs, vec_length, bias)
+PyObject* py_stacked(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        constexpr Py_ssize_t kMost = 4;
+        long V;
+        if (n != 8 || modes_active() || !small_int(a[6], 1, 1 << 20, &V) || !PyList_CheckExact(a[0]) || !PyList_CheckExact(a[1]) ||
+            !PyList_CheckExact(a[2]))
+            Py_RETURN_NONE;
+        const Py_ssize_t pieces = PyList_GET_SIZE(a[0]);
+        if (pieces < 1 || pieces > kMost || PyList_GET_SIZE(a[1]) != pieces || PyList_GET_SIZE(a[2]) != pieces) Py_RETURN_NONE;
+        const at::Tensor *col = plain(a[3], at::kInt), *val = plain(a[4], at::kHalf), *rhs = plain(a[5], at::kHalf), *bias = plain(a[7], at::kHalf);
+        if (!col || !val || !rhs || !bias || rhs->dim() != 2) Py_RETURN_NONE;
+        const int *offsets[kMost], *orders[kMost];
+        int64_t nvec[kMost], m_vec = 0;
+        long before = 0;
+        for (Py_ssize_t i = 0; i < pieces; ++i) {
+            const at::Tensor *ptr = plain(PyList_GET_ITEM(a[0], i), at::kInt), *order = plain(PyList_GET_ITEM(a[1], i), at::kInt);
+            long end;
+            if (!ptr || !order || ptr->device() != rhs->device() || order->device() != rhs->device() ||
+                !small_int(PyList_GET_ITEM(a[2], i), before, 0x7fffffff, &end))
+                Py_RETURN_NONE;
+            if (i == 0) m_vec = ptr->numel() - 1;
+            if (ptr->numel() - 1 != m_vec || order->numel() != m_vec) Py_RETURN_NONE;
+            offsets[i] = static_cast<const int*>(ptr->data_ptr());
+            orders[i] = static_cast<const int*>(order->data_ptr());
+            nvec[i] = end - before;
+            before = end;
+        }
+        const int64_t K = rhs->size(0), N = rhs->size(1), most = 0x7fffffff;
+        if (m_vec < 1 || m_vec > most / V / pieces || K > most || N > most || col->numel() != before || val->numel() != before * V ||
+            bias->numel() != pieces * m_vec * V || bias->device() != rhs->device() || col->device() != rhs->device() || val->device() != rhs->device())
+            Py_RETURN_NONE;
+        at::Tensor out = at::empty({pieces * m_vec * V, N}, rhs->options().requires_grad(false));
+        int taken = 0;
+        const int rc = launch(rhs->get_device(), [&](void* st) {
+            return sspmm_stacked((int)pieces, (int)m_vec, (int)V, (int)N, (int)K, nvec, orders, offsets, static_cast<const int*>(col->data_ptr()),
+                                 val->data_ptr(), rhs->data_ptr(), bias->data_ptr(), out.data_ptr(), 1, st, &taken);
+        });
+        if (rc == 0 && !taken) Py_RETURN_NONE;
+        return result(rc, out);
+    });
+}
+
 // bspmm(row_indices, row_offsets, column_indices, values, rhs_matrix, vec_length)
 PyObject* py_bspmm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -255,6 +298,7 @@ PyMethodDef methods[] = {
     {"svc", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_svc)), METH_FASTCALL, nullptr},
     {"sorted_row_swizzle", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sorted_row_swizzle)), METH_FASTCALL, nullptr},
     {"sspmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sspmm)), METH_FASTCALL, nullptr},
+    {"stacked", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_stacked)), METH_FASTCALL, nullptr},
     {"bspmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bspmm)), METH_FASTCALL, nullptr},
     {"planned", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_planned)), METH_FASTCALL, nullptr},
     {"group_run", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_group_run)), METH_FASTCALL, nullptr},

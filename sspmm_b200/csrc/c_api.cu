@@ -95,6 +95,15 @@ static bool block_kernel_is_faster(long long nvec, const SpmmArgs& a) {
     return t_block < t_rows;
 }
 
+// Whether the block kernel can take the call at all (rhs_ok: the dense operand lies on 16-byte boundaries; TMA reads whole batches
+// with one stride).
+static bool block_fits(const SpmmArgs& a, bool rhs_ok) {
+    const int64_t oes = a.out_f16 ? 2 : 4;
+    const bool out_ok = aligned16(a.out) && ((int64_t)a.n_out * oes) % 16 == 0;
+    return rhs_ok && out_ok && (a.batch == 1 || (a.values_stride == 0 && a.rhs_stride == (int64_t)a.K * a.n_out && (a.out_stride * oes) % 16 == 0)) &&
+           sspmm_block_scratch_bytes(a) <= ((size_t)2 << 30);
+}
+
 // Length-sorted scheduling order: rank by (length descending, row id ascending).
 __global__ void __launch_bounds__(256)
 row_swizzle_kernel(int m_vec, const int* __restrict__ row_offsets, int* __restrict__ row_indices) {
@@ -226,14 +235,11 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
             a.N = (int)ld;
             a.rhs_stride = batch > 1 ? (int64_t)K * ld : 0;
         }
-        const int64_t oes = out_f16 ? 2 : 4;
-        const bool out_ok = aligned16(out) && ((int64_t)N * oes) % 16 == 0;
-        // TMA reads whole batches with one stride.  A copied operand stays with the row-gather kernel: like the CUDA-core kernel
+        // A copied operand stays with the row-gather kernel: like the CUDA-core kernel
         // it sums fp32 results in round-to-nearest (2048 x 4608 half full, N = 1001, distance from 64 bits: 1.3e-7, the matrix
         // unit's truncated sums over all of K 2.7e-6, the CUDA cores 8.5e-7; 172, 53 and 1863 us) and multiplies no
         // infinity of B by a zero that is not in the list.
-        const bool block_ok = rhs_ok && out_ok && (batch == 1 || (values_stride == 0 && rhs_stride == (int64_t)K * N && (out_stride * oes) % 16 == 0)) &&
-                              sspmm_block_scratch_bytes(a) <= ((size_t)2 << 30);
+        const bool block_ok = block_fits(a, rhs_ok);
         if (choice == 3 && !block_ok && rhs_ok) {
             set_error("block kernel needs 16-byte aligned output, a shared value array for batches and <= 2 GiB of scratch");
             return (int)cudaErrorInvalidValue;
@@ -345,6 +351,60 @@ int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nv
     ex.nvec = nvec; ex.bias = bias_f16;
     return spmm_entry(m_vec, vec_length, N, K, batch, row_indices, row_offsets, column_indices, values_f16, values_stride, rhs_f16,
                       rhs_stride, out, out_stride, out_is_f16 != 0, stream, ex);
+}
+
+int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int64_t* nvec, const int* const* row_indices,
+                  const int* const* row_offsets, const int* column_indices, const void* values_f16, const void* rhs_f16,
+                  const void* bias_f16, void* out, int out_is_f16, void* stream, int* taken) {
+    g_err[0] = 0;
+    if (!taken || !nvec || !row_offsets || pieces < 1) { set_error("null pointer or no pieces"); return (int)cudaErrorInvalidValue; }
+    *taken = 0;
+    const int choice = g_kernel_choice.load();
+    const int V = vec_length;
+    if (pieces > kMaxPieces || (V != 8 && V != 16) || m_vec <= 0 || N <= 0 || K <= 0 || m_vec > 0x7fffffff / V / pieces || N % 8 != 0 ||
+        !column_indices || !values_f16 || !rhs_f16 || !out || !aligned16(values_f16) || !aligned16(rhs_f16) || !aligned16(out) ||
+        choice == 1 || choice == 2)
+        return 0;
+    SpmmArgs a;
+    a.m_vec = pieces * m_vec; a.V = V; a.N = N; a.n_out = N; a.K = K;
+    a.row_indices = nullptr; a.row_offsets = row_offsets[0]; a.column_indices = column_indices;
+    a.values = static_cast<const __half*>(values_f16); a.rhs = static_cast<const __half*>(rhs_f16);
+    a.out = out; a.out_f16 = out_is_f16 != 0; a.bias = static_cast<const __half*>(bias_f16); a.batch = 1;
+    a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
+    a.stream = static_cast<cudaStream_t>(stream);
+    a.pieces = pieces;
+    SpmmArgs each[kMaxPieces];
+    int64_t total = 0;
+    for (int i = 0; i < pieces; ++i) {
+        if (!row_offsets[i] || nvec[i] < 0 || total + nvec[i] > 0x7fffffffLL) return 0;
+        a.piece_offsets[i] = row_offsets[i];
+        a.piece_first[i] = (int)total;
+        SpmmArgs& s = each[i];
+        s = a;
+        s.pieces = 1; s.m_vec = m_vec;
+        s.row_indices = row_indices ? row_indices[i] : nullptr; s.row_offsets = row_offsets[i];
+        s.column_indices = column_indices + total; s.values = a.values + total * V;
+        s.out = static_cast<uint8_t*>(out) + (size_t)i * m_vec * V * N * (out_is_f16 ? 2 : 4);
+        s.bias = a.bias ? a.bias + (size_t)i * m_vec * V : nullptr;
+        if (sspmm_rows_scratch_bytes(s, nvec[i])) return 0;                 // long rows are cut: not in a launch of several products
+        total += nvec[i];
+    }
+    cudaError_t e;
+    if (choice == 3 || (choice == 0 && block_kernel_is_faster(total, a))) {
+        if (!block_fits(a, true)) return 0;
+        void* scratch = nullptr;
+        const size_t bytes = sspmm_block_scratch_bytes(a);
+        keep_pool_memory();
+        e = cudaMallocAsync(&scratch, bytes, a.stream);
+        if (e != cudaSuccess) { cudaGetLastError(); return 0; }
+        e = launch_sspmm_block(a, scratch, bytes);
+        cudaFreeAsync(scratch, a.stream);
+    } else {
+        e = launch_sspmm_rows_set(each, pieces, total);
+    }
+    if (e != cudaSuccess) return fail(e, "SpMM launch");
+    *taken = 1;
+    return 0;
 }
 
 int sspmm_workspace_bytes(int m_vec, int vec_length, int N, int K, int64_t nvec, int out_is_f16, int64_t* bytes) {

@@ -8,6 +8,8 @@
 
 namespace sspmm_b200 {
 
+constexpr int kMaxPieces = 4;
+
 struct SpmmArgs {
     int m_vec;                 // vector rows
     int V;                     // rows per vector (8 or 16)
@@ -28,6 +30,11 @@ struct SpmmArgs {
     int64_t rhs_stride;
     int64_t out_stride;
     cudaStream_t stream;
+    // The operand may be several of one height, one below the other, that share column_indices and values but keep their own row
+    // pointers (block kernel only): piece p starts at vector piece_first[p].  pieces <= 1: row_offsets are those of the operand.
+    int pieces = 1;
+    const int* piece_offsets[kMaxPieces] = {};
+    int piece_first[kMaxPieces] = {};
 };
 
 // tcgen05 row-gather kernel.  Requires N % 8 == 0, 16-byte aligned rhs/values.

@@ -48,9 +48,16 @@ std::atomic<bool> g_block_pairs{true};
 // V = 16: 6.3 us in 48 CTAs, 5.1 in 144).
 constexpr int kExpandChunk = 1024;           // longest
 
+// Row pointers of the pieces of an operand, `rows` vector rows each.
+struct PieceRows {
+    int rows;
+    const int* offsets[kMaxPieces];
+    int first[kMaxPieces];
+};
+
 template <int V>
 __global__ void __launch_bounds__(256)
-expand_transposed_kernel(int m_vec, int K, int chunk, const int* __restrict__ row_offsets, const int* __restrict__ col,
+expand_transposed_kernel(int m_vec, int K, int chunk, const __grid_constant__ PieceRows pieces, const int* __restrict__ col,
                          const __half* __restrict__ values, __half* __restrict__ at) {
     __shared__ int slot[kExpandChunk];
     const int64_t mp = (int64_t)m_vec * V;
@@ -59,7 +66,9 @@ expand_transposed_kernel(int m_vec, int K, int chunk, const int* __restrict__ ro
     for (int i = blockIdx.y; i < m_vec; i += gridDim.y) {
         for (int k = threadIdx.x; k < chunk; k += blockDim.x) slot[k] = -1;
         __syncthreads();
-        const int j0 = row_offsets[i], j1 = row_offsets[i + 1];
+        const int piece = i / pieces.rows;
+        const int* const row = pieces.offsets[piece] + (i - piece * pieces.rows);
+        const int j0 = pieces.first[piece] + row[0], j1 = pieces.first[piece] + row[1];
         // four independent loads in flight per thread: the kernel is a chain of dependent reads otherwise
         for (int j = j0 + threadIdx.x; j < j1; j += 4 * blockDim.x) {
             int c[4];
@@ -829,8 +838,13 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
         int chunk = kExpandChunk;
         while (chunk > 256 && (int64_t)by * ((a.K + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
         const dim3 grid((a.K + chunk - 1) / chunk, by);
-        if (a.V == 16) expand_transposed_kernel<16><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, a.row_offsets, a.column_indices, a.values, at);
-        else expand_transposed_kernel<8><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, a.row_offsets, a.column_indices, a.values, at);
+        PieceRows r = {a.m_vec, {a.row_offsets}, {0}};
+        if (a.pieces > 1) {
+            r.rows = a.m_vec / a.pieces;
+            for (int i = 0; i < a.pieces; ++i) { r.offsets[i] = a.piece_offsets[i]; r.first[i] = a.piece_first[i]; }
+        }
+        if (a.V == 16) expand_transposed_kernel<16><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, r, a.column_indices, a.values, at);
+        else expand_transposed_kernel<8><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, r, a.column_indices, a.values, at);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

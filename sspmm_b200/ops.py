@@ -100,6 +100,14 @@ def sspmm_bias(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: 
     return out
 
 
+def sspmm_stacked(row_offsets, row_indices, ends, column_indices: torch.Tensor, values: torch.Tensor, rhs: torch.Tensor, vec_length: int,
+                  bias: torch.Tensor) -> Optional[torch.Tensor]:
+    """Operands of one shape, their vectors one after another up to ``ends``, times the same rhs as one product (``sspmm_stacked``):
+    results one below the other, or None when they have to be multiplied one by one.  ``row_offsets`` and ``row_indices`` are lists."""
+    got = capi.native().stacked(row_offsets, row_indices, ends, column_indices, values, rhs, vec_length, bias)
+    return None if got is None else _made(got)
+
+
 def svc(row_ptr: torch.Tensor, col_idx: torch.Tensor, values: Optional[torch.Tensor], M: int, K: int,
         vec_length: int) -> Tuple[torch.Tensor, torch.Tensor, Optional[torch.Tensor], int]:
     """Sparse vector compression of a CSR matrix held on the GPU.

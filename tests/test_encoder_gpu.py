@@ -237,6 +237,27 @@ def test_stacked_linears_follow_their_tensors(lib):
     check(False)
 
 
+@pytest.mark.parametrize("hidden,tokens", [(128, 144), (256, 16384)])
+def test_stacked_linears_follow_row_pointers_changed_in_place(lib, hidden, tokens):
+    """The first row loses its last vector to the second, once with and once without torch noticing; row-gather and block kernel.
+    The stacked product and the linear's own round the same sums, taken in another order, to fp16."""
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=hidden, ffn=4 * hidden, heads=hidden // 64, sparsity=0.9, vec_length=16)
+    x = torch.randn(hidden, tokens, device="cuda:0", dtype=torch.float16)
+    L = layer.linears[:3]
+    l, end = L[0], int(L[0].row_offsets[1])
+    free = sorted(set(range(hidden)) - set(l.col[: int(l.row_offsets[2])].tolist()))
+    l.col[end - 2: end] = torch.tensor(free[:2], dtype=torch.int32, device="cuda:0")       # columns that neither row names
+    before = layer.qkv(L, x)[0].clone()
+    for change in (lambda t: t[1].sub_(1), lambda t: t.data[1].sub_(1)):
+        change(l.row_offsets)
+        got = layer.qkv(L, x)
+        for y, own in zip(got, L):
+            want = own(x).double()
+            assert (y.double() - want).norm() <= 2 * 2.0 ** -11 * want.norm()
+        assert (before[:32].double() - got[0][:32].double()).norm() > 0.05 * before[:32].double().norm()
+
+
 @pytest.mark.parametrize("heads,batch,seq,scale", [(3, 75, 72, 3.0), (2, 112, 120, 1.0), (4, 56, 128, 1.0), (2, 40, 136, 0.1), (1, 80, 200, 1.0),
                                                    (3, 3, 512, 6.0), (1, 10, 1928, 1.0), (8, 40, 64, 1.0)])
 def test_attention_with_many_tiles(lib, heads, batch, seq, scale):
