@@ -74,8 +74,9 @@ int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nv
  * sspmm_counted for several operands of one height and width that multiply the same rhs: `pieces` of m_vec vector rows each, results
  * one below the other in out [pieces * m_vec*V][N], as one product.  column_indices, values and bias hold the pieces one after
  * another (nvec[i] vectors, m_vec*V biases); each keeps its own row pointers, which start at 0, and row order (either pointer of
- * row_indices, or the array, may be NULL).  taken = 0: not a call for one product (more than four pieces, unaligned operands, rows
- * long enough to be cut, no room for the scratch); nothing was launched, and sspmm_counted takes the pieces one by one.
+ * row_indices, or the array, may be NULL).  The kernel is the one that each piece would get from sspmm_counted.  taken = 0: not a call
+ * for one product (more than four pieces, unaligned operands, rows long enough to be cut, pieces for different kernels, no room for
+ * the scratch); nothing was launched, and sspmm_counted takes the pieces one by one.
  */
 int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int64_t* nvec, const int* const* row_indices,
                   const int* const* row_offsets, const int* column_indices, const void* values_f16, const void* rhs_f16,

@@ -375,6 +375,9 @@ int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int
     a.pieces = pieces;
     SpmmArgs each[kMaxPieces];
     int64_t total = 0;
+    // The pieces go to the kernel that they would go to one by one, not to the one that is faster for all of them: the block kernel
+    // multiplies an infinity of rhs by zeros that are in no list, and a call's results must not depend on being stacked.
+    int block = 0;
     for (int i = 0; i < pieces; ++i) {
         if (!row_offsets[i] || nvec[i] < 0 || total + nvec[i] > 0x7fffffffLL) return 0;
         a.piece_offsets[i] = row_offsets[i];
@@ -386,12 +389,13 @@ int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int
         s.column_indices = column_indices + total; s.values = a.values + total * V;
         s.out = static_cast<uint8_t*>(out) + (size_t)i * m_vec * V * N * (out_is_f16 ? 2 : 4);
         s.bias = a.bias ? a.bias + (size_t)i * m_vec * V : nullptr;
-        if (sspmm_rows_scratch_bytes(s, nvec[i])) return 0;                 // long rows are cut: not in a launch of several products
+        if (block_fits(s, true) && (choice == 3 || (choice == 0 && block_kernel_is_faster(nvec[i], s)))) ++block;
+        else if (choice == 3 || sspmm_rows_scratch_bytes(s, nvec[i])) return 0;    // long rows are cut: not in a launch of several products
         total += nvec[i];
     }
+    if (block != 0 && (block != pieces || !block_fits(a, true))) return 0;
     cudaError_t e;
-    if (choice == 3 || (choice == 0 && block_kernel_is_faster(total, a))) {
-        if (!block_fits(a, true)) return 0;
+    if (block) {
         void* scratch = nullptr;
         const size_t bytes = sspmm_block_scratch_bytes(a);
         keep_pool_memory();

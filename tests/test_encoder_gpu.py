@@ -258,6 +258,21 @@ def test_stacked_linears_follow_row_pointers_changed_in_place(lib, hidden, token
         assert (before[:32].double() - got[0][:32].double()).norm() > 0.05 * before[:32].double().norm()
 
 
+@pytest.mark.parametrize("tokens", [512, 768, 1024, 1536, 2048, 2560, 3072, 4096])
+def test_stacked_linears_keep_infinities_where_their_rows_name_them(lib, tokens):
+    """Token counts around the one from which the dense-tile kernel, which multiplies an infinity by zeros that are in no list, is the
+    faster one for three products, and the one from which it is for one: NaN and infinity come out as from the products one by one."""
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=512, ffn=512, heads=8, sparsity=0.9, vec_length=16)
+    x = torch.randn(512, tokens, device="cuda:0", dtype=torch.float16)
+    x[3, 5], x[100, tokens - 1] = float("inf"), -float("inf")
+    got = layer.qkv(layer.linears[:3], x)
+    for y, l in zip(got or [], layer.linears):
+        want = l(x)
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isposinf(), want.isposinf()) and torch.equal(y.isneginf(), want.isneginf())
+    assert got is not None
+
+
 @pytest.mark.parametrize("heads,batch,seq,scale", [(3, 75, 72, 3.0), (2, 112, 120, 1.0), (4, 56, 128, 1.0), (2, 40, 136, 0.1), (1, 80, 200, 1.0),
                                                    (3, 3, 512, 6.0), (1, 10, 1928, 1.0), (8, 40, 64, 1.0)])
 def test_attention_with_many_tiles(lib, heads, batch, seq, scale):
