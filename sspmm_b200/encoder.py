@@ -173,10 +173,13 @@ class SparseEncoderLayer:
 
     def _groups_for(self, tokens: int):
         """Activation buffers of fixed shape and, bound to them, one group per dependency level of the layer:
-        {Q, K, V} share their input and run as one launch, then O, FFN1, FFN2."""
-        if getattr(self, "_tokens", None) == tokens:
-            return
+        {Q, K, V} share their input and run as one launch, then O, FFN1, FFN2.  Groups keep addresses, so they are made again when a
+        linear has another plan or other values (``.data`` gives a tensor another address)."""
         L = self.linears
+        bound = [l.plan for l in L], [l.values.data_ptr() for l in L]
+        if getattr(self, "_tokens", None) == tokens and bound == self._bound:
+            return
+        self._tokens = None
         z = lambda rows: torch.empty((rows, tokens), dtype=torch.float16, device=self.dev)
         b = self.buf = {"ln1": z(self.hidden), "q": z(self.hidden), "k": z(self.hidden), "v": z(self.hidden),
                         "att": z(self.hidden), "o": z(self.hidden), "sum": z(self.hidden), "ln2": z(self.hidden),
@@ -187,7 +190,7 @@ class SparseEncoderLayer:
             self.groups = [ops.Group([item(L[0], "ln1", "q"), item(L[1], "ln1", "k"), item(L[2], "ln1", "v")]),
                            ops.Group([item(L[3], "att", "o")]), ops.Group([item(L[4], "ln2", "h")]),
                            ops.Group([item(L[5], "h", "y")])]
-        self._tokens = tokens
+        self._tokens, self._bound = tokens, bound
 
     def forward_grouped(self, x: torch.Tensor, batch: int, seq: int) -> torch.Tensor:
         """Same layer with the linears run as groups (sspmm_group_run) on preallocated activation buffers.  The biases of

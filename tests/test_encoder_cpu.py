@@ -150,3 +150,34 @@ def test_dense_evaluation_uses_none_of_the_kernels(monkeypatch):
     assert (y.double() - ref).norm() <= 4e-3 * ref.norm()            # eight roundings to fp16 of at most 2^-11 each
     y.sum().backward()
     assert x.grad is not None and x.grad.any()
+
+
+class Linear:
+    def __init__(self, plan):
+        self.plan, self.values, self.bias = plan, torch.zeros(4).half(), None
+        self.V, self.out_features = 8, 8
+
+
+def test_groups_are_made_again_for_other_values_and_plans(monkeypatch):
+    class Plan:
+        one_launch = True
+    made = []
+    monkeypatch.setattr(encoder.ops, "Group", lambda products: made.append([p[1].data_ptr() for p in products]) or made[-1])
+    L = layer()
+    L.linears = [Linear(Plan()) for _ in range(6)]
+
+    def bound():
+        L._groups_for(8)
+        return [a for g in L.groups for a in g]
+    first = bound()
+    assert bound() == first and len(made) == 4
+    L.linears[3].values = torch.ones(4).half()
+    assert bound() == [l.values.data_ptr() for l in L.linears] and len(made) == 8
+    keep, L.linears[0].values.data = L.linears[0].values.data, torch.ones(4).half()
+    assert bound() == [l.values.data_ptr() for l in L.linears] and len(made) == 12 and keep is not None
+    L.linears[5].plan = Plan()
+    bound()
+    assert len(made) == 16
+    L.linears[1].values.mul_(2)
+    bound()
+    assert len(made) == 16
