@@ -91,7 +91,10 @@ class StackedLinears:
                    l.bias is not None for l in linears)
 
     def _holds(self, linears) -> bool:
-        """Whether the linears' tensors are still the views of what is stacked (one may have been replaced)."""
+        """Whether these are still linears whose tensors are the views of what is stacked (a tensor or a linear may have been replaced)."""
+        if any(type(l) is not SparseLinear for l in linears):
+            return False
+
         def view(t, whole, at, end):
             return t.numel() == end - at and t.dtype == whole.dtype and t.is_contiguous() and \
                 t.data_ptr() == whole.data_ptr() + at * whole.element_size()

@@ -181,3 +181,12 @@ def test_groups_are_made_again_for_other_values_and_plans(monkeypatch):
     L.linears[1].values.mul_(2)
     bound()
     assert len(made) == 16
+
+
+def test_stacked_linears_leave_other_callables_alone():
+    class Scaled(encoder.SparseLinear):
+        def __call__(self, x):
+            return 2 * super().__call__(x)
+    stack = encoder.StackedLinears.__new__(encoder.StackedLinears)
+    for other in (lambda x: x, Scaled.__new__(Scaled)):
+        assert stack([other] * 3, fm(8, 8)) is None
