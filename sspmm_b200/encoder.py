@@ -83,6 +83,7 @@ class StackedLinears:
         for i, (l, at, end) in enumerate(zip(linears, self.ends, self.ends[1:])):
             l.col, l.values = self.col[at:end], self.values[at * self.V: end * self.V]
             l.bias = self.bias[i * self.rows: (i + 1) * self.rows]
+            l.plan = ops.Plan(l.row_offsets, l.col, l.V, l.in_features)
 
     @staticmethod
     def fits(linears) -> bool:

@@ -258,6 +258,13 @@ def test_stacked_linears_follow_row_pointers_changed_in_place(lib, hidden, token
         assert (before[:32].double() - got[0][:32].double()).norm() > 0.05 * before[:32].double().norm()
 
 
+def test_plans_of_stacked_linears_read_the_stacked_columns(lib):
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=128, ffn=512, heads=2, sparsity=0.9, vec_length=16)
+    for l in layer.linears:
+        assert l.plan.column_indices.data_ptr() == l.col.data_ptr() and l.plan.row_offsets is l.row_offsets and l.plan.one_launch
+
+
 @pytest.mark.parametrize("tokens", [512, 768, 1024, 1536, 2048, 2560, 3072, 4096])
 def test_stacked_linears_keep_infinities_where_their_rows_name_them(lib, tokens):
     """Token counts around the one from which the dense-tile kernel, which multiplies an infinity by zeros that are in no list, is the
