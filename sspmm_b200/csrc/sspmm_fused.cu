@@ -1003,9 +1003,52 @@ bool fill_problem(Problem* P, const sspmm_plan* plan, const void* values, const 
 
 // ---- how a group is divided -----------------------------------------------------------------
 struct Shape { int m_tiles, k_steps, N; };
-struct GroupChoice { int BN, cut; double us; };      // tile width, K steps above which a tile's range is cut (0: never), modelled time
+struct GroupChoice {
+    int BN;                          // tile width
+    std::vector<int> parts;          // of each product's K range; every part has a step
+    double us;                       // modelled time, negative: nothing chosen
+};
 
 int parts_of(int k_steps, int cut) { return cut > 0 && k_steps > cut ? std::min(16, (k_steps + cut - 1) / cut) : 1; }
+int with_a_step_each(int k_steps, int parts) {
+    const int steps = (k_steps + parts - 1) / parts;
+    return steps > 0 ? (k_steps + steps - 1) / steps : 1;
+}
+
+// How many parts the K ranges are cut into at least where results are fp32: the tensor unit truncates when it adds, parts are added in
+// round-to-nearest, so what a result loses grows with the steps of a part (K = 4608: 5.5e-6 of the result whole, 4.2e-7 in parts of 5
+// steps; fp16 results, rounded by 2.1e-4, do not show it).  A part is at most a third of the work per SM, tiles being as
+// wide as gives every SM two; one product alone is cut where that shortens its critical path (an item costs its steps and two
+// for the hand-over, summing 17 steps' worth for a part of 128 x 256).
+std::vector<int> least_parts(const std::vector<Shape>& shapes, int units, int sms, bool pair) {
+    const int count = (int)shapes.size();
+    int BN = 256;
+    int64_t tiles = 0;
+    double work = 0;
+    for (;; BN >>= 1) {
+        tiles = 0; work = 0;
+        for (const Shape& s : shapes) {
+            const int64_t t = (int64_t)s.m_tiles * ((s.N + BN - 1) / BN);
+            tiles += t;
+            work += (double)t * (s.k_steps + 2);
+        }
+        if (pair || tiles >= 2 * sms || BN == 64) break;
+    }
+    const int cut = std::max(8, (int)(work / units / 3.0));
+    std::vector<int> least((size_t)count, 1);
+    if (count == 1) {
+        const int64_t extra = 17 * BN / 256 + 1;
+        int64_t best = -1;
+        for (int q = 1; q <= 16 && q <= shapes[0].k_steps; ++q) {
+            const int64_t rounds = (tiles * q + units - 1) / units;
+            const int64_t cost = rounds * ((shapes[0].k_steps + q - 1) / q + 2 + (q > 1 ? extra : 0));
+            if (best < 0 || cost < best) { best = cost; least[0] = q; }
+        }
+    } else if (tiles < 8 * (int64_t)units) {
+        for (int i = 0; i < count; ++i) least[(size_t)i] = parts_of(shapes[(size_t)i].k_steps, cut);
+    }
+    return least;
+}
 
 // Modelled time of the tile kernel with A tiles from the loader warps, in microseconds.  Fitted to groups of the conv layers at
 // N = 64 to 5000 and of encoder products (256 to 768 wide, 256 to 8192 columns), every width with and without cuts: a K
@@ -1014,15 +1057,18 @@ int parts_of(int k_steps, int cut) { return cut > 0 && k_steps > cut ? std::min(
 // So tiles are as wide as leaves the rounds of items few, and only ranges much longer than an SM's share are cut: conv layers
 // at N = 800 take 67 us with 608 whole tiles of 256 columns, 133 with 1976 of 64 (as many tiles as give every SM two, the rule before);
 // N = 64: 47 with whole tiles, 29 cut; 768 x 3072 at N = 4096: 33 with 96 tiles of 256, 90 with 384 of 64.
-GroupChoice choose_tiles(const std::vector<Shape>& shapes, int units, bool only_256) {
-    GroupChoice best{256, 0, -1.0};
+GroupChoice choose_tiles(const std::vector<Shape>& shapes, const std::vector<int>& least, int units, bool only_256) {
+    GroupChoice best{256, {}, -1.0};
+    std::vector<int> cuts(shapes.size());
     for (int BN = 256; BN >= (only_256 ? 256 : 64); BN /= 2)
         for (int cut : {0, 36, 24, 16, 12, 8}) {
             double longest = 0, total = 0, last_sum = 0, first_item = -1;
             int64_t n = 0;
             bool uniform = true;
-            for (const Shape& s : shapes) {
-                const int parts = parts_of(s.k_steps, cut), steps = (s.k_steps + parts - 1) / parts;
+            for (size_t i = 0; i < shapes.size(); ++i) {
+                const Shape& s = shapes[i];
+                const int parts = with_a_step_each(s.k_steps, std::max(parts_of(s.k_steps, cut), least[i])), steps = (s.k_steps + parts - 1) / parts;
+                cuts[i] = parts;
                 const int64_t tiles = (int64_t)s.m_tiles * ((s.N + BN - 1) / BN);
                 const double item = 0.515 * steps + 1.2;
                 const double sum = parts > 1 ? ((std::min(BN, s.N) + 63) / 64) * (1.1 + 0.85 * parts) : 0.0;
@@ -1035,7 +1081,7 @@ GroupChoice choose_tiles(const std::vector<Shape>& shapes, int units, bool only_
             }
             const double spread = uniform ? (double)((n + units - 1) / units) * first_item + last_sum : total / units;
             const double us = (BN == 256 ? 7.2 : BN == 128 ? 6.3 : 6.0) + std::max(longest, spread);
-            if (best.us < 0 || us < best.us) best = GroupChoice{BN, cut, us};
+            if (best.us < 0 || us < best.us) best = GroupChoice{BN, cuts, us};
         }
     return best;
 }
@@ -1235,7 +1281,8 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
     std::vector<fused::Shape> shapes((size_t)count);
     for (int i = 0; i < count; ++i)
         shapes[i] = fused::Shape{pair ? (items[i].plan->m_tiles + 1) / 2 : items[i].plan->m_tiles, items[i].plan->k_steps, items[i].N};
-    const fused::GroupChoice choice = fused::choose_tiles(shapes, units, pair);
+    const std::vector<int> least = out_is_f16 ? std::vector<int>((size_t)count, 1) : fused::least_parts(shapes, units, sms, pair);
+    const fused::GroupChoice choice = fused::choose_tiles(shapes, least, units, pair);
     const int BN = choice.BN;
     // Small groups go to the row-gather kernel, which spreads every vector row over the chip instead of walking a tile's K range
     // (launch and look-ups, then 2 * nvec * N bytes of gathers at 6 TB/s: 768 x 3072 at N = 128 10 us against 24, three 256 x 256 at 128
@@ -1280,8 +1327,7 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
         tiles += (int64_t)probs[i].m_tiles * probs[i].n_tiles;
     }
     if (tiles > (1 << 26)) { set_error("group too large (%lld tiles)", (long long)tiles); return (int)cudaErrorInvalidValue; }
-    // Tiles longer than choice.cut K steps are cut into parts; the parts' fp32 partial tiles are summed by whichever part
-    // finishes last.
+    // The fp32 partial tiles of a tile that is cut into parts are summed by whichever part finishes last.
     std::vector<fused::Item> list;
     list.reserve((size_t)tiles + 1024);
     int pslots = 0, cslots = 0;
@@ -1312,9 +1358,7 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
             }
         }
         const fused::Problem& L = probs[lead];
-        int parts = fused::parts_of(L.k_steps, choice.cut);
-        const int sps = (L.k_steps + parts - 1) / parts;
-        parts = (L.k_steps + sps - 1) / sps;
+        const int parts = choice.parts[(size_t)lead], sps = (L.k_steps + parts - 1) / parts;
         for (int nt = 0; nt < L.n_tiles; ++nt)
             for (int i : bundle) {
                 const fused::Problem& P = probs[i];
@@ -1349,7 +1393,7 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
         steps += (int64_t)probs[i].m_tiles * probs[i].n_tiles * probs[i].k_steps;
     }
     const double rounds_of_copies = (double)copy_blocks / g->grid;
-    g->expanded = pair || mode == 2 || (mode == 0 && BN == 256 && choice.cut == 0 &&
+    g->expanded = pair || mode == 2 || (mode == 0 && BN == 256 && cslots == 0 &&
                                         0.3 * (double)steps / sms > 10.0 + 4.5 * std::max(0.0, rounds_of_copies - 1.0));
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     std::vector<fused::ExpandJob> jobs;

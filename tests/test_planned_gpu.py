@@ -249,3 +249,25 @@ def test_automatic_group_with_a_long_row(lib, longest, rows):
     assert plan.one_launch and (g.work_items == 40) == rows
     g.run()
     assert_close(out.cpu().numpy(), spmm_oracle.sspmm_host(8, ptr, col, vals, rhs), fp32=True)
+
+
+@pytest.mark.parametrize("mode", [ops.Group.AUTO, ops.Group.COMPRESSED, ops.Group.EXPANDED])
+def test_fp32_groups_keep_their_sums_short(lib, mode):
+    """Eight products of 512 x 4608 at N = 200: parts of at most 18 steps of 64 columns, which the tensor unit adds in 72 additions that
+    truncate.  One loses 0.72 * 2^-24 of the sum so far on average (half a unit in the last place, over all mantissas), and the sum of
+    products of random sign after j of n additions is sqrt(j / n) of the last one, 2/3 on average; the parts are added in
+    round-to-nearest.  Parts of 36 steps lose twice as much."""
+    rng = np.random.default_rng(31)
+    K, g = 4608, torch.Generator(device=DEV).manual_seed(31)
+    d_ptr, d_col, d_val = dev(*random_cvse(rng, 32, K, 16, [3700] * 32))
+    d_val = torch.randn(d_val.numel(), device=DEV, generator=g).half()
+    dense = torch.zeros((32, 16, K), dtype=torch.float64, device=DEV)
+    dense[torch.arange(32, device=DEV).repeat_interleave(3700), :, d_col.long()] = d_val.double().view(-1, 16)
+    dense = dense.view(512, K)
+    plan = ops.Plan(d_ptr, d_col, 16, K)
+    prods = [(plan, d_val, torch.randn(K, 200, device=DEV, generator=g).half(), torch.empty((512, 200), device=DEV)) for _ in range(8)]
+    ops.Group(prods, mode=mode).run()
+    for _, _, rhs, out in prods:
+        ref = dense @ rhs.double()
+        assert (out.double() - ref).norm() <= 2 / 3 * 0.72 * 72 * 2.0 ** -24 * ref.norm()
+    assert ops.device_status() == 0
