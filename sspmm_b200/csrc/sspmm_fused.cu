@@ -1061,9 +1061,9 @@ GroupChoice choose_tiles(const std::vector<Shape>& shapes, const std::vector<int
     GroupChoice best{256, {}, -1.0};
     std::vector<int> cuts(shapes.size());
     for (int BN = 256; BN >= (only_256 ? 256 : 64); BN /= 2)
-        for (int cut : {0, 36, 24, 16, 12, 8}) {
-            double longest = 0, total = 0, last_sum = 0, first_item = -1;
-            int64_t n = 0;
+        for (int cut : {0, 36, 24, 18, 16, 12, 9, 8}) {
+            double longest = 0, total = 0, most_sum = 0, first_item = -1;
+            int64_t n = 0, tiles_total = 0;
             bool uniform = true;
             for (size_t i = 0; i < shapes.size(); ++i) {
                 const Shape& s = shapes[i];
@@ -1073,13 +1073,16 @@ GroupChoice choose_tiles(const std::vector<Shape>& shapes, const std::vector<int
                 const double item = 0.515 * steps + 1.2;
                 const double sum = parts > 1 ? ((std::min(BN, s.N) + 63) / 64) * (1.1 + 0.85 * parts) : 0.0;
                 longest = std::max(longest, item + sum);
-                last_sum = std::max(last_sum, sum);
+                most_sum = std::max(most_sum, sum);
                 total += tiles * (parts * item + sum);
                 n += tiles * parts;
+                tiles_total += tiles;
                 uniform = uniform && (first_item < 0 || first_item == item);
                 first_item = item;
             }
-            const double spread = uniform ? (double)((n + units - 1) / units) * first_item + last_sum : total / units;
+            // items of one length run in rounds, and so do the sums
+            const double spread = uniform ? (double)((n + units - 1) / units) * first_item + (double)((tiles_total + units - 1) / units) * most_sum
+                                          : total / units;
             const double us = (BN == 256 ? 7.2 : BN == 128 ? 6.3 : 6.0) + std::max(longest, spread);
             if (best.us < 0 || us < best.us) best = GroupChoice{BN, cuts, us};
         }

@@ -271,3 +271,17 @@ def test_fp32_groups_keep_their_sums_short(lib, mode):
         ref = dense @ rhs.double()
         assert (out.double() - ref).norm() <= 2 / 3 * 0.72 * 72 * 2.0 ** -24 * ref.norm()
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("N,tiles", [(9984, 4 * 39), (19200, 4 * 75)])
+@pytest.mark.parametrize("mode", [ops.Group.AUTO, ops.Group.COMPRESSED])
+def test_deep_tiles_of_several_rounds_stay_whole(lib, mode, N, tiles):
+    """512 x 4608 at just over one and two rounds of tiles: whole tiles of 256 columns; in parts every round of tiles has its round of
+    sums (N = 19200: 258 us in three parts, 125 whole)."""
+    rng = np.random.default_rng(N)
+    d_ptr, d_col, d_val = dev(*random_cvse(rng, 32, 4608, 16, [3700] * 32))
+    rhs, out = torch.zeros((4608, N), dtype=torch.float16, device=DEV), torch.full((512, N), float("nan"), dtype=torch.float16, device=DEV)
+    g = ops.Group([(ops.Plan(d_ptr, d_col, 16, 4608), d_val, rhs, out)], mode=mode)
+    assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or (g.tile_columns, g.work_items) == (256, tiles)
+    g.run()
+    assert not out.any() and ops.device_status() == 0
