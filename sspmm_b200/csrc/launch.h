@@ -46,6 +46,9 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch);
 // Several products with vectors of one length and outputs of one type in one launch; no scratch.  nvec: vectors of all of them.
 constexpr int kRowsMaxSet = 8;
 cudaError_t launch_sspmm_rows_set(const SpmmArgs* a, int count, long long nvec);
+// How that launch divides the products: columns of a tile, warps that share an item (a vector row of a tile), items, CTAs.
+struct RowsShape { int columns, warps; long long items, ctas; };
+RowsShape sspmm_rows_set_shape(const SpmmArgs* a, int count, long long nvec);
 // Copy of the dense operand with rows of `ld` columns (a multiple of 8, zeros in the columns added).
 cudaError_t launch_align_rows(const SpmmArgs& a, int ld, __half* dst);
 // tcgen05 block kernel on a dense transposed copy of A held in `scratch` (caller-owned, stream-ordered).

@@ -1287,13 +1287,16 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
     const std::vector<int> least = out_is_f16 ? std::vector<int>((size_t)count, 1) : fused::least_parts(shapes, units, sms, pair);
     const fused::GroupChoice choice = fused::choose_tiles(shapes, least, units, pair);
     const int BN = choice.BN;
-    // Small groups go to the row-gather kernel, which spreads every vector row over the chip instead of walking a tile's K range
-    // (launch and look-ups, then 2 * nvec * N bytes of gathers at 6 TB/s: 768 x 3072 at N = 128 10 us against 24, three 256 x 256 at 128
-    // 4 against 9; they meet at 13 to 15 us).  Its warps share the rows by the mean, so matrices with rows far longer than
-    // that stay with the tiles, which do not see them.
+    // Small groups go to the row-gather kernel, which spreads every vector row over the chip instead of walking a tile's K range: launch
+    // and look-ups, then 2 * nvec * N bytes of gathers at 6 TB/s, or the 16-vector steps of the longest row, one after another in the
+    // warps that share it, 0.53 us each for 64 columns (graph replays: 768 x 3072 at N = 128 10.5 us against 22.4 as tiles, three 256 x
+    // 256 at 128 4.1 against 8.8, 300 x 700 at N = 2048 15.2 against 13.0, 256 x 256 at 4096 9.3 against 9.5).  All products get the
+    // division of their mean, so a deep product of few rows among shallow ones of many stays with the tiles (4608 columns among
+    // rows of a tenth of that: 143 us against 33), and so do matrices with rows far longer than the mean.
     if (mode == 0 && count <= kRowsMaxSet) {
         double gathers = 0;
         long long nvec = 0;
+        int longest = 0;
         bool ok = true;
         std::vector<SpmmArgs> args((size_t)count);
         for (int i = 0; i < count; ++i) {
@@ -1306,10 +1309,14 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
             a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0; a.stream = nullptr;
             gathers += 2.0 * (double)pl->nvec * items[i].N;
             nvec += pl->nvec;
+            longest = std::max(longest, pl->max_len);
             ok = ok && pl->max_len <= 4 * (pl->nvec / pl->m_vec) + 64 && pl->V == items[0].plan->V && items[i].N % 8 == 0 && a.values && a.rhs && a.out && fused::aligned16(a.values) &&
                  fused::aligned16(a.rhs) && fused::aligned16(a.out);
         }
-        if (ok && 4.0 + gathers / 6.0e6 < choice.us) {
+        const RowsShape shape = sspmm_rows_set_shape(args.data(), count, nvec);
+        const int halves = shape.columns / 64;
+        const double chain = 3.9 + (halves > 1 ? 1.6 : 0.0) + 0.53 * halves * ((longest + 15) / 16) / shape.warps;
+        if (ok && std::max(4.0 + gathers / 6.0e6, chain) < choice.us) {
             sspmm_group* g = new (std::nothrow) sspmm_group();
             if (!g) return (int)cudaErrorMemoryAllocation;
             g->device = dev; g->count = count; g->out_f16 = out_is_f16 != 0; g->rows_nvec = nvec;

@@ -796,6 +796,15 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
     return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, split, d, sms) : rows::launch_typed<8, float>(a, p, H, split, d, sms);
 }
 
+RowsShape sspmm_rows_set_shape(const SpmmArgs* a, int count, long long nvec) {
+    const rows::Division d = rows::divide(a, count, nvec, current_device_sm_count() > 0 ? current_device_sm_count() : 148);
+    RowsShape r;
+    r.columns = 64 * d.H; r.warps = d.team * d.cluster;
+    r.items = rows::count_items(a, count, d.H);
+    r.ctas = (r.items * d.team + rows::kWarps - 1) / rows::kWarps * d.cluster;
+    return r;
+}
+
 cudaError_t launch_sspmm_rows_set(const SpmmArgs* a, int count, long long nvec) {
     const int sms = current_device_sm_count();
     if (sms <= 0) return cudaErrorNoDevice;

@@ -285,3 +285,23 @@ def test_deep_tiles_of_several_rounds_stay_whole(lib, mode, N, tiles):
     assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or (g.tile_columns, g.work_items) == (256, tiles)
     g.run()
     assert not out.any() and ops.device_status() == 0
+
+
+def test_automatic_group_with_a_deep_product_of_few_rows(lib):
+    """A warp would walk 230 steps of the deep product's rows while the others are done after eight: a tile group (row-gather groups
+    add biases, the others say that they do not)."""
+    rng = np.random.default_rng(9)
+    prods, refs = [], []
+    for (m_vec, K, n, N) in ((8, 4608, 3700, 64), (256, 300, 120, 256), (256, 300, 120, 256)):
+        ptr, col, vals = random_cvse(rng, m_vec, K, 8, [n] * m_vec)
+        rhs = rng.normal(0, 1, (K, N)).astype(np.float16)
+        d_ptr, d_col, d_val, d_rhs = dev(ptr, col, vals, rhs)
+        prods.append((ops.Plan(d_ptr, d_col, 8, K), d_val, d_rhs, torch.empty((m_vec * 8, N), device=DEV)))
+        refs.append(spmm_oracle.sspmm_host(8, ptr, col, vals, rhs, threads=8))
+    g, shallow = ops.Group(prods), ops.Group(prods[1:2])
+    assert not g.bias(0, None) and shallow.bias(0, None)
+    g.run()
+    for p, ref in zip(prods, refs):
+        assert_close(p[3].cpu().numpy(), ref, fp32=True)
+    shallow.run()
+    assert_close(prods[1][3].cpu().numpy(), refs[1], fp32=True)
