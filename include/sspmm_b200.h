@@ -176,7 +176,7 @@ int sspmm_planned(const sspmm_plan* plan, const void* values_f16, const void* rh
 
 /*
  * A GROUP binds several products (the layers of a model step, the members of a batch) to their
- * operands and runs all of them as one persistent tensor-core launch: the tiles of all products
+ * operands and runs all of them as one launch.  Tile groups are persistent: the tiles of all products
  * form one work list, longest first, taken by the CTAs from a shared queue, so that small products
  * fill the SMs a large one leaves idle; tiles with a long K range are cut into parts whose fp32
  * partial tiles are added, in part order, by whichever part finishes last.
@@ -192,7 +192,9 @@ int sspmm_planned(const sspmm_plan* plan, const void* values_f16, const void* rh
  *     CTAs of a cluster (tcgen05 cta_group::2, each CTA fetching its own 128 rows of A and half of
  *     the B tile).  Measured no faster than mode 2 on the conv workload (products with fewer than
  *     256 rows pay for the padding), so never chosen automatically;
- * mode 0: 1 or 2, chosen from the amount of work per SM.
+ * mode 0: 1 or 2 by a model of their times, or, for up to eight products with vectors of one length, aligned
+ *     operands and little work, the row-gather kernel of the calls above (no tiles, no scratch; it reads the plans'
+ *     row_offsets and column_indices and adds biases, see sspmm_group_bias).
  * Products of one group that multiply the same dense operand (same rhs pointer, N and K) are
  * scheduled panel by panel, so that a column panel of B is fetched from HBM once for all of them.
  * sspmm_group_create allocates the descriptors and the scratch once (and synchronises);
@@ -214,7 +216,8 @@ int sspmm_group_run(sspmm_group* group, void* stream);
 /* A number per output row of product `item` (fp16, m_vec*V of them; NULL: none), added to the fp32 sums before the conversion in
  * the runs that follow.  taken = 0: this group's kernel adds no biases (groups of the tile kernels), nothing has changed. */
 int sspmm_group_bias(sspmm_group* group, int item, const void* bias_f16, int* taken);
-/* Any output pointer may be NULL.  launches = kernels per run (always 1). */
+/* Any output pointer may be NULL.  launches = kernels per run (always 1).  tile_columns, work_items (tiles, or vector rows of a tile in
+ * row-gather groups, or parts of either) and ctas are those of the launch. */
 int sspmm_group_info(const sspmm_group* group, int* tile_columns, int* work_items, int* ctas, int* launches,
                      int64_t* scratch_bytes);
 int sspmm_group_destroy(sspmm_group* group);

@@ -1320,9 +1320,8 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
             sspmm_group* g = new (std::nothrow) sspmm_group();
             if (!g) return (int)cudaErrorMemoryAllocation;
             g->device = dev; g->count = count; g->out_f16 = out_is_f16 != 0; g->rows_nvec = nvec;
-            g->BN = 64; g->n_items = 0;
-            for (const SpmmArgs& a : args) g->n_items += a.m_vec * ((a.N + 63) / 64);
-            g->grid = std::min(g->n_items, sms);
+            g->BN = shape.columns; g->n_items = (int)std::min<long long>(shape.items, 0x7fffffff);
+            g->grid = (int)std::min<long long>(shape.ctas, 0x7fffffff);
             g->rows = std::move(args);
             *group = g;
             return 0;

@@ -300,6 +300,8 @@ def test_automatic_group_with_a_deep_product_of_few_rows(lib):
         refs.append(spmm_oracle.sspmm_host(8, ptr, col, vals, rhs, threads=8))
     g, shallow = ops.Group(prods), ops.Group(prods[1:2])
     assert not g.bias(0, None) and shallow.bias(0, None)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:        # 256 rows x 2 tiles, two items of four warps in a CTA
+        assert (shallow.tile_columns, shallow.work_items, shallow.ctas) == (128, 512, 256)
     g.run()
     for p, ref in zip(prods, refs):
         assert_close(p[3].cpu().numpy(), ref, fp32=True)
