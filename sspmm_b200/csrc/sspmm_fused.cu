@@ -1395,14 +1395,17 @@ int sspmm_group_create(const sspmm_group_item* items, int count, int out_is_f16,
     // With A tiles by TMA from a dense copy a K step of a loaded chip takes about 0.3 us less per SM than when the loader warps
     // build them; against that stands the writing of the copies: 10 us, and 4.5 for every further round of blocks (the
     // first items wait for theirs).  Conv layers, 15 steps per SM and 256 columns: N = 1200 74 us built, 92 copied; 1600 97 and 92;
-    // 3136 163 and 138.  768 x 768 at 8192: 43 and 38; 3072 x 768 at 4096: 30 and 34.
-    int64_t copy_blocks = 0, steps = 0;
+    // 3136 163 and 138.  Where tiles are few and alike the loaders keep up, so there are no copies below 48 steps per SM, a tile
+    // counting two more: 512 x 1024 at N = 25088 36 us built, 42 copied (fp32 results 39 and 43), 256 x 2304 at 18944 30 and 32; 768 x 768
+    // three times at 8192 40 and 40, 3072 x 768 at 8192 52 and 46.
+    int64_t copy_blocks = 0, steps = 0, with_hand_over = 0;
     for (int i = 0; i < count; ++i) {
         copy_blocks += ((int64_t)items[i].plan->m_vec * 8 * items[i].plan->k_steps + 255) / 256;
         steps += (int64_t)probs[i].m_tiles * probs[i].n_tiles * probs[i].k_steps;
+        with_hand_over += (int64_t)probs[i].m_tiles * probs[i].n_tiles * (probs[i].k_steps + 2);
     }
     const double rounds_of_copies = (double)copy_blocks / g->grid;
-    g->expanded = pair || mode == 2 || (mode == 0 && BN == 256 && cslots == 0 &&
+    g->expanded = pair || mode == 2 || (mode == 0 && BN == 256 && cslots == 0 && with_hand_over >= 48LL * sms &&
                                         0.3 * (double)steps / sms > 10.0 + 4.5 * std::max(0.0, rounds_of_copies - 1.0));
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     std::vector<fused::ExpandJob> jobs;

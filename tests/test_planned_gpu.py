@@ -307,3 +307,15 @@ def test_automatic_group_with_a_deep_product_of_few_rows(lib):
         assert_close(p[3].cpu().numpy(), ref, fp32=True)
     shallow.run()
     assert_close(prods[1][3].cpu().numpy(), refs[1], fp32=True)
+
+
+def test_no_copies_where_the_loaders_keep_up(lib):
+    """512 x 1024 at N = 25088: 392 equal tiles, 47.7 steps per SM of 148."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the figures are those of 148 SMs")
+    d_ptr, d_col, d_val = dev(*random_cvse(np.random.default_rng(2), 32, 1024, 16, [830] * 32))
+    rhs, out = torch.zeros((1024, 25088), dtype=torch.float16, device=DEV), torch.full((512, 25088), float("nan"), device=DEV)
+    g = ops.Group([(ops.Plan(d_ptr, d_col, 16, 1024), d_val, rhs, out)])
+    assert (g.tile_columns, g.work_items, g.scratch_bytes) == (256, 392, 0)
+    g.run()
+    assert not out.any() and ops.device_status() == 0
