@@ -235,6 +235,10 @@ struct BlockTeam {
 // each taking the groups that pass its filter (0 = all, 1 = at most kBigGroup entries, 2 = more).
 constexpr int kBigGroup = 1024;
 constexpr int kBigTeam = 1024;             // threads of such a CTA
+// Where every group gets a CTA it has 1024 threads as long as all are resident at once, else 256: with 2250 groups of 256 to 8000 entries
+// the larger ones took 116 to 131 us a call, 60 to 72 now (59 to 75 before groups got 1024 threads), with 256 groups of 37 k entries
+// (V = 16) 108 against 125.  Either fills an SM's threads, so neither may use more than 32 registers.
+constexpr int kTeam = 256;
 __device__ __forceinline__ bool group_passes(int filter, int entries) {
     return filter == 0 || (filter == 1) == (entries <= kBigGroup);
 }
@@ -242,7 +246,7 @@ __device__ __forceinline__ bool group_passes(int filter, int entries) {
 // ---------------------------------------------------------------- pass 1: count
 constexpr int kLookAt = 64;
 template <class Team>
-__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock)
+__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock, 2048 / (Team::kSize * Team::kPerBlock))
 svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, int* __restrict__ mode,
                  int* __restrict__ tbl_len) {
     extern __shared__ unsigned int sm_words[];
@@ -517,7 +521,7 @@ __device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* r
 // Bound by the latency of its look-ups, so the large groups get 1024 threads and every thread four entries at a time (conv weight of
 // 512 x 4608, 64 groups: 14.7 us with 256 threads and an entry each, 10.6 now, zeroing included).
 template <class Team>
-__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock)
+__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock, 2048 / (Team::kSize * Team::kPerBlock))
 svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restrict__ vec_ptr,
                        const int* __restrict__ mode, int* __restrict__ out_col, __half* __restrict__ out_vals,
                        const int* __restrict__ list, int n_list) {
@@ -1220,15 +1224,17 @@ cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool /*
     if (p.m_vec > 0) {
         const int words = (p.K + 31) / 32;
         const int sms = device_sm_count();
-        static DeviceOnce once_block, once_warp;
+        static DeviceOnce once_block, once_small, once_warp;
         cudaError_t e = allow_big_smem(svc_count_kernel<BlockTeam<kBigTeam>>, once_block, 200 * 1024);
+        if (e == cudaSuccess) e = allow_big_smem(svc_count_kernel<BlockTeam<kTeam>>, once_small, 200 * 1024);
         if (e == cudaSuccess) e = allow_big_smem(svc_count_kernel<WarpTeam>, once_warp, 200 * 1024);
         if (e != cudaSuccess) return e;
         const size_t warp_smem = (size_t)WarpTeam::kPerBlock * words * 4;
         if (p.m_vec <= 16 * sms || warp_smem > 200 * 1024) {
             // few groups (or bitmaps too large for eight per block): one CTA per group
             const int grid = p.m_vec < sms * 16 ? p.m_vec : sms * 16;
-            svc_count_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 4, stream>>>(p, words, 0, s.vec_ptr, s.mode, s.tbl_len);
+            if (p.m_vec <= 2 * sms) svc_count_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 4, stream>>>(p, words, 0, s.vec_ptr, s.mode, s.tbl_len);
+            else svc_count_kernel<BlockTeam<kTeam>><<<grid, kTeam, (size_t)words * 4, stream>>>(p, words, 0, s.vec_ptr, s.mode, s.tbl_len);
             e = cudaGetLastError();
         } else {
             std::lock_guard<std::mutex> lk(g_aux_mu);
@@ -1259,8 +1265,9 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
     if (p.m_vec == 0) return cudaSuccess;
     const int sms = device_sm_count();
     const int words = (p.K + 31) / 32;
-    static DeviceOnce once_block, once_warp;
+    static DeviceOnce once_block, once_small, once_warp;
     cudaError_t e = allow_big_smem(svc_emit_sorted_kernel<BlockTeam<kBigTeam>>, once_block, 208 * 1024);
+    if (e == cudaSuccess) e = allow_big_smem(svc_emit_sorted_kernel<BlockTeam<kTeam>>, once_small, 208 * 1024);
     if (e == cudaSuccess) e = allow_big_smem(svc_emit_sorted_kernel<WarpTeam>, once_warp, 208 * 1024);
     if (e != cudaSuccess) return e;
 
@@ -1286,8 +1293,8 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
         const size_t warp_smem = (size_t)WarpTeam::kPerBlock * words * 8;
         if (p.m_vec <= 16 * sms || warp_smem > 200 * 1024) {
             const int grid = p.m_vec < sms * 16 ? p.m_vec : sms * 16;
-            svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals,
-                                                                                             nullptr, 0);
+            if (p.m_vec <= 2 * sms) svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals, nullptr, 0);
+            else svc_emit_sorted_kernel<BlockTeam<kTeam>><<<grid, kTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals, nullptr, 0);
         } else {
             int grid = (p.m_vec + WarpTeam::kPerBlock - 1) / WarpTeam::kPerBlock;
             if (grid > sms * 8) grid = sms * 8;

@@ -279,3 +279,16 @@ def test_value_vectors_off_their_boundary(lib):
     lib.svc_free(job)
     assert torch.equal(ptr, want[0]) and torch.equal(col, want[1]) and torch.equal(room[3: 3 + want[2].numel()], want[2])
     assert (room[:3] == 7).all() and (room[3 + want[2].numel():] == 7).all()
+
+
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("groups,K,most", [(296, 200, 150), (297, 200, 150), (300, 3000, 900), (2368, 40, 9), (2369, 40, 9)])
+def test_svc_with_few_and_many_groups(lib, V, groups, K, most):
+    """Both team sizes of the launches with a CTA per group, on 148 SMs: 296 groups and one more, 2368 and one more; a last group of
+    one row, empty rows, ascending and replayed groups."""
+    rng = np.random.default_rng(groups)
+    rows = [np.sort(rng.permutation(K)[:n]) for n in rng.integers(0, most + 1, (groups - 1) * V + 1)]
+    rows[3:7] = [r[:0] for r in rows[3:7]]
+    ptr = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+    col = np.concatenate(rows).astype(np.int32)
+    check_against_oracle(synthetic.CSR(len(rows), K, ptr, col, rng.uniform(-1, 1, col.size).astype(np.float16)), V)
