@@ -151,6 +151,8 @@ struct Tile {
         const unsigned idx = (unsigned)(step + (lane >> 4) * stride) * kStep + (lane & 15);
         return idx < (unsigned)len ? __ldg(col + j0 + idx) : -1;
     }
+    // (The rings have to start on 128-byte boundaries, also behind a kernel's other shared variables: 16 bytes off, a copied row of 128
+    // bytes is written in two pieces; 4000 rows of 160 vectors, N = 128, 47 us, 21 as it is.)
     // Rows of the step land as [16 vectors][NT] with their 16-byte pieces XOR-swizzled by the vector number, so that the
     // copies (eight lanes per 128 bytes) and ldmatrix (eight rows per matrix) both touch every bank once.
     static __device__ __forceinline__ void copy_step(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs,
@@ -198,15 +200,10 @@ struct Tile {
     // Adds steps first, first + stride, ... of vectors [j0, j0 + len).  The whole warp takes part; `mem` is its shared memory.
     __device__ __forceinline__ void accumulate(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs, int n0,
                                                int j0, int len, int first, int stride, int lane, uint32_t mem) {
-        accumulate(p, values, rhs, n0, j0, len, first, stride, lane, mem, load_cols(p.col, j0, len, first, stride, lane), [] {});
-    }
-    // cols: load_cols of the first two steps.  meanwhile() is called once, when the first steps are under way.
-    template <class F>
-    __device__ __forceinline__ void accumulate(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs, int n0,
-                                               int j0, int len, int first, int stride, int lane, uint32_t mem, int cols, F&& meanwhile) {
         const int steps = (int)(((unsigned)len + kStep - 1) / kStep);
-        if (first >= steps) { meanwhile(); return; }
+        if (first >= steps) return;
         const int mine = (steps - first + stride - 1) / stride;         // steps of this warp
+        int cols = load_cols(p.col, j0, len, first, stride, lane);
         int next = load_cols(p.col, j0, len, first + 2 * stride, stride, lane);
         int issued = 0;
         uint32_t fill = 0, use = 0;                                     // ring slots
@@ -223,7 +220,6 @@ struct Tile {
         };
 #pragma unroll
         for (int k = 0; k < kStages - 1; ++k) issue();
-        meanwhile();
         for (int k = 0; k < mine; ++k) {
             cp_async_wait<kStages - 2>();
             __syncwarp();                           // everyone's copies are in, and the slot refilled next has been read
@@ -345,7 +341,7 @@ struct Tile {
 template <int V, typename OutT, int H>
 __device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ out, long long cta_item, int team, int cluster) {
     using T = Tile<V, H, sizeof(OutT) == 4>;
-    extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
+    extern __shared__ __align__(128) uint8_t smem[];    // [warp][T::kWarpBytes]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = cluster > 1 ? (int)cluster_cta_rank() : 0;
     const int member = warp % team;
@@ -404,35 +400,50 @@ sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int
     do_items<V, OutT, H>(p, out, (long long)(blockIdx.x / cluster) * (kWarps / team), team, cluster);
 }
 
-// More items than warps, one warp each: every warp walks over its items, and looks up the columns of the next one and the place of
-// the one after that while the first steps of its item are under way.  (With a CTA for every eight items the look-ups, four
-// dependent loads, were paid for by every round of CTAs: 96 products of 512 x 512 at 90 %, N = 64, 12.6 us, now 10.6.)
-// Neighbouring items go to different SMs: rows are often ordered by length.
+// More items than warps, one warp each: a CTA has its share of the items from the start, looks all of them up at once (a thread each, the
+// first column ids on their way to L1), and its warps take them one after another from a counter in shared memory.  With a CTA for
+// every eight items the look-ups, four dependent loads, were paid for by every round of CTAs, and a warp that was done waited for
+// the longest of its eight rows.  96 products of 512 x 512 at 90 %, N = 64: 12.6 us, now 10.3.
+// Nothing is known of the rows' lengths here, so nothing is dealt to a warp ahead of time: with the items dealt to the warps in turn and
+// the next two looked up early, one row in a hundred of 512 vectors among rows of 5 took 32 us where the CTAs of eight took 19 (now
+// 15); what look-ups are left, half a microsecond a launch, shows with rows of ten vectors (7.7 us, dealt in turn 7.1).
+// The CTAs' shares are staggered: rows are often ordered by length, and their number may divide the number of CTAs.
+// (Vectors of 16 rows lost by walking when items were dealt in turn: 2048 x 512 at 98 %, N = 8192 46 us, 48; not tried with the counter.)
+constexpr int kStagger = 113;
 template <typename OutT, int H>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_walk_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
     constexpr int V = 8;
     using T = Tile<V, H, sizeof(OutT) == 4>;
-    extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
+    extern __shared__ __align__(128) uint8_t smem[];    // [warp][T::kWarpBytes]
+    __shared__ Where table[kThreads];
+    __shared__ int next;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint8_t* const mem = smem + warp * T::kWarpBytes;
-    const long long stride = (long long)gridDim.x * kWarps;
-    long long item = (long long)warp * gridDim.x + blockIdx.x;
-    Where w = locate(p, item, T::NT);
-    int cols = T::load_cols(p.col, w.j0, w.len, 0, 1, lane);
-    Where w1 = locate(p, item + stride, T::NT);
-    for (; item < p.items; item += stride) {
-        Where w2;
-        int cols1;
-        T tile;
-        tile.clear();
-        tile.accumulate(p, p.values + w.batch * p.values_stride, p.rhs + w.batch * p.rhs_stride, w.n0, w.j0, w.len, 0, 1, lane, smem_u32(mem), cols,
-                        [&] {
-                            cols1 = T::load_cols(p.col, w1.j0, w1.len, 0, 1, lane);
-                            w2 = locate(p, item + 2 * stride, T::NT);
-                        });
-        if (w.row >= 0) tile.store(p, out + w.batch * p.out_stride, (int64_t)w.row * V, w.n0, reinterpret_cast<float*>(mem), lane);
-        w = w1; cols = cols1; w1 = w2;
+    const long long rounds = (p.items + gridDim.x - 1) / gridDim.x;
+    for (long long r0 = 0; r0 < rounds; r0 += kThreads) {
+        const long long r = r0 + threadIdx.x;
+        if (r0 > 0) __syncthreads();                     // the table has been read
+        if (r < rounds) {
+            const Where w = locate(p, r * gridDim.x + (blockIdx.x + r * kStagger) % gridDim.x, T::NT);
+            if (w.len > 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(p.col + w.j0));
+            table[threadIdx.x] = w;
+        }
+        if (threadIdx.x == 0) next = 0;
+        __syncthreads();
+        const int count = (int)min((long long)kThreads, rounds - r0);
+        for (;;) {
+            int x = 0;
+            if (lane == 0) x = atomicAdd(&next, 1);
+            x = __shfl_sync(0xffffffffu, x, 0);
+            if (x >= count) break;
+            const Where w = table[x];
+            if (w.row < 0) continue;
+            T tile;
+            tile.clear();
+            tile.accumulate(p, p.values + w.batch * p.values_stride, p.rhs + w.batch * p.rhs_stride, w.n0, w.j0, w.len, 0, 1, lane, smem_u32(mem));
+            tile.store(p, out + w.batch * p.out_stride, (int64_t)w.row * V, w.n0, reinterpret_cast<float*>(mem), lane);
+        }
     }
 }
 
@@ -465,7 +476,7 @@ template <int V, typename OutT, int H>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_split_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
     using T = Tile<V, H, sizeof(OutT) == 4>;
-    extern __shared__ __align__(16) uint8_t smem[];     // [warp][T::kWarpBytes]
+    extern __shared__ __align__(128) uint8_t smem[];    // [warp][T::kWarpBytes]
     __shared__ int seen;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint8_t* const mem = smem + warp * T::kWarpBytes;
@@ -642,7 +653,6 @@ cudaError_t launch_items(Kern kern, DeviceOnce& once, long long items, const Div
 
 template <int V, typename OutT, int H>
 cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d, int sms) {
-    // (vectors of 16 rows leave no registers for the look-ahead: 2048 x 512 at 98 %, N = 8192 46 us, walking 48)
     if constexpr (V == 8) {
         static DeviceOnce once_walk;
         if (d.team == 1 && p.items > (long long)sms * kResident * kWarps) {

@@ -257,3 +257,42 @@ def test_unaligned_dense_operand_with_infinities(lib, N, offset, dtype):
         assert hit.any() and not hit.all()
         want[:, n] = hit
     assert torch.equal(~got.isfinite(), want)
+
+
+@pytest.mark.parametrize("m,longest,K,N", [(2369, 40, 300, 64), (2400, 150, 160, 72), (800, 200, 256, 264), (37888, 3, 64, 128), (76032, 2, 64, 40)])
+def test_more_items_than_warps(lib, m, longest, K, N):
+    """One warp per item: a few more items than warps, empty rows and long ones among short ones, row orders, partial column tiles, as
+    many rounds of CTAs as a table of look-ups holds (37888 items of 128 columns: 128; 76032: 257, one more than fit)."""
+    rng = np.random.default_rng(m)
+    lens = np.where(rng.random(m) < 0.05, longest, rng.integers(0, min(longest, 6), m))
+    ptr, col, val, rhs = operands_fast(lens, K, 8, N, m)
+    ops.set_kernel(ops.KERNEL_GATHER_LSU)
+    try:
+        for order in (None, ops.sorted_row_swizzle(ptr)):
+            for dt in (torch.float16, torch.float32):
+                check(ops.sspmm(ptr, col, val, rhs, 8, row_indices=order, out_dtype=dt), ptr, col, val, rhs, 8)
+    finally:
+        ops.set_kernel(ops.KERNEL_AUTO)
+
+
+def operands_fast(lens, K, V, N, seed):
+    """operands() for many rows: columns at a random place, one after another (wrapped)."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    n = torch.as_tensor(lens, device=DEV)
+    ptr = torch.zeros(n.numel() + 1, dtype=torch.int32, device=DEV)
+    ptr[1:] = torch.cumsum(n, 0)
+    at = torch.arange(int(ptr[-1]), device=DEV) - torch.repeat_interleave(ptr[:-1].long(), n)
+    col = ((at + torch.repeat_interleave(torch.randint(K, (n.numel(),), device=DEV, generator=g), n)) % K).int()
+    return ptr, col, (torch.rand(col.numel() * V, device=DEV, generator=g) * 2 - 1).half(), torch.randn(K, N, device=DEV, generator=g).half()
+
+
+def test_batch_of_more_items_than_warps(lib):
+    """The longest row of every batch entry would fall to one warp if items were dealt out in turn: 64 rows, 2368 warps."""
+    lens = [512] + [7] * 62 + [0]
+    ptr, col, _, _ = operands_fast(lens, 512, 8, 64, 1)
+    g = torch.Generator(device=DEV).manual_seed(2)
+    val = torch.rand(96, col.numel() * 8, device=DEV, generator=g).half()
+    rhs = torch.randn(96, 512, 72, device=DEV, generator=g).half()
+    out = bspmm(ops.sorted_row_swizzle(ptr), ptr, col, val, rhs, 8)
+    for b in (0, 1, 37, 95):
+        check(out[b], ptr, col, val[b], rhs[b], 8)
