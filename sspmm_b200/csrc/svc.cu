@@ -257,9 +257,11 @@ svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, 
         const int r0 = min(i * p.V, p.M), r1 = min(i * p.V + p.V, p.M);
         const int e0 = p.row_ptr[r0], e1 = p.row_ptr[r1];
         if (!group_passes(filter, e1 - e0)) return;
+        const int* const cols = p.col_idx + e0;
+        const unsigned n_entries = (unsigned)max(0, e1 - e0);             // (an entry's number may come within a step of 2^31)
         if (e1 - e0 < words) {
-            for (int e = e0 + tid; e < e1; e += Team::kSize) {
-                const unsigned c = (unsigned)p.col_idx[e];
+            for (unsigned e = tid; e < n_entries; e += Team::kSize) {
+                const unsigned c = (unsigned)cols[e];
                 if (c < (unsigned)p.K) bm[c >> 5] = 0u;
             }
         } else {
@@ -267,10 +269,10 @@ svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, 
         }
         Team::sync();
         int cnt = 0, mx = -1, bad = 0;
-        for (int e = e0 + tid; e < e1; e += 4 * Team::kSize) {             // four loads in flight
+        for (unsigned e = tid; e < n_entries; e += 4 * Team::kSize) {      // four loads in flight
             int c4[4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) c4[b] = e + b * Team::kSize < e1 ? p.col_idx[e + b * Team::kSize] : -1;
+            for (int b = 0; b < 4; ++b) c4[b] = e + b * Team::kSize < n_entries ? cols[e + b * Team::kSize] : -1;
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 const int c = c4[b];
@@ -279,7 +281,7 @@ svc_count_kernel(SvcProblem p, int words, int filter, int* __restrict__ counts, 
                     const unsigned old = atomicOr(&bm[c >> 5], bit);
                     cnt += (old & bit) ? 0 : 1;
                     mx = max(mx, c);
-                } else if (e + b * Team::kSize < e1) {
+                } else if (e + b * Team::kSize < n_entries) {
                     bad = 1;
                 }
             }
@@ -502,19 +504,20 @@ __device__ __forceinline__ int row_of_entry(const int* rows, int n_rows, int e) 
 // Calls f(row, column, value) for the group's entries, four in flight per thread.
 template <class Team, class F>
 __device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* rows, int n_rows, F&& f) {
-    const int e1 = rows[n_rows];
-    for (int e = rows[0] + Team::tid(); e < e1; e += 4 * Team::kSize) {
+    const int e0 = rows[0];
+    const unsigned n_entries = (unsigned)max(0, rows[n_rows] - e0);
+    for (unsigned e = Team::tid(); e < n_entries; e += 4 * Team::kSize) {
         int c[4];
         __half v[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int x = e + b * Team::kSize;
-            c[b] = x < e1 ? p.col_idx[x] : -1;
-            v[b] = x < e1 ? p.vals[x] : __half(0);
+            const unsigned x = e + b * Team::kSize;
+            c[b] = x < n_entries ? p.col_idx[e0 + x] : -1;
+            v[b] = x < n_entries ? p.vals[e0 + x] : __half(0);
         }
 #pragma unroll
         for (int b = 0; b < 4; ++b)
-            if ((unsigned)c[b] < (unsigned)p.K) f(row_of_entry(rows, n_rows, e + b * Team::kSize), c[b], v[b]);
+            if ((unsigned)c[b] < (unsigned)p.K) f(row_of_entry(rows, n_rows, (int)(e0 + e + b * Team::kSize)), c[b], v[b]);
     }
 }
 
@@ -544,10 +547,12 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
         for (int w = tid; w < words; w += Team::kSize) bm[w] = 0u;
         if (out_vals && p.zero_values) zero_values<Team>(out_vals, base, vec_ptr[i + 1] - base, p.V);
         Team::sync();
-        for (int e = e0 + tid; e < e1; e += 4 * Team::kSize) {
+        const int* const cols = p.col_idx + e0;
+        const unsigned n_entries = (unsigned)max(0, e1 - e0);
+        for (unsigned e = tid; e < n_entries; e += 4 * Team::kSize) {
             int c[4];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) c[b] = e + b * Team::kSize < e1 ? p.col_idx[e + b * Team::kSize] : -1;
+            for (int b = 0; b < 4; ++b) c[b] = e + b * Team::kSize < n_entries ? cols[e + b * Team::kSize] : -1;
 #pragma unroll
             for (int b = 0; b < 4; ++b)
                 if ((unsigned)c[b] < (unsigned)p.K) atomicOr(&bm[c[b] >> 5], 1u << (c[b] & 31));

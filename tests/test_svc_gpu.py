@@ -292,3 +292,21 @@ def test_svc_with_few_and_many_groups(lib, V, groups, K, most):
     ptr = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
     col = np.concatenate(rows).astype(np.int32)
     check_against_oracle(synthetic.CSR(len(rows), K, ptr, col, rng.uniform(-1, 1, col.size).astype(np.float16)), V)
+
+
+def test_svc_with_almost_two_to_the_31_entries(lib):
+    """Entry numbers are 32-bit: the last group ends a hundred entries before 2^31, closer than one step of a team's loop."""
+    if torch.cuda.mem_get_info()[0] < 48 << 30:
+        pytest.skip("needs 30 GB on the device")
+    K, rows, short = 16384, 131072, 100
+    nnz = rows * K - short
+    col = torch.arange(K, dtype=torch.int32, device="cuda:0").repeat(rows)[:nnz]
+    val = torch.ones(nnz, dtype=torch.float16, device="cuda:0")
+    ptr = torch.arange(0, rows, device="cuda:0") * K
+    ptr = torch.cat([ptr, ptr.new_tensor([nnz])]).int()
+    vec_ptr, vec_col, vec_val, _ = ops.svc(ptr, col, val, rows, K, 8)
+    assert torch.equal(vec_ptr, torch.arange(0, rows // 8 + 1, device="cuda:0", dtype=torch.int32) * K)
+    assert torch.equal(vec_col, col[: K].repeat(rows // 8))
+    assert (vec_val[: -8 * K] == 1).all()
+    last = vec_val[-8 * K:].view(K, 8)
+    assert (last[:, :7] == 1).all() and (last[: K - short, 7] == 1).all() and not last[K - short:, 7].any()
