@@ -448,7 +448,8 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
     tc_fence_after_sync();
     const uint32_t tmem = *tmem_at;
 
-    bool nan = false;
+    bool nan = false, done = false;
+    float o[kHd], l[4] = {0.f, 0.f, 0.f, 0.f};                      // of the softmax warps
     if (warp == 4) {
         if (lane == 0) {
             // queries are in when the softmax warps say so (they add the bias first): their arrival is the first phase of o_free[0]
@@ -511,7 +512,7 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_o_free);
-        float o[kHd], m = -INFINITY, l[4] = {0.f, 0.f, 0.f, 0.f}, keep = 1.f;
+        float m = -INFINITY, keep = 1.f;
 #pragma unroll
         for (int f = 0; f < kHd; ++f) o[f] = 0.f;
         // adds the partial output of block it: o = o * factor + partial
@@ -584,22 +585,23 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
             if (lane == 0) mbar_arrive(bar_p_full + 8 * buf);
             if (it > 0 && !join(it - 1, last)) { ok = false; break; }
         }
-        ok = ok && join(rounds - 1, keep);
-        if (ok && q0 + row < seq) {
-            const float inv = 1.f / ((l[0] + l[1]) + (l[2] + l[3]));
+        done = ok && join(rounds - 1, keep) && q0 + row < seq;
+        if (done)
 #pragma unroll
             for (int f = 0; f < kHd; ++f) nan |= isnan(o[f]);
-            __half* dst = out + (int64_t)head * kHd * tokens + (int64_t)b * seq + q0 + row;
-#pragma unroll
-            for (int f = 0; f < kHd; ++f)
-                dst[f * tokens] = __float2half_rn(fmaf(o[f], inv, bias_v ? __half2float(bias_v[head * kHd + f]) : 0.f));
-        }
     }
     tc_fence_before_sync();
     nan = __syncthreads_or(nan);
     if (warp == 4) {
         tc_fence_after_sync();
         tmem_dealloc(tmem, kTcTmemCols);
+    }
+    if (done && !nan) {                                             // (out may be q, which a second pass reads again)
+        const float inv = 1.f / ((l[0] + l[1]) + (l[2] + l[3]));
+        __half* dst = out + (int64_t)head * kHd * tokens + (int64_t)b * seq + q0 + threadIdx.x;
+#pragma unroll
+        for (int f = 0; f < kHd; ++f)
+            dst[f * tokens] = __float2half_rn(fmaf(o[f], inv, bias_v ? __half2float(bias_v[head * kHd + f]) : 0.f));
     }
     // something infinite or NaN went in: again, with infinities and NaNs of v apart, 64 queries at a time
     if (nan && warp < 4) {

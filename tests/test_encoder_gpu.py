@@ -309,3 +309,18 @@ def test_attention_infinities_and_nans_with_many_tiles(lib, seq, scale):
     fin = ref.isfinite()
     slack = 2.0 ** -20 * (1 + score[score.isfinite()].abs().amax()) * (p @ split(v).abs())
     assert ((got - ref).abs()[fin] <= (2.0 ** -11 * ref.abs() + 2.0 ** -24 + slack)[fin]).all()
+
+
+@pytest.mark.parametrize("batch,seq", [(2, 72), (112, 136)])
+@pytest.mark.parametrize("finite", [True, False])
+def test_attention_into_its_queries(lib, batch, seq, finite):
+    """The result may take the queries' place, also where a tile is done twice because something infinite or NaN went in."""
+    from sspmm_b200 import ops
+    g = torch.Generator(device="cuda:0").manual_seed(seq)
+    q, k, v = (torch.randn(128, batch * seq, device="cuda:0", generator=g).half() for _ in range(3))
+    if not finite:
+        v[3, 5], v[70, seq - 1], v[90, 1] = float("inf"), -float("inf"), float("nan")
+    out = torch.empty_like(q)
+    ops.attention_fm(q, k, v, 2, batch, seq, out)
+    ops.attention_fm(q, k, v, 2, batch, seq, q)
+    assert torch.equal(q.view(torch.int16), out.view(torch.int16))
