@@ -266,6 +266,10 @@ int sspmm_add_bias_fm(int rows, int tokens, const void* x_f16, const void* bias_
  */
 int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* q_f16, const void* k_f16, const void* v_f16,
                        const void* bias_q_f16, const void* bias_v_f16, void* out_f16, void* stream);
+/* The same by a chosen kernel: 1 = 64 queries per CTA (mma.sync), 2 = 128 queries per CTA (tcgen05, operands by TMA), 0 = by size, as
+ * above.  taken (may be NULL): the one that was launched, 0 for none.  For tests and profiling. */
+int sspmm_attention_fm_as(int kernel, int heads, int head_dim, int batch, int seq, const void* q_f16, const void* k_f16, const void* v_f16,
+                          const void* bias_q_f16, const void* bias_v_f16, void* out_f16, void* stream, int* taken);
 
 /* ------------------------------------------------------------------- SVC --- */
 

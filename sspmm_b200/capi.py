@@ -32,6 +32,7 @@ SIGNATURES = {
     "sspmm_layer_norm_fm": (C.c_int, [C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, _vp, C.c_float, _vp, _vp]),
     "sspmm_add_bias_fm": (C.c_int, [C.c_int] * 2 + [_vp] * 5),
     "sspmm_attention_fm": (C.c_int, [C.c_int] * 4 + [_vp] * 7),
+    "sspmm_attention_fm_as": (C.c_int, [C.c_int] * 5 + [_vp] * 7 + [c_int_p]),
     "sspmm_group_run": (C.c_int, [_vp, _vp]),
     "sspmm_group_bias": (C.c_int, [_vp, C.c_int, _vp, c_int_p]),
     "sspmm_group_info": (C.c_int, [_vp, c_int_p, c_int_p, c_int_p, c_int_p, C.POINTER(C.c_int64)]),

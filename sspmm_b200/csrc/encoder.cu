@@ -698,7 +698,14 @@ int sspmm_add_bias_fm(int rows, int tokens, const void* x, const void* bias, con
 
 int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* q, const void* k, const void* v, const void* bias_q,
                        const void* bias_v, void* out, void* stream) {
+    return sspmm_attention_fm_as(0, heads, head_dim, batch, seq, q, k, v, bias_q, bias_v, out, stream, nullptr);
+}
+
+int sspmm_attention_fm_as(int kernel, int heads, int head_dim, int batch, int seq, const void* q, const void* k, const void* v,
+                          const void* bias_q, const void* bias_v, void* out, void* stream, int* taken) {
     set_error("%s", "");
+    if (taken) *taken = 0;
+    if (kernel < 0 || kernel > 2) { set_error("attention kernel must be 0, 1 or 2"); return (int)cudaErrorInvalidValue; }
     if (heads < 0 || batch < 0 || seq < 0 || head_dim != enc::kHd || seq % 8 != 0 || heads > 65535 || batch > 65535 || !q || !k || !v || !out ||
         !enc::piece_aligned(q) || !enc::piece_aligned(k) || !enc::piece_aligned(v) || !enc::piece_aligned(out)) {
         set_error("attention: bad argument (heads=%d head_dim=%d batch=%d seq=%d)", heads, head_dim, batch, seq);
@@ -716,7 +723,8 @@ int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* 
     const dim3 wide((seq + enc::kTcQueries - 1) / enc::kTcQueries, heads, batch);
     const int64_t tiles = (int64_t)wide.x * heads * batch;
     CUtensorMap tq, tk, tv;
-    enc::EncodeFn encode = 2 * tiles * ((seq - 1) / enc::kTile) >= 3 * sms ? enc::encode_fn() : nullptr;
+    const bool wanted = kernel == 2 || (kernel == 0 && 2 * tiles * ((seq - 1) / enc::kTile) >= 3 * sms);
+    enc::EncodeFn encode = wanted ? enc::encode_fn() : nullptr;
     if (encode && enc::encode_tokens(encode, &tq, q, heads * head_dim, batch, seq) &&
         enc::encode_tokens(encode, &tk, k, heads * head_dim, batch, seq) && enc::encode_tokens(encode, &tv, v, heads * head_dim, batch, seq)) {
         static DeviceOnce once;
@@ -727,9 +735,14 @@ int sspmm_attention_fm(int heads, int head_dim, int batch, int seq, const void* 
         }
         enc::attention_tc_kernel<<<wide, enc::kTcThreads, enc::TcSmem::kDynamic, st>>>(seq, tokens, tq, tk, tv, hq, hk, hv, bq, bv,
                                                                                         static_cast<__half*>(out));
+        if (taken) *taken = 2;
+    } else if (kernel == 2) {
+        set_error("attention: no tensor maps for these operands");
+        return (int)cudaErrorNotSupported;
     } else {
         const dim3 grid((seq + enc::kTile - 1) / enc::kTile, heads, batch);
         enc::attention_fm_kernel<<<grid, enc::kAttnThreads, 0, st>>>(seq, tokens, hq, hk, hv, bq, bv, static_cast<__half*>(out));
+        if (taken) *taken = 1;
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("attention launch: %s", cudaGetErrorString(e)); return (int)e; }

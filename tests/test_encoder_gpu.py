@@ -324,3 +324,50 @@ def test_attention_into_its_queries(lib, batch, seq, finite):
     ops.attention_fm(q, k, v, 2, batch, seq, out)
     ops.attention_fm(q, k, v, 2, batch, seq, q)
     assert torch.equal(q.view(torch.int16), out.view(torch.int16))
+
+
+def attend_by(lib, kernel, q, k, v, heads, batch, seq, biases=(None, None)):
+    import ctypes as C
+    out, taken = torch.full_like(q, float("nan")), C.c_int()
+    rc = lib.sspmm_attention_fm_as(kernel, heads, 64, batch, seq, q.data_ptr(), k.data_ptr(), v.data_ptr(),
+                                   *(None if b is None else b.data_ptr() for b in biases), out.data_ptr(),
+                                   torch.cuda.current_stream().cuda_stream, C.byref(taken))
+    assert rc == 0
+    return out, taken.value
+
+
+@pytest.mark.parametrize("heads,batch,seq,tc", [(8, 40, 64, False), (1, 1, 512, False), (3, 75, 72, True), (2, 120, 120, True), (4, 60, 128, True),
+                                                (1, 80, 200, True), (3, 3, 512, None), (1, 10, 1928, True)])
+def test_attention_takes_the_kernel_of_its_size(lib, heads, batch, seq, tc):
+    """Two thirds of the SMs times the blocks of keys after the first decide; the sizes are 3 % or more from the line of 148 SMs."""
+    q, k, v = (torch.randn(heads * 64, batch * seq, device="cuda:0").half() for _ in range(3))
+    out, taken = attend_by(lib, 0, q, k, v, heads, batch, seq)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert taken == (2 if 2 * -(-seq // 128) * heads * batch * ((seq - 1) // 64) >= 3 * sms else 1)
+    assert tc is None or sms != 148 or taken == (2 if tc else 1)
+    assert torch.equal(out, attend_by(lib, taken, q, k, v, heads, batch, seq)[0])
+
+
+@pytest.mark.parametrize("kernel", [1, 2])
+@pytest.mark.parametrize("heads,batch,seq,scale,finite", [(1, 1, 8, 1.0, True), (2, 3, 64, 1.0, True), (4, 2, 72, 3.0, True), (1, 2, 136, 6.0, True),
+                                                          (3, 1, 200, 0.1, True), (2, 1, 520, 1.0, True), (2, 2, 72, 1.0, False), (2, 3, 328, 0.5, False)])
+def test_attention_by_either_kernel(lib, kernel, heads, batch, seq, scale, finite):
+    """The same operands through both kernels, at sizes that the choice gives to one of them only; infinities and NaNs come out as in
+    the plain formula.  Bound: see test_attention_feature_major."""
+    g = torch.Generator(device="cuda:0").manual_seed(seq)
+    r = lambda s: (torch.randn((heads * 64, batch * seq), device="cuda:0", generator=g) * s).half()
+    q, k, v = r(scale), r(scale), r(1.0)
+    bq, bv = (torch.randn(heads * 64, device="cuda:0", generator=g).half() for _ in range(2))
+    if not finite:
+        inf = float("inf")
+        v[3, 5], v[10, seq - 1], v[70, 0], v[90, 1], v[90, seq - 2], v[127, seq + 7] = inf, -inf, inf, inf, -inf, float("nan")
+    out, taken = attend_by(lib, kernel, q, k, v, heads, batch, seq, (bq, bv))
+    assert taken == kernel
+    split = lambda t: t.double().view(heads, 64, batch, seq).permute(2, 0, 3, 1)
+    score = split(q + bq[:, None]) @ split(k).transpose(-1, -2) / 8
+    p = torch.softmax(score, -1)
+    ref, got = p @ split(v) + bv.double().view(heads, 64)[None, :, None, :], split(out)
+    assert torch.equal(ref.isnan(), got.isnan()) and torch.equal(ref.isposinf(), got.isposinf()) and torch.equal(ref.isneginf(), got.isneginf())
+    fin = ref.isfinite()
+    slack = 2.0 ** -20 * (1 + score.abs().amax()) * (p @ split(v).abs() + bv.double().abs().view(heads, 64)[None, :, None, :])
+    assert ((got - ref).abs()[fin] <= (2.0 ** -11 * ref.abs() + 2.0 ** -24 + slack)[fin]).all()
