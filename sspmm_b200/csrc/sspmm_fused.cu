@@ -1050,13 +1050,17 @@ std::vector<int> least_parts(const std::vector<Shape>& shapes, int units, int sm
     return least;
 }
 
-// Modelled time of the tile kernel with A tiles from the loader warps, in microseconds.  Fitted to groups of the conv layers at
-// N = 64 to 5000 and of encoder products (256 to 768 wide, 256 to 8192 columns), every width with and without cuts: a K
-// step takes 0.515 us whatever the width (the loaders set the pace), an item 1.2 more, the launch 6 to 7.  A cut tile's
-// parts are added by the CTA that finishes last, 0.85 us per part and 64 columns, and that is what cuts cost.
-// So tiles are as wide as leaves the rounds of items few, and only ranges much longer than an SM's share are cut: conv layers
-// at N = 800 take 67 us with 608 whole tiles of 256 columns, 133 with 1976 of 64 (as many tiles as give every SM two, the rule before);
-// N = 64: 47 with whole tiles, 29 cut; 768 x 3072 at N = 4096: 33 with 96 tiles of 256, 90 with 384 of 64.
+// Modelled time of the tile kernel with A tiles from the loader warps, in microseconds.  Fitted to encoder products (256 to 768 wide, 256
+// to 8192 columns) and, for the order of the candidates, to groups of the conv layers at N = 64 to 5000, every width with and
+// without cuts: a K step takes 0.515 us whatever the width (the loaders set the pace), an item 1.2 more, the launch 6 to 7.  A cut
+// tile's parts are added by the CTA that finishes last, 0.85 us per part and 64 columns, and that is what cuts cost.
+// Single products come out within 10 %, groups whose operands pass through HBM a quarter to a third too short (conv layers at N = 64 20
+// for 25, N = 800 45 for 68, N = 3136 124 for 173).
+// So tiles are as wide as leaves the rounds of items few, and only ranges much longer than an SM's share are cut.  Before, tiles
+// were as wide as left every SM two and cut to a third of an SM's work: conv layers at N = 400 94 us (552 items in up to seven
+// parts), 47 now (384); N = 800 132 (832, and copies of A), 68 (608 whole tiles); 768 x 3072 at N = 4096 91 (384 tiles of 64), 34 (96 of
+// 256).  Modes 1 to 3 get the same division: mode 2 65 for 94 us at N = 200, mode 3 71 for 123; small losses are left (three of
+// 768 x 768 at N = 128, mode 3, 33 us for 30).
 GroupChoice choose_tiles(const std::vector<Shape>& shapes, const std::vector<int>& least, int units, bool only_256) {
     GroupChoice best{256, {}, -1.0};
     std::vector<int> cuts(shapes.size());

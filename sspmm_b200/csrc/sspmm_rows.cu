@@ -403,7 +403,7 @@ sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int
 // More items than warps, one warp each: a CTA has its share of the items from the start, looks all of them up at once (a thread each, the
 // first column ids on their way to L1), and its warps take them one after another from a counter in shared memory.  With a CTA for
 // every eight items the look-ups, four dependent loads, were paid for by every round of CTAs, and a warp that was done waited for
-// the longest of its eight rows.  96 products of 512 x 512 at 90 %, N = 64: 12.6 us, now 10.3.
+// the longest of its eight rows.  96 products of 512 x 512 at 90 %, N = 64: 12.5 us, now 10.5.
 // Nothing is known of the rows' lengths here, so nothing is dealt to a warp ahead of time: with the items dealt to the warps in turn and
 // the next two looked up early, one row in a hundred of 512 vectors among rows of 5 took 32 us where the CTAs of eight took 19 (now
 // 15); what look-ups are left, half a microsecond a launch, shows with rows of ten vectors (7.7 us, dealt in turn 7.1).
@@ -467,7 +467,7 @@ sspmm_rows_set_kernel(const __grid_constant__ ProblemSet s, int team, int cluste
 }
 
 // Matrices whose rows differ in length by orders of magnitude (power-law matrices: half of the rows have fewer than 50
-// vectors, the longest tens of thousands; n = 51970, V = 8, N = 128: 46.8 us, with one CTA of tcgen05 stages per SM 67.8).
+// vectors, the longest tens of thousands; n = 51970, V = 8, N = 128: 40.8 us, with one CTA of tcgen05 stages per SM 67.8).
 // Rows longer than kLightRow are cut into parts of at most p.chunk vectors (listed by list_parts_kernel); a CTA does a
 // part with all its warps, the parts dealt out in turn since they are of one size, and whoever finishes the last part of
 // a row adds the parts up in order.  Rows of a single part follow those with several: they write C themselves and have no
