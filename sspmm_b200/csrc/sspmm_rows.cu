@@ -721,7 +721,8 @@ Scratch plan_scratch(const SpmmArgs& a, long long nvec) {
     }
     const long long nt = a.N <= 64 ? 64 : 128, n_tiles = (a.N + nt - 1) / nt;
     // A part: a quarter of an SM's share of the vectors, at least four steps per warp.  n = 51970 (820 k vectors, V = 8,
-    // N = 128) takes 46.8 us with a quarter, 52.1 with an eighth and 78 with a sixteenth (every part drains the rings once).
+    // N = 128) took 46.8 us with a quarter, 52.1 with an eighth and 78 with a sixteenth (every part drains the rings once; measured
+    // before the rings were on 128-byte boundaries, 40.8 now).
     long long c = nvec * n_tiles / ((long long)sms * 4) / 128 * 128;
     if (c < 512) c = 512;
     // A row with several parts has at most one that is not full, so its parts are fewer than twice its vectors / c; their

@@ -103,3 +103,20 @@ def test_wrapped_tensors_and_modes_are_left_to_python(product):
         got = ops.sspmm(ptr, col, val, torch.nn.Parameter(rhs), 8)
     s.synchronize()
     assert torch.equal(got, want) and not got.requires_grad
+
+
+def test_stacked_operands(product):
+    """Two operands one below the other against their products one by one, row orders included; what is not such a call is left alone."""
+    ptr, col, val, rhs = product
+    order, n = ops.sorted_row_swizzle(ptr), col.numel()
+    ptr2 = torch.cat([ptr[:1], ptr[1:-1] - (ptr[1:-1] > 0).int(), ptr[-1:]])              # other row ends, the same columns
+    cols, vals, bias = torch.cat([col, col]), torch.cat([val, val * 2]), torch.randn(144, device=DEV).half()
+    call = lambda ptrs=(ptr, ptr2), orders=(order, order), ends=(n, 2 * n), c=cols, v=vals, r=rhs, V=8, b=bias: \
+        ops.sspmm_stacked(list(ptrs), list(orders), list(ends), c, v, r, V, b)
+    want = torch.cat([ops.sspmm_bias(ptr, col, val, rhs, 8, bias[:72], order), ops.sspmm_bias(ptr2, col, val * 2, rhs, 8, bias[72:], order)])
+    assert torch.equal(call(), want)
+    five = [ptr] * 5
+    for other in (dict(ends=(n, 2 * n - 1)), dict(ends=(n + 1, n)), dict(ptrs=(ptr, ptr[:-1])), dict(orders=(order, order[:-1])), dict(c=cols[:-1]), dict(v=vals[8:]),
+                  dict(r=rhs.float()), dict(r=rhs.t()), dict(r=rhs.cpu()), dict(b=bias[:-1]), dict(b=None), dict(ptrs=(ptr, ptr.long())), dict(r=rhs[:, :20].contiguous()),
+                  dict(ptrs=five, orders=[order] * 5, ends=[n * i for i in range(1, 6)], c=col.repeat(5), v=val.repeat(5), b=bias[:72].repeat(5)), dict(ptrs=(), orders=(), ends=())):
+        assert call(**other) is None
