@@ -237,7 +237,8 @@ constexpr int kBigGroup = 1024;
 constexpr int kBigTeam = 1024;             // threads of such a CTA
 // Where every group gets a CTA it has 1024 threads as long as all are resident at once, else 256: with 2250 groups of 256 to 8000 entries
 // the larger ones took 116 to 131 us a call, 60 to 72 now (59 to 75 before groups got 1024 threads), with 256 groups of 37 k entries
-// (V = 16) 108 against 125.  Either fills an SM's threads, so neither may use more than 32 registers.
+// (V = 16) 108 against 125.  Those of 256 have to fill an SM's threads, with at most 32 registers (1000 groups of 18 k entries: 271 us
+// with 40, 241 with 32); those of 1024 are faster with what they take (the large groups of a stack of 16: 60 us, 62.5 with 32).
 constexpr int kTeam = 256;
 __device__ __forceinline__ bool group_passes(int filter, int entries) {
     return filter == 0 || (filter == 1) == (entries <= kBigGroup);
@@ -505,6 +506,8 @@ __device__ __forceinline__ int row_of_entry(const int* rows, int n_rows, int e) 
 template <class Team, class F>
 __device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* rows, int n_rows, F&& f) {
     const int e0 = rows[0];
+    const int* const cols = p.col_idx + e0;
+    const __half* const vals = p.vals + e0;
     const unsigned n_entries = (unsigned)max(0, rows[n_rows] - e0);
     for (unsigned e = Team::tid(); e < n_entries; e += 4 * Team::kSize) {
         int c[4];
@@ -512,8 +515,8 @@ __device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* r
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const unsigned x = e + b * Team::kSize;
-            c[b] = x < n_entries ? p.col_idx[e0 + x] : -1;
-            v[b] = x < n_entries ? p.vals[e0 + x] : __half(0);
+            c[b] = x < n_entries ? cols[x] : -1;
+            v[b] = x < n_entries ? vals[x] : __half(0);
         }
 #pragma unroll
         for (int b = 0; b < 4; ++b)
@@ -524,7 +527,7 @@ __device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* r
 // Bound by the latency of its look-ups, so the large groups get 1024 threads and every thread four entries at a time (conv weight of
 // 512 x 4608, 64 groups: 14.7 us with 256 threads and an entry each, 10.6 now, zeroing included).
 template <class Team>
-__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock, 2048 / (Team::kSize * Team::kPerBlock))
+__global__ void __launch_bounds__(Team::kSize * Team::kPerBlock, Team::kSize == kTeam ? 2048 / kTeam : 1)
 svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restrict__ vec_ptr,
                        const int* __restrict__ mode, int* __restrict__ out_col, __half* __restrict__ out_vals,
                        const int* __restrict__ list, int n_list) {
