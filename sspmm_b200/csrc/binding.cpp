@@ -15,6 +15,8 @@
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <vector>
+
 #include "../../include/sspmm_b200.h"
 
 namespace {
@@ -281,6 +283,82 @@ PyObject* py_svc(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// svc_batch(list of (row_ptr, col_idx, values or None, M, K), vec_length, list of entries per matrix or None)
+//   -> (list of (vec_ptr, vec_col, vec_values or None), replayed rows)
+PyObject* py_svc_batch(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long V;
+        if (n != 3 || modes_active() || !PyList_CheckExact(a[0]) || !small_int(a[1], 1, 1 << 20, &V) || (a[2] != Py_None && !PyList_CheckExact(a[2])))
+            Py_RETURN_NONE;
+        const Py_ssize_t count = PyList_GET_SIZE(a[0]);
+        if (count < 1 || count > 0x7fffffff || (a[2] != Py_None && PyList_GET_SIZE(a[2]) != count)) Py_RETURN_NONE;
+        std::vector<int> M((size_t)count), K((size_t)count), nnz((size_t)count);
+        std::vector<const int*> ptrs((size_t)count), cols((size_t)count);
+        std::vector<const void*> vals((size_t)count);
+        bool with_values = true;
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            PyObject* const m = PyList_GET_ITEM(a[0], i);
+            if (!PyTuple_CheckExact(m) || PyTuple_GET_SIZE(m) != 5) Py_RETURN_NONE;
+            with_values = with_values && PyTuple_GET_ITEM(m, 2) != Py_None;
+        }
+        const at::Tensor* first = nullptr;
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            PyObject* const m = PyList_GET_ITEM(a[0], i);
+            long rows, width, entries;
+            const at::Tensor *ptr = plain(PyTuple_GET_ITEM(m, 0), at::kInt), *col = plain(PyTuple_GET_ITEM(m, 1), at::kInt);
+            const at::Tensor* val = with_values ? plain(PyTuple_GET_ITEM(m, 2), at::kHalf) : nullptr;
+            if (!ptr || !col || (with_values && !val) || !small_int(PyTuple_GET_ITEM(m, 3), 0, 0x7ffffff0, &rows) ||
+                !small_int(PyTuple_GET_ITEM(m, 4), 0, 0x7fffffff, &width))
+                Py_RETURN_NONE;
+            if (a[2] == Py_None) entries = col->numel() <= 0x7fffffff ? (long)col->numel() : -1;
+            else if (!small_int(PyList_GET_ITEM(a[2], i), 0, 0x7fffffff, &entries)) Py_RETURN_NONE;
+            if (!first) first = ptr;
+            if (entries < 0 || ptr->device() != first->device() || col->device() != first->device() || (val && val->device() != first->device()))
+                Py_RETURN_NONE;
+            M[i] = (int)rows; K[i] = (int)width; nnz[i] = (int)entries;
+            ptrs[i] = static_cast<const int*>(ptr->data_ptr());
+            cols[i] = static_cast<const int*>(col->data_ptr());
+            vals[i] = val ? val->data_ptr() : nullptr;
+        }
+        const c10::cuda::CUDAGuard guard(first->device());
+        struct Job {
+            svc_batch_job* job = nullptr;
+            ~Job() { svc_batch_free(job); }
+        } j;
+        std::vector<int64_t> nvec((size_t)count);
+        int64_t replayed = 0, total = 0, vec_rows = 0;
+        const auto ints = first->options().requires_grad(false);
+        int rc = launch(first->get_device(), [&](void* st) {
+            return svc_batch_begin((int)count, (int)V, M.data(), K.data(), nnz.data(), ptrs.data(), cols.data(), with_values ? vals.data() : nullptr, st,
+                                   &j.job, nvec.data());
+        });
+        if (rc != 0) return PyLong_FromLong(rc);
+        for (Py_ssize_t i = 0; i < count; ++i) { total += nvec[i]; vec_rows += (M[i] + V - 1) / V; }
+        at::Tensor out_ptr = at::empty({vec_rows + (int64_t)count}, ints), out_col = at::empty({total}, ints), out_val;
+        if (with_values) out_val = at::empty({total * V}, ints.dtype(at::kHalf));
+        rc = launch(first->get_device(), [&](void* st) {
+            const int e = svc_batch_replayed_rows(j.job, &replayed);
+            return e != 0 ? e : svc_batch_finish(j.job, static_cast<int*>(out_ptr.data_ptr()), static_cast<int*>(out_col.data_ptr()),
+                                                 with_values ? out_val.data_ptr() : nullptr, st);
+        });
+        if (rc != 0) return PyLong_FromLong(rc);
+        PyObject* const list = PyList_New(count);
+        if (!list) return nullptr;
+        int64_t po = 0, vo = 0;
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            const int64_t rows = (M[i] + V - 1) / V + 1;
+            PyObject* values = Py_None;
+            if (with_values) values = THPVariable_Wrap(out_val.narrow(0, vo * V, nvec[i] * V)); else Py_INCREF(Py_None);
+            PyObject* const item = Py_BuildValue("(NNN)", THPVariable_Wrap(out_ptr.narrow(0, po, rows)), THPVariable_Wrap(out_col.narrow(0, vo, nvec[i])), values);
+            if (!item) { Py_DECREF(list); return nullptr; }
+            PyList_SET_ITEM(list, i, item);
+            po += rows;
+            vo += nvec[i];
+        }
+        return Py_BuildValue("(NL)", list, (long long)replayed);
+    });
+}
+
 // sorted_row_swizzle(row_offsets)
 PyObject* py_sorted_row_swizzle(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -296,6 +374,7 @@ PyObject* py_sorted_row_swizzle(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyMethodDef methods[] = {
     {"svc", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_svc)), METH_FASTCALL, nullptr},
+    {"svc_batch", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_svc_batch)), METH_FASTCALL, nullptr},
     {"sorted_row_swizzle", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sorted_row_swizzle)), METH_FASTCALL, nullptr},
     {"sspmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sspmm)), METH_FASTCALL, nullptr},
     {"stacked", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_stacked)), METH_FASTCALL, nullptr},

@@ -294,6 +294,45 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
     return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
 }
 
+// Host memory that kernels write the numbers to which the host waits for (counts of a compression): the copy that came after the
+// scans, into pageable memory, took as long as they did.  64 slots, 256 KB, allocated at the first use; a compression
+// holds one while it waits, and copies to its own memory when there is none.
+class HostSlots {
+public:
+    static constexpr size_t kBytes = 4096;
+    void* take() {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (!base_ && !failed_) {
+            void* p = nullptr;
+            if (cudaHostAlloc(&p, 64 * kBytes, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) base_ = static_cast<uint8_t*>(p);
+            else { cudaGetLastError(); failed_ = true; }
+        }
+        if (!base_ || used_ == ~0ull) return nullptr;
+        int k = 0;
+        while (used_ >> k & 1ull) ++k;
+        used_ |= 1ull << k;
+        return base_ + k * kBytes;
+    }
+    void give_back(void* slot) {
+        if (!slot) return;
+        std::lock_guard<std::mutex> lk(mu_);
+        used_ &= ~(1ull << ((static_cast<uint8_t*>(slot) - base_) / kBytes));
+    }
+private:
+    std::mutex mu_;
+    uint8_t* base_ = nullptr;
+    unsigned long long used_ = 0;
+    bool failed_ = false;
+};
+static HostSlots g_slots;
+struct HostSlot {
+    void* const at = g_slots.take();
+    ~HostSlot() { g_slots.give_back(at); }
+    HostSlot() = default;
+    HostSlot(const HostSlot&) = delete;
+    HostSlot& operator=(const HostSlot&) = delete;
+};
+
 }  // namespace sspmm_b200
 
 using namespace sspmm_b200;
@@ -319,6 +358,83 @@ struct svc_batch_job {
     long long* d_cuts;
     cudaStream_t stream;
 };
+
+// First half of a compression: counting and scans are enqueued.  slot: host memory for the totals, or null.
+static int svc_count(int M, int K, int vec_length, const int* d_csr_row_ptr, const int* d_csr_col_idx, const void* d_csr_values_f16, void* stream,
+                     void* slot, svc_job** job) {
+    if (vec_length != 8 && vec_length != 16) {
+        set_error("vec_length must be 8 or 16 (got %d)", vec_length);
+        return (int)cudaErrorInvalidValue;
+    }
+    if (M < 0 || K < 0) { set_error("negative dimension"); return (int)cudaErrorInvalidValue; }
+    if (K > kSvcMaxK) {
+        set_error("K = %d exceeds the supported maximum of %d columns", K, kSvcMaxK);
+        return (int)cudaErrorInvalidValue;
+    }
+    // d_csr_col_idx may be NULL when the matrix has no entries (it is then never read)
+    if (!d_csr_row_ptr) { set_error("null CSR row pointer"); return (int)cudaErrorInvalidValue; }
+    svc_job* j = new (std::nothrow) svc_job();
+    if (!j) return (int)cudaErrorMemoryAllocation;
+    memset(j, 0, sizeof *j);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    j->stream = st;
+    cudaGetDevice(&j->device);
+    j->p.M = M; j->p.K = K; j->p.V = vec_length; j->p.m_vec = (M + vec_length - 1) / vec_length;
+    j->p.row_ptr = d_csr_row_ptr; j->p.col_idx = d_csr_col_idx;
+    j->p.vals = static_cast<const __half*>(d_csr_values_f16);
+    j->with_values = d_csr_values_f16 != nullptr;
+    const size_t mv = (size_t)j->p.m_vec;
+    // one allocation: vec_ptr[mv+1] | mode[mv] | tbl_len[mv] | class_list[mv] | queue[8] | pad | tbl_off[mv+1] | totals
+    const size_t ints = (mv + 1) + mv + mv + mv + 8;
+    const size_t ints_padded = (ints + 3) & ~(size_t)3;
+    const size_t scan_blocks = (size_t)svc_scan_blocks((long long)mv);
+    const size_t bytes = ints_padded * 4 + (mv + 1 + kSvcTotals + scan_blocks * kSvcScanFields) * 8;
+    void* base = nullptr;
+    keep_pool_memory();
+    cudaError_t e = cudaMallocAsync(&base, bytes, st);
+    if (e != cudaSuccess) { delete j; return fail(e, "scratch allocation"); }
+    j->s.vec_ptr = static_cast<int*>(base);
+    j->s.mode = j->s.vec_ptr + mv + 1;
+    j->s.tbl_len = j->s.mode + mv;
+    j->s.class_list = j->s.tbl_len + mv;
+    j->s.queue = j->s.class_list + mv;
+    j->s.tbl_off = reinterpret_cast<long long*>(static_cast<int*>(base) + ints_padded);
+    j->s.totals = j->s.tbl_off + mv + 1;
+    j->s.block_sums = j->s.totals + kSvcTotals;
+    j->s.tables = nullptr;
+    j->s.host_totals = static_cast<long long*>(slot);
+    e = svc_count_and_scan(j->p, j->s, j->with_values, st);
+    if (e != cudaSuccess) {
+        if (slot) cudaStreamSynchronize(st);          // what was launched may write to the slot
+        cudaFreeAsync(base, st);
+        delete j;
+        return fail(e, "SVC counting pass");
+    }
+    *job = j;
+    return 0;
+}
+
+// Second half: waits for the totals, and checks them.  The job is gone when this fails.
+static int svc_counted(svc_job* j, const void* slot, cudaStream_t st) {
+    long long totals[kSvcTotals] = {0};
+    cudaError_t e = slot ? cudaSuccess : cudaMemcpyAsync(totals, j->s.totals, sizeof totals, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess && slot) memcpy(totals, slot, sizeof totals);
+    j->s.host_totals = nullptr;
+    const int bad = (int)totals[2 + kSvcSegs];
+    if (e != cudaSuccess || bad || totals[0] > 0x7fffffffLL) {
+        cudaFreeAsync(j->s.vec_ptr, st);
+        delete j;
+        if (e != cudaSuccess) return fail(e, "SVC counting pass");
+        if (bad) set_error("CSR column id outside [0, K)");
+        else set_error("more than 2^31-1 vectors");
+        return (int)cudaErrorInvalidValue;
+    }
+    j->nvec = totals[0];
+    j->table_ints = totals[1];
+    for (int c = 0; c < kSvcSegs; ++c) j->class_groups[c] = totals[2 + c];
+    return 0;
+}
 
 extern "C" {
 
@@ -489,63 +605,12 @@ int svc_begin(int M, int K, int vec_length, const int* d_csr_row_ptr, const int*
     g_err[0] = 0;
     if (!job || !nvec) { set_error("null output pointer"); return (int)cudaErrorInvalidValue; }
     *job = nullptr;
-    if (vec_length != 8 && vec_length != 16) {
-        set_error("vec_length must be 8 or 16 (got %d)", vec_length);
-        return (int)cudaErrorInvalidValue;
-    }
-    if (M < 0 || K < 0) { set_error("negative dimension"); return (int)cudaErrorInvalidValue; }
-    if (K > kSvcMaxK) {
-        set_error("K = %d exceeds the supported maximum of %d columns", K, kSvcMaxK);
-        return (int)cudaErrorInvalidValue;
-    }
-    // d_csr_col_idx may be NULL when the matrix has no entries (it is then never read)
-    if (!d_csr_row_ptr) { set_error("null CSR row pointer"); return (int)cudaErrorInvalidValue; }
-    svc_job* j = new (std::nothrow) svc_job();
-    if (!j) return (int)cudaErrorMemoryAllocation;
-    memset(j, 0, sizeof *j);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    j->stream = st;
-    cudaGetDevice(&j->device);
-    j->p.M = M; j->p.K = K; j->p.V = vec_length; j->p.m_vec = (M + vec_length - 1) / vec_length;
-    j->p.row_ptr = d_csr_row_ptr; j->p.col_idx = d_csr_col_idx;
-    j->p.vals = static_cast<const __half*>(d_csr_values_f16);
-    j->with_values = d_csr_values_f16 != nullptr;
-    const size_t mv = (size_t)j->p.m_vec;
-    // one allocation: vec_ptr[mv+1] | mode[mv] | tbl_len[mv] | class_list[mv] | queue[8] | pad | tbl_off[mv+1] | totals
-    const size_t ints = (mv + 1) + mv + mv + mv + 8;
-    const size_t ints_padded = (ints + 3) & ~(size_t)3;
-    const size_t scan_blocks = (size_t)svc_scan_blocks((long long)mv);
-    const size_t bytes = ints_padded * 4 + (mv + 1 + kSvcTotals + scan_blocks * kSvcScanFields) * 8;
-    void* base = nullptr;
-    keep_pool_memory();
-    cudaError_t e = cudaMallocAsync(&base, bytes, st);
-    if (e != cudaSuccess) { delete j; return fail(e, "scratch allocation"); }
-    j->s.vec_ptr = static_cast<int*>(base);
-    j->s.mode = j->s.vec_ptr + mv + 1;
-    j->s.tbl_len = j->s.mode + mv;
-    j->s.class_list = j->s.tbl_len + mv;
-    j->s.queue = j->s.class_list + mv;
-    j->s.tbl_off = reinterpret_cast<long long*>(static_cast<int*>(base) + ints_padded);
-    j->s.totals = j->s.tbl_off + mv + 1;
-    j->s.block_sums = j->s.totals + kSvcTotals;
-    j->s.tables = nullptr;
-    e = svc_count_and_scan(j->p, j->s, j->with_values, st);
-    long long totals[kSvcTotals] = {0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(totals, j->s.totals, sizeof totals, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    const int bad = (int)totals[2 + kSvcSegs];
-    if (e != cudaSuccess || bad || totals[0] > 0x7fffffffLL) {
-        cudaFreeAsync(base, st);
-        delete j;
-        if (e != cudaSuccess) return fail(e, "SVC counting pass");
-        if (bad) set_error("CSR column id outside [0, K)");
-        else set_error("more than 2^31-1 vectors");
-        return (int)cudaErrorInvalidValue;
-    }
-    j->nvec = totals[0];
-    j->table_ints = totals[1];
-    for (int c = 0; c < kSvcSegs; ++c) j->class_groups[c] = totals[2 + c];
-    *nvec = totals[0];
+    const HostSlot slot;
+    svc_job* j = nullptr;
+    int rc = svc_count(M, K, vec_length, d_csr_row_ptr, d_csr_col_idx, d_csr_values_f16, stream, slot.at, &j);
+    if (rc == 0) rc = svc_counted(j, slot.at, static_cast<cudaStream_t>(stream));
+    if (rc != 0) return rc;
+    *nvec = j->nvec;
     *job = j;
     return 0;
 }
@@ -554,9 +619,11 @@ int svc_finish(svc_job* j, int* d_vec_row_ptr, int* d_vec_col, void* d_vec_value
     g_err[0] = 0;
     if (!j || !d_vec_row_ptr || (j->nvec > 0 && !d_vec_col)) { set_error("null pointer"); return (int)cudaErrorInvalidValue; }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t e = cudaMemcpyAsync(d_vec_row_ptr, j->s.vec_ptr, ((size_t)j->p.m_vec + 1) * 4, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) return fail(e, "row pointer copy");
-    if (j->nvec == 0) return 0;
+    cudaError_t e = cudaSuccess;
+    if (j->nvec == 0) {
+        e = cudaMemcpyAsync(d_vec_row_ptr, j->s.vec_ptr, ((size_t)j->p.m_vec + 1) * 4, cudaMemcpyDeviceToDevice, st);
+        return e == cudaSuccess ? 0 : fail(e, "row pointer copy");
+    }
     __half* ov = j->with_values ? static_cast<__half*>(d_vec_values_f16) : nullptr;
     j->p.zero_values = aligned16(ov);
     if (ov && !j->p.zero_values) {
@@ -567,7 +634,7 @@ int svc_finish(svc_job* j, int* d_vec_row_ptr, int* d_vec_col, void* d_vec_value
         e = cudaMallocAsync(reinterpret_cast<void**>(&j->s.tables), (size_t)j->table_ints * 4, st);
         if (e != cudaSuccess) return fail(e, "table scratch allocation");
     }
-    e = svc_emit(j->p, j->s, j->class_groups, d_vec_col, ov, st);
+    e = svc_emit(j->p, j->s, j->class_groups, d_vec_row_ptr, d_vec_col, ov, st);
     if (e != cudaSuccess) return fail(e, "SVC emit");
     j->stream = st;
     return 0;
@@ -642,21 +709,31 @@ int svc_batch_begin(int count, int vec_length, const int* M, const int* K, const
     int* s_ptr = reinterpret_cast<int*>(base + off_ptr);
     int* s_col = reinterpret_cast<int*>(base + off_col);
     __half* s_val = with_values ? reinterpret_cast<__half*>(base + off_val) : nullptr;
-    e = cudaMemcpyAsync(b->d_tab, tab.data(), tab.size() * sizeof(SvcBatchEntry), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);          // `tab` is pageable host memory about to go out of scope
-    if (e == cudaSuccess) e = svc_stack(b->d_tab, count, rows, entries, V, s_ptr, s_col, s_val, st);
-    int64_t total_nvec = 0;
+    e = svc_stack(tab.data(), b->d_tab, count, rows, entries, s_ptr, s_col, s_val, st);
+    // the cuts go to the slot behind the totals, where there is room, and one wait is for both
+    const HostSlot slot;
+    constexpr size_t kCutsAt = 256;
+    static_assert(kSvcTotals * 8 <= kCutsAt, "cuts behind the totals");
+    long long* const near = slot.at && kCutsAt + ((size_t)count + 1) * 8 <= HostSlots::kBytes
+                                ? reinterpret_cast<long long*>(static_cast<uint8_t*>(slot.at) + kCutsAt) : nullptr;
     int rc = 0;
     if (e == cudaSuccess) {
-        rc = svc_begin((int)rows, k_max, V, s_ptr, s_col, s_val, stream, &b->inner, &total_nvec);
+        rc = svc_count((int)rows, k_max, V, s_ptr, s_col, s_val, stream, slot.at, &b->inner);
         if (rc == 0) {
-            e = svc_batch_cuts(b->d_tab, count, b->inner->s.vec_ptr, b->d_cuts, st);
-            std::vector<long long> cuts((size_t)count + 1);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(cuts.data(), b->d_cuts, cuts.size() * 8, cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            if (e == cudaSuccess)
-                for (int i = 0; i < count; ++i) nvec[i] = cuts[i + 1] - cuts[i];
+            e = svc_batch_cuts(b->d_tab, count, b->inner->s.vec_ptr, b->d_cuts, near, st);
+            rc = svc_counted(b->inner, slot.at, st);
+            if (rc != 0) b->inner = nullptr;
         }
+        std::vector<long long> copied;
+        const long long* cuts = near;
+        if (e == cudaSuccess && rc == 0 && !near) {
+            copied.resize((size_t)count + 1);
+            e = cudaMemcpyAsync(copied.data(), b->d_cuts, copied.size() * 8, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            cuts = copied.data();
+        }
+        if (e == cudaSuccess && rc == 0)
+            for (int i = 0; i < count; ++i) nvec[i] = cuts[i + 1] - cuts[i];
     }
     if (e != cudaSuccess || rc != 0) {
         if (b->inner) svc_free(b->inner);
@@ -689,7 +766,7 @@ int svc_batch_finish(svc_batch_job* b, int* d_vec_row_ptr, int* d_vec_col, void*
         e = cudaMallocAsync(reinterpret_cast<void**>(&j->s.tables), (size_t)j->table_ints * 4, st);
         if (e != cudaSuccess) return fail(e, "table scratch allocation");
     }
-    e = svc_emit(j->p, j->s, j->class_groups, d_vec_col, ov, st);
+    e = svc_emit(j->p, j->s, j->class_groups, nullptr, d_vec_col, ov, st);
     if (e != cudaSuccess) return fail(e, "SVC emit");
     j->stream = st;
     b->stream = st;

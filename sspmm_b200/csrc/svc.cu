@@ -410,7 +410,7 @@ svc_scan_sums_kernel(int m_vec, const int* __restrict__ counts, const int* __res
 
 // One CTA: block_sums -> exclusive prefixes in place, and the totals; a warp per field.
 __global__ void __launch_bounds__(32 * kScanFields)
-svc_scan_blocks_kernel(int n_blocks, long long* __restrict__ block_sums, long long* __restrict__ totals) {
+svc_scan_blocks_kernel(int n_blocks, long long* __restrict__ block_sums, long long* __restrict__ totals, long long* __restrict__ host_totals) {
     const int field = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long carry = 0;
     for (int b0 = 0; b0 < n_blocks; b0 += 32) {
@@ -425,9 +425,13 @@ svc_scan_blocks_kernel(int n_blocks, long long* __restrict__ block_sums, long lo
         if (b < n_blocks) block_sums[(size_t)b * kScanFields + field] = carry + inc - v;
         carry += __shfl_sync(0xffffffffu, inc, 31);
     }
-    if (lane == 0) totals[field] = carry;
+    if (lane == 0) {
+        totals[field] = carry;
+        if (host_totals) host_totals[field] = carry;
+    }
     if (threadIdx.x == 0) {
         totals[kScanFields] = g_svc_bad_column;          // reported with the totals, then cleared
+        if (host_totals) host_totals[kScanFields] = g_svc_bad_column;
         g_svc_bad_column = 0;
     }
 }
@@ -438,7 +442,7 @@ template <bool ALONE>
 __global__ void __launch_bounds__(kScanThreads)
 svc_scan_place_kernel(int m_vec, int* __restrict__ vec_ptr, const int* __restrict__ tbl_len,
                       long long* __restrict__ tbl_off, const long long* __restrict__ block_sums,
-                      long long* __restrict__ totals, int* __restrict__ class_list) {
+                      long long* __restrict__ totals, long long* __restrict__ host_totals, int* __restrict__ class_list) {
     __shared__ long long sh[2][32];
     __shared__ int seg[kNumSegs], seg_at[kNumSegs];
     if (threadIdx.x < kNumSegs) seg[threadIdx.x] = 0;
@@ -471,12 +475,17 @@ svc_scan_place_kernel(int m_vec, int* __restrict__ vec_ptr, const int* __restric
         if (it.cls[j] > 0) class_list[seg_at[it.cls[j]] + it.rank[j]] = i;
     }
     if (ALONE) {
-        if (threadIdx.x < kNumSegs) totals[2 + threadIdx.x] = seg[threadIdx.x];
+        auto report = [&](int field, long long v) {
+            totals[field] = v;
+            if (host_totals) host_totals[field] = v;
+        };
+        if (threadIdx.x < kNumSegs) report(2 + threadIdx.x, seg[threadIdx.x]);
         if (threadIdx.x == 0) {
-            totals[0] = total_a; totals[1] = total_b;
+            report(0, total_a);
+            report(1, total_b);
             vec_ptr[m_vec] = (int)total_a;
             tbl_off[m_vec] = total_b;
-            totals[kScanFields] = g_svc_bad_column;          // reported with the totals, then cleared
+            report(kScanFields, g_svc_bad_column);           // reported with the totals, then cleared
             g_svc_bad_column = 0;
         }
     } else if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -529,7 +538,7 @@ __device__ __forceinline__ void for_each_value(const SvcProblem& p, const int* r
 template <class Team>
 __global__ void __launch_bounds__(Team::kSize * Team::kPerBlock, Team::kSize == kTeam ? 2048 / kTeam : 1)
 svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restrict__ vec_ptr,
-                       const int* __restrict__ mode, int* __restrict__ out_col, __half* __restrict__ out_vals,
+                       const int* __restrict__ mode, int* __restrict__ out_ptr, int* __restrict__ out_col, __half* __restrict__ out_vals,
                        const int* __restrict__ list, int n_list) {
     extern __shared__ unsigned int sm_words[];
     __shared__ int red[33], all_rows[Team::kPerBlock * kRowInts];
@@ -541,6 +550,10 @@ svc_emit_sorted_kernel(SvcProblem p, int words, int filter, const int* __restric
     const int n_loop = list ? n_list : p.m_vec;
     for (int k = blockIdx.x * Team::kPerBlock + Team::index_in_block(); k < n_loop; k += gridDim.x * Team::kPerBlock) {
         const int i = list ? list[k] : k;
+        if (out_ptr && tid == 0) {
+            out_ptr[i] = vec_ptr[i];
+            if (i == p.m_vec - 1) out_ptr[p.m_vec] = vec_ptr[p.m_vec];
+        }
         if (mode[i] != 0) continue;
         const int r0 = min(i * p.V, p.M), n_rows = min(i * p.V + p.V, p.M) - r0;
         const int e0 = p.row_ptr[r0], e1 = p.row_ptr[r0 + n_rows];
@@ -1258,17 +1271,17 @@ cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool /*
     }
     const int n_blocks = p.m_vec > 0 ? (p.m_vec + kScanBlock - 1) / kScanBlock : 1;
     if (n_blocks == 1) {
-        svc_scan_place_kernel<true><<<1, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, nullptr, s.totals, s.class_list);
+        svc_scan_place_kernel<true><<<1, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, nullptr, s.totals, s.host_totals, s.class_list);
         return cudaGetLastError();
     }
     svc_scan_sums_kernel<<<n_blocks, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.block_sums);
-    svc_scan_blocks_kernel<<<1, 32 * kScanFields, 0, stream>>>(n_blocks, s.block_sums, s.totals);
-    svc_scan_place_kernel<false><<<n_blocks, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, s.block_sums, s.totals,
+    svc_scan_blocks_kernel<<<1, 32 * kScanFields, 0, stream>>>(n_blocks, s.block_sums, s.totals, s.host_totals);
+    svc_scan_place_kernel<false><<<n_blocks, kScanThreads, 0, stream>>>(p.m_vec, s.vec_ptr, s.tbl_len, s.tbl_off, s.block_sums, s.totals, nullptr,
                                                                  s.class_list);
     return cudaGetLastError();
 }
 
-cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* seg_groups, int* out_col,
+cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* seg_groups, int* out_ptr, int* out_col,
                      __half* out_vals, cudaStream_t stream) {
     if (p.m_vec == 0) return cudaSuccess;
     const int sms = device_sm_count();
@@ -1279,11 +1292,6 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
     if (e == cudaSuccess) e = allow_big_smem(svc_emit_sorted_kernel<WarpTeam>, once_warp, 208 * 1024);
     if (e != cudaSuccess) return e;
 
-    // the work counters of the replay classes, cleared before the side streams fork off
-    e = cudaMemsetAsync(s.queue, 0, 8 * sizeof(int), stream);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(g_aux_mu);
-    Fork f(aux_for_device(), stream);
     // groups per class and where the class starts in the list of replayed groups
     long long class_groups[kNumClasses] = {0}, first[kNumClasses] = {0};
     class_groups[kClassSorted] = seg_groups[0] + seg_groups[kSegSortedBig];
@@ -1297,19 +1305,37 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
         for (int k = 1; k < s0; ++k) first[c] += seg_groups[k];
         for (int k = s0; k < s1; ++k) class_groups[c] += seg_groups[k];
     }
+    long long replayed = 0;
+    for (int c = 1; c < kNumClasses; ++c) replayed += class_groups[c];
+    // the work counters of the replay classes, cleared before the side streams fork off
+    if (replayed > 0) {
+        e = cudaMemsetAsync(s.queue, 0, 8 * sizeof(int), stream);
+        if (e != cudaSuccess) return e;
+    }
+    // Side streams only for launches that there are: a record or a wait costs the caller half a microsecond and the device's front end
+    // more (weights without replayed groups: 6 records and 10 waits around one launch).
+    const bool one_cta_each = p.m_vec <= 16 * sms || (size_t)WarpTeam::kPerBlock * words * 8 > 200 * 1024;
+    const bool forks = replayed > 0 || (n_big > 0 && !one_cta_each);
+    std::unique_lock<std::mutex> lk(g_aux_mu, std::defer_lock);
+    if (forks) lk.lock();
+    Fork f(forks ? aux_for_device() : nullptr, stream);
+    if (out_ptr && class_groups[kClassSorted] == 0) {
+        e = cudaMemcpyAsync(out_ptr, s.vec_ptr, ((size_t)p.m_vec + 1) * 4, cudaMemcpyDeviceToDevice, stream);
+        if (e != cudaSuccess) return e;
+    }
     if (class_groups[kClassSorted] > 0) {
         const size_t warp_smem = (size_t)WarpTeam::kPerBlock * words * 8;
-        if (p.m_vec <= 16 * sms || warp_smem > 200 * 1024) {
+        if (one_cta_each) {
             const int grid = p.m_vec < sms * 16 ? p.m_vec : sms * 16;
-            if (p.m_vec <= 2 * sms) svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals, nullptr, 0);
-            else svc_emit_sorted_kernel<BlockTeam<kTeam>><<<grid, kTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_col, out_vals, nullptr, 0);
+            if (p.m_vec <= 2 * sms) svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<grid, kBigTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_ptr, out_col, out_vals, nullptr, 0);
+            else svc_emit_sorted_kernel<BlockTeam<kTeam>><<<grid, kTeam, (size_t)words * 8, stream>>>(p, words, 0, s.vec_ptr, s.mode, out_ptr, out_col, out_vals, nullptr, 0);
         } else {
             int grid = (p.m_vec + WarpTeam::kPerBlock - 1) / WarpTeam::kPerBlock;
             if (grid > sms * 8) grid = sms * 8;
-            svc_emit_sorted_kernel<WarpTeam><<<grid, 256, warp_smem, stream>>>(p, words, 1, s.vec_ptr, s.mode, out_col, out_vals, nullptr, 0);
+            svc_emit_sorted_kernel<WarpTeam><<<grid, 256, warp_smem, stream>>>(p, words, 1, s.vec_ptr, s.mode, out_ptr, out_col, out_vals, nullptr, 0);
             if (n_big > 0) {
                 const int big_grid = n_big < sms * 2 ? n_big : sms * 2;
-                svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<big_grid, kBigTeam, (size_t)words * 8, f.next()>>>(p, words, 2, s.vec_ptr, s.mode, out_col,
+                svc_emit_sorted_kernel<BlockTeam<kBigTeam>><<<big_grid, kBigTeam, (size_t)words * 8, f.next()>>>(p, words, 2, s.vec_ptr, s.mode, nullptr, out_col,
                                                                                                      out_vals, big_list, n_big);
             }
         }
@@ -1317,15 +1343,15 @@ cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* 
         if (e != cudaSuccess) return e;
     }
     // the largest groups first: they are the critical path
-    auto replay = [&](auto kernel, int c, cudaStream_t st) {
-        if (e == cudaSuccess) e = kernel(p, s, out_col, out_vals, class_groups[c], first[c], st);
+    auto replay = [&](auto kernel, int c, bool aside) {
+        if (e == cudaSuccess && class_groups[c] > 0) e = kernel(p, s, out_col, out_vals, class_groups[c], first[c], aside ? f.next() : stream);
     };
-    replay(launch_replay<kClassXL, 0>, kClassXL, f.next());
-    replay(p.K <= 1 << 17 ? launch_replay<kClassL, 17> : launch_replay<kClassL, 0>, kClassL, f.next());
-    replay(launch_replay<kClassM2, 18>, kClassM2, f.next());
-    replay(launch_replay<kClassM1, 18>, kClassM1, f.next());
-    replay(launch_replay<kClassS, 18>, kClassS, f.next());
-    replay(launch_replay<kClassXS, 18>, kClassXS, stream);
+    replay(launch_replay<kClassXL, 0>, kClassXL, true);
+    replay(p.K <= 1 << 17 ? launch_replay<kClassL, 17> : launch_replay<kClassL, 0>, kClassL, true);
+    replay(launch_replay<kClassM2, 18>, kClassM2, true);
+    replay(launch_replay<kClassM1, 18>, kClassM1, true);
+    replay(launch_replay<kClassS, 18>, kClassS, true);
+    replay(launch_replay<kClassXS, 18>, kClassXS, false);
     if (e != cudaSuccess) return e;
     return f.join();
 }
@@ -1344,29 +1370,72 @@ __device__ __forceinline__ int owner_of(long long x, int count, F base_of) {
     return lo;
 }
 
+// Bound by its copies (6 bytes per entry each way).  A CTA takes runs of kStackRun positions: it looks the matrix of a run's first
+// position up in the table (in shared memory when it came with the launch) and the threads walk on from there, four loads of each array under way.  Stack of 16,
+// 5.3 M entries: 24 us with a search in global memory for every entry.
+constexpr int kStackRun = 1024;
+struct SvcStackTable {
+    SvcBatchEntry e[kSvcParamEntries + 1];
+};
+// in_params: the table is in `given`, and CTA 0 also writes it to d_tab; else it is in d_tab.
 __global__ void __launch_bounds__(256)
-svc_stack_kernel(const SvcBatchEntry* __restrict__ tab, int count, long long rows, long long entries, int* __restrict__ row_ptr,
-                 int* __restrict__ col_idx, __half* __restrict__ vals) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (long long r = t0; r <= rows; r += stride) {
-        if (r == rows) { row_ptr[r] = (int)entries; continue; }
-        const int m = owner_of(r, count, [&](int k) { return tab[k].row_base; });
-        const long long lr = r - tab[m].row_base;
-        row_ptr[r] = (int)(tab[m].nnz_base + (lr < tab[m].M ? tab[m].row_ptr[lr] : tab[m].nnz));
+svc_stack_kernel(const __grid_constant__ SvcStackTable given, bool in_params, SvcBatchEntry* __restrict__ d_tab, int count, long long rows,
+                 long long entries, int* __restrict__ row_ptr, int* __restrict__ col_idx, __half* __restrict__ vals) {
+    __shared__ SvcBatchEntry near[kSvcParamEntries + 1];
+    const SvcBatchEntry* tab = d_tab;
+    if (in_params) {
+        constexpr int kWords = sizeof(SvcBatchEntry) / 4;
+        for (int x = threadIdx.x; x < (count + 1) * kWords; x += 256) {
+            const int v = reinterpret_cast<const int*>(given.e)[x];
+            reinterpret_cast<int*>(near)[x] = v;
+            if (blockIdx.x == 0) reinterpret_cast<int*>(d_tab)[x] = v;
+        }
+        __syncthreads();
+        tab = near;
     }
-    for (long long e = t0; e < entries; e += stride) {
-        const int m = owner_of(e, count, [&](int k) { return tab[k].nnz_base; });
-        const long long le = e - tab[m].nnz_base;
-        col_idx[e] = tab[m].col_idx[le];
-        if (vals) vals[e] = tab[m].vals[le];
+    const long long step = (long long)gridDim.x * kStackRun;
+    for (long long r0 = (long long)blockIdx.x * kStackRun; r0 <= rows; r0 += step) {
+        int m = owner_of(r0, count, [&](int k) { return tab[k].row_base; });
+#pragma unroll
+        for (int b = 0; b < kStackRun / 256; ++b) {
+            const long long r = r0 + b * 256 + threadIdx.x;
+            if (r > rows) break;
+            if (r == rows) { row_ptr[r] = (int)entries; break; }
+            while (m + 1 < count && tab[m + 1].row_base <= r) ++m;
+            const long long lr = r - tab[m].row_base;
+            row_ptr[r] = (int)(tab[m].nnz_base + (lr < tab[m].M ? tab[m].row_ptr[lr] : tab[m].nnz));
+        }
+    }
+    for (long long e0 = (long long)blockIdx.x * kStackRun; e0 < entries; e0 += step) {
+        int m = owner_of(e0, count, [&](int k) { return tab[k].nnz_base; });
+        int c[kStackRun / 256];
+        __half v[kStackRun / 256];
+#pragma unroll
+        for (int b = 0; b < kStackRun / 256; ++b) {
+            const long long e = e0 + b * 256 + threadIdx.x;
+            if (e >= entries) break;
+            while (m + 1 < count && tab[m + 1].nnz_base <= e) ++m;
+            const long long le = e - tab[m].nnz_base;
+            c[b] = __ldg(tab[m].col_idx + le);
+            if (vals) v[b] = tab[m].vals[le];
+        }
+#pragma unroll
+        for (int b = 0; b < kStackRun / 256; ++b) {
+            const long long e = e0 + b * 256 + threadIdx.x;
+            if (e >= entries) break;
+            col_idx[e] = c[b];
+            if (vals) vals[e] = v[b];
+        }
     }
 }
 
 __global__ void svc_batch_cuts_kernel(const SvcBatchEntry* __restrict__ tab, int count, const int* __restrict__ vec_ptr,
-                                      long long* __restrict__ cuts) {
+                                      long long* __restrict__ cuts, long long* __restrict__ host_cuts) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m <= count) cuts[m] = vec_ptr[tab[m].vec_row_base];
+    if (m > count) return;
+    const long long v = vec_ptr[tab[m].vec_row_base];
+    cuts[m] = v;
+    if (host_cuts) host_cuts[m] = v;
 }
 
 __global__ void __launch_bounds__(256)
@@ -1382,20 +1451,29 @@ svc_batch_row_ptrs_kernel(const SvcBatchEntry* __restrict__ tab, int count, long
 }
 }  // namespace
 
-cudaError_t svc_stack(const SvcBatchEntry* tab, int count, long long rows, long long entries, int V, int* row_ptr,
+cudaError_t svc_stack(const SvcBatchEntry* tab, SvcBatchEntry* d_tab, int count, long long rows, long long entries, int* row_ptr,
                       int* col_idx, __half* vals, cudaStream_t stream) {
-    (void)V;
     const long long work = (rows + 1 > entries ? rows + 1 : entries);
-    long long blocks = (work + 255) / 256;
-    const long long cap = (long long)device_sm_count() * 16;
+    long long blocks = (work + kStackRun - 1) / kStackRun;
+    const long long cap = (long long)device_sm_count() * 8;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
-    svc_stack_kernel<<<(int)blocks, 256, 0, stream>>>(tab, count, rows, entries, row_ptr, col_idx, vals);
+    static_assert(sizeof(SvcStackTable) <= 4000, "the table fits the parameters of a launch");
+    SvcStackTable given;
+    const bool in_params = count <= kSvcParamEntries;
+    if (in_params) {
+        for (int k = 0; k <= count; ++k) given.e[k] = tab[k];
+    } else {
+        cudaError_t e = cudaMemcpyAsync(d_tab, tab, ((size_t)count + 1) * sizeof(SvcBatchEntry), cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);          // `tab` is pageable memory of the caller
+        if (e != cudaSuccess) return e;
+    }
+    svc_stack_kernel<<<(int)blocks, 256, 0, stream>>>(given, in_params, d_tab, count, rows, entries, row_ptr, col_idx, vals);
     return cudaGetLastError();
 }
 
-cudaError_t svc_batch_cuts(const SvcBatchEntry* tab, int count, const int* vec_ptr, long long* cuts, cudaStream_t stream) {
-    svc_batch_cuts_kernel<<<(count + 1 + 255) / 256, 256, 0, stream>>>(tab, count, vec_ptr, cuts);
+cudaError_t svc_batch_cuts(const SvcBatchEntry* tab, int count, const int* vec_ptr, long long* cuts, long long* host_cuts, cudaStream_t stream) {
+    svc_batch_cuts_kernel<<<(count + 1 + 255) / 256, 256, 0, stream>>>(tab, count, vec_ptr, cuts, host_cuts);
     return cudaGetLastError();
 }
 

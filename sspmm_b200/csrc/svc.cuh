@@ -34,6 +34,7 @@ struct SvcScratch {
     int* class_list;      // [m_vec]    replayed groups, class by class (written by the scan)
     int* queue;           // [8]        work counters of the replay classes
     long long* block_sums;  // [svc_scan_blocks(m_vec) * kSvcScanFields] partial sums of the scans
+    long long* host_totals; // null, or host memory that the scans write the totals to as well
 };
 
 // Number of blocks the scan kernels cut m_vec groups into.
@@ -48,7 +49,8 @@ constexpr int kSvcScanFields = 2 + kSvcSegs;   // numbers per block of the scans
 cudaError_t svc_count_and_scan(const SvcProblem& p, const SvcScratch& s, bool with_values, cudaStream_t stream);
 // Pass 2: emits column lists (and value vectors when out_vals != null, which must be zero-filled unless p.zero_values).
 // seg_groups = totals[2..2+kSvcSegs) read back by the host (launches are skipped for empty classes).
-cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* seg_groups, int* out_col,
+// out_ptr: null, or where the vector row pointers are copied to.
+cudaError_t svc_emit(const SvcProblem& p, const SvcScratch& s, const long long* seg_groups, int* out_ptr, int* out_col,
                      __half* out_vals, cudaStream_t stream);
 
 // ---- batches: several independent matrices compressed as one stacked matrix ----------------
@@ -64,11 +66,14 @@ struct SvcBatchEntry {
     long long vec_row_base;  // first stacked vector row
     int M, nnz;
 };
-// tab has count + 1 entries (the last one carries the totals).  Builds the stacked CSR.
-cudaError_t svc_stack(const SvcBatchEntry* tab, int count, long long rows, long long entries, int V, int* row_ptr,
+// tab has count + 1 entries (the last one carries the totals) in host memory; device memory for them is written.  Builds the stacked
+// CSR.  Up to kSvcParamEntries of them travel with the launch;
+// more are copied, and the call waits for the copy.
+constexpr int kSvcParamEntries = 60;
+cudaError_t svc_stack(const SvcBatchEntry* tab, SvcBatchEntry* d_tab, int count, long long rows, long long entries, int* row_ptr,
                       int* col_idx, __half* vals, cudaStream_t stream);
-// cuts[m] = vec_ptr[first vector row of matrix m] for m in 0..count.
-cudaError_t svc_batch_cuts(const SvcBatchEntry* tab, int count, const int* vec_ptr, long long* cuts, cudaStream_t stream);
+// cuts[m] = vec_ptr[first vector row of matrix m] for m in 0..count; host_cuts: null, or host memory that gets them as well.
+cudaError_t svc_batch_cuts(const SvcBatchEntry* tab, int count, const int* vec_ptr, long long* cuts, long long* host_cuts, cudaStream_t stream);
 // out: for every matrix its m_vec + 1 row pointers, rebased to 0, matrices one after another.
 cudaError_t svc_batch_row_ptrs(const SvcBatchEntry* tab, int count, long long vec_rows, const int* vec_ptr,
                                const long long* cuts, int* out, cudaStream_t stream);

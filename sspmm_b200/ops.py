@@ -153,6 +153,9 @@ def svc_batch(mats, vec_length: int, nnz=None):
     import ctypes as C
     if not mats:
         return [], 0
+    got = capi.native().svc_batch(mats, vec_length, nnz)
+    if got is not None:
+        return _made(got)
     V = vec_length
     n = len(mats)
     dev = mats[0][0].device
