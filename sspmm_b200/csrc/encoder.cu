@@ -33,12 +33,14 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 // ---- LayerNorm ------------------------------------------------------------------------------------
-// Bound by memory: x (and add) read once, out (and the sum) written once.  A CTA takes TT tokens and keeps their features in
-// shared memory between the passes for the mean, the variance and the result, so nothing is read twice; a thread works on
-// eight tokens (16 bytes) of every (256 * 8 / TT)-th feature.  TT = 32 gives 64-byte runs; with few tokens TT = 8 spreads
-// them over more SMs.  768 x 16384: 300 us as eleven torch launches (fp32 copies, mean, variance, five broadcasts),
-// 20 us here.
-constexpr int kLnThreads = 256;
+// Bound by memory: x (and add) read once, out (and the sum) written once.  A CTA takes TT tokens and keeps what it has read for the passes
+// for the mean, the variance and the result: in shared memory, or, where 32 tokens per CTA give every SM one and there are
+// at most 1024 features, in the registers of 512 threads.  32 tokens give 64-byte runs; with few tokens TT = 8 spreads
+// them over more SMs.  Through shared memory, 768 x 16384 took 24.0 us, with a sum 40.2: every thread added up the warps' sums for
+// itself (64 reads twice), converted every element three times and worked on one element per instruction.  From registers, with pairs
+// of elements per instruction and sums that are added up once, 16.6 and 24.8 (operands that change from call to call; 5000 tokens 14.0
+// and 20.1, now 9.5 and 12.5; 256 x 16384 10.6 and 14.5, now 10.3 and 12.3).  256 threads with twice the registers take 17.1 and 36.6.
+constexpr int kLnThreads = 256, kLnWideThreads = 512;
 template <int TT>
 __global__ void __launch_bounds__(kLnThreads)
 layer_norm_fm_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
@@ -118,6 +120,164 @@ layer_norm_fm_kernel(int hidden, int tokens, const __half* __restrict__ x, const
         for (int e = 0; e < 8; ++e) f[e] = (f[e] - mean[e]) * var[e] * g + b;
         if (in) *reinterpret_cast<uint4*>(out + (int64_t)r * tokens + t0) = pack8(f);
     }
+}
+
+// Two fp32 numbers in one register pair; an instruction works on both, each rounded to nearest as by itself.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair_of(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 floats_of(f32x2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ void unpack4(const uint4& x, f32x2 (&f)[4]) {
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        f[i] = pair_of(v.x, v.y);
+    }
+}
+__device__ __forceinline__ uint4 pack4(const f32x2 (&f)[4]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 v = floats_of(f[i]);
+        const __half2 h = __floats2half2_rn(v.x, v.y);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The same with a thread's share in registers: 32 tokens, up to 128 * NV features.
+template <int NV>
+__global__ void __launch_bounds__(kLnWideThreads, 2)
+layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
+                          __half* __restrict__ sum_out, const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps,
+                          __half* __restrict__ out) {
+    constexpr int TT = 32, P = TT / 8, kRows = kLnWideThreads / P;
+    __shared__ float red[kLnWideThreads / 32][TT];
+    __shared__ __align__(16) float whole[2][TT];
+    const int piece = threadIdx.x % P, r0 = threadIdx.x / P, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * TT + piece * 8;
+    const bool in = t0 < tokens;
+    // Sums over the features of eight numbers per token, the same in every thread of the piece.  A lane hands on half of what it has at each
+    // step (7 shuffles; 24 with every sum in every lane), and one warp adds up for the CTA.
+    auto total = [&](f32x2 (&f)[4], float (&sums)[TT]) {
+        f32x2 h[2];
+        const bool upper = lane & 16, odd = lane & 8;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) h[e] = add2(upper ? f[2 + e] : f[e], __shfl_xor_sync(0xffffffffu, upper ? f[e] : f[2 + e], 16));
+        const float2 q = floats_of(add2(odd ? h[1] : h[0], __shfl_xor_sync(0xffffffffu, odd ? h[0] : h[1], 8)));
+        const float own = lane & 4 ? q.y : q.x, other = lane & 4 ? q.x : q.y;
+        red[warp][piece * 8 + (lane >> 4) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1)] = own + __shfl_xor_sync(0xffffffffu, other, 4);
+        __syncthreads();
+        if (warp == 0) {
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < kLnWideThreads / 32; ++w) t += red[w][lane];
+            sums[lane] = t;
+        }
+        __syncthreads();
+        const float4 lo = *reinterpret_cast<const float4*>(&sums[piece * 8]), hi = *reinterpret_cast<const float4*>(&sums[piece * 8 + 4]);
+        f[0] = pair_of(lo.x, lo.y); f[1] = pair_of(lo.z, lo.w); f[2] = pair_of(hi.x, hi.y); f[3] = pair_of(hi.z, hi.w);
+    };
+    const int last = in ? (hidden - r0 + kRows - 1) / kRows : 0;               // pieces of this thread
+    const int64_t at0 = (int64_t)r0 * tokens + t0, turn = (int64_t)kRows * tokens;
+    uint4 v[NV];
+    // The passes unpack v anew: without this the compiler keeps 8 * NV floats from one to the next, and spills.
+    auto forget = [&]() {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) asm volatile("" : "+r"(v[j].x), "+r"(v[j].y), "+r"(v[j].z), "+r"(v[j].w));
+    };
+#pragma unroll
+    for (int j = 0; j < NV; ++j) v[j] = j < last ? __ldg(reinterpret_cast<const uint4*>(x + at0 + j * turn)) : make_uint4(0, 0, 0, 0);
+    if (bias)
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+            if (j < last) {
+                f32x2 f[4];
+                unpack4(v[j], f);
+                const float b = __half2float(__ldg(bias + r0 + j * kRows));
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f[e] = add2(f[e], pair_of(b, b));
+                v[j] = pack4(f);
+            }
+    if (add)
+#pragma unroll
+        for (int j0 = 0; j0 < NV; j0 += 2) {
+            uint4 a[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) a[q] = j0 + q < last ? __ldg(reinterpret_cast<const uint4*>(add + at0 + (j0 + q) * turn)) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                f32x2 f[4], g[4];
+                unpack4(v[j0 + q], f);
+                unpack4(a[q], g);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f[e] = add2(f[e], g[e]);
+                v[j0 + q] = pack4(f);
+                if (j0 + q < last) *reinterpret_cast<uint4*>(sum_out + at0 + (j0 + q) * turn) = v[j0 + q];
+            }
+        }
+    forget();
+    f32x2 mean[4] = {0, 0, 0, 0}, var[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        f32x2 f[4];
+        unpack4(v[j], f);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mean[e] = add2(mean[e], f[e]);                 // (pieces past the last are zeros)
+    }
+    total(mean, whole[0]);
+    forget();
+    const float inv = 1.f / (float)hidden;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) mean[e] = mul2(mean[e], pair_of(-inv, -inv));      // its negative
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+        if (j < last) {
+            f32x2 f[4];
+            unpack4(v[j], f);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { const f32x2 d = add2(f[e], mean[e]); var[e] = fma2(d, d, var[e]); }
+        }
+    total(var, whole[1]);
+    forget();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 s = floats_of(var[e]);
+        var[e] = pair_of(rsqrtf(fmaf(s.x, inv, eps)), rsqrtf(fmaf(s.y, inv, eps)));
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+        if (j < last) {
+            f32x2 f[4];
+            unpack4(v[j], f);
+            const float g = __half2float(__ldg(gamma + r0 + j * kRows)), b = __half2float(__ldg(beta + r0 + j * kRows));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) f[e] = fma2(mul2(add2(f[e], mean[e]), var[e]), pair_of(g, g), pair_of(b, b));
+            *reinterpret_cast<uint4*>(out + at0 + j * turn) = pack4(f);
+        }
 }
 
 // out = x + bias + add, rounded after each addition; one 16-byte piece per thread.
@@ -659,19 +819,28 @@ int sspmm_layer_norm_fm(int hidden, int tokens, const void* x, const void* bias,
     if (sms <= 0) return (int)cudaErrorNoDevice;
     // 32 tokens per CTA once that gives every SM one
     const bool wide = tokens >= 32 * sms;
-    auto kern = wide ? enc::layer_norm_fm_kernel<32> : enc::layer_norm_fm_kernel<8>;
-    const int TT = wide ? 32 : 8;
-    const size_t smem = (size_t)hidden * TT * 2;
-    static DeviceOnce once_wide, once_narrow;
-    DeviceOnce& once = wide ? once_wide : once_narrow;
-    if (!once.done()) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * TT * 2);
-        if (e != cudaSuccess) { set_error("LayerNorm: %s", cudaGetErrorString(e)); return (int)e; }
-        once.mark();
+    auto go = [&](auto kern, int TT, int threads, size_t smem) {
+        kern<<<(tokens + TT - 1) / TT, threads, smem, static_cast<cudaStream_t>(stream)>>>(
+            hidden, tokens, static_cast<const __half*>(x), static_cast<const __half*>(bias), static_cast<const __half*>(add), static_cast<__half*>(sum_out),
+            static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, static_cast<__half*>(out));
+    };
+    if (wide && hidden <= 1024) {
+        if (hidden <= 256) go(enc::layer_norm_fm_regs_kernel<2>, 32, enc::kLnWideThreads, 0);
+        else if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<4>, 32, enc::kLnWideThreads, 0);
+        else if (hidden <= 768) go(enc::layer_norm_fm_regs_kernel<6>, 32, enc::kLnWideThreads, 0);
+        else go(enc::layer_norm_fm_regs_kernel<8>, 32, enc::kLnWideThreads, 0);
+    } else {
+        auto kern = wide ? enc::layer_norm_fm_kernel<32> : enc::layer_norm_fm_kernel<8>;
+        const int TT = wide ? 32 : 8;
+        static DeviceOnce once_wide, once_narrow;
+        DeviceOnce& once = wide ? once_wide : once_narrow;
+        if (!once.done()) {
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * TT * 2);
+            if (e != cudaSuccess) { set_error("LayerNorm: %s", cudaGetErrorString(e)); return (int)e; }
+            once.mark();
+        }
+        go(kern, TT, enc::kLnThreads, (size_t)hidden * TT * 2);
     }
-    kern<<<(tokens + TT - 1) / TT, enc::kLnThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        hidden, tokens, static_cast<const __half*>(x), static_cast<const __half*>(bias), static_cast<const __half*>(add), static_cast<__half*>(sum_out),
-        static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, static_cast<__half*>(out));
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("LayerNorm launch: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
