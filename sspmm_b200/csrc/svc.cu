@@ -27,16 +27,17 @@
 //                      fixed length is "first come, first served" along each key's
 //                      probe path, which has a unique fixed point: slot = the first
 //                      one on my path not held by an earlier element.  The team finds
-//                      it in parallel with atomicMin on words that hold the element's
+//                      it in parallel with atomic minima on words that hold the element's
 //                      sequence number and its column; table growth steps are replayed
-//                      level by level (8, 32, 128, ...).  What bounds it is the longest
-//                      chain of elements that push one another on, one after another
-//                      (rows are ascending and so come to sit in runs), so the tables
-//                      of a rebuild are kept and the next one starts from them.
+//                      level by level (8, 32, 128, ...).  Small tables are filled in batches
+//                      of the sequence whose losers go on in rounds (BitTable,
+//                      insert_batches); the tables of large sets are kept from one rebuild
+//                      to the next, which starts from them (relevel).
 //                      Stack of 16 power-law matrices (n 4096 to 65536, V = 8), whole
-//                      call: 3080 to 3450 us with every rebuild from free tables and
-//                      sequences apart from the tables, 1141 now; per launch, classes L,
-//                      M2, M1, S, XS 680, 573, 367, 235, 295 us one after another.
+//                      call: 877 us; 1033 with every small table filled by all elements at
+//                      once, 3080 to 3450 also with free tables at every rebuild.  Per launch,
+//                      classes L, M2, M1, S, XS 613, 454, 276, 189, 199 us one after another
+//                      (600, 503, 436, 228, 286 before batches).
 // The replay kernels take their groups from per-class lists (written by the scan kernel)
 // through a work counter, so a CTA never walks over groups of other classes and the
 // groups of a class, whose cost differs by an order of magnitude, balance themselves.
@@ -180,7 +181,6 @@ struct WarpTeam {
     __device__ static int tid() { return threadIdx.x & 31; }
     __device__ static int index_in_block() { return threadIdx.x >> 5; }
     __device__ static void sync() { __syncwarp(); }
-    __device__ static bool any(bool p, int*) { return __any_sync(0xffffffffu, p); }
     __device__ static int sum(int v, int*) { return warp_sum(v); }
     __device__ static int max_of(int v, int*) { return warp_max(v); }
     __device__ static int broadcast(int v, int*) { return __shfl_sync(0xffffffffu, v, 0); }   // value of thread 0
@@ -189,7 +189,7 @@ struct WarpTeam {
 template <int THREADS>
 struct BlockTeam {
     static constexpr int kSize = THREADS;
-    static constexpr int kPerBlock = 1;
+    [[maybe_unused]] static constexpr int kPerBlock = 1;
     __device__ static int tid() { return threadIdx.x; }
     __device__ static int index_in_block() { return 0; }
     __device__ static void sync() { __syncthreads(); }
@@ -673,6 +673,8 @@ struct SharedWords {
         asm volatile("atom.shared.min.u32 %0, [%1], %2;" : "=r"(old) : "r"(at + 4u * i), "r"(v) : "memory");
         return old;
     }
+    __device__ __forceinline__ void claim(unsigned i, unsigned v) const { asm volatile("red.shared.min.u32 [%0], %1;" ::"r"(at + 4u * i), "r"(v) : "memory"); }
+    __device__ __forceinline__ void set(unsigned i, unsigned v) const { asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(at + 4u * i), "r"(v) : "memory"); }
     __device__ __forceinline__ bool give_up(unsigned i, unsigned v) const {        // frees the slot if it still holds v
         unsigned old;
         asm volatile("atom.shared.cas.b32 %0, [%1], %2, %3;" : "=r"(old) : "r"(at + 4u * i), "r"(v), "r"(kFree) : "memory");
@@ -686,6 +688,7 @@ struct GlobalWords {
     __device__ __forceinline__ void st(unsigned i, unsigned v) const { __stcg(at + i, v); }
     __device__ __forceinline__ void free4(unsigned i) const { __stcg(reinterpret_cast<uint4*>(at + i), make_uint4(kFree, kFree, kFree, kFree)); }
     __device__ __forceinline__ unsigned take(unsigned i, unsigned v) const { return atomicMin(at + i, v); }
+    __device__ __forceinline__ void claim(unsigned i, unsigned v) const { atomicMin(at + i, v); }
     __device__ __forceinline__ bool give_up(unsigned i, unsigned v) const { return atomicCAS(at + i, v, kFree) == v; }
 };
 
@@ -700,25 +703,151 @@ struct GlobalList {
     __device__ __forceinline__ void st(unsigned i, unsigned v) const { asm volatile("st.global.u32 [%0], %1;" ::"l"(at + i), "r"(v) : "memory"); }
 };
 
-constexpr int kWarpLevels = 128;      // tables up to this length are done by one warp also in a CTA team
+// A bit per slot that is taken; a word more than the table needs, since windows are read as two words.
+// to_free: to the first free slot on the path from position p on (a table is never more than 60 % full, and the jumps reach every slot).
+__device__ __forceinline__ void to_free(const SharedWords& bits, Probe& p, unsigned mask) {
+    for (;;) {
+        const unsigned at = p.i >> 5;
+        const unsigned window = __funnelshift_r(bits.ld(at), bits.ld(at + 1), p.i & 31u);
+        const unsigned open = ~window & (p.i + kLinearProbes <= mask ? (2u << kLinearProbes) - 1u : 1u) & (~0u << p.w);
+        if (open) {
+            p.w = __ffs(open) - 1;
+            return;
+        }
+        p.perturb >>= kPerturbShift;
+        p.i = (p.i * 5u + 1u + p.perturb) & mask;
+        p.w = 0;
+    }
+}
+
+// A table that one warp fills in insertion order, 32 elements at a time: a word per slot, (number << 18 | column) or kFree.  Lanes claim
+// their slots by an atomic minimum and look who has them; those that lost go on, all at once.  Few rounds do (2.5 to 5 per batch
+// for sets from power-law matrices, whatever the length of the table), and there is no chain of elements that push one another
+// on.  Elements of later batches come after all that is in the table: a bit per slot says what is taken, and a lane reads the ten
+// bits of its window and has its first free slot.  (A match of the lanes' slots in place of the claims holds the warp for some 230 cycles: twice
+// the time.  The first batch, which is all of most sets, through the bits as well: 258 us for 31 k sets of up to 76 columns, now 196.)
+struct BitTable {
+    static constexpr int kShift = 18;
+    SharedWords words, bits;
+    __device__ __forceinline__ static unsigned column_of(unsigned w) { return w & ((1u << kShift) - 1u); }
+    // The first n columns of the list into the table, emptied to `size` slots, and back to the list in slot order.
+    template <class List>
+    __device__ __forceinline__ void reorder(const List& list, int n, int size) const {
+        const unsigned mask = (unsigned)size - 1u;
+        const int lane = threadIdx.x & 31;
+        for (int w = lane * 4; w < size; w += 128) words.free4(w);
+        {
+            const bool in = lane < n;
+            const unsigned column = in ? list.ld(lane) : 0u, me = (unsigned)lane << kShift | column;
+            Probe p = probe_begin(column, mask);
+            __syncwarp();
+            if (in) words.claim(p.i, me);
+            for (;;) {
+                __syncwarp();
+                const bool lost = in && words.ld(p.i + p.w) != me;
+                if (!__any_sync(0xffffffffu, lost)) break;
+                if (lost) {
+                    probe_advance(p, mask);
+                    words.claim(p.i + p.w, me);
+                }
+            }
+            if (n > 32) {
+                for (int w = lane; w <= size >> 5; w += 32) bits.st(w, 0u);
+                __syncwarp();
+                bits.set((p.i + p.w) >> 5, 1u << ((p.i + p.w) & 31u));
+                __syncwarp();
+            }
+        }
+        for (int q0 = 32; q0 < n; q0 += 32) {
+            const bool in = q0 + lane < n;
+            const unsigned column = in ? list.ld(q0 + lane) : 0u, me = (unsigned)(q0 + lane) << kShift | column;
+            Probe p = probe_begin(column, mask);
+            if (in) {
+                to_free(bits, p, mask);
+                words.claim(p.i + p.w, me);
+            }
+            for (;;) {
+                __syncwarp();
+                const bool lost = in && words.ld(p.i + p.w) != me;
+                if (!__any_sync(0xffffffffu, lost)) break;
+                if (lost) {
+                    ++p.w;
+                    to_free(bits, p, mask);
+                    words.claim(p.i + p.w, me);
+                }
+            }
+            if (in) bits.set((p.i + p.w) >> 5, 1u << ((p.i + p.w) & 31u));
+            __syncwarp();
+        }
+        int done = 0;
+#pragma unroll 4
+        for (int s0 = 0; s0 < size; s0 += 32) {
+            const unsigned w = s0 + lane < size ? words.ld(s0 + lane) : kFree;
+            const unsigned taken = __ballot_sync(0xffffffffu, w != kFree);
+            if (w != kFree) list.st(done + __popc(taken & ((1u << lane) - 1u)), column_of(w));
+            done += __popc(taken);
+        }
+        __syncwarp();
+    }
+    // Slot of a column; false: it is not in the table.
+    __device__ __forceinline__ bool find(unsigned mask, unsigned column, unsigned& slot) const {
+        Probe p = probe_begin(column, mask);
+        for (unsigned n = 0; n <= 8u * mask + 64u; ++n) {
+            slot = p.i + p.w;
+            const unsigned w = words.ld(slot);
+            if (w == kFree) return false;
+            if (column_of(w) == column) return true;
+            probe_advance(p, mask);
+        }
+        return false;
+    }
+    // The bits of the whole table, and in counts how many slots are taken before each word of them; then rank is a slot's place in the order.
+    __device__ __forceinline__ void index(const SharedWords& counts, int size) const {
+        const int lane = threadIdx.x & 31;
+        int done = 0;
+        for (int s0 = 0; s0 < size; s0 += 32) {
+            const unsigned taken = __ballot_sync(0xffffffffu, s0 + lane < size && words.ld(s0 + lane) != kFree);
+            if (lane == 0) {
+                bits.st(s0 >> 5, taken);
+                counts.st(s0 >> 5, (unsigned)done);
+            }
+            done += __popc(taken);
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ int rank(const SharedWords& counts, unsigned slot) const {
+        return (int)counts.ld(slot >> 5) + __popc(bits.ld(slot >> 5) & ((1u << (slot & 31u)) - 1u));
+    }
+};
+
+constexpr int kWarpLevels = 128;      // CTA teams: tables up to this length are done by one warp
+constexpr int kWarpLevelBits = 8;     // words of their bits (five are in use)
+// Longer tables, up to this length, are filled in batches by teams of up to 512 threads, and are empty at the start of every level; the others
+// are kept from one rebuild to the next.  Rows of neighbours take as many rounds as they are long, which a CTA of 1024 pays for most: stack of 16
+// (V = 8), classes M1 and M2 394 and 487 us with kept tables, 263 and 453 so (12 matrices, V = 16: 502 and 937, 527 and 701), class L 578
+// with kept tables, 1110 with batches up to 2048 slots, 1772 at all lengths.
+constexpr int kBatchLevels = 2048;
 
 // A set being rebuilt.  `list` is the insertion sequence: what the set held, in its order, then the row's new columns; a level's
 // extraction writes the order of its table over the part that the level inserted.  A slot's word is the number of its
 // element in the list and, packed (SHIFT bits), its column; unpacked the column is looked up in the list.  After the last level
 // of the last rebuild the number is the position in the ordered set, so a word also answers where a column went.
-// Packed, every level above kWarpLevels has a table of its own, which stays for the next rebuild: between two rebuilds its words
-// have the number kVacant (later than every element's), which a new element takes like a free slot.
+// Tables up to BATCH slots are empty at the start of a level.  Packed, every longer level has a table of its own behind them, which
+// stays for the next rebuild: between two rebuilds its words have the number kVacant (later than every element's), which a new element takes
+// like a free slot.
 enum class After { kFreed, kVacated, kNumbered };     // what becomes of a level's words when its order has been read
-template <class Words, class List, int SHIFT>
+template <class Words, class List, int SHIFT, int BATCH>
 struct HashSet {
     Words tab;
     List list;
+    SharedWords bits;         // of the table of a batch level
     GlobalWords ext;          // unpacked only: extraction goes here first, since words refer to the list
     static constexpr bool kPacked = SHIFT > 0;
+    static constexpr int kBatch = BATCH;
     static constexpr unsigned kVacant = kPacked ? ((1u << (32 - SHIFT)) - 2u) << SHIFT : kFree;      // words from here on name no element
-    // where the table of a level starts (lengths above kWarpLevels grow by four as long as words are packed)
-    __device__ __forceinline__ static unsigned start(int size) { return kPacked && size > kWarpLevels ? (unsigned)(size - kWarpLevels) / 3u : 0u; }
-    __device__ __forceinline__ HashSet level(int size) const { return HashSet{tab.part(start(size)), list, ext}; }
+    // where the table of a level starts (lengths grow by four as long as words are packed)
+    __device__ __forceinline__ static unsigned start(int size) { return kPacked && size > BATCH ? (unsigned)(BATCH + (size - 4 * BATCH) / 3) : 0u; }
+    __device__ __forceinline__ HashSet level(int size) const { return HashSet{tab.part(start(size)), list, bits, ext}; }
     __device__ __forceinline__ unsigned word(unsigned number, unsigned key) const { return kPacked ? number << SHIFT | key : number; }
     __device__ __forceinline__ unsigned key_of(unsigned w) const { return kPacked ? w & ((1u << SHIFT) - 1u) : list.ld(w); }
     __device__ __forceinline__ static unsigned number_of(unsigned w) { return w >> SHIFT; }
@@ -815,6 +944,38 @@ struct HashSet {
         }
         return false;
     }
+    // The first n elements into an empty table, as BitTable's batches, of one element per thread.  A round is a barrier: whoever lost its
+    // slot goes on and claims the next one, and when nobody has, all are in place.  (insert and relevel walk the losers one link after
+    // another, on one thread each.)
+    template <class Team>
+    __device__ __forceinline__ void insert_batches(int n, int size) const {
+        const unsigned mask = (unsigned)size - 1u;
+        for (int w = threadIdx.x; w <= size >> 5; w += Team::kSize) bits.st(w, 0u);
+        for (int q0 = 0; q0 < n; q0 += Team::kSize) {
+            const bool in = q0 + (int)threadIdx.x < n;
+            const unsigned key = in ? list.ld(q0 + threadIdx.x) : 0u, me = word(q0 + threadIdx.x, key);
+            Probe p = probe_begin(key, mask);
+            if (in) {
+                if (q0 > 0) to_free(bits, p, mask);
+                tab.claim(p.i + p.w, me);
+            }
+            bool lost = in;
+            while (Team::any(lost, nullptr)) {
+                lost = in && tab.ld(p.i + p.w) != me;
+                if (lost) {
+                    if (q0 > 0) {
+                        ++p.w;
+                        to_free(bits, p, mask);
+                    } else {
+                        probe_advance(p, mask);
+                    }
+                    tab.claim(p.i + p.w, me);
+                }
+            }
+            if (in) bits.set((p.i + p.w) >> 5, 1u << ((p.i + p.w) & 31u));
+            Team::sync();
+        }
+    }
     // Whether every slot on the path of the element in `slot` before that one has an earlier element.
     __device__ __forceinline__ bool in_place(unsigned w, unsigned slot, unsigned mask) const {
         Probe p = probe_begin(key_of(w), mask);
@@ -824,43 +985,18 @@ struct HashSet {
         }
         return true;
     }
-    // One warp: the table's columns in slot order to the list.
-    template <After AFTER>
-    __device__ __forceinline__ void extract_warp(int size) const {
+    // One warp: levels from length 8 up to `last`; the level of length `final` is kept, in this table's first slots, which are free otherwise.
+    __device__ __forceinline__ void warp_levels(const BitTable& b, int n_total, int last, int final) const {
         const int lane = threadIdx.x & 31;
-        int n = 0;
-        for (int s0 = 0; s0 < size; s0 += 128) {
-            unsigned w[4];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) w[b] = s0 + b * 32 + lane < size ? tab.ld(s0 + b * 32 + lane) : kFree;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                if (s0 + b * 32 >= size) break;
-                const unsigned m = __ballot_sync(0xffffffffu, w[b] != kFree);
-                if (w[b] != kFree) {
-                    const int pos = n + __popc(m & ((1u << lane) - 1u));
-                    const unsigned key = key_of(w[b]);
-                    if (kPacked) list.st(pos, key); else ext.st(pos, key);
-                    tab.st(s0 + b * 32 + lane, AFTER == After::kNumbered ? word(pos, key) : kFree);
-                }
-                n += __popc(m);
-            }
+        for (int size = kMinTable; size <= last; size = level_next(size)) b.reorder(list, min(level_trigger(size), n_total), size);
+        int done = 0;
+        for (int s0 = 0; s0 < (final <= last ? final : 0); s0 += 32) {
+            const unsigned w = s0 + lane < final ? b.words.ld(s0 + lane) : kFree;
+            const unsigned taken = __ballot_sync(0xffffffffu, w != kFree);
+            if (s0 + lane < final) tab.st(s0 + lane, w != kFree ? word(done + __popc(taken & ((1u << lane) - 1u)), BitTable::column_of(w)) : kFree);
+            done += __popc(taken);
         }
         __syncwarp();
-        if (!kPacked) {
-            for (int q = lane; q < n; q += 32) list.st(q, ext.ld(q));
-            __syncwarp();
-        }
-    }
-    // One warp: levels from length 8 up to `last`, each in the same free table; the level of length `final` is kept.
-    __device__ __forceinline__ bool levels_warp(int n_total, int last, int final) const {
-        for (int size = kMinTable; size <= last; size = level_next(size)) {
-            const bool again = insert(min(level_trigger(size), n_total), (unsigned)size - 1u, threadIdx.x & 31, 32);
-            if (__any_sync(0xffffffffu, again)) return true;
-            __syncwarp();
-            if (size == final) extract_warp<After::kNumbered>(size); else extract_warp<After::kFreed>(size);
-        }
-        return false;
     }
 };
 
@@ -918,7 +1054,9 @@ __device__ __forceinline__ void extract_cta(const Set& t, int size, After after,
     const int first = warp * rows * 32 + lane;
     const bool in = warp * rows * 32 < size;
     int cnt = 0;
-    if (in)
+    if (in && size <= Set::kBatch)
+        cnt = warp_sum(lane < rows ? __popc(t.bits.ld(warp * rows + lane)) : 0);        // (at most eight rows of a warp)
+    else if (in)
 #pragma unroll 4
         for (int j = 0; j < rows; ++j) cnt += __popc(__ballot_sync(0xffffffffu, t.tab.ld(first + j * 32) < Set::kVacant));
     int total;
@@ -1006,18 +1144,17 @@ __device__ __forceinline__ bool relevel(const Set& t, int n, int size, int* red)
     return Team::any(t.insert(n, mask, tid, Team::kSize), red);
 }
 
-// One group.  rows: kRowInts ints of shared memory; red: 96.
+// One group, by a CTA.  rows: kRowInts ints of shared memory; red: 96; small: kWarpLevels + kWarpLevelBits words.
 template <class Team, class Set>
-__device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, int base, const Set& t, int* rows, int* red,
+__device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, int base, const Set& t, const SharedWords& small, int* rows, int* red,
                              int* __restrict__ out_col, __half* __restrict__ out_vals) {
-    constexpr bool kWarp = Team::kSize == 32, kKeep = !kWarp && Set::kPacked;
-    const int tid = Team::tid(), lane = threadIdx.x & 31;
+    constexpr bool kKeep = Set::kPacked;
+    const int tid = Team::tid(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = min(i * p.V, p.M), n_rows = min(i * p.V + p.V, p.M) - r0;
     if (tid <= n_rows) rows[tid] = p.row_ptr[r0 + tid];
-    for (int s = tid * 4; s < (int)(kKeep ? Set::start(cap) : 0u) + cap; s += Team::kSize * 4) t.tab.free4(s);
+    for (int s = tid * 4; s < (int)Set::start(cap) + cap; s += Team::kSize * 4) t.tab.free4(s);
     if (out_vals && p.zero_values) zero_values<Team>(out_vals, base, u_final, p.V);
     Team::sync();
-    // a warp team does all levels in one table
     auto table = [&](int size) { return kKeep ? t.level(size) : t; };
 
     int n_cur = 0, size = 0;                   // length of the table of the last rebuild (0: none yet, all slots free)
@@ -1031,19 +1168,18 @@ __device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, i
         // ---- columns of this row that are not in the set yet, in row order
         const Set held = table(size);
         int n_new = 0;
+        bool ascending = true;
         for (int t0 = 0; t0 < rlen; t0 += Team::kSize) {
-            if (t0 > 0) key = t0 + tid < rlen ? p.col_idx[rs + t0 + tid] : -1;
+            const bool in = t0 + tid < rlen;
+            if (t0 > 0) key = in ? p.col_idx[rs + t0 + tid] : -1;
+            if (in && t0 + tid > 0) ascending = ascending && p.col_idx[rs + t0 + tid - 1] < key;
             const bool fresh = (unsigned)key < (unsigned)p.K && (n_cur == 0 || !held.contains((unsigned)size - 1u, (unsigned)key));
             const unsigned b = __ballot_sync(0xffffffffu, fresh);
             int at = n_cur + n_new + __popc(b & ((1u << lane) - 1u));
-            if constexpr (kWarp) {
-                n_new += __popc(b);
-            } else {
-                int total;
-                at += Team::before(__popc(b), total, red + 32 + 32 * turn);
-                n_new += total;
-                turn ^= 1;
-            }
+            int total;
+            at += Team::before(__popc(b), total, red + 32 + 32 * turn);
+            n_new += total;
+            turn ^= 1;
             if (fresh && at < u_final) t.list.st(at, (unsigned)key);
         }
         const int n_total = n_cur + n_new;
@@ -1052,30 +1188,39 @@ __device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, i
         int final = kMinTable;
         while (n_total >= level_trigger(final)) final = level_next(final);
         // ---- set(list), level by level
-        if constexpr (kWarp) {
+        const bool unsorted = Team::any(!ascending, red);   // (the barrier: the list is complete, the table has been read)
+        const int used = Set::start(size) > 0 ? 0 : size;   // tables of their own stay
+        if (warp == 0) {
+            for (int s = lane * 4; s < min(used, kWarpLevels); s += 128) t.tab.free4(s);
             __syncwarp();
-            for (int s = lane * 4; s < size; s += 128) t.tab.free4(s);
-            __syncwarp();
-            again = t.levels_warp(n_total, final, final);
+            t.warp_levels(BitTable{small, small.part(kWarpLevels)}, n_total, min(final, kWarpLevels), final);
         } else {
-            Team::sync();                                   // the list is complete, the table has been read
-            const int used = kKeep && size > kWarpLevels ? 0 : size;          // tables of their own stay
-            if (threadIdx.x < 32) {
-                for (int s = lane * 4; s < min(used, kWarpLevels); s += 128) t.tab.free4(s);
-                __syncwarp();
-                again = t.levels_warp(n_total, min(final, kWarpLevels), final);
-            } else {
-                for (int s = kWarpLevels + (tid - 32) * 4; s < used; s += (Team::kSize - 32) * 4) t.tab.free4(s);
+            for (int s = kWarpLevels + (tid - 32) * 4; s < used; s += (Team::kSize - 32) * 4) t.tab.free4(s);
+        }
+        Team::sync();
+        for (int level = level_next(kWarpLevels); level <= final && !again; level = level_next(level)) {
+            const int n = min(level_trigger(level), n_total);
+            if (level <= Set::kBatch) {
+                t.template insert_batches<Team>(n, level);
+                extract_cta<Team>(t, level, level == final ? After::kNumbered : After::kFreed, red);
+                continue;
             }
-            again = Team::any(again, red);
-            for (int level = level_next(kWarpLevels); level <= final && !again; level = level_next(level)) {
-                const Set l = table(level);
-                const int n = min(level_trigger(level), n_total);
-                if (kKeep && level <= size) again = relevel<Team>(l, n, level, red);
-                else again = Team::any(l.insert(n, (unsigned)level - 1u, tid, Team::kSize), red);
-                if (!again)
-                    extract_cta<Team>(l, level, level == final && (!kKeep || r + 1 == n_rows) ? After::kNumbered : kKeep ? After::kVacated : After::kFreed, red);
+            const Set l = table(level);
+            if (kKeep && level <= size) again = relevel<Team>(l, n, level, red);
+            else again = Team::any(l.insert(n, (unsigned)level - 1u, tid, Team::kSize), red);
+            if (!again)
+                extract_cta<Team>(l, level, level == final && (!kKeep || r + 1 == n_rows) ? After::kNumbered : kKeep ? After::kVacated : After::kFreed, red);
+        }
+        // A column that a row repeats is met in the tables above BATCH; in the others it has two slots, and only the first is found.
+        if (unsorted && final <= Set::kBatch) {
+            const Set now = table(final);
+            bool twice = false;
+            for (int q = tid; q < n_total; q += Team::kSize) {
+                unsigned w;
+                now.find((unsigned)final - 1u, t.list.ld(q), w);
+                twice = twice || w == kFree || Set::number_of(w) != (unsigned)q;
             }
+            again = Team::any(twice, red);
         }
         if (again) break;
         n_cur = n_total;
@@ -1100,25 +1245,101 @@ __device__ void replay_group(const SvcProblem& p, int i, int u_final, int cap, i
     Team::sync();
 }
 
+// One group, by a warp.  What bounds it is the issue of instructions: 30 to 48 warps per SM, a few hundred instructions per rebuild.
+// counts: a word per word of the table's bits.
+__device__ void replay_group_by_warp(const SvcProblem& p, int i, int u_final, int cap, int base, const BitTable& t, const SharedWords& list,
+                                     const SharedWords& counts, int* rows, int* __restrict__ out_col, __half* __restrict__ out_vals) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int r0 = min(i * p.V, p.M), n_rows = min(i * p.V + p.V, p.M) - r0;
+    if (lane <= n_rows) rows[lane] = p.row_ptr[r0 + lane];
+    if (out_vals && p.zero_values) zero_values<WarpTeam>(out_vals, base, u_final, p.V);
+    __syncwarp();
+    int n_cur = 0, size = kMinTable;
+    bool again = false;
+    int next_key = lane < rows[1] - rows[0] ? p.col_idx[rows[0] + lane] : -1;          // the next row's columns are under way early
+    for (int r = 0; r < n_rows; ++r) {
+        const int rs = rows[r], rlen = rows[r + 1] - rs;
+        int key = next_key;
+        if (r + 1 < n_rows) next_key = lane < rows[r + 2] - rows[r + 1] ? p.col_idx[rows[r + 1] + lane] : -1;
+        // ---- columns of this row that are not in the set yet, in row order
+        int n_total = n_cur, last = -1;
+        bool ascending = true;
+        for (int t0 = 0; t0 < rlen; t0 += 32) {
+            const bool in = t0 + lane < rlen;
+            if (t0 > 0) key = in ? p.col_idx[rs + t0 + lane] : -1;
+            const int left = __shfl_up_sync(0xffffffffu, key, 1);
+            ascending = ascending && (!in || (lane > 0 ? left : last) < key);
+            last = __shfl_sync(0xffffffffu, key, 31);
+            unsigned slot;
+            const bool fresh = (unsigned)key < (unsigned)p.K && (n_cur == 0 || !t.find((unsigned)size - 1u, (unsigned)key, slot));
+            const unsigned b = __ballot_sync(0xffffffffu, fresh);
+            const int at = n_total + __popc(b & below);
+            if (fresh && at < u_final) list.st(at, (unsigned)key);
+            n_total += __popc(b);
+        }
+        if (n_total > u_final) { again = true; break; }     // only possible when the row repeats a column
+        if (n_total == 0) continue;
+        int final = kMinTable;
+        while (n_total >= level_trigger(final)) final = level_next(final);
+        __syncwarp();
+        for (int level = kMinTable; level <= final; level = level_next(level)) t.reorder(list, min(level_trigger(level), n_total), level);
+        n_cur = n_total;
+        size = final;
+        // a column that occurs twice has two slots now, and only the first of them is found
+        if (!__all_sync(0xffffffffu, ascending)) {
+            t.index(counts, size);
+            for (int q0 = 0; q0 < n_cur && !again; q0 += 32) {
+                unsigned slot = 0;
+                const bool twice = q0 + lane < n_cur && (!t.find((unsigned)size - 1u, list.ld(q0 + lane), slot) || t.rank(counts, slot) != q0 + lane);
+                again = __any_sync(0xffffffffu, twice);
+            }
+        }
+        if (again) break;
+    }
+    if (again) {
+        unsigned mask = 0;
+        __syncwarp();
+        if (lane == 0) n_cur = replay_sequential(p, rows, n_rows, HashSet<SharedWords, SharedWords, BitTable::kShift, kWarpLevels>{t.words, list, t.bits, GlobalWords{nullptr}}, cap, mask);
+        n_cur = __shfl_sync(0xffffffffu, n_cur, 0);
+        size = (int)__shfl_sync(0xffffffffu, mask, 0) + 1;
+        __syncwarp();
+    }
+    for (int q = lane; q < n_cur; q += 32) out_col[base + q] = (int)list.ld(q);
+    if (out_vals && n_cur > 0) {
+        t.index(counts, size);
+        for_each_value<WarpTeam>(p, rows, n_rows, [&](int r, int c, __half v) {
+            unsigned slot;
+            if (t.find((unsigned)size - 1u, (unsigned)c, slot)) out_vals[((int64_t)base + t.rank(counts, slot)) * p.V + r] = v;
+        });
+    }
+    __syncwarp();
+}
+
 // What a team of a class has in shared memory: its tables, a list and the row ends of its group.  Class L with a table per level
 // leaves no room for the list, and class XL has everything, in global scratch.
 // SHIFT: bits of a column in a word; numbers of a list and two more fit the others (0: unpacked).
 template <int CLASS, int SHIFT>
 struct ClassShape {
-    static constexpr int kTeam = CLASS == kClassM1 ? 256 : CLASS == kClassM2 ? 512 : CLASS == kClassL || CLASS == kClassXL ? 1024 : 32;
+    static constexpr bool kWarp = CLASS == kClassXS || CLASS == kClassS;
+    static constexpr int kTeam = kWarp ? 32 : CLASS == kClassM1 ? 256 : CLASS == kClassM2 ? 512 : 1024;
     static constexpr int kCapU = CLASS == kClassXS ? kXSCapU : CLASS == kClassS ? kSCapU : CLASS == kClassM1 ? kM1CapU : CLASS == kClassM2 ? kM2CapU : kLCapU;
     static constexpr int kCapT = CLASS == kClassXS ? kXSCapT : CLASS == kClassS ? kSCapT : CLASS == kClassM1 ? kM1CapT : CLASS == kClassM2 ? kM2CapT : kLCapT;
     static constexpr bool kListInSmem = CLASS != kClassXL && !(CLASS == kClassL && SHIFT > 0);
-    static constexpr int kTable = CLASS == kClassXL ? 0 : kTeam > 32 && SHIFT > 0 ? kCapT + (kCapT - kWarpLevels) / 3 : kCapT;
+    static constexpr int kBatch = kTeam <= 512 ? kBatchLevels : kWarpLevels;       // a CTA: tables filled in batches
+    static constexpr int kTable = CLASS == kClassXL ? 0 : !kWarp && SHIFT > 0 && kCapT > kBatch ? kCapT + kBatch + (kCapT - 4 * kBatch) / 3 : kCapT;
     static constexpr int kList = kListInSmem ? (kCapU + 3) & ~3 : 0;
-    static constexpr int kInts = kTable + kList + kRowInts;          // of a team, in shared memory
-    static constexpr int kThreads = kTeam == 32 ? 256 : kTeam;       // of a block
+    static constexpr int kBits = (kWarp ? kCapT : kBatch) / 32 + 4;         // (the word after the last is read)
+    static constexpr int kCounts = kWarp ? kCapT / 32 : kWarpLevels + kWarpLevelBits;      // a CTA: the table of the small levels
+    static constexpr int kInts = kTable + kList + kBits + kCounts + kRowInts;     // of a team, in shared memory
+    static constexpr int kThreads = kWarp ? 256 : kTeam;          // of a block
     static constexpr int kBlocks = (kTeam == 1024 ? 1024 : 1536) / kThreads;      // per SM
-    using Team = std::conditional_t<kTeam == 32, WarpTeam, BlockTeam<kTeam>>;
+    using Team = std::conditional_t<kWarp, WarpTeam, BlockTeam<kTeam>>;
+    static constexpr int kPerBlock = kThreads / kTeam;
     using Words = std::conditional_t<CLASS == kClassXL, GlobalWords, SharedWords>;
     using List = std::conditional_t<kListInSmem, SharedWords, GlobalList>;
     static_assert(SHIFT == 0 || kCapU < (1ll << (32 - SHIFT)) - 2, "numbers of a list fit the words");
-    static_assert(SHIFT == 0 || (kCapU <= 32 * kTeam && kCapT <= 32 * kTeam), "relevel: a bit per element and slot of a thread");
+    static_assert(kWarp || SHIFT == 0 || (kCapU <= 32 * kTeam && kCapT <= 32 * kTeam), "relevel: a bit per element and slot of a thread");
 };
 
 template <int CLASS, int SHIFT>
@@ -1132,6 +1353,8 @@ svc_emit_replay_kernel(SvcProblem p, const int* __restrict__ vec_ptr, const int*
     extern __shared__ __align__(16) int sm_ints[];
     __shared__ int red[96];
     int* mine = sm_ints + (size_t)Team::index_in_block() * Shape::kInts;
+    const SharedWords bits{smem_u32(mine + Shape::kTable + Shape::kList)};
+    int* const rows = mine + Shape::kTable + Shape::kList + Shape::kBits + Shape::kCounts;
     for (;;) {
         int k = 0;
         if (Team::tid() == 0) k = atomicAdd(queue, 1);
@@ -1141,14 +1364,20 @@ svc_emit_replay_kernel(SvcProblem p, const int* __restrict__ vec_ptr, const int*
         const int base = vec_ptr[i];
         const int u = vec_ptr[i + 1] - base;
         const int cap = tbl_len[i];
-        unsigned* g = reinterpret_cast<unsigned*>(scratch) + (CLASS == kClassL || CLASS == kClassXL ? tbl_off[i] : 0);
-        HashSet<typename Shape::Words, typename Shape::List, SHIFT> t;
-        if constexpr (CLASS == kClassXL) { t.tab.at = g; g += cap; }
-        else t.tab.at = smem_u32(mine);
-        if constexpr (Shape::kListInSmem) t.list.at = smem_u32(mine + Shape::kTable);
-        else { t.list.at = g; g += u; }
-        t.ext.at = g;
-        replay_group<Team>(p, i, u, cap, base, t, mine + Shape::kTable + Shape::kList, red, out_col, out_vals);
+        if constexpr (Shape::kWarp) {
+            replay_group_by_warp(p, i, u, cap, base, BitTable{SharedWords{smem_u32(mine)}, bits}, SharedWords{smem_u32(mine + Shape::kTable)},
+                                 bits.part(Shape::kBits), rows, out_col, out_vals);
+        } else {
+            unsigned* g = reinterpret_cast<unsigned*>(scratch) + (CLASS == kClassL || CLASS == kClassXL ? tbl_off[i] : 0);
+            HashSet<typename Shape::Words, typename Shape::List, SHIFT, Shape::kBatch> t;
+            if constexpr (CLASS == kClassXL) { t.tab.at = g; g += cap; }
+            else t.tab.at = smem_u32(mine);
+            if constexpr (Shape::kListInSmem) t.list.at = smem_u32(mine + Shape::kTable);
+            else { t.list.at = g; g += u; }
+            t.bits = bits;
+            t.ext.at = g;
+            replay_group<Team>(p, i, u, cap, base, t, bits.part(Shape::kBits), rows, red, out_col, out_vals);
+        }
     }
 }
 
@@ -1209,9 +1438,8 @@ cudaError_t launch_replay(const SvcProblem& p, const SvcScratch& s, int* out_col
                           long long first, cudaStream_t stream) {
     if (groups <= 0) return cudaSuccess;
     using Shape = ClassShape<CLASS, SHIFT>;
-    using Team = typename Shape::Team;
     auto kern = svc_emit_replay_kernel<CLASS, SHIFT>;
-    const size_t smem = (size_t)Team::kPerBlock * Shape::kInts * sizeof(int);
+    const size_t smem = (size_t)Shape::kPerBlock * Shape::kInts * sizeof(int);
     static DeviceOnce once;
     if (!once.done()) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1222,7 +1450,7 @@ cudaError_t launch_replay(const SvcProblem& p, const SvcScratch& s, int* out_col
         once.mark();
     }
     // as many blocks as can be resident: the groups are handed out through the class's work counter
-    const long long want = (groups + Team::kPerBlock - 1) / Team::kPerBlock;
+    const long long want = (groups + Shape::kPerBlock - 1) / Shape::kPerBlock;
     const long long most = (long long)device_sm_count() * Shape::kBlocks;
     kern<<<(unsigned)(want < most ? want : most), Shape::kThreads, smem, stream>>>(p, s.vec_ptr, s.tbl_len, s.tbl_off, s.tables, out_col, out_vals,
                                                                             s.class_list + first, (int)groups, s.queue + CLASS);

@@ -264,6 +264,36 @@ def test_replay_of_rows_that_repeat_columns(lib, K, big):
         check_against_oracle(_one_group(K, [4, 9, 3, big, 6], K + repeat, repeat=repeat), 8)
 
 
+@pytest.mark.parametrize("u", [5, 19, 31, 32, 33, 64, 65, 76, 77, 97, 256, 257, 306, 307, 512, 513, 1228, 1229, 2600])
+def test_replay_at_the_edges_of_batches(lib, u):
+    """Sets around the sizes of a batch (32, 256 and 512 elements) and of the classes, ascending and not, without and with a column
+    that its row repeats."""
+    for order, repeat in (("ascending", 0), ("any", 0), ("any", 1)):
+        for lens in ([u, 0, 1, 2], [2, 1, u - 3], [u // 2, u - u // 2, 0, 3]):
+            check_against_oracle(_one_group(200000, lens, u, repeat=repeat, order=order), 8)
+
+
+@pytest.mark.parametrize("count", [1, 60, 61])
+def test_batches_around_the_table_of_a_launch(lib, count):
+    """Up to 60 matrices travel with the launch, more are copied; with matrices of no rows and no entries, and without values."""
+    dev, rng = torch.device("cuda:0"), np.random.default_rng(count)
+    mats = []
+    for i in range(count):
+        m, k = (0 if i == 7 else 8 * int(rng.integers(1, 8))), int(rng.integers(50, 400))
+        n = np.zeros(m, dtype=np.int64) if i == 9 else rng.integers(0, 30, m)
+        ptr = np.concatenate([[0], np.cumsum(n)]).astype(np.int32)
+        col = np.concatenate([np.sort(rng.permutation(k)[:x]) for x in n] + [np.zeros(0, dtype=np.int64)]).astype(np.int32)
+        mats.append(tuple(torch.from_numpy(x).to(dev) for x in (ptr, col, rng.uniform(-1, 1, col.size).astype(np.float16))) + (m, k))
+    for with_values in (True, False):
+        given = [x if with_values else x[:2] + (None,) + x[3:] for x in mats]
+        res, replayed = ops.svc_batch(given, 8)
+        single = [ops.svc(*x, 8) for x in given]
+        assert replayed == sum(x[3] for x in single)
+        for got, want in zip(res, single):
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+            assert got[2] is None and want[2] is None if not with_values else torch.equal(got[2], want[2])
+
+
 def test_value_vectors_off_their_boundary(lib):
     """The caller's value array need not start on a 16-byte boundary; nothing before or after it is written."""
     import ctypes as C
