@@ -531,9 +531,10 @@ attention_fm_kernel(int seq, int64_t tokens, const __half* __restrict__ q, const
 // three stages of 64 tokens; scores and partial outputs have two buffers each in tensor memory, so the scores of the
 // next block are computed while this block's probabilities are, and a partial output is taken one block later.
 // The arithmetic is attend's: blocks of 64 keys, sums of a block from zero, joined in round-to-nearest.
-// Bound by the softmax warps: about ten instructions per score, and the waits between them and the products, which two CTAs per SM
-// do not fill.  12 heads, 32 x 512 tokens: 75 us (attention_fm_kernel 141; 85 with the first requests after the set-up); 16 x 512 40 (75),
-// 1 x 2048 44 (83).  Distance from 64 bits as there: 2.074969e-4 against 2.074970e-4 (scores of size 1), 2.073688e-4 against 2.073688e-4
+// Bound by the softmax warps: about seven instructions per score (additions, products and the joining of outputs work on pairs of
+// numbers, each rounded as by itself; one number at a time it was ten), and the waits between them and the products, which two CTAs per SM
+// do not fill.  12 heads, 32 x 512 tokens: 71 us, 78 one number at a time (attention_fm_kernel 141; 85 with the first requests after the
+// set-up); one number at a time 16 x 512 40 (75), 1 x 2048 44 (83).  Distance from 64 bits as there: 2.074969e-4 against 2.074970e-4 (scores of size 1), 2.073688e-4 against 2.073688e-4
 // (size 5).  A CTA that walks over tiles with the next one's operands on their way takes 96 us.
 constexpr int kTcQueries = 128, kTcStages = 3, kTcThreads = 160;
 struct TcSmem {
@@ -609,7 +610,7 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
     const uint32_t tmem = *tmem_at;
 
     bool nan = false, done = false;
-    float o[kHd], l[4] = {0.f, 0.f, 0.f, 0.f};                      // of the softmax warps
+    f32x2 o[kHd / 2], l[2] = {0, 0};                                // of the softmax warps, in pairs
     if (warp == 4) {
         if (lane == 0) {
             // queries are in when the softmax warps say so (they add the bias first): their arrival is the first phase of o_free[0]
@@ -674,19 +675,21 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
         if (lane == 0) mbar_arrive(bar_o_free);
         float m = -INFINITY, keep = 1.f;
 #pragma unroll
-        for (int f = 0; f < kHd; ++f) o[f] = 0.f;
+        for (int f = 0; f < kHd / 2; ++f) o[f] = 0;
         // adds the partial output of block it: o = o * factor + partial
         auto join = [&](int it, float factor) -> bool {
             const int buf = it & 1;
             if (!__all_sync(0xffffffffu, mbar_wait(bar_o_full + 8 * buf, (it >> 1) & 1, abort_flag, kStatusWaitAttention))) return false;
             tc_fence_after_sync();
+            const f32x2 both = pair_of(factor, factor);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 uint32_t d[32];
                 tmem_ld_x32(tmem + lanes + 2 * kTile + buf * kHd + h * 32, d);
                 tc_wait_ld();
 #pragma unroll
-                for (int f = 0; f < 32; ++f) o[h * 32 + f] = fmaf(o[h * 32 + f], factor, __uint_as_float(d[f]));
+                for (int f = 0; f < 16; ++f)
+                    o[h * 16 + f] = fma2(o[h * 16 + f], both, pair_of(__uint_as_float(d[2 * f]), __uint_as_float(d[2 * f + 1])));
             }
             tc_fence_before_sync();
             __syncwarp();
@@ -720,19 +723,22 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
             m = mx[0];
             const float shift = m == -INFINITY ? 0.f : m;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) l[e] *= keep;
+            for (int e = 0; e < 2; ++e) l[e] = mul2(l[e], pair_of(keep, keep));
+            const f32x2 less = pair_of(-shift, -shift), scale = pair_of(kScale, kScale), lift = pair_of(kLift, kLift);
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
                 uint32_t hi[8], lo[8];
 #pragma unroll
                 for (int n = 0; n < 8; ++n) {
-                    const float p0 = ex2(fmaf(__uint_as_float(s[h >> 1][(h & 1) * 16 + 2 * n]) - shift, kScale, kLift));
-                    const float p1 = ex2(fmaf(__uint_as_float(s[h >> 1][(h & 1) * 16 + 2 * n + 1]) - shift, kScale, kLift));
-                    l[(2 * n) & 3] += p0;
-                    l[(2 * n + 1) & 3] += p1;
+                    const uint32_t* const at2 = &s[h >> 1][(h & 1) * 16 + 2 * n];
+                    const float2 x = floats_of(fma2(add2(pair_of(__uint_as_float(at2[0]), __uint_as_float(at2[1])), less), scale, lift));
+                    const float p0 = ex2(x.x), p1 = ex2(x.y);
+                    const f32x2 p = pair_of(p0, p1);
+                    l[n & 1] = add2(l[n & 1], p);
                     const __half2 ph = __floats2half2_rn(p0, p1);
                     const float2 back = __half22float2(ph);
-                    const __half2 pl = __floats2half2_rn(p0 - back.x, p1 - back.y);
+                    const float2 rest = floats_of(add2(p, pair_of(-back.x, -back.y)));
+                    const __half2 pl = __floats2half2_rn(rest.x, rest.y);
                     hi[n] = *reinterpret_cast<const uint32_t*>(&ph);
                     lo[n] = *reinterpret_cast<const uint32_t*>(&pl);
                 }
@@ -748,7 +754,7 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
         done = ok && join(rounds - 1, keep) && q0 + row < seq;
         if (done)
 #pragma unroll
-            for (int f = 0; f < kHd; ++f) nan |= isnan(o[f]);
+            for (int f = 0; f < kHd / 2; ++f) { const float2 x = floats_of(o[f]); nan |= isnan(x.x) || isnan(x.y); }
     }
     tc_fence_before_sync();
     nan = __syncthreads_or(nan);
@@ -757,11 +763,14 @@ attention_tc_kernel(int seq, int64_t tokens, const __grid_constant__ CUtensorMap
         tmem_dealloc(tmem, kTcTmemCols);
     }
     if (done && !nan) {                                             // (out may be q, which a second pass reads again)
-        const float inv = 1.f / ((l[0] + l[1]) + (l[2] + l[3]));
+        const float2 l01 = floats_of(l[0]), l23 = floats_of(l[1]);
+        const float inv = 1.f / ((l01.x + l01.y) + (l23.x + l23.y));
         __half* dst = out + (int64_t)head * kHd * tokens + (int64_t)b * seq + q0 + threadIdx.x;
 #pragma unroll
-        for (int f = 0; f < kHd; ++f)
-            dst[f * tokens] = __float2half_rn(fmaf(o[f], inv, bias_v ? __half2float(bias_v[head * kHd + f]) : 0.f));
+        for (int f = 0; f < kHd; ++f) {
+            const float2 x = floats_of(o[f >> 1]);
+            dst[f * tokens] = __float2half_rn(fmaf(f & 1 ? x.y : x.x, inv, bias_v ? __half2float(bias_v[head * kHd + f]) : 0.f));
+        }
     }
     // something infinite or NaN went in: again, with infinities and NaNs of v apart, 64 queries at a time
     if (nan && warp < 4) {
