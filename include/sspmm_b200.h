@@ -71,6 +71,34 @@ int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nv
                   const void* bias_f16, void* out, int64_t out_stride, int out_is_f16, void* stream);
 
 /*
+ * sspmm_counted for one product with fp16 results, with add[m_vec*V][N] (fp16) added to the fp32 sums before the conversion, as the
+ * bias is.  The kernel is the one that sspmm_counted takes.  taken = 0: not a call for it (unaligned operands, rows long enough
+ * to be cut, another kernel forced, no room for the scratch); nothing was launched.
+ */
+int sspmm_counted_sum(int m_vec, int vec_length, int N, int K, int64_t nvec, const int* row_indices, const int* row_offsets,
+                      const int* column_indices, const void* values_f16, const void* rhs_f16, const void* bias_f16, const void* add_f16,
+                      void* out_f16, void* stream, int* taken);
+
+/*
+ * Products whose operands are known ahead of the first of them (the linears of a layer): the dense transposed copies that the block
+ * kernel works on, of up to eight operands for right-hand sides of N columns, made by one launch.  An operand is `pieces` of
+ * m_vec vector rows each, one below the other, as in sspmm_stacked.  offsets[i] is where its copy [K][pieces * m_vec*V] (fp16) starts in
+ * room, in bytes, or -1 where sspmm_counted would not take the block kernel; *bytes is what the copies need.  room NULL: only that, nothing is
+ * launched; else 256-byte aligned.
+ * sspmm_of_copy: the product of such a copy, with bias and add (either may be NULL) as in sspmm_counted_sum; fp16 results.
+ */
+typedef struct sspmm_dense_operand {
+    int pieces, m_vec, vec_length, K;
+    const int64_t* nvec;               /* of each piece */
+    const int* const* row_offsets;     /* of each piece */
+    const int* column_indices;
+    const void* values_f16;
+} sspmm_dense_operand;
+int sspmm_dense_copies(int count, const sspmm_dense_operand* operands, int N, void* room, int64_t* offsets, int64_t* bytes, void* stream);
+int sspmm_of_copy(int m_vec, int vec_length, int N, int K, const void* copy_f16, const void* rhs_f16, const void* bias_f16, const void* add_f16,
+                  void* out_f16, void* stream);
+
+/*
  * sspmm_counted for several operands of one height and width that multiply the same rhs: `pieces` of m_vec vector rows each, results
  * one below the other in out [pieces * m_vec*V][N], as one product.  column_indices, values and bias hold the pieces one after
  * another (nvec[i] vectors, m_vec*V biases); each keeps its own row pointers, which start at 0, and row order (either pointer of
@@ -216,6 +244,9 @@ int sspmm_group_run(sspmm_group* group, void* stream);
 /* A number per output row of product `item` (fp16, m_vec*V of them; NULL: none), added to the fp32 sums before the conversion in
  * the runs that follow.  taken = 0: this group's kernel adds no biases (groups of the tile kernels), nothing has changed. */
 int sspmm_group_bias(sspmm_group* group, int item, const void* bias_f16, int* taken);
+/* One run of a group of one product with fp16 results whose sums go to out (like the group's own output, which keeps what it has) with
+ * this bias (NULL: none; the group's own is not looked at) and add[m_vec*V][N] (fp16) added before the conversion; 16-byte aligned.  taken = 0: this group's kernel does not, nothing was launched. */
+int sspmm_group_run_sum(sspmm_group* group, const void* bias_f16, const void* add_f16, void* out_f16, void* stream, int* taken);
 /* Any output pointer may be NULL.  launches = kernels per run (always 1).  tile_columns, work_items (tiles, or vector rows of a tile in
  * row-gather groups, or parts of either) and ctas are those of the launch. */
 int sspmm_group_info(const sspmm_group* group, int* tile_columns, int* work_items, int* ctas, int* launches,

@@ -179,6 +179,136 @@ PyObject* py_planned(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
+// sspmm_sum(row_offsets, column_indices, values, rhs, vec_length, bias, row_indices, add)
+PyObject* py_sspmm_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long V;
+        if (n != 8 || modes_active() || !small_int(a[4], 1, 1 << 20, &V)) Py_RETURN_NONE;
+        const at::Tensor *ptr = plain(a[0], at::kInt), *col = plain(a[1], at::kInt), *val = plain(a[2], at::kHalf), *rhs = plain(a[3], at::kHalf),
+                         *bias = plain(a[5], at::kHalf), *order = plain(a[6], at::kInt), *add = plain(a[7], at::kHalf);
+        if (!ptr || !col || !val || !rhs || !bias || !order || !add || rhs->dim() != 2) Py_RETURN_NONE;
+        const int64_t m_vec = ptr->numel() - 1, K = rhs->size(0), N = rhs->size(1), most = 0x7fffffff;
+        if (m_vec < 0 || m_vec > most / V || K > most || N > most || bias->numel() != m_vec * V || add->dim() != 2 || add->size(0) != m_vec * V ||
+            add->size(1) != N)
+            Py_RETURN_NONE;
+        for (const at::Tensor* t : {ptr, col, val, bias, order, add})
+            if (t->device() != rhs->device()) Py_RETURN_NONE;
+        at::Tensor out = at::empty({m_vec * V, N}, rhs->options().requires_grad(false));
+        int taken = 0;
+        const int rc = launch(rhs->get_device(), [&](void* st) {
+            return sspmm_counted_sum((int)m_vec, (int)V, (int)N, (int)K, col->numel(), static_cast<const int*>(order->data_ptr()),
+                                     static_cast<const int*>(ptr->data_ptr()), static_cast<const int*>(col->data_ptr()), val->data_ptr(), rhs->data_ptr(),
+                                     bias->data_ptr(), add->data_ptr(), out.data_ptr(), st, &taken);
+        });
+        if (rc == 0 && !taken) Py_RETURN_NONE;
+        return result(rc, out);
+    });
+}
+
+// dense_copies([(row_offsets of each piece, where the pieces' vectors end, column_indices, values, vec_length, K), ...], N)
+//   -> a copy [K, rows] per operand, or None where the product does not work on one; None: not operands for it
+PyObject* py_dense_copies(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        constexpr Py_ssize_t kMost = 8, kPieces = 4;
+        long N;
+        if (n != 2 || modes_active() || !PyList_CheckExact(a[0]) || !small_int(a[1], 1, 0x7fffffff, &N)) Py_RETURN_NONE;
+        const Py_ssize_t count = PyList_GET_SIZE(a[0]);
+        if (count < 1 || count > kMost) Py_RETURN_NONE;
+        sspmm_dense_operand op[kMost];
+        const int* offsets[kMost][kPieces];
+        int64_t nvec[kMost][kPieces], at[kMost], bytes = 0;
+        const at::Tensor* first = nullptr;
+        for (Py_ssize_t k = 0; k < count; ++k) {
+            PyObject* const t = PyList_GET_ITEM(a[0], k);
+            if (!PyTuple_CheckExact(t) || PyTuple_GET_SIZE(t) != 6) Py_RETURN_NONE;
+            PyObject *ptrs = PyTuple_GET_ITEM(t, 0), *ends = PyTuple_GET_ITEM(t, 1);
+            const at::Tensor *col = plain(PyTuple_GET_ITEM(t, 2), at::kInt), *val = plain(PyTuple_GET_ITEM(t, 3), at::kHalf);
+            long V, K, before = 0;
+            if (!PyList_CheckExact(ptrs) || !PyList_CheckExact(ends) || !col || !val || !small_int(PyTuple_GET_ITEM(t, 4), 8, 16, &V) ||
+                !small_int(PyTuple_GET_ITEM(t, 5), 1, 0x7fffffff, &K))
+                Py_RETURN_NONE;
+            const Py_ssize_t pieces = PyList_GET_SIZE(ptrs);
+            if (pieces < 1 || pieces > kPieces || PyList_GET_SIZE(ends) != pieces) Py_RETURN_NONE;
+            if (!first) first = col;
+            if (col->device() != first->device() || val->device() != first->device()) Py_RETURN_NONE;
+            int64_t m_vec = 0;
+            for (Py_ssize_t i = 0; i < pieces; ++i) {
+                const at::Tensor* ptr = plain(PyList_GET_ITEM(ptrs, i), at::kInt);
+                long end;
+                if (!ptr || ptr->device() != first->device() || !small_int(PyList_GET_ITEM(ends, i), before, 0x7fffffff, &end)) Py_RETURN_NONE;
+                if (i == 0) m_vec = ptr->numel() - 1;
+                if (ptr->numel() - 1 != m_vec || m_vec < 1 || m_vec > 0x7fffffff / V / pieces) Py_RETURN_NONE;
+                offsets[k][i] = static_cast<const int*>(ptr->data_ptr());
+                nvec[k][i] = end - before;
+                before = end;
+            }
+            if (col->numel() != before || val->numel() != before * V) Py_RETURN_NONE;
+            op[k] = sspmm_dense_operand{(int)pieces, (int)m_vec, (int)V, (int)K, nvec[k], offsets[k], static_cast<const int*>(col->data_ptr()), val->data_ptr()};
+        }
+        int rc = sspmm_dense_copies((int)count, op, (int)N, nullptr, at, &bytes, nullptr);
+        if (rc != 0) return PyLong_FromLong(rc);
+        at::Tensor room;
+        if (bytes) {
+            room = at::empty({bytes / 2}, first->options().dtype(at::kHalf).requires_grad(false));
+            rc = launch(first->get_device(), [&](void* st) { return sspmm_dense_copies((int)count, op, (int)N, room.data_ptr(), at, &bytes, st); });
+            if (rc != 0) return PyLong_FromLong(rc);
+        }
+        PyObject* const list = PyList_New(count);
+        if (!list) return nullptr;
+        for (Py_ssize_t k = 0; k < count; ++k) {
+            PyObject* item = Py_None;
+            if (at[k] >= 0) {
+                const int64_t rows = (int64_t)op[k].pieces * op[k].m_vec * op[k].vec_length;
+                item = THPVariable_Wrap(room.narrow(0, at[k] / 2, op[k].K * rows).view({op[k].K, rows}));
+            } else {
+                Py_INCREF(item);
+            }
+            PyList_SET_ITEM(list, k, item);
+        }
+        return list;
+    });
+}
+
+// of_copy(copy, rhs, vec_length, bias, add or None)
+PyObject* py_of_copy(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long V;
+        if (n != 5 || modes_active() || !small_int(a[2], 8, 16, &V)) Py_RETURN_NONE;
+        const at::Tensor *copy = plain(a[0], at::kHalf), *rhs = plain(a[1], at::kHalf), *bias = plain(a[3], at::kHalf),
+                         *add = a[4] == Py_None ? nullptr : plain(a[4], at::kHalf);
+        if (!copy || !rhs || !bias || (a[4] != Py_None && !add) || copy->dim() != 2 || rhs->dim() != 2 || rhs->size(0) != copy->size(0)) Py_RETURN_NONE;
+        const int64_t K = copy->size(0), rows = copy->size(1), N = rhs->size(1), most = 0x7fffffff;
+        if (rows % V != 0 || rows > most || K > most || N > most || N % 8 != 0 || bias->numel() != rows || reinterpret_cast<uintptr_t>(rhs->data_ptr()) % 16 != 0 ||
+            copy->device() != rhs->device() || bias->device() != rhs->device())
+            Py_RETURN_NONE;
+        if (add && (add->dim() != 2 || add->size(0) != rows || add->size(1) != N || add->device() != rhs->device() ||
+                    reinterpret_cast<uintptr_t>(add->data_ptr()) % 16 != 0))
+            Py_RETURN_NONE;
+        at::Tensor out = at::empty({rows, N}, rhs->options().requires_grad(false));
+        return result(launch(rhs->get_device(), [&](void* st) {
+            return sspmm_of_copy((int)(rows / V), (int)V, (int)N, (int)K, copy->data_ptr(), rhs->data_ptr(), bias->data_ptr(),
+                                 add ? add->data_ptr() : nullptr, out.data_ptr(), st);
+        }), out);
+    });
+}
+
+// group_run_sum(handle, rows of the output, bias or None, add) -> the sum, or None
+PyObject* py_group_run_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        long rows;
+        if (n != 4 || modes_active() || !PyLong_CheckExact(a[0]) || !small_int(a[1], 0, 0x7fffffff, &rows)) Py_RETURN_NONE;
+        const at::Tensor *add = plain(a[3], at::kHalf), *bias = a[2] == Py_None ? nullptr : plain(a[2], at::kHalf);
+        sspmm_group* group = static_cast<sspmm_group*>(PyLong_AsVoidPtr(a[0]));
+        if (!group || !add || add->dim() != 2 || add->size(0) != rows || (a[2] != Py_None && (!bias || bias->numel() != rows || bias->device() != add->device())))
+            Py_RETURN_NONE;
+        at::Tensor out = at::empty({rows, add->size(1)}, add->options().requires_grad(false));
+        int taken = 0;
+        const int rc = launch(add->get_device(), [&](void* st) { return sspmm_group_run_sum(group, bias ? bias->data_ptr() : nullptr, add->data_ptr(), out.data_ptr(), st, &taken); });
+        if (rc == 0 && !taken) Py_RETURN_NONE;
+        return result(rc, out);
+    });
+}
+
 // group_run(handle, device index) -> error code
 PyObject* py_group_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -380,6 +510,10 @@ PyMethodDef methods[] = {
     {"stacked", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_stacked)), METH_FASTCALL, nullptr},
     {"bspmm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bspmm)), METH_FASTCALL, nullptr},
     {"planned", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_planned)), METH_FASTCALL, nullptr},
+    {"dense_copies", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_dense_copies)), METH_FASTCALL, nullptr},
+    {"of_copy", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_of_copy)), METH_FASTCALL, nullptr},
+    {"sspmm_sum", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_sspmm_sum)), METH_FASTCALL, nullptr},
+    {"group_run_sum", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_group_run_sum)), METH_FASTCALL, nullptr},
     {"group_run", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_group_run)), METH_FASTCALL, nullptr},
     {"same_plain", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_same_plain)), METH_FASTCALL, nullptr},
     {"layer_norm_fm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_layer_norm_fm)), METH_FASTCALL, nullptr},

@@ -469,6 +469,121 @@ int sspmm_counted(int m_vec, int vec_length, int N, int K, int batch, int64_t nv
                       rhs_stride, out, out_stride, out_is_f16 != 0, stream, ex);
 }
 
+int sspmm_counted_sum(int m_vec, int vec_length, int N, int K, int64_t nvec, const int* row_indices, const int* row_offsets,
+                      const int* column_indices, const void* values_f16, const void* rhs_f16, const void* bias_f16, const void* add_f16,
+                      void* out_f16, void* stream, int* taken) {
+    g_err[0] = 0;
+    if (!taken || nvec < 0) { set_error("null pointer or negative nvec"); return (int)cudaErrorInvalidValue; }
+    *taken = 0;
+    const int choice = g_kernel_choice.load();
+    if ((vec_length != 8 && vec_length != 16) || m_vec <= 0 || N <= 0 || K <= 0 || m_vec > 0x7fffffff / vec_length || N % 8 != 0 || !row_offsets ||
+        !column_indices || !values_f16 || !rhs_f16 || !add_f16 || !out_f16 || !aligned16(values_f16) || !aligned16(rhs_f16) || !aligned16(add_f16) ||
+        !aligned16(out_f16) || choice == 1 || choice == 2)
+        return 0;
+    SpmmArgs a;
+    a.m_vec = m_vec; a.V = vec_length; a.N = N; a.n_out = N; a.K = K;
+    a.row_indices = row_indices; a.row_offsets = row_offsets; a.column_indices = column_indices;
+    a.values = static_cast<const __half*>(values_f16); a.rhs = static_cast<const __half*>(rhs_f16);
+    a.out = out_f16; a.out_f16 = true; a.bias = static_cast<const __half*>(bias_f16); a.add = static_cast<const __half*>(add_f16); a.batch = 1;
+    a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
+    a.stream = static_cast<cudaStream_t>(stream);
+    // the kernel that sspmm_counted takes
+    const bool fits = block_fits(a, true);
+    cudaError_t e;
+    if (fits && (choice == 3 || (choice == 0 && block_kernel_is_faster(nvec, a)))) {
+        void* scratch = nullptr;
+        const size_t bytes = sspmm_block_scratch_bytes(a);
+        keep_pool_memory();
+        e = cudaMallocAsync(&scratch, bytes, a.stream);
+        if (e != cudaSuccess) { cudaGetLastError(); return 0; }
+        e = launch_sspmm_block(a, scratch, bytes);
+        cudaFreeAsync(scratch, a.stream);
+    } else {
+        if (choice == 3 || sspmm_rows_scratch_bytes(a, nvec)) return 0;        // long rows are cut there
+        e = launch_sspmm_rows_set(&a, 1, nvec);
+    }
+    if (e != cudaSuccess) return fail(e, "SpMM launch");
+    *taken = 1;
+    return 0;
+}
+
+int sspmm_dense_copies(int count, const sspmm_dense_operand* operands, int N, void* room, int64_t* offsets, int64_t* bytes, void* stream) {
+    g_err[0] = 0;
+    if (count < 0 || count > kMaxCopies || !operands || !offsets || !bytes) { set_error("null pointer or more than %d operands", kMaxCopies); return (int)cudaErrorInvalidValue; }
+    const int choice = g_kernel_choice.load();
+    SpmmArgs a[kMaxCopies];
+    __half* at[kMaxCopies];
+    int64_t room_for = 0;
+    int copies = 0;
+    for (int k = 0; k < count; ++k) {
+        const sspmm_dense_operand& o = operands[k];
+        offsets[k] = -1;
+        if ((o.vec_length != 8 && o.vec_length != 16) || o.pieces < 1 || o.pieces > kMaxPieces || o.m_vec <= 0 || o.K <= 0 || N <= 0 || N % 8 != 0 ||
+            o.m_vec > 0x7fffffff / o.vec_length / o.pieces || !o.row_offsets || !o.nvec || !o.column_indices || !o.values_f16 ||
+            !aligned16(o.values_f16) || choice == 1 || choice == 2 || choice == 4)
+            continue;
+        SpmmArgs& s = a[copies];
+        s = SpmmArgs{};
+        s.m_vec = o.m_vec; s.V = o.vec_length; s.N = N; s.n_out = N; s.K = o.K;
+        s.row_indices = nullptr; s.row_offsets = o.row_offsets[0]; s.column_indices = o.column_indices;
+        s.values = static_cast<const __half*>(o.values_f16); s.rhs = s.values;
+        s.out = room; s.out_f16 = true; s.bias = nullptr; s.batch = 1;
+        s.values_stride = 0; s.rhs_stride = 0; s.out_stride = 0; s.stream = static_cast<cudaStream_t>(stream);
+        // every piece would go to the block kernel by itself
+        bool block = true;
+        int64_t total = 0;
+        for (int i = 0; i < o.pieces && block; ++i) {
+            block = o.row_offsets[i] && o.nvec[i] >= 0 && total + o.nvec[i] <= 0x7fffffffLL && sspmm_block_scratch_bytes(s) <= ((size_t)2 << 30) &&
+                    (choice == 3 || block_kernel_is_faster(o.nvec[i], s));
+            s.piece_offsets[i] = o.row_offsets[i];
+            s.piece_first[i] = (int)total;
+            total += o.nvec[i];
+        }
+        if (!block) continue;
+        s.m_vec = o.pieces * o.m_vec;
+        s.pieces = o.pieces;
+        if (sspmm_block_scratch_bytes(s) > ((size_t)2 << 30)) continue;
+        offsets[k] = room_for;
+        at[copies] = reinterpret_cast<__half*>(static_cast<uint8_t*>(room) + room_for);
+        room_for += (int64_t)(((size_t)o.K * s.m_vec * s.V * sizeof(__half) + 255) & ~(size_t)255);
+        ++copies;
+    }
+    *bytes = room_for;
+    if (!room || copies == 0) return 0;
+    if (reinterpret_cast<uintptr_t>(room) % 256 != 0) { set_error("copies need room on a 256-byte boundary"); return (int)cudaErrorInvalidValue; }
+    const cudaError_t e = launch_expand_set(a, at, copies, static_cast<cudaStream_t>(stream));
+    return e == cudaSuccess ? 0 : fail(e, "dense copies");
+}
+
+int sspmm_of_copy(int m_vec, int vec_length, int N, int K, const void* copy_f16, const void* rhs_f16, const void* bias_f16, const void* add_f16,
+                  void* out_f16, void* stream) {
+    g_err[0] = 0;
+    if ((vec_length != 8 && vec_length != 16) || m_vec <= 0 || N <= 0 || K <= 0 || m_vec > 0x7fffffff / vec_length || N % 8 != 0 || !copy_f16 || !rhs_f16 ||
+        !out_f16 || !aligned16(copy_f16) || !aligned16(rhs_f16) || !aligned16(add_f16) || !aligned16(out_f16)) {
+        set_error("a product of a dense copy needs N %% 8 == 0 and 16-byte aligned operands");
+        return (int)cudaErrorInvalidValue;
+    }
+    SpmmArgs a;
+    a.m_vec = m_vec; a.V = vec_length; a.N = N; a.n_out = N; a.K = K;
+    a.row_indices = nullptr; a.row_offsets = nullptr; a.column_indices = nullptr; a.values = nullptr;
+    a.rhs = static_cast<const __half*>(rhs_f16);
+    a.out = out_f16; a.out_f16 = true; a.bias = static_cast<const __half*>(bias_f16); a.add = static_cast<const __half*>(add_f16); a.batch = 1;
+    a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
+    a.stream = static_cast<cudaStream_t>(stream);
+    a.copy = static_cast<const __half*>(copy_f16);
+    const size_t bytes = sspmm_block_scratch_bytes(a);              // partial tiles of a cut K range
+    void* scratch = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (bytes) {
+        keep_pool_memory();
+        e = cudaMallocAsync(&scratch, bytes, a.stream);
+        if (e != cudaSuccess) return fail(e, "scratch allocation for the SpMM");
+    }
+    e = launch_sspmm_block(a, scratch, bytes);
+    if (scratch) cudaFreeAsync(scratch, a.stream);
+    return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
+}
+
 int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int64_t* nvec, const int* const* row_indices,
                   const int* const* row_offsets, const int* column_indices, const void* values_f16, const void* rhs_f16,
                   const void* bias_f16, void* out, int out_is_f16, void* stream, int* taken) {

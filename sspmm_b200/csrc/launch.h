@@ -24,6 +24,7 @@ struct SpmmArgs {
     void* out;                 // [m_vec * V * N] row-major, fp32 or fp16
     bool out_f16;
     const __half* bias;        // per row of the output, added before the conversion; may be null
+    const __half* add = nullptr;   // like the output, added as well (fp16 results of one product; block kernel and launch_sspmm_rows_set)
     // batching (one launch, grid z-less: tiles enumerate the batch too)
     int batch;                 // >= 1
     int64_t values_stride;     // elements between batches (0 = shared)
@@ -35,6 +36,8 @@ struct SpmmArgs {
     int pieces = 1;
     const int* piece_offsets[kMaxPieces] = {};
     int piece_first[kMaxPieces] = {};
+    // Block kernel: the dense transposed copy [K][m_vec*V] of the operand (launch_expand_set); null: it makes its own from the operand.
+    const __half* copy = nullptr;
 };
 
 // tcgen05 row-gather kernel.  Requires N % 8 == 0, 16-byte aligned rhs/values.
@@ -56,6 +59,10 @@ cudaError_t launch_align_rows(const SpmmArgs& a, int ld, __half* dst);
 // (at least K * m_vec*V halfs) it runs without split-K.
 size_t sspmm_block_scratch_bytes(const SpmmArgs& a);
 cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_bytes);
+// Dense transposed copies of several operands (m_vec, V, K, column_indices, values and the row offsets of their pieces count) in one
+// launch; at[i] holds K * m_vec*V halfs.
+constexpr int kMaxCopies = 8;
+cudaError_t launch_expand_set(const SpmmArgs* a, __half* const* at, int count, cudaStream_t stream);
 // Allows (default) or forbids the CTA-pair variant of the block kernel.  Process-wide.
 void sspmm_block_allow_pairs(bool allow);
 // CUDA-core kernel without alignment requirements.

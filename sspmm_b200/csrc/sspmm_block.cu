@@ -56,52 +56,80 @@ struct PieceRows {
 };
 
 template <int V>
+__device__ __forceinline__ void expand_row(int m_vec, int K, int chunk, int i, int k_begin, const PieceRows& pieces, const int* __restrict__ col,
+                                           const __half* __restrict__ values, __half* __restrict__ at, int (&slot)[kExpandChunk]) {
+    const int64_t mp = (int64_t)m_vec * V;
+    const int k_end = min(K, k_begin + chunk);
+            for (int k = threadIdx.x; k < chunk; k += blockDim.x) slot[k] = -1;
+            __syncthreads();
+            const int piece = i / pieces.rows;
+            const int* const row = pieces.offsets[piece] + (i - piece * pieces.rows);
+            const int j0 = pieces.first[piece] + row[0], j1 = pieces.first[piece] + row[1];
+            // four independent loads in flight per thread: the kernel is a chain of dependent reads otherwise
+            for (int j = j0 + threadIdx.x; j < j1; j += 4 * blockDim.x) {
+                int c[4];
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) c[q] = (j + q * (int)blockDim.x < j1) ? __ldg(col + j + q * blockDim.x) : -1;
+    #pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (c[q] >= k_begin && c[q] < k_end) slot[c[q] - k_begin] = j + q * blockDim.x;   // duplicates: one of them wins
+            }
+            __syncthreads();
+            for (int k = k_begin + threadIdx.x; k < k_end; k += 4 * blockDim.x) {
+                int js[4];
+                uint4 v[4][V / 8];
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) js[q] = (k + q * (int)blockDim.x < k_end) ? slot[k + q * blockDim.x - k_begin] : -1;
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint4* src = reinterpret_cast<const uint4*>(values + (int64_t)(js[q] >= 0 ? js[q] : 0) * V);
+    #pragma unroll
+                    for (int h = 0; h < V / 8; ++h) v[q][h] = js[q] >= 0 ? __ldg(src + h) : make_uint4(0, 0, 0, 0);
+                }
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int kq = k + q * (int)blockDim.x;
+                    if (kq < k_end) {
+                        uint4* dst = reinterpret_cast<uint4*>(at + (int64_t)kq * mp + (int64_t)i * V);
+    #pragma unroll
+                        for (int h = 0; h < V / 8; ++h) dst[h] = v[q][h];
+                    }
+                }
+            }
+}
+
+template <int V>
 __global__ void __launch_bounds__(256)
 expand_transposed_kernel(int m_vec, int K, int chunk, const __grid_constant__ PieceRows pieces, const int* __restrict__ col,
                          const __half* __restrict__ values, __half* __restrict__ at) {
     __shared__ int slot[kExpandChunk];
-    const int64_t mp = (int64_t)m_vec * V;
-    const int k_begin = blockIdx.x * chunk;
-    const int k_end = min(K, k_begin + chunk);
     for (int i = blockIdx.y; i < m_vec; i += gridDim.y) {
-        for (int k = threadIdx.x; k < chunk; k += blockDim.x) slot[k] = -1;
-        __syncthreads();
-        const int piece = i / pieces.rows;
-        const int* const row = pieces.offsets[piece] + (i - piece * pieces.rows);
-        const int j0 = pieces.first[piece] + row[0], j1 = pieces.first[piece] + row[1];
-        // four independent loads in flight per thread: the kernel is a chain of dependent reads otherwise
-        for (int j = j0 + threadIdx.x; j < j1; j += 4 * blockDim.x) {
-            int c[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) c[q] = (j + q * (int)blockDim.x < j1) ? __ldg(col + j + q * blockDim.x) : -1;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (c[q] >= k_begin && c[q] < k_end) slot[c[q] - k_begin] = j + q * blockDim.x;   // duplicates: one of them wins
-        }
-        __syncthreads();
-        for (int k = k_begin + threadIdx.x; k < k_end; k += 4 * blockDim.x) {
-            int js[4];
-            uint4 v[4][V / 8];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) js[q] = (k + q * (int)blockDim.x < k_end) ? slot[k + q * blockDim.x - k_begin] : -1;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint4* src = reinterpret_cast<const uint4*>(values + (int64_t)(js[q] >= 0 ? js[q] : 0) * V);
-#pragma unroll
-                for (int h = 0; h < V / 8; ++h) v[q][h] = js[q] >= 0 ? __ldg(src + h) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int kq = k + q * (int)blockDim.x;
-                if (kq < k_end) {
-                    uint4* dst = reinterpret_cast<uint4*>(at + (int64_t)kq * mp + (int64_t)i * V);
-#pragma unroll
-                    for (int h = 0; h < V / 8; ++h) dst[h] = v[q][h];
-                }
-            }
-        }
+        expand_row<V>(m_vec, K, chunk, i, blockIdx.x * chunk, pieces, col, values, at, slot);
         __syncthreads();
     }
+}
+
+// Several operands in one launch, a CTA per row and chunk of each: the operands of an encoder layer (768 wide, 14 MB of copies), which
+// took a launch of 5.9 us before each product, take one of 12.4.
+struct ExpandSet {
+    int count, first[kMaxCopies + 1];        // first CTA of each operand, and the end
+    struct Operand {
+        int m_vec, K, V, chunk, chunks;
+        const int* col;
+        const __half* values;
+        __half* at;
+        PieceRows pieces;
+    } op[kMaxCopies];
+};
+__global__ void __launch_bounds__(256)
+expand_set_kernel(const __grid_constant__ ExpandSet s) {
+    __shared__ int slot[kExpandChunk];
+    int o = 0;
+    while (o + 1 < s.count && (int)blockIdx.x >= s.first[o + 1]) ++o;
+    const ExpandSet::Operand& op = s.op[o];
+    const int b = (int)blockIdx.x - s.first[o], i = b / op.chunks, k_begin = (b - i * op.chunks) * op.chunk;
+    if (op.V == 16) expand_row<16>(op.m_vec, op.K, op.chunk, i, k_begin, op.pieces, op.col, op.values, op.at, slot);
+    else expand_row<8>(op.m_vec, op.K, op.chunk, i, k_begin, op.pieces, op.col, op.values, op.at, slot);
 }
 
 template <int BN, int STAGES>
@@ -130,12 +158,34 @@ struct BlockProblem {
                              // per operand and stage brings all 64-wide chunks; 0: one instruction per chunk
     int64_t out_stride;      // per batch, elements
     const __half* bias;      // per row of C, added before the conversion; null: none (or added by the reduction)
+    const __half* add;       // [Mp][N] fp16, added before the conversion (fp16 results); null: none (or added by the reduction)
 };
 
 __device__ __forceinline__ void add_bias(uint32_t (&w)[32], float bias) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) + bias);
 }
+
+// 32 columns of a row that is added to C, from column n on; they are asked for a chunk ahead of their use.
+struct AddChunk {
+    uint4 v[4];
+    __device__ __forceinline__ void load(const __half* row, int n, int N) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) v[g] = row && n + 8 * g < N ? __ldg(reinterpret_cast<const uint4*>(row + n) + g) : make_uint4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ void add_to(uint32_t (&w)[32]) const {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const uint32_t x[4] = {v[g].x, v[g].y, v[g].z, v[g].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&x[i]));
+                w[8 * g + 2 * i] = __float_as_uint(__uint_as_float(w[8 * g + 2 * i]) + f.x);
+                w[8 * g + 2 * i + 1] = __float_as_uint(__uint_as_float(w[8 * g + 2 * i + 1]) + f.y);
+            }
+        }
+    }
+};
 
 template <int BN, int STAGES, typename OutT>
 __global__ void __launch_bounds__(kBlockThreads, 1)
@@ -262,6 +312,9 @@ sspmm_block_kernel(const __grid_constant__ CUtensorMap tmap_at, const __grid_con
             const int m0 = (r % p.m_tiles) * kBM, n0 = (r / p.m_tiles) * BN;
             const uint32_t buf = acc_it & 1u, acc_phase = (acc_it >> 1) & 1u;
             // the four warps must agree on leaving: they meet at named barriers below
+            const __half* const add_row = sizeof(OutT) == 2 && p.add && m0 + row < p.Mp ? p.add + (int64_t)(m0 + row) * p.N : nullptr;
+            AddChunk next;
+            if (sizeof(OutT) == 2 && p.add) next.load(add_row, n0, p.N);
             if (!named_barrier_and(2, 128, mbar_wait(bar_acc_full + 8 * buf, acc_phase, abort_flag, kStatusWaitBlock))) break;
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN;
@@ -270,6 +323,8 @@ sspmm_block_kernel(const __grid_constant__ CUtensorMap tmap_at, const __grid_con
             tmem_ld_x32(taddr, v[0]);
 #pragma unroll
             for (int cc = 0; cc < BN / 32; ++cc) {
+                AddChunk now = next;
+                if (sizeof(OutT) == 2 && p.add && cc + 1 < BN / 32) next.load(add_row, n0 + (cc + 1) * 32, p.N);
                 tc_wait_ld();
                 if (cc + 1 < BN / 32) {
                     tmem_ld_x32(taddr + (cc + 1) * 32, v[(cc + 1) & 1]);       // in flight while this chunk is stored
@@ -280,6 +335,7 @@ sspmm_block_kernel(const __grid_constant__ CUtensorMap tmap_at, const __grid_con
                 }
                 uint32_t(&w)[32] = v[cc & 1];
                 if (p.bias) add_bias(w, bias);
+                if (sizeof(OutT) == 2 && p.add) now.add_to(w);
 #pragma unroll
                 for (int h = 0; h < kStoresPerLoad; ++h) {
                     const uint32_t sb = st_it & 1u;
@@ -484,6 +540,9 @@ sspmm_block_pair_kernel(const __grid_constant__ CUtensorMap tmap_at, const __gri
             const int m0 = (r % p.m_tiles) * (2 * kBM) + (int)rank * kBM, n0 = (r / p.m_tiles) * BN;
             const bool rows_exist = m0 < p.Mp;                   // an odd number of 128-row tiles leaves the last half empty
             const uint32_t buf = acc_it & 1u, acc_phase = (acc_it >> 1) & 1u;
+            const __half* const add_row = sizeof(OutT) == 2 && p.add && m0 + row < p.Mp ? p.add + (int64_t)(m0 + row) * p.N : nullptr;
+            AddChunk next;
+            if (sizeof(OutT) == 2 && p.add) next.load(add_row, n0, p.N);
             if (!named_barrier_and(2, 128, mbar_wait(bar_acc_full + 8 * buf, acc_phase, abort_flag, kStatusWaitBlock))) break;
             tc_fence_after_sync();
             const uint32_t drained = cluster_map_shared(bar_acc_empty + 8 * buf, 0);
@@ -493,6 +552,8 @@ sspmm_block_pair_kernel(const __grid_constant__ CUtensorMap tmap_at, const __gri
             tmem_ld_x32(taddr, v[0]);
 #pragma unroll
             for (int cc = 0; cc < BN / 32; ++cc) {
+                AddChunk now = next;
+                if (sizeof(OutT) == 2 && p.add && cc + 1 < BN / 32) next.load(add_row, n0 + (cc + 1) * 32, p.N);
                 tc_wait_ld();
                 if (cc + 1 < BN / 32) {
                     tmem_ld_x32(taddr + (cc + 1) * 32, v[(cc + 1) & 1]);
@@ -503,6 +564,7 @@ sspmm_block_pair_kernel(const __grid_constant__ CUtensorMap tmap_at, const __gri
                 }
                 uint32_t(&w)[32] = v[cc & 1];
                 if (p.bias) add_bias(w, bias);
+                if (sizeof(OutT) == 2 && p.add) now.add_to(w);
 #pragma unroll
                 for (int h = 0; h < kStoresPerLoad; ++h) {
                     const uint32_t sb = st_it & 1u;
@@ -669,7 +731,7 @@ cudaError_t launch_block_pair(const SpmmArgs& a, const CUtensorMap& ta, const CU
 template <typename OutT>
 __global__ void __launch_bounds__(256)
 reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, int64_t elems, int splits, int N,
-                     const __half* __restrict__ bias) {
+                     const __half* __restrict__ bias, const __half* __restrict__ add) {
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= elems) return;                                      // elems is a multiple of 4 (N % 8 == 0)
     float4 acc = *reinterpret_cast<const float4*>(partial + i);
@@ -682,6 +744,11 @@ reduce_splits_kernel(const float* __restrict__ partial, OutT* __restrict__ out, 
         acc.x += b; acc.y += b; acc.z += b; acc.w += b;
     }
     if constexpr (sizeof(OutT) == 2) {
+        if (add) {
+            const uint2 a = __ldg(reinterpret_cast<const uint2*>(add + i));
+            const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&a.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&a.y));
+            acc.x += f0.x; acc.y += f0.y; acc.z += f1.x; acc.w += f1.y;
+        }
         __half2 lo = __floats2half2_rn(acc.x, acc.y), hi = __floats2half2_rn(acc.z, acc.w);
         uint2 w;
         w.x = *reinterpret_cast<uint32_t*>(&lo); w.y = *reinterpret_cast<uint32_t*>(&hi);
@@ -721,7 +788,7 @@ BlockPlan plan_block(const SpmmArgs& a, int sms, size_t budget) {
     pl.splits = 1;
     const int k_steps = (a.K + kBK - 1) / kBK;
     pl.steps_per_split = k_steps;
-    pl.at_bytes = (((size_t)a.K * Mp * sizeof(__half)) + 255) & ~(size_t)255;
+    pl.at_bytes = a.copy ? 0 : (((size_t)a.K * Mp * sizeof(__half)) + 255) & ~(size_t)255;
     pl.partial_bytes = 0;
     if (pl.pair || a.batch != 1 || tiles256 >= units || k_steps < 8) return pl;
     // Fewer 256-column tiles than SMs: pick tile width and split-K factor by a small time model
@@ -760,6 +827,46 @@ size_t sspmm_block_scratch_bytes(const SpmmArgs& a) {
     return pl.at_bytes + pl.partial_bytes;
 }
 
+namespace {
+int expand_chunk(int rows, int K, int sms) {
+    int chunk = kExpandChunk;
+    while (chunk > 256 && (int64_t)rows * ((K + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
+    return chunk;
+}
+PieceRows piece_rows(const SpmmArgs& a) {
+    PieceRows r = {a.m_vec, {a.row_offsets}, {0}};
+    if (a.pieces > 1) {
+        r.rows = a.m_vec / a.pieces;
+        for (int i = 0; i < a.pieces; ++i) { r.offsets[i] = a.piece_offsets[i]; r.first[i] = a.piece_first[i]; }
+    }
+    return r;
+}
+}  // namespace
+
+cudaError_t launch_expand_set(const SpmmArgs* a, __half* const* at, int count, cudaStream_t stream) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    ExpandSet s = {};
+    s.count = count;
+    int64_t blocks = 0, rows = 0;
+    for (int k = 0; k < count; ++k) rows += a[k].m_vec;
+    for (int k = 0; k < count; ++k) {
+        ExpandSet::Operand& op = s.op[k];
+        op.m_vec = a[k].m_vec; op.K = a[k].K; op.V = a[k].V;
+        op.chunk = expand_chunk((int)(rows < 0x7fffffff ? rows : 0x7fffffff), a[k].K, sms);
+        op.chunks = (a[k].K + op.chunk - 1) / op.chunk;
+        op.col = a[k].column_indices; op.values = a[k].values; op.at = at[k];
+        op.pieces = piece_rows(a[k]);
+        s.first[k] = (int)blocks;
+        blocks += (int64_t)op.m_vec * op.chunks;
+        if (blocks > 0x7fffffffLL) { set_error("too many rows for dense copies in one launch"); return cudaErrorInvalidValue; }
+        s.first[k + 1] = (int)blocks;
+    }
+    if (blocks == 0) return cudaSuccess;
+    expand_set_kernel<<<(unsigned)blocks, 256, 0, stream>>>(s);
+    return cudaGetLastError();
+}
+
 // `scratch` (scratch_bytes long, owned by the caller) holds the transposed dense copy of A
 // (K * m_vec*V halfs) and, when split-K is used, the fp32 partial tiles after it.
 // Every check and every tensor-map encode comes before the first launch: an error return has
@@ -775,10 +882,10 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
         return cudaErrorInvalidValue;
     }
     const int Mp = a.m_vec * a.V;
-    __half* at = static_cast<__half*>(scratch);
+    __half* at = a.copy ? const_cast<__half*>(a.copy) : static_cast<__half*>(scratch);
     const int sms = current_device_sm_count();
     if (sms <= 0) return cudaErrorNoDevice;
-    if (!scratch || (size_t)a.K * Mp * sizeof(__half) > scratch_bytes) {
+    if (!a.copy && (!scratch || (size_t)a.K * Mp * sizeof(__half) > scratch_bytes)) {
         set_error("scratch too small for the block kernel");
         return cudaErrorInvalidValue;
     }
@@ -795,6 +902,7 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     p.total_tiles = (int)total;
     p.out_stride = a.out_stride;
     p.bias = pl.splits > 1 ? nullptr : a.bias;
+    p.add = pl.splits > 1 ? nullptr : a.add;
     CUtensorMap ta, tb, tc;
     const bool split = pl.splits > 1;
     if (split && pl.at_bytes + pl.partial_bytes > scratch_bytes) {
@@ -833,16 +941,11 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     };
     cudaError_t e = gemm(true);
     if (e != cudaSuccess) return e;
-    {
+    if (!a.copy) {
         const int by = a.m_vec < 32768 ? a.m_vec : 32768;
-        int chunk = kExpandChunk;
-        while (chunk > 256 && (int64_t)by * ((a.K + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
+        const int chunk = expand_chunk(by, a.K, sms);
         const dim3 grid((a.K + chunk - 1) / chunk, by);
-        PieceRows r = {a.m_vec, {a.row_offsets}, {0}};
-        if (a.pieces > 1) {
-            r.rows = a.m_vec / a.pieces;
-            for (int i = 0; i < a.pieces; ++i) { r.offsets[i] = a.piece_offsets[i]; r.first[i] = a.piece_first[i]; }
-        }
+        const PieceRows r = piece_rows(a);
         if (a.V == 16) expand_transposed_kernel<16><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, r, a.column_indices, a.values, at);
         else expand_transposed_kernel<8><<<grid, 256, 0, a.stream>>>(a.m_vec, a.K, chunk, r, a.column_indices, a.values, at);
         e = cudaGetLastError();
@@ -852,8 +955,8 @@ cudaError_t launch_sspmm_block(const SpmmArgs& a, void* scratch, size_t scratch_
     if (e != cudaSuccess || !split) return e;
     const int64_t elems = (int64_t)Mp * a.N;
     const unsigned rgrid = (unsigned)((elems / 4 + 255) / 256);
-    if (a.out_f16) reduce_splits_kernel<__half><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<__half*>(a.out), elems, pl.splits, a.N, a.bias);
-    else reduce_splits_kernel<float><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<float*>(a.out), elems, pl.splits, a.N, a.bias);
+    if (a.out_f16) reduce_splits_kernel<__half><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<__half*>(a.out), elems, pl.splits, a.N, a.bias, a.add);
+    else reduce_splits_kernel<float><<<rgrid, 256, 0, a.stream>>>(partial, static_cast<float*>(a.out), elems, pl.splits, a.N, a.bias, nullptr);
     return cudaGetLastError();
 }
 

@@ -1523,6 +1523,22 @@ int sspmm_group_bias(sspmm_group* group, int item, const void* bias_f16, int* ta
     return 0;
 }
 
+int sspmm_group_run_sum(sspmm_group* group, const void* bias_f16, const void* add_f16, void* out_f16, void* stream, int* taken) {
+    set_error("%s", "");
+    if (!group || !taken || !add_f16 || !out_f16) { set_error("null group, operand or output pointer"); return (int)cudaErrorInvalidValue; }
+    *taken = 0;
+    if (group->rows.empty() || group->count != 1 || !group->out_f16 || !fused::aligned16(add_f16) || !fused::aligned16(out_f16)) return 0;
+    SpmmArgs a = group->rows[0];
+    a.stream = static_cast<cudaStream_t>(stream);
+    a.bias = static_cast<const __half*>(bias_f16);
+    a.add = static_cast<const __half*>(add_f16);
+    a.out = out_f16;
+    const cudaError_t e = launch_sspmm_rows_set(&a, 1, group->rows_nvec);
+    if (e != cudaSuccess) { set_error("group launch: %s", cudaGetErrorString(e)); return (int)e; }
+    *taken = 1;
+    return 0;
+}
+
 int sspmm_group_info(const sspmm_group* group, int* tile_columns, int* work_items, int* ctas, int* launches,
                      int64_t* scratch_bytes) {
     if (!group) return (int)cudaErrorInvalidValue;

@@ -252,14 +252,23 @@ struct Tile {
         o[4] += hi.x; o[5] += hi.y; o[6] += hi.z; o[7] += hi.w;
     }
     // Writes this lane's piece of unit u to C (first_row: the first of the vector row's V rows).
-    template <typename OutT>
+    template <typename OutT, bool ADD = false>
     static __device__ __forceinline__ void store_unit(const Problem& p, OutT* __restrict__ out, int64_t first_row, int n0, int u, int lane,
-                                                      float (&o)[8]) {
+                                                      float (&o)[8], const __half* add = nullptr) {
         const int id = u * 32 + lane, n = n0 + (id % kPieces) * 8;
         if (p.bias) {
             const float b = __half2float(p.bias[first_row + id / kPieces]);
 #pragma unroll
             for (int e = 0; e < 8; ++e) o[e] += b;
+        }
+        if (ADD && add && n < p.N) {                             // (rows are whole pieces)
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(add + (first_row + id / kPieces) * p.N + n));
+            const uint32_t x[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&x[e]));
+                o[2 * e] += f.x; o[2 * e + 1] += f.y;
+            }
         }
         OutT* dst = out + (first_row + id / kPieces) * p.N + n;
         if (p.out_pieces) {
@@ -311,8 +320,9 @@ struct Tile {
         }
     }
     // A warp's own tile to C, eight rows at a time through one slot of its ring.
-    template <typename OutT>
-    __device__ __forceinline__ void store(const Problem& p, OutT* __restrict__ out, int64_t first_row, int n0, float* slot, int lane) const {
+    template <typename OutT, bool ADD = false>
+    __device__ __forceinline__ void store(const Problem& p, OutT* __restrict__ out, int64_t first_row, int n0, float* slot, int lane,
+                                          const __half* add = nullptr) const {
         static_assert(8 * kPitch * 4 <= kWarpBytes, "eight rows of sums fit the ring");
         const int g = lane >> 2, t = lane & 3;
 #pragma unroll
@@ -326,7 +336,7 @@ struct Tile {
             for (int u = 0; u < kUnits / VB; ++u) {
                 float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 add_piece(slot + piece_at(u, lane), o);
-                store_unit(p, out, first_row + vb * 8, n0, u, lane, o);
+                store_unit<OutT, ADD>(p, out, first_row + vb * 8, n0, u, lane, o, add);
             }
             __syncwarp();
         }
@@ -338,8 +348,9 @@ struct Tile {
 // warp order through shared memory (of the cluster), so results do not depend on timing.
 // cta_item: the first of the CTA's (or cluster's) items, of problem p.  (With the warp's own item in its place the plain kernel of V = 16
 // took another register and 2 to 5 % more time: 2048 x 4608 at 90 %, N = 2048 225 us, 216 as it is; 1500 x 2500 at 80 %, N = 800 60.3 and 57.0.)
-template <int V, typename OutT, int H>
-__device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ out, long long cta_item, int team, int cluster) {
+template <int V, typename OutT, int H, bool ADD = false>
+__device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ out, long long cta_item, int team, int cluster,
+                                         const __half* add = nullptr) {
     using T = Tile<V, H, sizeof(OutT) == 4>;
     extern __shared__ __align__(128) uint8_t smem[];    // [warp][T::kWarpBytes]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -355,7 +366,7 @@ __device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ ou
     OutT* const cbase = out + w.batch * p.out_stride;
     const int64_t first_row = (int64_t)w.row * V;
     if (team == 1) {
-        if (w.row >= 0) tile.store(p, cbase, first_row, w.n0, reinterpret_cast<float*>(mem), lane);
+        if (w.row >= 0) tile.template store<OutT, ADD>(p, cbase, first_row, w.n0, reinterpret_cast<float*>(mem), lane, add);
         return;
     }
     tile.spill(reinterpret_cast<float*>(mem), lane);
@@ -367,7 +378,7 @@ __device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ ou
         for (int m = 0; m < team; ++m)
             T::add_piece(reinterpret_cast<const float*>(smem + (warp - member + m) * T::kWarpBytes) + T::piece_at(u, lane), o);
         if (cluster == 1) {
-            if (w.row >= 0) T::store_unit(p, cbase, first_row, w.n0, u, lane, o);
+            if (w.row >= 0) T::template store_unit<OutT, ADD>(p, cbase, first_row, w.n0, u, lane, o, add);
         } else {
 #pragma unroll
             for (int e = 0; e < 8; ++e) kept[e] = o[e];
@@ -389,7 +400,7 @@ __device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ ou
 #pragma unroll
             for (int e = 0; e < 8; ++e) o[e] += ld_cluster_f32(remote + e * 128);
         }
-        if (w.row >= 0) T::store_unit(p, cbase, first_row, w.n0, u, lane, o);
+        if (w.row >= 0) T::template store_unit<OutT, ADD>(p, cbase, first_row, w.n0, u, lane, o, add);
     }
     cluster_sync_all();                                   // nobody leaves while its tile is being read
 }
@@ -454,16 +465,18 @@ struct ProblemSet {
     int count;
     int first[kRowsMaxSet + 1];           // first item of each product, and the end
     void* out[kRowsMaxSet];
+    const __half* add[kRowsMaxSet];       // like C, added to the sums; or null (only looked at with ADD)
     Problem p[kRowsMaxSet];
 };
-template <int V, typename OutT, int H>
+template <int V, typename OutT, int H, bool ADD>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_set_kernel(const __grid_constant__ ProblemSet s, int team, int cluster) {
     const int per_cta = kWarps / team, warp = threadIdx.x >> 5;
     const long long item = (long long)(blockIdx.x / cluster) * per_cta + warp / team;
     int k = 0;
     while (k + 1 < s.count && item >= s.first[k + 1]) ++k;
-    do_items<V, OutT, H>(s.p[k], static_cast<OutT*>(s.out[k]), item - warp / team - s.first[k], team, cluster);
+    do_items<V, OutT, H, ADD>(s.p[k], static_cast<OutT*>(s.out[k]), item - warp / team - s.first[k], team, cluster,
+                            ADD ? s.add[k] : nullptr);
 }
 
 // Matrices whose rows differ in length by orders of magnitude (power-law matrices: half of the rows have fewer than 50
@@ -668,11 +681,11 @@ cudaError_t launch_plain(const SpmmArgs& a, const Problem& p, const Division& d,
     return launch_items<V, OutT, H>(sspmm_rows_kernel<V, OutT, H>, once, p.items, d, a.stream, p, static_cast<OutT*>(a.out));
 }
 
-template <int V, typename OutT>
+template <int V, typename OutT, bool ADD>
 cudaError_t launch_set(const ProblemSet& s, const Division& d, cudaStream_t stream) {
     static DeviceOnce once_wide, once_narrow;
-    if (d.H == 2) return launch_items<V, OutT, 2>(sspmm_rows_set_kernel<V, OutT, 2>, once_wide, s.first[s.count], d, stream, s);
-    return launch_items<V, OutT, 1>(sspmm_rows_set_kernel<V, OutT, 1>, once_narrow, s.first[s.count], d, stream, s);
+    if (d.H == 2) return launch_items<V, OutT, 2>(sspmm_rows_set_kernel<V, OutT, 2, ADD>, once_wide, s.first[s.count], d, stream, s);
+    return launch_items<V, OutT, 1>(sspmm_rows_set_kernel<V, OutT, 1, ADD>, once_narrow, s.first[s.count], d, stream, s);
 }
 
 template <int V, typename OutT, int H>
@@ -827,10 +840,17 @@ cudaError_t launch_sspmm_rows_set(const SpmmArgs* a, int count, long long nvec) 
     for (int k = 0; k < count; ++k) {
         s.p[k] = rows::problem_of(a[k], d.H);
         s.out[k] = a[k].out;
+        s.add[k] = a[k].add;
         s.first[k + 1] = s.first[k] + (int)s.p[k].items;
     }
-    if (a->V == 16) return a->out_f16 ? rows::launch_set<16, __half>(s, d, a->stream) : rows::launch_set<16, float>(s, d, a->stream);
-    return a->out_f16 ? rows::launch_set<8, __half>(s, d, a->stream) : rows::launch_set<8, float>(s, d, a->stream);
+    bool add = false;
+    for (int k = 0; k < count; ++k) add = add || a[k].add;
+    if (add) {
+        if (!a->out_f16) { set_error("sums are added to fp16 results only"); return cudaErrorInvalidValue; }
+        return a->V == 16 ? rows::launch_set<16, __half, true>(s, d, a->stream) : rows::launch_set<8, __half, true>(s, d, a->stream);
+    }
+    if (a->V == 16) return a->out_f16 ? rows::launch_set<16, __half, false>(s, d, a->stream) : rows::launch_set<16, float, false>(s, d, a->stream);
+    return a->out_f16 ? rows::launch_set<8, __half, false>(s, d, a->stream) : rows::launch_set<8, float, false>(s, d, a->stream);
 }
 
 // ---- dense operands whose rows do not start on 16-byte boundaries -------------------------------

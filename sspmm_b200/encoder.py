@@ -55,6 +55,12 @@ class SparseLinear:
         pad = -self.out_features % self.V
         return F.pad(b, (0, pad)) if pad else b
 
+    def of_copy(self, copy: Optional[torch.Tensor], x: torch.Tensor, add: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+        """``self(x)``, plus ``add``, from the dense copy of this linear that ``_copies`` made for this call; None: there is none, or
+        these are not tensors for it."""
+        rows = None if copy is None or not (_plain(x) if add is None else _plain(x, add)) else self.bias_rows()
+        return None if rows is None else ops.of_copy(copy, x, self.V, rows, add)
+
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         rows = self.bias_rows()
         if rows is not None:
@@ -62,6 +68,14 @@ class SparseLinear:
         y = ops.sspmm(self.row_offsets, self.col, self.values, x, self.V, row_indices=self.row_indices)
         y = y[: self.out_features]
         return y if self.bias is None else y + self.bias[:, None]
+
+    def plus(self, x: torch.Tensor, add: torch.Tensor) -> torch.Tensor:
+        """``self(x) + add``, rounded once where the product's kernel adds it to its sums."""
+        rows = self.bias_rows() if self.out_features % self.V == 0 and _plain(x, add) else None
+        got = None
+        if rows is not None:
+            got = ops.sspmm_sum(self.row_offsets, self.col, self.values, x, self.V, rows, self.row_indices, add)
+        return self(x) + add if got is None else got
 
     def dense_forward(self, x: torch.Tensor) -> torch.Tensor:
         y = self.dense @ x
@@ -104,6 +118,17 @@ class StackedLinears:
         return all(view(l.col, self.col, at, end) and view(l.values, self.values, at * self.V, end * self.V) and
                    view(l.bias, self.bias, i * self.rows, (i + 1) * self.rows)
                    for i, (l, at, end) in enumerate(zip(linears, self.ends, self.ends[1:])))
+
+    def operand(self, linears):
+        """What ``ops.dense_copies`` takes, or None."""
+        if not self._holds(linears):
+            return None
+        return [l.row_offsets for l in linears], self.ends[1:], self.col, self.values, self.V, linears[0].in_features
+
+    def of_copy(self, copy: Optional[torch.Tensor], x: torch.Tensor):
+        """The linears' results from the copy of what ``operand`` gave in this call, or None."""
+        y = ops.of_copy(copy, x, self.V, self.bias) if copy is not None and _plain(x) else None
+        return None if y is None else y.split(self.rows)
 
     def __call__(self, linears, x: torch.Tensor):
         """The linears' results, or None when these are not the operands that were stacked, a bias is not plain or the call is not
@@ -175,6 +200,20 @@ class SparseEncoderLayer:
         att = self._attention(q, k, v, batch, seq)
         return att.contiguous() if out is None else out.copy_(att)
 
+    def _copies(self, tokens: int):
+        """Dense copies of the operands of this call's products, by one launch: of Q, K and V together, O, FFN1 and FFN2; None for a
+        product that does not work on one.  (Below 512 tokens none does.)"""
+        L = self.linears
+        qkv = getattr(self, "qkv", None)
+        if tokens < 512 or any(type(l) is not SparseLinear or l.out_features % l.V for l in L[3:]):
+            return [None] * 4
+        first = qkv.operand(L[:3]) if qkv else None
+        each = [([l.row_offsets], [l.col.numel()], l.col, l.values, l.V, l.in_features) for l in L[3:]]
+        made = ops.dense_copies(([first] if first else []) + each, tokens)
+        if made is None:
+            return [None] * 4
+        return made if first else [None] + made
+
     def _groups_for(self, tokens: int):
         """Activation buffers of fixed shape and, bound to them, one group per dependency level of the layer:
         {Q, K, V} share their input and run as one launch, then O, FFN1, FFN2.  Groups keep addresses, so they are made again when a
@@ -215,9 +254,13 @@ class SparseEncoderLayer:
         g[2].run()
         if L[4].bias is not None and not added:
             b["h"] += L[4].bias[:, None]
-        g[3].run()
         bias = L[5].bias_rows()
-        if bias is not None and out is b["sum"] and bias.get_device() == out.get_device():       # as LayerNorm's kernel left it
+        plain = bias is not None and out is b["sum"] and bias.get_device() == out.get_device()    # as LayerNorm's kernel left it
+        y = g[3].run_sum(bias, out) if plain else None
+        if y is not None:
+            return y
+        g[3].run()
+        if plain:
             return ops.launch_add_bias_fm(b["y"], bias, out)
         return (b["y"] if L[5].bias is None else b["y"] + L[5].bias[:, None]) + out
 
@@ -230,9 +273,18 @@ class SparseEncoderLayer:
             q, k, v = (l.dense_forward(y) for l in L[:3])
             out = L[3].dense_forward(self._attention(q, k, v, batch, seq).contiguous()) + x
             return L[5].dense_forward(L[4].dense_forward(self._layer_norm_fm(out, self.ln2))) + out
+        copies = self._copies(x.shape[-1])
+
+        def product(i, a):
+            y = L[i].of_copy(copies[i - 2], a) if copies[i - 2] is not None else None
+            return L[i](a) if y is None else y
         _, y = self._norm(x, self.ln1)
         qkv = getattr(self, "qkv", None)
-        q, k, v = (qkv and qkv(L[:3], y)) or [l(y) for l in L[:3]]
-        att = L[3](self._attend(q, k, v, batch, seq))
+        q, k, v = (qkv and (qkv.of_copy(copies[0], y) or qkv(L[:3], y))) or [l(y) for l in L[:3]]
+        att = product(3, self._attend(q, k, v, batch, seq))
         out, y = self._norm(att, self.ln2, add=x)
-        return L[5](L[4](y)) + out
+        h = product(4, y)
+        if type(L[5]) is not SparseLinear:
+            return L[5](h) + out
+        y = L[5].of_copy(copies[3], h, out)
+        return L[5].plus(h, out) if y is None else y

@@ -100,6 +100,27 @@ def sspmm_bias(row_offsets: torch.Tensor, column_indices: torch.Tensor, values: 
     return out
 
 
+def sspmm_sum(row_offsets, column_indices, values, rhs, vec_length: int, bias, row_indices, add) -> Optional[torch.Tensor]:
+    """``sspmm_bias`` with a matrix like the result added to the fp32 sums before they are rounded (``sspmm_counted_sum``), or None
+    when the sum has to be made from the product's result."""
+    got = capi.native().sspmm_sum(row_offsets, column_indices, values, rhs, vec_length, bias, row_indices, add)
+    return None if got is None else _made(got)
+
+
+def dense_copies(operands, N: int):
+    """The dense copies that the block kernel works on, of operands whose products with N columns are still to come, by one launch
+    (``sspmm_dense_copies``).  ``operands``: (list of row offsets, where their vectors end, column_indices, values, vec_length, K).  A copy or
+    None (the product does not work on one) for each; None: not operands for it."""
+    got = capi.native().dense_copies(operands, N)
+    return None if got is None else _made(got)
+
+
+def of_copy(copy: torch.Tensor, rhs: torch.Tensor, vec_length: int, bias: torch.Tensor, add: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """The product of an operand's copy and rhs, plus bias and ``add`` (``sspmm_of_copy``); None: not tensors for it."""
+    got = capi.native().of_copy(copy, rhs, vec_length, bias, add)
+    return None if got is None else _made(got)
+
+
 def sspmm_stacked(row_offsets, row_indices, ends, column_indices: torch.Tensor, values: torch.Tensor, rhs: torch.Tensor, vec_length: int,
                   bias: torch.Tensor) -> Optional[torch.Tensor]:
     """Operands of one shape, their vectors one after another up to ``ends``, times the same rhs as one product (``sspmm_stacked``):
@@ -388,6 +409,15 @@ class Group:
         if taken.value:
             self._biases[item] = bias
         return bool(taken.value)
+
+    def run_sum(self, bias: Optional[torch.Tensor], add: torch.Tensor) -> Optional[torch.Tensor]:
+        """A run of a group of one product whose result, with this bias and ``add`` added before it is rounded, goes to a new tensor;
+        None: this group's kernel does not do that, or ``add`` is not like the output, and nothing was launched."""
+        out = self._keep[0][3]
+        if not self._h or len(self._keep) != 1 or add.shape != out.shape or add.device != out.device:
+            return None
+        got = capi.native().group_run_sum(self._h.value, out.shape[0], bias, add)
+        return None if got is None else _made(got)
 
     def run(self) -> None:
         rc = capi.native().group_run(self._h.value if self._h else 0, self.device.index)

@@ -1,5 +1,6 @@
 """Encoder layer with pruned, SVC-compressed weights against the same layer evaluated with dense
 matrices (torch.matmul on the densified pruned weights)."""
+import numpy as np
 import pytest
 import torch
 
@@ -217,6 +218,95 @@ def test_layer_norm_with_features_in_registers(lib, hidden):
     ops.layer_norm_fm(x, w, w, 1e-5, out)
     ops.layer_norm_fm(x, w, w, 1e-5, x)
     assert torch.equal(out, x)
+
+
+@pytest.mark.parametrize("M,K,N,V,sparsity,kernel", [
+    (64, 64, 8, 8, 0.5, 0), (256, 1024, 128, 16, 0.9, 0), (200, 300, 72, 8, 0.9, 0), (768, 3072, 200, 16, 0.95, 0),     # rows by warps
+    (256, 512, 128, 8, 0.9, 3), (136, 520, 264, 8, 0.5, 3), (768, 3072, 128, 16, 0.9, 3),                             # tiles, K cut or not
+    (768, 3072, 8192, 16, 0.9, 0), (272, 640, 19000, 16, 0.9, 3)])                                                    # CTA pairs, a half empty one
+def test_product_plus_a_matrix(lib, M, K, N, V, sparsity, kernel):
+    """Against the same product with fp32 results: the sum is rounded once, and the fp32 sums of two launches differ by 1e-5 of the
+    operands' sizes at most (order of the parts, truncation of the tensor unit over K <= 3072)."""
+    from sspmm_b200 import ops, synthetic
+    w = synthetic.magnitude_pruned(M, K, sparsity, np.random.default_rng(M + N))
+    d = lambda a: torch.from_numpy(a).to("cuda:0")
+    ptr, col, val, _ = ops.svc(d(w.row_ptr), d(w.col_idx), d(w.values), M, K, V)
+    rows = (ptr.numel() - 1) * V
+    g = torch.Generator(device="cuda:0").manual_seed(N)
+    r = lambda *s: torch.randn(s, device="cuda:0", generator=g).half()
+    rhs, add, bias, order = r(K, N), r(rows, N) * 4, r(rows), ops.sorted_row_swizzle(ptr)
+    ops.set_kernel(kernel)
+    try:
+        got = ops.sspmm_sum(ptr, col, val, rhs, V, bias, order, add)
+        want = ops.sspmm_bias(ptr, col, val, rhs, V, bias, row_indices=order, out_dtype=torch.float32).double() + add.double()
+    finally:
+        ops.set_kernel(0)
+    assert got is not None and got.dtype == torch.float16
+    assert ((got.double() - want).abs() <= 2.0 ** -11 * want.abs() + 1e-5 * (1 + want.abs().max())).all()
+    if kernel == 0 and K <= 1024:
+        plan = ops.Plan(ptr, col, V, K)
+        group = ops.Group([(plan, val, rhs, torch.full((rows, N), 7.0, device="cuda:0", dtype=torch.float16))])
+        if plan.one_launch and group.run_sum(None, add) is not None:
+            assert torch.equal(group.run_sum(bias, add), got) or N % 64            # the same division, or another tile width
+            assert (group._keep[0][3] == 7).all()
+    assert ops.sspmm_sum(ptr, col, val, rhs, V, bias, order, add[:, : N - 8]) is None
+    assert ops.sspmm_sum(ptr, col, val, rhs, V, bias, order, add.float()) is None
+
+
+@pytest.mark.parametrize("V,N,shapes", [(8, 264, [(64, 64), (136, 1300), (512, 100)]), (16, 136, [(768, 3072), (48, 1024), (16, 8), (3072, 768)]),
+                                        (16, 8192, [(768, 3072), (256, 1040)])])
+def test_products_of_copies_made_by_one_launch(lib, V, N, shapes):
+    """Rows and chunks of several operands in one launch, one of them three pieces: bit by bit the product that makes its own copy."""
+    from sspmm_b200 import ops, synthetic
+    d = lambda a: torch.from_numpy(a).to("cuda:0")
+    g = torch.Generator(device="cuda:0").manual_seed(N)
+    r = lambda *s: torch.randn(s, device="cuda:0", generator=g).half()
+    operands, products = [], []
+    for i, (M, K) in enumerate(shapes):
+        pieces = [ops.svc(d(w.row_ptr), d(w.col_idx), d(w.values), M, K, V)
+                  for w in (synthetic.magnitude_pruned(M, K, 0.8, np.random.default_rng(M + K + x)) for x in range(3 if i == 0 else 1))]
+        ends = torch.cumsum(torch.tensor([p[1].numel() for p in pieces]), 0).tolist()
+        col, val = torch.cat([p[1] for p in pieces]), torch.cat([p[2] for p in pieces])
+        operands.append(([p[0] for p in pieces], ends, col, val, V, K))
+        products.append((pieces, r(K, N), r(len(pieces) * (pieces[0][0].numel() - 1) * V)))
+    ops.set_kernel(3)
+    try:
+        copies = ops.dense_copies(operands, N)
+        assert all(c is not None and c.data_ptr() % 256 == 0 for c in copies)
+        for copy, (pieces, rhs, bias) in zip(copies, products):
+            rows = bias.numel() // len(pieces)
+            got = ops.of_copy(copy, rhs, V, bias)
+            for i, (ptr, col, val, _) in enumerate(pieces):
+                dense = copy[:, i * rows: (i + 1) * rows].contiguous()
+                own = ops.sspmm_bias(ptr, col, val, rhs, V, bias[i * rows: (i + 1) * rows].contiguous())
+                one = ops.of_copy(dense, rhs, V, bias[i * rows: (i + 1) * rows].contiguous())
+                assert torch.equal(one, own)
+                assert (got[i * rows: (i + 1) * rows].double() - own.double()).norm() <= 2 * 2.0 ** -11 * own.double().norm()
+                if len(pieces) == 1:
+                    assert torch.equal(got, own)
+    finally:
+        ops.set_kernel(0)
+    assert ops.dense_copies([([torch.tensor([0, 1], device="cuda:0", dtype=torch.int32)], [1], *[t[:n].contiguous() for t, n in
+                            ((products[0][0][0][1], 1), (products[0][0][0][2], V))], V, 64)], 512) == [None]
+
+
+def test_layer_of_copies_is_the_layer(lib, monkeypatch):
+    """The same layer with every product making its own copy, and one whose linears were replaced."""
+    from sspmm_b200.encoder import SparseEncoderLayer
+    layer = SparseEncoderLayer(hidden=512, ffn=2048, heads=8, sparsity=0.9, vec_length=16)
+    x = torch.randn(512, 4096, device="cuda:0", dtype=torch.float16)
+    assert all(c is not None for c in layer._copies(4096)) and layer._copies(64) == [None] * 4
+    y = layer.forward(x, 8, 512)
+    layer.linears[4].values.mul_(2)
+    scaled = layer.forward(x, 8, 512)
+    layer.linears[4].values.div_(2)
+    monkeypatch.setattr(layer, "_copies", lambda tokens: [None] * 4)
+    assert torch.equal(y, layer.forward(x, 8, 512)) and not torch.equal(y, scaled)
+    monkeypatch.undo()
+    own = layer.linears[5]
+    layer.linears[5] = lambda a: own(a)
+    assert layer._copies(4096) == [None] * 4
+    assert (layer.forward(x, 8, 512).double() - y.double()).norm() <= 4 * 2.0 ** -11 * y.double().norm()
 
 
 def test_stacked_linears_follow_their_tensors(lib):
