@@ -33,13 +33,14 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 // ---- LayerNorm ------------------------------------------------------------------------------------
-// Bound by memory: x (and add) read once, out (and the sum) written once.  A CTA takes TT tokens and keeps what it has read for the passes
-// for the mean, the variance and the result: in shared memory, or, where 32 tokens per CTA give every SM one and there are
-// at most 1024 features, in the registers of 512 threads.  32 tokens give 64-byte runs; with few tokens TT = 8 spreads
-// them over more SMs.  Through shared memory, 768 x 16384 took 24.0 us, with a sum 40.2: every thread added up the warps' sums for
-// itself (64 reads twice), converted every element three times and worked on one element per instruction.  From registers, with pairs
-// of elements per instruction and sums that are added up once, 16.6 and 24.8 (operands that change from call to call; 5000 tokens 14.0
-// and 20.1, now 9.5 and 12.5; 256 x 16384 10.6 and 14.5, now 10.3 and 12.3).  256 threads with twice the registers take 17.1 and 36.6.
+// Bound by memory: x (and add) read once, out (and the sum) written once.  A CTA takes TT tokens, as many as give every SM a CTA (8, 16 or
+// 32: runs of 16, 32 or 64 bytes), and keeps what it has read for the passes for the mean, the variance and the result in the registers of
+// 512 threads; 32 tokens of more than 1024 features go through shared memory.  Through shared memory, 768 x 16384 took 24.0 us,
+// with a sum 40.2: every thread added up the warps' sums for itself (64 reads twice), converted every element three times and worked
+// on one element per instruction.  From registers, with pairs of elements per instruction and sums that are added up once, 16.6
+// and 24.8 (operands that change from call to call); 256 threads with twice the registers take 17.1 and 36.6.  In graph replays 256 x 128 2.75 us
+// and 3.19, now 2.28 and 2.63; 768 x 1024 4.68 and 6.15, now 3.77 and 4.77; 512 x 4000 7.36 and 9.83, now 4.10 and 5.14; 3072 x 512 9.25 and
+// 15.3, now 7.07 and 11.1.
 constexpr int kLnThreads = 256, kLnWideThreads = 512;
 template <int TT>
 __global__ void __launch_bounds__(kLnThreads)
@@ -168,13 +169,14 @@ __device__ __forceinline__ uint4 pack4(const f32x2 (&f)[4]) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// The same with a thread's share in registers: 32 tokens, up to 128 * NV features.
-template <int NV>
+// The same with a thread's share in registers: TT tokens, up to 4096 / TT * NV features.
+template <int TT, int NV>
 __global__ void __launch_bounds__(kLnWideThreads, 2)
 layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
                           __half* __restrict__ sum_out, const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps,
                           __half* __restrict__ out) {
-    constexpr int TT = 32, P = TT / 8, kRows = kLnWideThreads / P;
+    constexpr int P = TT / 8, kRows = kLnWideThreads / P, kPair = NV < 2 ? 1 : 2;
+    static_assert(NV % kPair == 0, "whole pairs");
     __shared__ float red[kLnWideThreads / 32][TT];
     __shared__ __align__(16) float whole[2][TT];
     const int piece = threadIdx.x % P, r0 = threadIdx.x / P, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -189,9 +191,12 @@ layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, 
         for (int e = 0; e < 2; ++e) h[e] = add2(upper ? f[2 + e] : f[e], __shfl_xor_sync(0xffffffffu, upper ? f[e] : f[2 + e], 16));
         const float2 q = floats_of(add2(odd ? h[1] : h[0], __shfl_xor_sync(0xffffffffu, odd ? h[0] : h[1], 8)));
         const float own = lane & 4 ? q.y : q.x, other = lane & 4 ? q.x : q.y;
-        red[warp][piece * 8 + (lane >> 4) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1)] = own + __shfl_xor_sync(0xffffffffu, other, 4);
+        float one = own + __shfl_xor_sync(0xffffffffu, other, 4);
+#pragma unroll
+        for (int o = P; o < 4; o <<= 1) one += __shfl_xor_sync(0xffffffffu, one, o);
+        red[warp][piece * 8 + (lane >> 4) * 4 + (lane >> 3 & 1) * 2 + (lane >> 2 & 1)] = one;
         __syncthreads();
-        if (warp == 0) {
+        if (threadIdx.x < TT) {
             float t = 0.f;
 #pragma unroll
             for (int w = 0; w < kLnWideThreads / 32; ++w) t += red[w][lane];
@@ -224,12 +229,12 @@ layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, 
             }
     if (add)
 #pragma unroll
-        for (int j0 = 0; j0 < NV; j0 += 2) {
-            uint4 a[2];
+        for (int j0 = 0; j0 < NV; j0 += kPair) {
+            uint4 a[kPair];
 #pragma unroll
-            for (int q = 0; q < 2; ++q) a[q] = j0 + q < last ? __ldg(reinterpret_cast<const uint4*>(add + at0 + (j0 + q) * turn)) : make_uint4(0, 0, 0, 0);
+            for (int q = 0; q < kPair; ++q) a[q] = j0 + q < last ? __ldg(reinterpret_cast<const uint4*>(add + at0 + (j0 + q) * turn)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
+            for (int q = 0; q < kPair; ++q) {
                 f32x2 f[4], g[4];
                 unpack4(v[j0 + q], f);
                 unpack4(a[q], g);
@@ -826,29 +831,34 @@ int sspmm_layer_norm_fm(int hidden, int tokens, const void* x, const void* bias,
     if (tokens == 0) return 0;
     const int sms = current_device_sm_count();
     if (sms <= 0) return (int)cudaErrorNoDevice;
-    // 32 tokens per CTA once that gives every SM one
-    const bool wide = tokens >= 32 * sms;
     auto go = [&](auto kern, int TT, int threads, size_t smem) {
         kern<<<(tokens + TT - 1) / TT, threads, smem, static_cast<cudaStream_t>(stream)>>>(
             hidden, tokens, static_cast<const __half*>(x), static_cast<const __half*>(bias), static_cast<const __half*>(add), static_cast<__half*>(sum_out),
             static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, static_cast<__half*>(out));
     };
-    if (wide && hidden <= 1024) {
-        if (hidden <= 256) go(enc::layer_norm_fm_regs_kernel<2>, 32, enc::kLnWideThreads, 0);
-        else if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<4>, 32, enc::kLnWideThreads, 0);
-        else if (hidden <= 768) go(enc::layer_norm_fm_regs_kernel<6>, 32, enc::kLnWideThreads, 0);
-        else go(enc::layer_norm_fm_regs_kernel<8>, 32, enc::kLnWideThreads, 0);
-    } else {
-        auto kern = wide ? enc::layer_norm_fm_kernel<32> : enc::layer_norm_fm_kernel<8>;
-        const int TT = wide ? 32 : 8;
-        static DeviceOnce once_wide, once_narrow;
-        DeviceOnce& once = wide ? once_wide : once_narrow;
+    constexpr int kT = enc::kLnWideThreads;
+    // as many tokens per CTA as give every SM one
+    if (tokens >= 32 * sms && hidden > 1024) {
+        static DeviceOnce once;
         if (!once.done()) {
-            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * TT * 2);
+            const cudaError_t e = cudaFuncSetAttribute(enc::layer_norm_fm_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * 32 * 2);
             if (e != cudaSuccess) { set_error("LayerNorm: %s", cudaGetErrorString(e)); return (int)e; }
             once.mark();
         }
-        go(kern, TT, enc::kLnThreads, (size_t)hidden * TT * 2);
+        go(enc::layer_norm_fm_kernel<32>, 32, enc::kLnThreads, (size_t)hidden * 32 * 2);
+    } else if (tokens >= 32 * sms) {
+        if (hidden <= 256) go(enc::layer_norm_fm_regs_kernel<32, 2>, 32, kT, 0);
+        else if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<32, 4>, 32, kT, 0);
+        else if (hidden <= 768) go(enc::layer_norm_fm_regs_kernel<32, 6>, 32, kT, 0);
+        else go(enc::layer_norm_fm_regs_kernel<32, 8>, 32, kT, 0);
+    } else if (tokens >= 16 * sms && hidden <= 1024) {
+        if (hidden <= 256) go(enc::layer_norm_fm_regs_kernel<16, 1>, 16, kT, 0);
+        else if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<16, 2>, 16, kT, 0);
+        else go(enc::layer_norm_fm_regs_kernel<16, 4>, 16, kT, 0);
+    } else {
+        if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<8, 1>, 8, kT, 0);
+        else if (hidden <= 1024) go(enc::layer_norm_fm_regs_kernel<8, 2>, 8, kT, 0);
+        else go(enc::layer_norm_fm_regs_kernel<8, 6>, 8, kT, 0);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("LayerNorm launch: %s", cudaGetErrorString(e)); return (int)e; }

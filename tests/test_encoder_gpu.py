@@ -206,12 +206,12 @@ def test_layer_norm_wide_tile_with_most_features(lib):
     assert ((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -19 * (1 + w.double().abs()[:, None] * 4)).all()
 
 
-@pytest.mark.parametrize("hidden", [1, 127, 129, 256, 257, 512, 768, 1000, 1024, 1025])
-def test_layer_norm_with_features_in_registers(lib, hidden):
-    """From 32 tokens per SM on: every number of features per thread, its edges, the first that goes through shared memory, and a
-    partly filled tile; then the result in place of the operand.  Bound as in test_layer_norm_feature_major."""
+@pytest.mark.parametrize("tokens", [40, 16 * 148 + 8, 32 * 148 + 8])
+@pytest.mark.parametrize("hidden", [1, 127, 129, 256, 257, 512, 513, 768, 1000, 1024, 1025, 3072])
+def test_layer_norm_with_features_in_registers(lib, hidden, tokens):
+    """8, 16 and 32 tokens per CTA on 148 SMs: every number of features per thread, its edges, the first that goes through shared memory,
+    and a partly filled tile; then the result in place of the operand.  Bound as in test_layer_norm_feature_major."""
     from sspmm_b200 import ops
-    tokens = 32 * 148 + 8
     test_layer_norm_feature_major(lib, hidden, tokens)
     x, w = torch.randn(hidden, tokens, device="cuda:0").half(), torch.ones(hidden, device="cuda:0").half()
     out = torch.empty_like(x)
