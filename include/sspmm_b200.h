@@ -95,6 +95,9 @@ typedef struct sspmm_dense_operand {
     const void* values_f16;
 } sspmm_dense_operand;
 int sspmm_dense_copies(int count, const sspmm_dense_operand* operands, int N, void* room, int64_t* offsets, int64_t* bytes, void* stream);
+/* sspmm_dense_copies and sspmm_layer_norm_fm (without bias and sum) by one launch. */
+int sspmm_layer_norm_copies(int count, const sspmm_dense_operand* operands, int N, void* room, int hidden, int tokens, const void* x,
+                            const void* gamma, const void* beta, float eps, void* out, void* stream);
 int sspmm_of_copy(int m_vec, int vec_length, int N, int K, const void* copy_f16, const void* rhs_f16, const void* bias_f16, const void* add_f16,
                   void* out_f16, void* stream);
 

@@ -36,6 +36,7 @@ SIGNATURES = {
     "sspmm_group_run": (C.c_int, [_vp, _vp]),
     "sspmm_group_bias": (C.c_int, [_vp, C.c_int, _vp, c_int_p]),
     "sspmm_dense_copies": (C.c_int, [C.c_int, _vp, C.c_int, _vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64), _vp]),
+    "sspmm_layer_norm_copies": (C.c_int, [C.c_int, _vp, C.c_int, _vp, C.c_int, C.c_int] + [_vp] * 3 + [C.c_float, _vp, _vp]),
     "sspmm_of_copy": (C.c_int, [C.c_int] * 4 + [_vp] * 6),
     "sspmm_group_run_sum": (C.c_int, [_vp] * 5 + [c_int_p]),
     "sspmm_counted_sum": (C.c_int, [C.c_int] * 4 + [C.c_int64] + [_vp] * 9 + [c_int_p]),

@@ -205,13 +205,17 @@ PyObject* py_sspmm_sum(PyObject*, PyObject* const* a, Py_ssize_t n) {
     });
 }
 
-// dense_copies([(row_offsets of each piece, where the pieces' vectors end, column_indices, values, vec_length, K), ...], N)
-//   -> a copy [K, rows] per operand, or None where the product does not work on one; None: not operands for it
+// dense_copies([(row_offsets of each piece, where the pieces' vectors end, column_indices, values, vec_length, K), ...], N, x, gamma, beta, eps)
+//   -> a copy [K, rows] per operand, or None where the product does not work on one, and then LayerNorm of x where there is a copy (x may be
+//   None: without it; the caller has compared its operands); None: not operands for it
 PyObject* py_dense_copies(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         constexpr Py_ssize_t kMost = 8, kPieces = 4;
         long N;
-        if (n != 2 || modes_active() || !PyList_CheckExact(a[0]) || !small_int(a[1], 1, 0x7fffffff, &N)) Py_RETURN_NONE;
+        if (n != 6 || modes_active() || !PyList_CheckExact(a[0]) || !small_int(a[1], 1, 0x7fffffff, &N) || !PyFloat_Check(a[5])) Py_RETURN_NONE;
+        const at::Tensor *x = a[2] == Py_None ? nullptr : plain(a[2], at::kHalf), *gamma = x ? plain(a[3], at::kHalf) : nullptr,
+                         *beta = x ? plain(a[4], at::kHalf) : nullptr;
+        if (a[2] != Py_None && (!x || !gamma || !beta || x->dim() != 2)) Py_RETURN_NONE;
         const Py_ssize_t count = PyList_GET_SIZE(a[0]);
         if (count < 1 || count > kMost) Py_RETURN_NONE;
         sspmm_dense_operand op[kMost];
@@ -247,13 +251,18 @@ PyObject* py_dense_copies(PyObject*, PyObject* const* a, Py_ssize_t n) {
         }
         int rc = sspmm_dense_copies((int)count, op, (int)N, nullptr, at, &bytes, nullptr);
         if (rc != 0) return PyLong_FromLong(rc);
-        at::Tensor room;
+        at::Tensor room, norm;
         if (bytes) {
             room = at::empty({bytes / 2}, first->options().dtype(at::kHalf).requires_grad(false));
-            rc = launch(first->get_device(), [&](void* st) { return sspmm_dense_copies((int)count, op, (int)N, room.data_ptr(), at, &bytes, st); });
+            if (x) norm = at::empty_like(*x, x->options().requires_grad(false));
+            rc = launch(first->get_device(), [&](void* st) {
+                return x ? sspmm_layer_norm_copies((int)count, op, (int)N, room.data_ptr(), (int)x->size(0), (int)x->size(1), x->data_ptr(),
+                                                   gamma->data_ptr(), beta->data_ptr(), (float)PyFloat_AS_DOUBLE(a[5]), norm.data_ptr(), st)
+                         : sspmm_dense_copies((int)count, op, (int)N, room.data_ptr(), at, &bytes, st);
+            });
             if (rc != 0) return PyLong_FromLong(rc);
         }
-        PyObject* const list = PyList_New(count);
+        PyObject* const list = PyList_New(count + (norm.defined() ? 1 : 0));
         if (!list) return nullptr;
         for (Py_ssize_t k = 0; k < count; ++k) {
             PyObject* item = Py_None;
@@ -265,6 +274,7 @@ PyObject* py_dense_copies(PyObject*, PyObject* const* a, Py_ssize_t n) {
             }
             PyList_SET_ITEM(list, k, item);
         }
+        if (norm.defined()) PyList_SET_ITEM(list, count, THPVariable_Wrap(norm));
         return list;
     });
 }

@@ -359,6 +359,52 @@ struct svc_batch_job {
     cudaStream_t stream;
 };
 
+// The operands whose products with N columns work on a copy, and where it goes in room.
+static int collect_copies(int count, const sspmm_dense_operand* operands, int N, void* room, SpmmArgs* a, __half** at, int* made, int64_t* offsets,
+                          int64_t* bytes) {
+    if (count < 0 || count > kMaxCopies || !operands || !offsets || !bytes) { set_error("null pointer or more than %d operands", kMaxCopies); return (int)cudaErrorInvalidValue; }
+    const int choice = g_kernel_choice.load();
+    int64_t room_for = 0;
+    int copies = 0;
+    for (int k = 0; k < count; ++k) {
+        const sspmm_dense_operand& o = operands[k];
+        offsets[k] = -1;
+        if ((o.vec_length != 8 && o.vec_length != 16) || o.pieces < 1 || o.pieces > kMaxPieces || o.m_vec <= 0 || o.K <= 0 || N <= 0 || N % 8 != 0 ||
+            o.m_vec > 0x7fffffff / o.vec_length / o.pieces || !o.row_offsets || !o.nvec || !o.column_indices || !o.values_f16 ||
+            !aligned16(o.values_f16) || choice == 1 || choice == 2 || choice == 4)
+            continue;
+        SpmmArgs& s = a[copies];
+        s = SpmmArgs{};
+        s.m_vec = o.m_vec; s.V = o.vec_length; s.N = N; s.n_out = N; s.K = o.K;
+        s.row_indices = nullptr; s.row_offsets = o.row_offsets[0]; s.column_indices = o.column_indices;
+        s.values = static_cast<const __half*>(o.values_f16); s.rhs = s.values;
+        s.out = room; s.out_f16 = true; s.bias = nullptr; s.batch = 1;
+        s.values_stride = 0; s.rhs_stride = 0; s.out_stride = 0; s.stream = nullptr;
+        // every piece would go to the block kernel by itself
+        bool block = true;
+        int64_t total = 0;
+        for (int i = 0; i < o.pieces && block; ++i) {
+            block = o.row_offsets[i] && o.nvec[i] >= 0 && total + o.nvec[i] <= 0x7fffffffLL && sspmm_block_scratch_bytes(s) <= ((size_t)2 << 30) &&
+                    (choice == 3 || block_kernel_is_faster(o.nvec[i], s));
+            s.piece_offsets[i] = o.row_offsets[i];
+            s.piece_first[i] = (int)total;
+            total += o.nvec[i];
+        }
+        if (!block) continue;
+        s.m_vec = o.pieces * o.m_vec;
+        s.pieces = o.pieces;
+        if (sspmm_block_scratch_bytes(s) > ((size_t)2 << 30)) continue;
+        offsets[k] = room_for;
+        at[copies] = reinterpret_cast<__half*>(static_cast<uint8_t*>(room) + room_for);
+        room_for += (int64_t)(((size_t)o.K * s.m_vec * s.V * sizeof(__half) + 255) & ~(size_t)255);
+        ++copies;
+    }
+    *bytes = room_for;
+    *made = copies;
+    if (room && reinterpret_cast<uintptr_t>(room) % 256 != 0) { set_error("copies need room on a 256-byte boundary"); return (int)cudaErrorInvalidValue; }
+    return 0;
+}
+
 // First half of a compression: counting and scans are enqueued.  slot: host memory for the totals, or null.
 static int svc_count(int M, int K, int vec_length, const int* d_csr_row_ptr, const int* d_csr_col_idx, const void* d_csr_values_f16, void* stream,
                      void* slot, svc_job** job) {
@@ -509,48 +555,11 @@ int sspmm_counted_sum(int m_vec, int vec_length, int N, int K, int64_t nvec, con
 
 int sspmm_dense_copies(int count, const sspmm_dense_operand* operands, int N, void* room, int64_t* offsets, int64_t* bytes, void* stream) {
     g_err[0] = 0;
-    if (count < 0 || count > kMaxCopies || !operands || !offsets || !bytes) { set_error("null pointer or more than %d operands", kMaxCopies); return (int)cudaErrorInvalidValue; }
-    const int choice = g_kernel_choice.load();
     SpmmArgs a[kMaxCopies];
     __half* at[kMaxCopies];
-    int64_t room_for = 0;
     int copies = 0;
-    for (int k = 0; k < count; ++k) {
-        const sspmm_dense_operand& o = operands[k];
-        offsets[k] = -1;
-        if ((o.vec_length != 8 && o.vec_length != 16) || o.pieces < 1 || o.pieces > kMaxPieces || o.m_vec <= 0 || o.K <= 0 || N <= 0 || N % 8 != 0 ||
-            o.m_vec > 0x7fffffff / o.vec_length / o.pieces || !o.row_offsets || !o.nvec || !o.column_indices || !o.values_f16 ||
-            !aligned16(o.values_f16) || choice == 1 || choice == 2 || choice == 4)
-            continue;
-        SpmmArgs& s = a[copies];
-        s = SpmmArgs{};
-        s.m_vec = o.m_vec; s.V = o.vec_length; s.N = N; s.n_out = N; s.K = o.K;
-        s.row_indices = nullptr; s.row_offsets = o.row_offsets[0]; s.column_indices = o.column_indices;
-        s.values = static_cast<const __half*>(o.values_f16); s.rhs = s.values;
-        s.out = room; s.out_f16 = true; s.bias = nullptr; s.batch = 1;
-        s.values_stride = 0; s.rhs_stride = 0; s.out_stride = 0; s.stream = static_cast<cudaStream_t>(stream);
-        // every piece would go to the block kernel by itself
-        bool block = true;
-        int64_t total = 0;
-        for (int i = 0; i < o.pieces && block; ++i) {
-            block = o.row_offsets[i] && o.nvec[i] >= 0 && total + o.nvec[i] <= 0x7fffffffLL && sspmm_block_scratch_bytes(s) <= ((size_t)2 << 30) &&
-                    (choice == 3 || block_kernel_is_faster(o.nvec[i], s));
-            s.piece_offsets[i] = o.row_offsets[i];
-            s.piece_first[i] = (int)total;
-            total += o.nvec[i];
-        }
-        if (!block) continue;
-        s.m_vec = o.pieces * o.m_vec;
-        s.pieces = o.pieces;
-        if (sspmm_block_scratch_bytes(s) > ((size_t)2 << 30)) continue;
-        offsets[k] = room_for;
-        at[copies] = reinterpret_cast<__half*>(static_cast<uint8_t*>(room) + room_for);
-        room_for += (int64_t)(((size_t)o.K * s.m_vec * s.V * sizeof(__half) + 255) & ~(size_t)255);
-        ++copies;
-    }
-    *bytes = room_for;
-    if (!room || copies == 0) return 0;
-    if (reinterpret_cast<uintptr_t>(room) % 256 != 0) { set_error("copies need room on a 256-byte boundary"); return (int)cudaErrorInvalidValue; }
+    const int rc = collect_copies(count, operands, N, room, a, at, &copies, offsets, bytes);
+    if (rc != 0 || !room || copies == 0) return rc;
     const cudaError_t e = launch_expand_set(a, at, copies, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? 0 : fail(e, "dense copies");
 }

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/sspmm_b200.h"
 #include "launch.h"
@@ -42,12 +43,11 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // and 3.19, now 2.28 and 2.63; 768 x 1024 4.68 and 6.15, now 3.77 and 4.77; 512 x 4000 7.36 and 9.83, now 4.10 and 5.14; 3072 x 512 9.25 and
 // 15.3, now 7.07 and 11.1.
 constexpr int kLnThreads = 256, kLnWideThreads = 512;
-template <int TT>
 __global__ void __launch_bounds__(kLnThreads)
 layer_norm_fm_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
                      __half* __restrict__ sum_out,
                      const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps, __half* __restrict__ out) {
-    constexpr int P = TT / 8, kRows = kLnThreads / P;      // pieces per feature, features per turn
+    constexpr int TT = 32, P = TT / 8, kRows = kLnThreads / P;      // pieces per feature, features per turn
     extern __shared__ uint4 tile[];                         // [hidden][P]
     __shared__ float red[kLnThreads / 32][TT];
     const int piece = threadIdx.x % P, r0 = threadIdx.x / P, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -171,16 +171,15 @@ __device__ __forceinline__ uint4 pack4(const f32x2 (&f)[4]) {
 
 // The same with a thread's share in registers: TT tokens, up to 4096 / TT * NV features.
 template <int TT, int NV>
-__global__ void __launch_bounds__(kLnWideThreads, 2)
-layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
-                          __half* __restrict__ sum_out, const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps,
-                          __half* __restrict__ out) {
+__device__ __forceinline__ void layer_norm_tile(int tile, int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias,
+                                                const __half* __restrict__ add, __half* __restrict__ sum_out, const __half* __restrict__ gamma,
+                                                const __half* __restrict__ beta, float eps, __half* __restrict__ out) {
     constexpr int P = TT / 8, kRows = kLnWideThreads / P, kPair = NV < 2 ? 1 : 2;
     static_assert(NV % kPair == 0, "whole pairs");
     __shared__ float red[kLnWideThreads / 32][TT];
     __shared__ __align__(16) float whole[2][TT];
     const int piece = threadIdx.x % P, r0 = threadIdx.x / P, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t0 = blockIdx.x * TT + piece * 8;
+    const int t0 = tile * TT + piece * 8;
     const bool in = t0 < tokens;
     // Sums over the features of eight numbers per token, the same in every thread of the piece.  A lane hands on half of what it has at each
     // step (7 shuffles; 24 with every sum in every lane), and one warp adds up for the CTA.
@@ -283,6 +282,48 @@ layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, 
             for (int e = 0; e < 4; ++e) f[e] = fma2(mul2(add2(f[e], mean[e]), var[e]), pair_of(g, g), pair_of(b, b));
             *reinterpret_cast<uint4*>(out + at0 + j * turn) = pack4(f);
         }
+}
+
+template <int TT, int NV>
+__global__ void __launch_bounds__(kLnWideThreads, 2)
+layer_norm_fm_regs_kernel(int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ bias, const __half* __restrict__ add,
+                          __half* __restrict__ sum_out, const __half* __restrict__ gamma, const __half* __restrict__ beta, float eps,
+                          __half* __restrict__ out) {
+    layer_norm_tile<TT, NV>(blockIdx.x, hidden, tokens, x, bias, add, sum_out, gamma, beta, eps, out);
+}
+
+// The first CTAs write the dense copies of a layer's operands, the others normalise its input: neither needs the other, the copies are chains
+// of look-ups and the input is traffic.  768 wide, 32 x 512 tokens: 14.0 and 12.4 us one after the other and a launch between, 23.6 together; the
+// layer takes 335 us where it takes 339, with 4 x 512 tokens 104.8 (107.2), 16 x 512 213.2 (216.9).
+template <int TT, int NV>
+__global__ void __launch_bounds__(kLnWideThreads, 2)
+layer_norm_copies_kernel(const __grid_constant__ ExpandSet s, int hidden, int tokens, const __half* __restrict__ x, const __half* __restrict__ gamma,
+                         const __half* __restrict__ beta, float eps, __half* __restrict__ out) {
+    __shared__ int slot[kExpandChunk];
+    const int copies = s.first[s.count];
+    if ((int)blockIdx.x < copies) expand_of_set(s, blockIdx.x, slot);
+    else layer_norm_tile<TT, NV>(blockIdx.x - copies, hidden, tokens, x, nullptr, nullptr, nullptr, gamma, beta, eps, out);
+}
+
+// Calls f with tokens per tile and pieces per thread of the kernels above; false: a tile goes through shared memory.
+template <typename F>
+bool with_tile(int hidden, int tokens, int sms, F&& f) {
+    using std::integral_constant;
+    auto go = [&](auto tt, auto nv) { f(tt, nv); return true; };
+    constexpr integral_constant<int, 1> k1{};
+    constexpr integral_constant<int, 2> k2{};
+    constexpr integral_constant<int, 4> k4{};
+    constexpr integral_constant<int, 6> k6{};
+    constexpr integral_constant<int, 8> k8{};
+    constexpr integral_constant<int, 16> k16{};
+    constexpr integral_constant<int, 32> k32{};
+    // as many tokens per CTA as give every SM one
+    if (tokens >= 32 * sms) {
+        if (hidden > 1024) return false;
+        return hidden <= 256 ? go(k32, k2) : hidden <= 512 ? go(k32, k4) : hidden <= 768 ? go(k32, k6) : go(k32, k8);
+    }
+    if (tokens >= 16 * sms && hidden <= 1024) return hidden <= 256 ? go(k16, k1) : hidden <= 512 ? go(k16, k2) : go(k16, k4);
+    return hidden <= 512 ? go(k8, k1) : hidden <= 1024 ? go(k8, k2) : go(k8, k6);
 }
 
 // out = x + bias + add, rounded after each addition; one 16-byte piece per thread.
@@ -831,38 +872,59 @@ int sspmm_layer_norm_fm(int hidden, int tokens, const void* x, const void* bias,
     if (tokens == 0) return 0;
     const int sms = current_device_sm_count();
     if (sms <= 0) return (int)cudaErrorNoDevice;
-    auto go = [&](auto kern, int TT, int threads, size_t smem) {
-        kern<<<(tokens + TT - 1) / TT, threads, smem, static_cast<cudaStream_t>(stream)>>>(
-            hidden, tokens, static_cast<const __half*>(x), static_cast<const __half*>(bias), static_cast<const __half*>(add), static_cast<__half*>(sum_out),
-            static_cast<const __half*>(gamma), static_cast<const __half*>(beta), eps, static_cast<__half*>(out));
-    };
-    constexpr int kT = enc::kLnWideThreads;
-    // as many tokens per CTA as give every SM one
-    if (tokens >= 32 * sms && hidden > 1024) {
+    const __half *hx = static_cast<const __half*>(x), *hb = static_cast<const __half*>(bias), *ha = static_cast<const __half*>(add);
+    const __half *hg = static_cast<const __half*>(gamma), *ht = static_cast<const __half*>(beta);
+    __half *hs = static_cast<__half*>(sum_out), *ho = static_cast<__half*>(out);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const bool done = enc::with_tile(hidden, tokens, sms, [&](auto tt, auto nv) {
+        enc::layer_norm_fm_regs_kernel<tt, nv><<<(tokens + tt - 1) / tt, enc::kLnWideThreads, 0, st>>>(hidden, tokens, hx, hb, ha, hs, hg, ht, eps, ho);
+    });
+    if (!done) {
         static DeviceOnce once;
         if (!once.done()) {
-            const cudaError_t e = cudaFuncSetAttribute(enc::layer_norm_fm_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * 32 * 2);
+            const cudaError_t e = cudaFuncSetAttribute(enc::layer_norm_fm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 3072 * 32 * 2);
             if (e != cudaSuccess) { set_error("LayerNorm: %s", cudaGetErrorString(e)); return (int)e; }
             once.mark();
         }
-        go(enc::layer_norm_fm_kernel<32>, 32, enc::kLnThreads, (size_t)hidden * 32 * 2);
-    } else if (tokens >= 32 * sms) {
-        if (hidden <= 256) go(enc::layer_norm_fm_regs_kernel<32, 2>, 32, kT, 0);
-        else if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<32, 4>, 32, kT, 0);
-        else if (hidden <= 768) go(enc::layer_norm_fm_regs_kernel<32, 6>, 32, kT, 0);
-        else go(enc::layer_norm_fm_regs_kernel<32, 8>, 32, kT, 0);
-    } else if (tokens >= 16 * sms && hidden <= 1024) {
-        if (hidden <= 256) go(enc::layer_norm_fm_regs_kernel<16, 1>, 16, kT, 0);
-        else if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<16, 2>, 16, kT, 0);
-        else go(enc::layer_norm_fm_regs_kernel<16, 4>, 16, kT, 0);
-    } else {
-        if (hidden <= 512) go(enc::layer_norm_fm_regs_kernel<8, 1>, 8, kT, 0);
-        else if (hidden <= 1024) go(enc::layer_norm_fm_regs_kernel<8, 2>, 8, kT, 0);
-        else go(enc::layer_norm_fm_regs_kernel<8, 6>, 8, kT, 0);
+        enc::layer_norm_fm_kernel<<<(tokens + 31) / 32, enc::kLnThreads, (size_t)hidden * 32 * 2, st>>>(hidden, tokens, hx, hb, ha, hs, hg, ht, eps, ho);
     }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("LayerNorm launch: %s", cudaGetErrorString(e)); return (int)e; }
     return 0;
+}
+
+int sspmm_layer_norm_copies(int count, const sspmm_dense_operand* operands, int N, void* room, int hidden, int tokens, const void* x, const void* gamma,
+                            const void* beta, float eps, void* out, void* stream) {
+    set_error("%s", "");
+    if (hidden <= 0 || hidden > 3072 || tokens <= 0 || tokens % 8 != 0 || !x || !gamma || !beta || !out || !room || !enc::piece_aligned(x) ||
+        !enc::piece_aligned(out)) {
+        set_error("LayerNorm with copies: bad argument (hidden=%d tokens=%d)", hidden, tokens);
+        return (int)cudaErrorInvalidValue;
+    }
+    SpmmArgs a[kMaxCopies];
+    __half* at[kMaxCopies];
+    int copies = 0;
+    int64_t offsets[kMaxCopies], bytes = 0;
+    const int rc = collect_copies(count, operands, N, room, a, at, &copies, offsets, &bytes);
+    if (rc != 0) return rc;
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return (int)cudaErrorNoDevice;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    ExpandSet s;
+    cudaError_t e = make_expand_set(a, at, copies, sms, &s);
+    if (e != cudaSuccess) { set_error("dense copies: %s", cudaGetErrorString(e)); return (int)e; }
+    const __half *hx = static_cast<const __half*>(x), *hg = static_cast<const __half*>(gamma), *hb = static_cast<const __half*>(beta);
+    if (enc::with_tile(hidden, tokens, sms, [&](auto tt, auto nv) {
+            enc::layer_norm_copies_kernel<tt, nv><<<s.first[s.count] + (tokens + tt - 1) / tt, enc::kLnWideThreads, 0, st>>>(
+                s, hidden, tokens, hx, hg, hb, eps, static_cast<__half*>(out));
+        })) {
+        e = cudaGetLastError();
+        if (e != cudaSuccess) { set_error("LayerNorm launch: %s", cudaGetErrorString(e)); return (int)e; }
+        return 0;
+    }
+    e = launch_expand_set(a, at, copies, st);
+    if (e != cudaSuccess) { set_error("dense copies: %s", cudaGetErrorString(e)); return (int)e; }
+    return sspmm_layer_norm_fm(hidden, tokens, x, nullptr, nullptr, nullptr, gamma, beta, eps, out, stream);
 }
 
 int sspmm_add_bias_fm(int rows, int tokens, const void* x, const void* bias, const void* add, void* out, void* stream) {

@@ -121,15 +121,18 @@ struct ExpandSet {
         PieceRows pieces;
     } op[kMaxCopies];
 };
+__device__ __forceinline__ void expand_of_set(const ExpandSet& s, int cta, int (&slot)[kExpandChunk]) {
+    int o = 0;
+    while (o + 1 < s.count && cta >= s.first[o + 1]) ++o;
+    const ExpandSet::Operand& op = s.op[o];
+    const int b = cta - s.first[o], i = b / op.chunks, k_begin = (b - i * op.chunks) * op.chunk;
+    if (op.V == 16) expand_row<16>(op.m_vec, op.K, op.chunk, i, k_begin, op.pieces, op.col, op.values, op.at, slot);
+    else expand_row<8>(op.m_vec, op.K, op.chunk, i, k_begin, op.pieces, op.col, op.values, op.at, slot);
+}
 __global__ void __launch_bounds__(256)
 expand_set_kernel(const __grid_constant__ ExpandSet s) {
     __shared__ int slot[kExpandChunk];
-    int o = 0;
-    while (o + 1 < s.count && (int)blockIdx.x >= s.first[o + 1]) ++o;
-    const ExpandSet::Operand& op = s.op[o];
-    const int b = (int)blockIdx.x - s.first[o], i = b / op.chunks, k_begin = (b - i * op.chunks) * op.chunk;
-    if (op.V == 16) expand_row<16>(op.m_vec, op.K, op.chunk, i, k_begin, op.pieces, op.col, op.values, op.at, slot);
-    else expand_row<8>(op.m_vec, op.K, op.chunk, i, k_begin, op.pieces, op.col, op.values, op.at, slot);
+    expand_of_set(s, blockIdx.x, slot);
 }
 
 template <int BN, int STAGES>
@@ -843,27 +846,35 @@ PieceRows piece_rows(const SpmmArgs& a) {
 }
 }  // namespace
 
-cudaError_t launch_expand_set(const SpmmArgs* a, __half* const* at, int count, cudaStream_t stream) {
-    const int sms = current_device_sm_count();
-    if (sms <= 0) return cudaErrorNoDevice;
-    ExpandSet s = {};
-    s.count = count;
+namespace {
+cudaError_t make_expand_set(const SpmmArgs* a, __half* const* at, int count, int sms, ExpandSet* set) {
+    *set = ExpandSet{};
+    set->count = count;
     int64_t blocks = 0, rows = 0;
     for (int k = 0; k < count; ++k) rows += a[k].m_vec;
     for (int k = 0; k < count; ++k) {
-        ExpandSet::Operand& op = s.op[k];
+        ExpandSet::Operand& op = set->op[k];
         op.m_vec = a[k].m_vec; op.K = a[k].K; op.V = a[k].V;
         op.chunk = expand_chunk((int)(rows < 0x7fffffff ? rows : 0x7fffffff), a[k].K, sms);
         op.chunks = (a[k].K + op.chunk - 1) / op.chunk;
         op.col = a[k].column_indices; op.values = a[k].values; op.at = at[k];
         op.pieces = piece_rows(a[k]);
-        s.first[k] = (int)blocks;
+        set->first[k] = (int)blocks;
         blocks += (int64_t)op.m_vec * op.chunks;
-        if (blocks > 0x7fffffffLL) { set_error("too many rows for dense copies in one launch"); return cudaErrorInvalidValue; }
-        s.first[k + 1] = (int)blocks;
+        if (blocks > 0x3fffffffLL) { set_error("too many rows for dense copies in one launch"); return cudaErrorInvalidValue; }
+        set->first[k + 1] = (int)blocks;
     }
-    if (blocks == 0) return cudaSuccess;
-    expand_set_kernel<<<(unsigned)blocks, 256, 0, stream>>>(s);
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t launch_expand_set(const SpmmArgs* a, __half* const* at, int count, cudaStream_t stream) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    ExpandSet s;
+    const cudaError_t e = make_expand_set(a, at, count, sms, &s);
+    if (e != cudaSuccess || s.first[count] == 0) return e;
+    expand_set_kernel<<<(unsigned)s.first[count], 256, 0, stream>>>(s);
     return cudaGetLastError();
 }
 

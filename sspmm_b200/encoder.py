@@ -168,13 +168,17 @@ class SparseEncoderLayer:
         o = F.scaled_dot_product_attention(split(q), split(k), split(v))
         return o.permute(1, 3, 0, 2).reshape(self.hidden, batch * seq)
 
+    @staticmethod
+    def _normable(x, tensors, rows) -> bool:
+        """Whether LayerNorm's kernel takes x, all these tensors, and these numbers per feature."""
+        return _plain(*tensors) and x.dim() == 2 and x.shape[1] % 8 == 0 and 0 < x.shape[0] <= 3072 and all(t.shape == x.shape[:1] for t in rows)
+
     def _norm(self, x, wb, add=None, bias=None, out=None, sum_out=None):
         """LayerNorm of x + bias + add: (what was normalised, the result)."""
         whole = [t for t in (x, add, out, sum_out) if t is not None]
         rows = [t for t in (bias, *wb) if t is not None]
         shape = x.shape
-        if _plain(*whole, *rows) and len(shape) == 2 and shape[1] % 8 == 0 and 0 < shape[0] <= 3072 and \
-                (bias is None or add is not None) and all(t.shape == shape for t in whole) and all(t.shape == shape[:1] for t in rows):
+        if self._normable(x, [*whole, *rows], rows) and (bias is None or add is not None) and all(t.shape == shape for t in whole):
             out = torch.empty_like(x) if out is None else out
             if add is not None and sum_out is None:
                 sum_out = torch.empty_like(x)
@@ -200,19 +204,21 @@ class SparseEncoderLayer:
         att = self._attention(q, k, v, batch, seq)
         return att.contiguous() if out is None else out.copy_(att)
 
-    def _copies(self, tokens: int):
-        """Dense copies of the operands of this call's products, by one launch: of Q, K and V together, O, FFN1 and FFN2; None for a
-        product that does not work on one.  (Below 512 tokens none does.)"""
-        L = self.linears
+    def _copies(self, x: torch.Tensor):
+        """Dense copies of the operands of this call's products, of Q, K and V together, O, FFN1 and FFN2 (None for a product that does
+        not work on one; below 512 tokens none does), and the LayerNorm of x, by one launch; None for that where there is none."""
+        L, tokens = self.linears, x.shape[-1]
         qkv = getattr(self, "qkv", None)
         if tokens < 512 or any(type(l) is not SparseLinear or l.out_features % l.V for l in L[3:]):
-            return [None] * 4
+            return [None] * 4, None
         first = qkv.operand(L[:3]) if qkv else None
         each = [([l.row_offsets], [l.col.numel()], l.col, l.values, l.V, l.in_features) for l in L[3:]]
-        made = ops.dense_copies(([first] if first else []) + each, tokens)
+        norm = (x, *self.ln1, 1e-5) if self._normable(x, [x, *self.ln1], self.ln1) else None
+        made = ops.dense_copies(([first] if first else []) + each, tokens, norm)
         if made is None:
-            return [None] * 4
-        return made if first else [None] + made
+            return [None] * 4, None
+        y = made.pop() if len(made) > len(each) + (first is not None) else None
+        return (made if first else [None] + made), y
 
     def _groups_for(self, tokens: int):
         """Activation buffers of fixed shape and, bound to them, one group per dependency level of the layer:
@@ -273,12 +279,13 @@ class SparseEncoderLayer:
             q, k, v = (l.dense_forward(y) for l in L[:3])
             out = L[3].dense_forward(self._attention(q, k, v, batch, seq).contiguous()) + x
             return L[5].dense_forward(L[4].dense_forward(self._layer_norm_fm(out, self.ln2))) + out
-        copies = self._copies(x.shape[-1])
+        copies, y = self._copies(x)
 
         def product(i, a):
             y = L[i].of_copy(copies[i - 2], a) if copies[i - 2] is not None else None
             return L[i](a) if y is None else y
-        _, y = self._norm(x, self.ln1)
+        if y is None:
+            _, y = self._norm(x, self.ln1)
         qkv = getattr(self, "qkv", None)
         q, k, v = (qkv and (qkv.of_copy(copies[0], y) or qkv(L[:3], y))) or [l(y) for l in L[:3]]
         att = product(3, self._attend(q, k, v, batch, seq))

@@ -107,11 +107,12 @@ def sspmm_sum(row_offsets, column_indices, values, rhs, vec_length: int, bias, r
     return None if got is None else _made(got)
 
 
-def dense_copies(operands, N: int):
+def dense_copies(operands, N: int, norm=None):
     """The dense copies that the block kernel works on, of operands whose products with N columns are still to come, by one launch
     (``sspmm_dense_copies``).  ``operands``: (list of row offsets, where their vectors end, column_indices, values, vec_length, K).  A copy or
-    None (the product does not work on one) for each; None: not operands for it."""
-    got = capi.native().dense_copies(operands, N)
+    None (the product does not work on one) for each; None: not operands for it.  ``norm``: (x, gamma, beta, eps), compared by the
+    caller; where there is a copy its LayerNorm is made by the same launch and follows the copies."""
+    got = capi.native().dense_copies(operands, N, *((None, None, None, 0.0) if norm is None else norm))
     return None if got is None else _made(got)
 
 

@@ -290,22 +290,44 @@ def test_products_of_copies_made_by_one_launch(lib, V, N, shapes):
                             ((products[0][0][0][1], 1), (products[0][0][0][2], V))], V, 64)], 512) == [None]
 
 
+@pytest.mark.parametrize("hidden,tokens", [(256, 640), (512, 2400), (768, 2408), (768, 4744), (1088, 4744)])
+def test_layer_norm_beside_copies(lib, hidden, tokens):
+    """One launch for both, at every tile width, and two where the tile goes through shared memory: bit by bit the launches of their own."""
+    from sspmm_b200 import ops, synthetic
+    d = lambda a: torch.from_numpy(a).to("cuda:0")
+    w = synthetic.magnitude_pruned(512, 1500, 0.8, np.random.default_rng(hidden))
+    ptr, col, val, _ = ops.svc(d(w.row_ptr), d(w.col_idx), d(w.values), 512, 1500, 16)
+    operands = [([ptr], [col.numel()], col, val, 16, 1500)] * 2
+    x, g, b = torch.randn(hidden, tokens, device="cuda:0").half(), torch.randn(hidden, device="cuda:0").half(), torch.randn(hidden, device="cuda:0").half()
+    want = torch.empty_like(x)
+    ops.layer_norm_fm(x, g, b, 1e-5, want)
+    ops.set_kernel(3)
+    try:
+        one, two, norm = ops.dense_copies(operands, tokens, (x, g, b, 1e-5))
+        alone, _ = ops.dense_copies(operands, tokens)
+    finally:
+        ops.set_kernel(0)
+    assert torch.equal(norm, want) and torch.equal(one, alone) and torch.equal(two, alone)
+
+
 def test_layer_of_copies_is_the_layer(lib, monkeypatch):
     """The same layer with every product making its own copy, and one whose linears were replaced."""
     from sspmm_b200.encoder import SparseEncoderLayer
     layer = SparseEncoderLayer(hidden=512, ffn=2048, heads=8, sparsity=0.9, vec_length=16)
     x = torch.randn(512, 4096, device="cuda:0", dtype=torch.float16)
-    assert all(c is not None for c in layer._copies(4096)) and layer._copies(64) == [None] * 4
+    copies, norm = layer._copies(x)
+    assert all(c is not None for c in copies) and layer._copies(x[:, :64].contiguous()) == ([None] * 4, None)
+    assert torch.equal(norm, layer._norm(x, layer.ln1)[1])
     y = layer.forward(x, 8, 512)
     layer.linears[4].values.mul_(2)
     scaled = layer.forward(x, 8, 512)
     layer.linears[4].values.div_(2)
-    monkeypatch.setattr(layer, "_copies", lambda tokens: [None] * 4)
+    monkeypatch.setattr(layer, "_copies", lambda x: ([None] * 4, None))
     assert torch.equal(y, layer.forward(x, 8, 512)) and not torch.equal(y, scaled)
     monkeypatch.undo()
     own = layer.linears[5]
     layer.linears[5] = lambda a: own(a)
-    assert layer._copies(4096) == [None] * 4
+    assert layer._copies(x) == ([None] * 4, None)
     assert (layer.forward(x, 8, 512).double() - y.double()).norm() <= 4 * 2.0 ** -11 * y.double().norm()
 
 
