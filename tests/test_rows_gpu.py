@@ -64,6 +64,16 @@ def test_tile_edges_teams_and_clusters(lib, V, lens, K, N, kernel):
 
 
 @pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("rows,len_,N", [(74, 560, 64), (75, 560, 64), (75, 1780, 64), (75, 1800, 64), (37, 640, 64), (38, 640, 64), (37, 630, 64), (9, 640, 200)])
+def test_edges_of_the_division_into_clusters(lib, V, rows, len_, N):
+    """148 SMs: items that get an SM each in clusters of two or not, and of four, rows of 112 steps and more, of 40 and fewer; a row that
+    is longer than the mean and an empty one."""
+    ptr, col, val, rhs = operands([len_] * (rows - 2) + [0, min(2 * len_, 2000)], 2000, V, N, rows)
+    for dt in (torch.float16, torch.float32):
+        check(ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt), ptr, col, val, rhs, V)
+
+
+@pytest.mark.parametrize("V", [8, 16])
 @pytest.mark.parametrize("lens,K,N,offset", [([5, 0, 40], 64, 1, 0), ([900] * 4, 1000, 49, 0), ([40] * 20, 64, 50, 0), ([40] * 20, 64, 64, 3),
                                              ([1000] * 64, 1024, 1001, 1)])
 def test_unaligned_dense_operand(lib, V, lens, K, N, offset):
