@@ -284,7 +284,7 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
                 a.rhs = static_cast<const __half*>(scratch);
                 rest += copy_bytes;
             }
-            if (e == cudaSuccess) e = use_block ? launch_sspmm_block(a, rest, room) : launch_sspmm_rows(a, nvec, want ? rest : nullptr);
+            if (e == cudaSuccess) e = use_block ? launch_sspmm_block(a, rest, room) : launch_sspmm_rows(a, nvec, want ? rest : nullptr, true);
             if (scratch && !ex.caller_workspace) cudaFreeAsync(scratch, st);
             return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
         }
@@ -545,7 +545,7 @@ int sspmm_counted_sum(int m_vec, int vec_length, int N, int K, int64_t nvec, con
         e = launch_sspmm_block(a, scratch, bytes);
         cudaFreeAsync(scratch, a.stream);
     } else {
-        if (choice == 3 || sspmm_rows_scratch_bytes(a, nvec)) return 0;        // long rows are cut there
+        if (choice == 3 || sspmm_rows_may_be_long(a, nvec)) return 0;
         e = launch_sspmm_rows_set(&a, 1, nvec);
     }
     if (e != cudaSuccess) return fail(e, "SpMM launch");
@@ -630,7 +630,7 @@ int sspmm_stacked(int pieces, int m_vec, int vec_length, int N, int K, const int
         s.out = static_cast<uint8_t*>(out) + (size_t)i * m_vec * V * N * (out_is_f16 ? 2 : 4);
         s.bias = a.bias ? a.bias + (size_t)i * m_vec * V : nullptr;
         if (block_fits(s, true) && (choice == 3 || (choice == 0 && block_kernel_is_faster(nvec[i], s)))) ++block;
-        else if (choice == 3 || sspmm_rows_scratch_bytes(s, nvec[i])) return 0;    // long rows are cut: not in a launch of several products
+        else if (choice == 3 || sspmm_rows_may_be_long(s, nvec[i])) return 0;    // not in a launch of several products
         total += nvec[i];
     }
     if (block != 0 && (block != pieces || !block_fits(a, true))) return 0;

@@ -45,7 +45,10 @@ cudaError_t launch_sspmm_gather(const SpmmArgs& a);
 // Row-gather kernel: N % 8 == 0, rhs and values 16-byte aligned; any n_out <= N.
 // scratch: null, or sspmm_rows_scratch_bytes() bytes when that is not 0 (long rows are then cut); nvec < 0: unknown.
 size_t sspmm_rows_scratch_bytes(const SpmmArgs& a, long long nvec);
-cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch);
+// spread: the warps are divided with a row in mind that is many times the mean, where there may be one.
+cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch, bool spread);
+// Whether there may be one.
+bool sspmm_rows_may_be_long(const SpmmArgs& a, long long nvec);
 // Several products with vectors of one length and outputs of one type in one launch; no scratch.  nvec: vectors of all of them.
 constexpr int kRowsMaxSet = 8;
 cudaError_t launch_sspmm_rows_set(const SpmmArgs* a, int count, long long nvec);

@@ -1247,7 +1247,7 @@ int sspmm_planned(const sspmm_plan* plan, const void* values_f16, const void* rh
             a.out = out; a.out_f16 = out_is_f16 != 0; a.bias = nullptr; a.batch = 1;
             a.values_stride = 0; a.rhs_stride = 0; a.out_stride = 0;
             a.stream = static_cast<cudaStream_t>(stream);
-            const cudaError_t e = launch_sspmm_rows(a, plan->nvec, nullptr);
+            const cudaError_t e = launch_sspmm_rows(a, plan->nvec, nullptr, false);
             if (e != cudaSuccess) { set_error("SpMM launch: %s", cudaGetErrorString(e)); return (int)e; }
             return 0;
         }

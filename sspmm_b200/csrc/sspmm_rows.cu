@@ -71,6 +71,11 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
     const uint32_t bytes = valid ? 16u : 0u;                       // 0: the destination is zero-filled, nothing is read
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -411,6 +416,78 @@ sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int
     do_items<V, OutT, H>(p, out, (long long)(blockIdx.x / cluster) * (kWarps / team), team, cluster);
 }
 
+// Few items, and a row of unknown length may be many times the mean: a cluster has up to sixteen items, and its 64 warps take them in numbers that
+// go with their steps (per_step warps each, 16 bits of fraction).  What does not fit the warps at once is done in another round;
+// even rows fit.  A row's warps depend on its own length alone, so results do not depend on the order of the rows.
+// One launch without scratch, where cutting such rows (below) is a list by one CTA and a launch that waits for it, and leaves
+// one warp to a row of 256 vectors: 128 rows of 230 of 4608, V = 8, N = 49 17 us, here 8.2; one of them full 15.2, 10.3; 32 rows of 115 of
+// 2304, N = 800 16.7, 8.2.  What bounds it are the chain of look-ups, a step or two, and the cluster's start and two barriers.
+// The items are dealt in turn and staggered, so that tiles of one row do not meet (32 rows, one full, N = 800: 20.5 us in plain
+// turns, 10.3).
+constexpr int kStagger = 113;
+constexpr int kPooled = 16;               // items per cluster
+constexpr int kPoolClusters = 32;         // all of them resident
+constexpr int kPoolWarps = kMaxCluster * kWarps;
+constexpr int kPoolMost = 40;             // warps of an item, so that others find room (all 64: 128 rows of 115, one full, 16.4 us, 10.3)
+template <int V, typename OutT, int H>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_pooled_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int per_step, int most) {
+    using T = Tile<V, H, sizeof(OutT) == 4>;
+    extern __shared__ __align__(128) uint8_t smem[];    // [warp][T::kWarpBytes]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int mine = (int)cluster_cta_rank() * kWarps + warp;
+    const int clusters = gridDim.x / kMaxCluster, id = blockIdx.x / kMaxCluster;
+    const int count = (int)((p.items + clusters - 1) / clusters);
+    // Every lane has one item, whose warps end before `end` (of the warps of all items, one after another).
+    Where own = {-1, 0, 0, 0, 0};
+    if (lane < count) own = locate(p, (long long)lane * clusters + (id + lane * kStagger) % clusters, T::NT);
+    const int steps = (int)(((unsigned)own.len + kStep - 1) / kStep);
+    const int share = own.row < 0 ? 0 : min(max((int)((long long)steps * per_step >> 16), 1), most);
+    int end = share;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, end, d);
+        if (lane >= d) end += below;
+    }
+    uint8_t* const mem = smem + warp * T::kWarpBytes;
+    const int all = __shfl_sync(0xffffffffu, end, 31);
+    for (int done = 0; done < all;) {                     // a round: the items that fit from here on (the same in every warp)
+        const unsigned fits = __ballot_sync(0xffffffffu, end > done && end <= done + kPoolWarps);
+        const unsigned before = __ballot_sync(0xffffffffu, end - share <= done + mine);
+        const int owner = 31 - __clz(before);             // (of items without warps the last, whose end is the same)
+        const int last = __shfl_sync(0xffffffffu, end, 31 - __clz(fits));
+        const int team = __shfl_sync(0xffffffffu, share, owner), first = __shfl_sync(0xffffffffu, end, owner) - team - done;
+        const int row = __shfl_sync(0xffffffffu, own.row, owner), n0 = __shfl_sync(0xffffffffu, own.n0, owner);
+        const int j0 = __shfl_sync(0xffffffffu, own.j0, owner), len = __shfl_sync(0xffffffffu, own.len, owner);
+        const bool works = done + mine < last;
+        const int64_t first_row = (int64_t)row * V;
+        if (works) {
+            T tile;
+            tile.clear();
+            tile.accumulate(p, p.values, p.rhs, n0, j0, len, mine - first, team, lane, smem_u32(mem));
+            if (team == 1) tile.store(p, out, first_row, n0, reinterpret_cast<float*>(mem), lane);
+            else tile.spill(reinterpret_cast<float*>(mem), lane);
+        }
+        cluster_sync_all();                               // every warp's tile is complete and visible
+        if (works && team > 1) {
+            constexpr int kFours = T::NT / 4;
+            for (int u = mine - first; u < V * kFours / 32; u += team) {
+                const int x = u * 32 + lane, r = x / kFours, n = x % kFours * 4;
+                const uint32_t piece = smem_u32(smem) + (r * T::kPitch + n) * 4;
+                float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+                for (int m = first; m < first + team; ++m) {
+                    const float4 v = ld_cluster_f32x4(cluster_map_shared(piece + m % kWarps * T::kWarpBytes, (uint32_t)(m / kWarps)));
+                    o.x += v.x; o.y += v.y; o.z += v.z; o.w += v.w;
+                }
+                T::store_four(p, out, first_row + r, n0 + n, o);
+            }
+        }
+        cluster_sync_all();                               // the tiles have been read: the rings may be used again, and a CTA may leave
+        done = last;
+    }
+}
+
 // More items than warps, one warp each: a CTA has its share of the items from the start, looks all of them up at once (a thread each, the
 // first column ids on their way to L1), and its warps take them one after another from a counter in shared memory.  With a CTA for
 // every eight items the look-ups, four dependent loads, were paid for by every round of CTAs, and a warp that was done waited for
@@ -420,7 +497,6 @@ sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int
 // 15); what look-ups are left, half a microsecond a launch, shows with rows of ten vectors (7.7 us, dealt in turn 7.1).
 // The CTAs' shares are staggered: rows are often ordered by length, and their number may divide the number of CTAs.
 // (Vectors of 16 rows lost by walking when items were dealt in turn: 2048 x 512 at 98 %, N = 8192 46 us, 48; not tried with the counter.)
-constexpr int kStagger = 113;
 template <typename OutT, int H>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_walk_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
@@ -720,10 +796,65 @@ cudaError_t launch_split(const SpmmArgs& a, const Problem& p, int sms) {
     return cudaGetLastError();
 }
 
+// Some row may be many times the mean: the columns bound a row's length, so K tells, and the vector count tells the mean.  Below 2048
+// columns that counts only where the plain division leaves a warp more than 48 steps of such a row (a step takes about
+// 0.65 us, the list of parts 5): eight rows of 2000 vectors among 1024 of 40, V = 16, N = 128, 41 to 46 us, cut 14; 512 rows of 36 of
+// 1200, V = 8, N = 1024, 11 us, listed in vain 15.
+// Then, in this order: more warps for every item, warps by length, cut rows.  64 rows of 460 of 4608, V = 8, N = 56: 6.6 us with 32 warps
+// per row, 8.2 by length, 10.3 cut; one of them full, 10.3, 10.3 and 16.  Eight rows of 1000 of 20000: 8.2 by length, 12.4 cut, one
+// full 14.4 both ways.
+struct Route {
+    enum Way { kPlain, kPooledWarps, kCut } way;
+    Division d;
+    bool long_rows;                                 // a row may be many times the mean
+    int per_step, most;                             // pooled warps: warps per step of an item (16 bits of fraction), and at most
+};
+Route route(const SpmmArgs& a, long long nvec, int sms) {
+    Route r{Route::kPlain, divide(&a, 1, nvec, sms), false, 0, 0};
+    if (nvec <= 0 || a.batch != 1) return r;
+    const long long mean = nvec / a.m_vec, slots = (long long)sms * kResident * kWarps, items = count_items(&a, 1, r.d.H);
+    if (a.K < 8 * (mean + 1)) return r;
+    if (a.K < 2048 && a.K <= 48LL * kStep * r.d.team * r.d.cluster) return r;
+    r.long_rows = true;
+    // As many warps per item as leave a full row at most twelve steps each, if there is room: a full one then takes no longer than cut.
+    Division w = r.d;
+    auto too_long = [&] { return a.K > 12LL * kStep * w.team * w.cluster; };
+    auto room = [&] { return 2 * items * w.team * w.cluster <= slots; };
+    while (too_long() && w.team < kWarps && room()) w.team *= 2;
+    while (too_long() && w.cluster < kMaxCluster && w.team == kWarps && room()) w.cluster *= 2;
+    if (!too_long()) { r.d = w; return r; }
+    // Warps by length, a warp for every two steps at most and so many that even rows take 92 % of them; a full row twelve steps per warp,
+    // or twenty where nothing else is in its cluster (eight rows of 1000 of 20000, one full: 14.4 us, and cut).
+    const long long pooled = (items + kPoolClusters - 1) / kPoolClusters;
+    r.per_step = (int)std::min<long long>(1 << 15, (long long)(0.92 * 65536 * kPoolWarps * kStep * a.m_vec / (pooled * (nvec + 8.0 * a.m_vec))));
+    r.most = pooled == 1 ? kPoolWarps : kPoolMost;
+    const long long full = std::min<long long>(r.most, std::max<long long>(1, (a.K / kStep * r.per_step) >> 16));
+    r.way = pooled <= kPooled && a.K <= (pooled == 1 ? 20 : 12) * kStep * full ? Route::kPooledWarps : Route::kCut;
+    return r;
+}
+
+template <int V, typename OutT, int H>
+cudaError_t launch_pooled(const SpmmArgs& a, const Problem& p, const Route& r) {
+    static DeviceOnce once;
+    constexpr int kBytes = kWarps * Tile<V, H, sizeof(OutT) == 4>::kWarpBytes;
+    cudaError_t e = allow_smem(sspmm_rows_pooled_kernel<V, OutT, H>, once, kBytes);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(std::min<long long>(p.items, kPoolClusters) * kMaxCluster));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)kBytes; cfg.stream = a.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)kMaxCluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, sspmm_rows_pooled_kernel<V, OutT, H>, p, static_cast<OutT*>(a.out), r.per_step, r.most);
+}
+
 template <int V, typename OutT>
-cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, bool split, const Division& d, int sms) {
-    if (split) return H == 2 ? launch_split<V, OutT, 2>(a, p, sms) : launch_split<V, OutT, 1>(a, p, sms);
-    return H == 2 ? launch_plain<V, OutT, 2>(a, p, d, sms) : launch_plain<V, OutT, 1>(a, p, d, sms);
+cudaError_t launch_typed(const SpmmArgs& a, const Problem& p, int H, const Route& r, int sms) {
+    if (r.way == Route::kCut) return H == 2 ? launch_split<V, OutT, 2>(a, p, sms) : launch_split<V, OutT, 1>(a, p, sms);
+    if (r.way == Route::kPooledWarps) return H == 2 ? launch_pooled<V, OutT, 2>(a, p, r) : launch_pooled<V, OutT, 1>(a, p, r);
+    return H == 2 ? launch_plain<V, OutT, 2>(a, p, r.d, sms) : launch_plain<V, OutT, 1>(a, p, r.d, sms);
 }
 
 // Scratch of the variant that cuts rows: [16 B header][cap_cut * n_tiles arrival counters][cap_cut + cap_whole entries]
@@ -732,19 +863,10 @@ struct Scratch {
     int chunk = 0, cap_cut = 0, cap_whole = 0;      // chunk = 0: not worth cutting
     size_t entries_at = 0, partial_at = 0, bytes = 0;
 };
-// Rows are worth cutting when some row may be many times the mean: the columns bound a row's length, so K tells, and the
-// vector count tells the mean.  Below 2048 columns that is so only where the one-launch kernel leaves a warp more than 48 steps of
-// such a row (a step takes about 0.65 us, the list of parts 5): eight rows of 2000 vectors among 1024 of 40, V = 16, N = 128,
-// 41 to 46 us, cut 14; 512 rows of 36 of 1200, V = 8, N = 1024, 11 us, listed in vain 15.
 Scratch plan_scratch(const SpmmArgs& a, long long nvec) {
     Scratch r;
-    if (nvec <= 0 || a.batch != 1) return r;
     const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;
-    if (a.K < 8 * (nvec / a.m_vec + 1)) return r;
-    if (a.K < 2048) {
-        const Division d = divide(&a, 1, nvec, sms);
-        if (a.K <= 48LL * kStep * d.team * d.cluster) return r;
-    }
+    if (a.m_vec <= 0 || route(a, nvec, sms).way != Route::kCut) return r;
     const long long nt = a.N <= 64 ? 64 : 128, n_tiles = (a.N + nt - 1) / nt;
     // A part: a quarter of an SM's share of the vectors, at least four steps per warp.  n = 51970 (820 k vectors, V = 8,
     // N = 128) took 46.8 us with a quarter, 52.1 with an eighth and 78 with a sixteenth (every part drains the rings once; measured
@@ -810,13 +932,21 @@ bool too_many(long long items, int sms) {
 }
 }  // namespace rows
 
+bool sspmm_rows_may_be_long(const SpmmArgs& a, long long nvec) {
+    const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;
+    return a.m_vec > 0 && rows::route(a, nvec, sms).long_rows;
+}
+
 // scratch: null, or sspmm_rows_scratch_bytes() bytes (long rows are then cut); nvec < 0: unknown.
-cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) {
+cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch, bool spread) {
     const int sms = current_device_sm_count();
     if (sms <= 0) return cudaErrorNoDevice;
     const bool split = scratch != nullptr;
-    const rows::Division d = rows::divide(&a, 1, nvec, sms);
-    const int H = split ? (a.N > 64 ? 2 : 1) : d.H;
+    rows::Route r = rows::route(a, nvec, sms);
+    if (!spread) r.d = rows::divide(&a, 1, nvec, sms);
+    if (split) r.way = rows::Route::kCut;
+    else if (!spread || r.way == rows::Route::kCut) r.way = rows::Route::kPlain;
+    const int H = split ? (a.N > 64 ? 2 : 1) : r.d.H;
     rows::Problem p = rows::problem_of(a, H);
     if (rows::too_many(p.items, sms)) return cudaErrorInvalidValue;
     if (split) {
@@ -829,8 +959,8 @@ cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch) 
         p.partial = reinterpret_cast<float*>(s + r.partial_at);
     }
     if (a.V == 16)
-        return a.out_f16 ? rows::launch_typed<16, __half>(a, p, H, split, d, sms) : rows::launch_typed<16, float>(a, p, H, split, d, sms);
-    return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, split, d, sms) : rows::launch_typed<8, float>(a, p, H, split, d, sms);
+        return a.out_f16 ? rows::launch_typed<16, __half>(a, p, H, r, sms) : rows::launch_typed<16, float>(a, p, H, r, sms);
+    return a.out_f16 ? rows::launch_typed<8, __half>(a, p, H, r, sms) : rows::launch_typed<8, float>(a, p, H, r, sms);
 }
 
 RowsShape sspmm_rows_set_shape(const SpmmArgs* a, int count, long long nvec) {

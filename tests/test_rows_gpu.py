@@ -306,3 +306,19 @@ def test_batch_of_more_items_than_warps(lib):
     out = bspmm(ops.sorted_row_swizzle(ptr), ptr, col, val, rhs, 8)
     for b in (0, 1, 37, 95):
         check(out[b], ptr, col, val[b], rhs[b], 8)
+
+
+# Rows that may be many times the mean: more warps for every item, warps by length (one round and several, empty rows, one item and
+# several per cluster, 512 items and one more, 20 steps per warp of a full row and more), cut rows.
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("lens,K,N", [
+    ([230] * 128, 4608, 72), ([0] * 127 + [2304], 2304, 48), ([2304] * 3 + [20] * 29, 2304, 800), ([4608] + [400] * 63, 4608, 56),
+    ([115, 0, 17, 1, 33, 32, 600] * 20, 2304, 200), ([25] * 512, 2048, 64), ([25] * 513, 2048, 64), ([1000] * 8, 20480, 24), ([1000] * 8, 20496, 24),
+    ([1], 2048, 8), ([1900] * 10 + [30] * 500, 2000, 64)])
+def test_rows_that_may_be_long(lib, V, lens, K, N):
+    ptr, col, val, rhs = operands(lens, K, V, N, 11)
+    order = torch.randperm(len(lens), device=DEV).int()
+    for dt in (torch.float16, torch.float32):
+        got = ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt)
+        check(got, ptr, col, val, rhs, V)
+        assert torch.equal(got, ops.sspmm(ptr, col, val, rhs, V, row_indices=order, out_dtype=dt))
