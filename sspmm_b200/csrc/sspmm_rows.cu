@@ -711,7 +711,8 @@ Division divide(const SpmmArgs* a, int count, long long nvec, int sms) {
     while (d.team < kWarps && (2 * d.team <= want || mean_steps > 32LL * d.team)) d.team *= 2;
     // Clusters leave each warp fewer steps, at least four, and cost about a microsecond.  The first doubling is not worth it where it gives
     // SMs a second CTA and saves no more than seven steps per warp (300 x 700, V = 8, N = 96 5.34 us in clusters of two, 4.52 without; 512 x 2048,
-    // V = 16, N = 200 8.82 and 8.41; 188 x 4491, N = 712, 18 steps saved, 15.2 and 17.0); the second is from two and a half steps on where every
+    // V = 16, N = 200 8.82 and 8.41; 188 x 4491, N = 712, 18 steps saved, 15.2 and 17.0), where a full row leaves no warp more than twenty
+    // (64 x 4608, V = 8, N = 1024, one row of eight full: 13.5 us in clusters, 18.5); the second is from two and a half steps on where every
     // CTA has an SM (256 x 1024, V = 16, N = 128 5.34, in clusters of four 4.92; 113 x 1191, V = 16, N = 8 5.17 and 4.63).  fp32 results keep their
     // clusters: their distance from 64 bits grows by 1 to 4 % with other chains (7.74e-8 to 8.04e-8, 336 x 878); fp16 ones show nothing.
     if (d.team == kWarps) {
@@ -719,7 +720,7 @@ Division divide(const SpmmArgs* a, int count, long long nvec, int sms) {
         const bool f16 = a->out_f16;
         while (d.cluster < kMaxCluster && (long long)d.cluster * 2 * d.team <= want) {
             const long long warps = (long long)d.cluster * d.team;
-            if (f16 && d.cluster == 1 && items <= sms && 2 * items > sms && mean_steps <= 14 * warps) break;
+            if (f16 && d.cluster == 1 && items <= sms && 2 * items > sms && mean_steps <= 14 * warps && a->K <= 20 * kStep * warps) break;
             if (mean_steps < 4 * warps && !(f16 && d.cluster == 2 && 2 * mean_steps >= 5 * warps && 4 * items <= sms)) break;
             d.cluster *= 2;
         }
