@@ -246,6 +246,11 @@ static int spmm_entry(int m_vec, int V, int N, int K, int batch, const int* row_
         }
         long long nvec = ex.nvec;
         if (nvec < 0 && !ex.query && (choice == 0 || choice == 4)) nvec = lookup_nvec(row_offsets, m_vec, st);
+        if (!rhs_ok && choice == 0 && sspmm_rows_reads_unaligned(a, nvec)) {
+            a.N = N;                                           // rows of B where they lie
+            e = launch_sspmm_rows_unaligned(a, nvec);
+            return e == cudaSuccess ? 0 : fail(e, "SpMM launch");
+        }
         const bool use_block = block_ok && (choice == 3 || (choice == 0 && nvec >= 0 && block_kernel_is_faster(nvec, a)));
         const size_t want = use_block ? sspmm_block_scratch_bytes(a) : sspmm_rows_scratch_bytes(a, nvec);
         if (ex.query) { *ex.query = want; return 0; }

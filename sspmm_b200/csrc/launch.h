@@ -49,6 +49,9 @@ size_t sspmm_rows_scratch_bytes(const SpmmArgs& a, long long nvec);
 cudaError_t launch_sspmm_rows(const SpmmArgs& a, long long nvec, void* scratch, bool spread);
 // Whether there may be one.
 bool sspmm_rows_may_be_long(const SpmmArgs& a, long long nvec);
+// The same for an rhs on a 16-byte boundary whose N is not a multiple of 8, one product without a copy of rhs; whether a call is one for it.
+bool sspmm_rows_reads_unaligned(const SpmmArgs& a, long long nvec);
+cudaError_t launch_sspmm_rows_unaligned(const SpmmArgs& a, long long nvec);
 // Several products with vectors of one length and outputs of one type in one launch; no scratch.  nvec: vectors of all of them.
 constexpr int kRowsMaxSet = 8;
 cudaError_t launch_sspmm_rows_set(const SpmmArgs* a, int count, long long nvec);

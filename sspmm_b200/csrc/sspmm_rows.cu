@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "launch.h"
 #include "ptx.cuh"
@@ -78,6 +79,9 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr) {
 }
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
     const uint32_t bytes = valid ? 16u : 0u;                       // 0: the destination is zero-filled, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_bytes(uint32_t dst, const void* src, uint32_t bytes) {      // up to 16 bytes, zeros after them
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
@@ -182,10 +186,11 @@ struct Tile {
                         ok ? values + ((int64_t)j0 + idx) * V + part * 8 : values, ok);
         }
     }
-    __device__ __forceinline__ void multiply_step(uint32_t slot, int lane) {
+    __device__ __forceinline__ void multiply_step(uint32_t slot, int lane) { multiply_step(slot, slot + kStep * kRowBytes, lane); }
+    __device__ __forceinline__ void multiply_step(uint32_t slot, uint32_t vectors, int lane) {
         uint32_t b[VB][2];
         const int k = lane & 15;
-        const uint32_t vrow = slot + kStep * kRowBytes + k * (V * 2);
+        const uint32_t vrow = vectors + k * (V * 2);
         if constexpr (V == 8) {
             ldmatrix_x2_trans(b[0][0], b[0][1], vrow);
         } else {
@@ -234,6 +239,88 @@ struct Tile {
         }
         cp_async_wait<0>();
         __syncwarp();                               // the ring may be used for something else
+    }
+    // The same from a B whose rows start anywhere (pitch p.ldb halfs, B itself on a 16-byte boundary and of less than 2 GiB), 64 columns: the
+    // aligned pieces that hold a row's columns land as they lie, nine per row, and a step's rows are shifted into place before it is
+    // multiplied, each piece by the lane that asked for it.  Nothing is read past a row's columns.
+    static constexpr int kRawRow = 9 * 16;
+    static constexpr int kRawStage = kStep * kRawRow + kStep * V * 2;                          // rows, vectors
+    static constexpr int kRawStages = 4;
+    static constexpr int kRawBytes = kStep * kRowBytes + kRawStages * kRawStage;               // a step's shifted rows, the ring
+    static constexpr int kRawWarpBytes = ((kRawBytes > kSumBytes ? kRawBytes : kSumBytes) + 127) & ~127;
+    __device__ __forceinline__ void accumulate_unaligned(const Problem& p, const __half* __restrict__ values, const __half* __restrict__ rhs, int n0,
+                                                         int j0, int len, int first, int stride, int lane, uint32_t mem) {
+        static_assert(H == 1 && kRawStages == 4, "eight pieces per row; the offsets of four steps in 64 bits");
+        const int steps = (int)(((unsigned)len + kStep - 1) / kStep);
+        if (first >= steps) return;
+        const int mine = (steps - first + stride - 1) / stride;
+        const int width = min(NT, p.ldb - n0) * 2, pitch = p.ldb * 2, at0 = n0 * 2;
+        const uint8_t* const base = reinterpret_cast<const uint8_t*>(rhs);
+        const uint32_t ring = mem + kStep * kRowBytes;
+        const int row = lane >> 3, piece = lane & 7;
+        int cols = load_cols(p.col, j0, len, first, stride, lane);
+        int next = load_cols(p.col, j0, len, first + 2 * stride, stride, lane);
+        int issued = 0;
+        uint32_t fill = ring, use = ring;
+        uint64_t offsets = 0;                       // of this lane's four rows, 4 bits each, of the last four steps asked for
+        auto issue = [&]() {
+            offsets >>= 16;
+            if (issued < mine) {
+                const int half = (issued & 1) * 16;
+                uint32_t mask = 0;
+#pragma unroll
+                for (int i = 0; i < 5; ++i) {       // four rows at a time; then the ninth pieces of all
+                    const int r = i < 4 ? i * 4 + row : lane & 15, x = i < 4 ? piece : 8;
+                    const int c = __shfl_sync(0xffffffffu, cols, half + r);
+                    const bool ok = (unsigned)c < (unsigned)p.K;
+                    const int at = c * pitch + at0, from = (at & ~15) + x * 16;
+                    const int bytes = ok ? min(max(at + width - from, 0), 16) : 0;
+                    if (i < 4 || lane < 16) cp_async_bytes(fill + r * kRawRow + x * 16, base + (bytes ? from : 0), (uint32_t)bytes);
+                    if (i < 4) mask |= (uint32_t)(at & 15) << (4 * i);
+                }
+                offsets |= (uint64_t)mask << 48;
+                const int k = lane / VB, part = lane % VB;
+                if (lane < kStep * VB) {
+                    const unsigned idx = (unsigned)(first + issued * stride) * kStep + k;
+                    const bool ok = idx < (unsigned)len;
+                    cp_async_16(fill + kStep * kRawRow + k * (V * 2) + ((V == 16 ? part ^ ((k >> 2) & 1) : 0) << 4),
+                                ok ? values + ((int64_t)j0 + idx) * V + part * 8 : values, ok);
+                }
+            }
+            cp_async_commit();
+            if (issued & 1) {
+                cols = next;
+                next = load_cols(p.col, j0, len, first + (issued + 3) * stride, stride, lane);
+            }
+            ++issued;
+            fill = fill == ring + (kRawStages - 1) * kRawStage ? ring : fill + kRawStage;
+        };
+#pragma unroll
+        for (int k = 0; k < kRawStages - 1; ++k) issue();
+        for (int k = 0; k < mine; ++k) {
+            cp_async_wait<kRawStages - 2>();
+            __syncwarp();                           // everyone's copies are in; the slot refilled next and the shifted rows have been read
+            issue();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = i * 4 + row;
+                const uint32_t by = (uint32_t)offsets >> (4 * i), at = use + r * kRawRow + piece * 16 + (by & 8);
+                uint32_t w[6];
+#pragma unroll
+                for (int x = 0; x < 6; x += 2) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[x]), "=r"(w[x + 1]) : "r"(at + x * 4) : "memory");
+#pragma unroll
+                for (int x = 0; x < 5; ++x) w[x] = (by & 4) ? w[x + 1] : w[x];
+#pragma unroll
+                for (int x = 0; x < 4; ++x) w[x] = __funnelshift_r(w[x], w[x + 1], (by & 2) * 8);
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(mem + r * kRowBytes + ((piece ^ (r & 7)) << 4)), "r"(w[0]), "r"(w[1]),
+                             "r"(w[2]), "r"(w[3]) : "memory");
+            }
+            __syncwarp();                           // the step's rows are in place
+            multiply_step(mem, use + kStep * kRawRow, lane);
+            use = use == ring + (kRawStages - 1) * kRawStage ? ring : use + kRawStage;
+        }
+        cp_async_wait<0>();
+        __syncwarp();
     }
     // This warp's accumulators to its tile of sums [V][kPitch].
     __device__ __forceinline__ void spill(float* dst, int lane) const {
@@ -353,21 +440,26 @@ struct Tile {
 // warp order through shared memory (of the cluster), so results do not depend on timing.
 // cta_item: the first of the CTA's (or cluster's) items, of problem p.  (With the warp's own item in its place the plain kernel of V = 16
 // took another register and 2 to 5 % more time: 2048 x 4608 at 90 %, N = 2048 225 us, 216 as it is; 1500 x 2500 at 80 %, N = 800 60.3 and 57.0.)
-template <int V, typename OutT, int H, bool ADD = false>
+template <int V, typename OutT, int H, bool ADD = false, bool UNALIGNED = false>
 __device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ out, long long cta_item, int team, int cluster,
                                          const __half* add = nullptr) {
     using T = Tile<V, H, sizeof(OutT) == 4>;
-    extern __shared__ __align__(128) uint8_t smem[];    // [warp][T::kWarpBytes]
+    constexpr int kMine = UNALIGNED ? T::kRawWarpBytes : T::kWarpBytes;
+    extern __shared__ __align__(128) uint8_t smem[];    // [warp][kMine]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = cluster > 1 ? (int)cluster_cta_rank() : 0;
     const int member = warp % team;
     const Where w = locate(p, cta_item + warp / team, T::NT);
-    uint8_t* const mem = smem + warp * T::kWarpBytes;
+    uint8_t* const mem = smem + warp * kMine;
     T tile;
     tile.clear();
-    if (w.row >= 0)
-        tile.accumulate(p, p.values + w.batch * p.values_stride, p.rhs + w.batch * p.rhs_stride, w.n0, w.j0, w.len, rank * team + member,
-                        team * cluster, lane, smem_u32(mem));
+    if (w.row >= 0) {
+        if constexpr (UNALIGNED)
+            tile.accumulate_unaligned(p, p.values, p.rhs, w.n0, w.j0, w.len, rank * team + member, team * cluster, lane, smem_u32(mem));
+        else
+            tile.accumulate(p, p.values + w.batch * p.values_stride, p.rhs + w.batch * p.rhs_stride, w.n0, w.j0, w.len, rank * team + member,
+                            team * cluster, lane, smem_u32(mem));
+    }
     OutT* const cbase = out + w.batch * p.out_stride;
     const int64_t first_row = (int64_t)w.row * V;
     if (team == 1) {
@@ -381,7 +473,7 @@ __device__ __forceinline__ void do_items(const Problem& p, OutT* __restrict__ ou
     for (int u = member; u < T::kUnits; u += team) {
         float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int m = 0; m < team; ++m)
-            T::add_piece(reinterpret_cast<const float*>(smem + (warp - member + m) * T::kWarpBytes) + T::piece_at(u, lane), o);
+            T::add_piece(reinterpret_cast<const float*>(smem + (warp - member + m) * kMine) + T::piece_at(u, lane), o);
         if (cluster == 1) {
             if (w.row >= 0) T::template store_unit<OutT, ADD>(p, cbase, first_row, w.n0, u, lane, o, add);
         } else {
@@ -414,6 +506,15 @@ template <int V, typename OutT, int H>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int team, int cluster) {
     do_items<V, OutT, H>(p, out, (long long)(blockIdx.x / cluster) * (kWarps / team), team, cluster);
+}
+
+// A dense operand whose rows start off 16-byte boundaries, read where it lies: the aligned copy is an allocation and a launch of its own.
+// 512 x 512 half full, V = 8, N = 49 9.8 us with the copy, 6.2 here (replayed from a graph 5.1 and 4.3); 512 x 4608 at 80 % 12.3 and 8.7 (7.1, 6.8).  A step costs
+// more than twice an aligned one, in shared memory: its rows are read from the ring, shifted and written once more.
+template <int V, typename OutT>
+__global__ void __launch_bounds__(kThreads, kResident)
+sspmm_rows_unaligned_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out, int team, int cluster) {
+    do_items<V, OutT, 1, false, true>(p, out, (long long)(blockIdx.x / cluster) * (kWarps / team), team, cluster);
 }
 
 // Few items, and a row of unknown length may be many times the mean: a cluster has up to sixteen items, and its 64 warps take them in numbers that
@@ -496,7 +597,7 @@ sspmm_rows_pooled_kernel(const __grid_constant__ Problem p, OutT* __restrict__ o
 // the next two looked up early, one row in a hundred of 512 vectors among rows of 5 took 32 us where the CTAs of eight took 19 (now
 // 15); what look-ups are left, half a microsecond a launch, shows with rows of ten vectors (7.7 us, dealt in turn 7.1).
 // The CTAs' shares are staggered: rows are often ordered by length, and their number may divide the number of CTAs.
-// (Vectors of 16 rows lost by walking when items were dealt in turn: 2048 x 512 at 98 %, N = 8192 46 us, 48; not tried with the counter.)
+// (Vectors of 16 rows do not gain: 96 products of 512 x 512 at 90 %, N = 64 8.3 us, walking 8.6; 1355 x 4242, N = 16200 192 and 217.)
 template <typename OutT, int H>
 __global__ void __launch_bounds__(kThreads, kResident)
 sspmm_rows_walk_kernel(const __grid_constant__ Problem p, OutT* __restrict__ out) {
@@ -737,9 +838,9 @@ cudaError_t allow_smem(Kern kern, DeviceOnce& once, int bytes) {
     return e;
 }
 
-template <int V, typename OutT, int H, typename Kern, typename... Args>
+template <int V, typename OutT, int H, int WARP_BYTES = 0, typename Kern, typename... Args>
 cudaError_t launch_items(Kern kern, DeviceOnce& once, long long items, const Division& d, cudaStream_t stream, Args... args) {
-    constexpr int kBytes = kWarps * Tile<V, H, sizeof(OutT) == 4>::kWarpBytes;
+    constexpr int kBytes = kWarps * (WARP_BYTES ? WARP_BYTES : Tile<V, H, sizeof(OutT) == 4>::kWarpBytes);
     cudaError_t e = allow_smem(kern, once, kBytes);
     if (e != cudaSuccess) return e;
     const int per_cta = kWarps / d.team;
@@ -932,6 +1033,38 @@ bool too_many(long long items, int sms) {
     return true;
 }
 }  // namespace rows
+
+// One wave of warps with few steps each: the copy is what counts.  Five steps per warp (2048 x 2048 half full, N = 49: 16.0 and 14.4 us; 1024 x 1024,
+// N = 100: 10.3 and 12.3, in a graph 8.3 and 7.3) are as good as even, ten (512 x 4608 at 43 %) 13.9 and 14.4, in a graph 11.1 and 9.0.
+// One or two columns are copied all the same: every warp asks for the same few lines (123 rows of 510 of 627, V = 16, N = 1 in a graph 11.7 us, copied 6.2;
+// N = 3 6.9 and 6.3, from a stream 8.2 and 11.5).
+constexpr long long kUnalignedSteps = 4;
+bool sspmm_rows_reads_unaligned(const SpmmArgs& a, long long nvec) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0 || nvec <= 0 || a.batch != 1 || a.m_vec <= 0 || a.n_out < 3 || reinterpret_cast<uintptr_t>(a.rhs) % 16 ||
+        (int64_t)a.K * a.N * 2 > INT_MAX) return false;
+    const rows::Route r = rows::route(a, nvec, sms);
+    const long long steps = (nvec / a.m_vec + rows::kStep) / rows::kStep, warps = (long long)r.d.team * r.d.cluster;
+    return r.way == rows::Route::kPlain && r.d.H == 1 && steps <= kUnalignedSteps * warps &&
+           rows::count_items(&a, 1, 1) * warps <= (long long)sms * rows::kResident * rows::kWarps;
+}
+cudaError_t launch_sspmm_rows_unaligned(const SpmmArgs& a, long long nvec) {
+    const int sms = current_device_sm_count();
+    if (sms <= 0) return cudaErrorNoDevice;
+    const rows::Division d = rows::route(a, nvec, sms).d;
+    const rows::Problem p = rows::problem_of(a, 1);
+    auto go = [&](auto v, auto out) {
+        using OutT = decltype(out);
+        constexpr int V = decltype(v)::value;
+        static DeviceOnce once;
+        return rows::launch_items<V, OutT, 1, rows::Tile<V, 1, sizeof(OutT) == 4>::kRawWarpBytes>(rows::sspmm_rows_unaligned_kernel<V, OutT>, once, p.items,
+                                                                                                 d, a.stream, p, static_cast<OutT*>(a.out));
+    };
+    constexpr std::integral_constant<int, 8> k8{};
+    constexpr std::integral_constant<int, 16> k16{};
+    if (a.V == 16) return a.out_f16 ? go(k16, __half()) : go(k16, float());
+    return a.out_f16 ? go(k8, __half()) : go(k8, float());
+}
 
 bool sspmm_rows_may_be_long(const SpmmArgs& a, long long nvec) {
     const int sms = current_device_sm_count() > 0 ? current_device_sm_count() : 148;

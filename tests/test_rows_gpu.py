@@ -322,3 +322,23 @@ def test_rows_that_may_be_long(lib, V, lens, K, N):
         got = ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt)
         check(got, ptr, col, val, rhs, V)
         assert torch.equal(got, ops.sspmm(ptr, col, val, rhs, V, row_indices=order, out_dtype=dt))
+
+
+# Rows of B read where they lie: every offset from a 16-byte boundary, one element, row ends at the last column of a tile and of B, steps
+# that do not fill a warp's share, clusters.  The same numbers in the same order as from an aligned copy of B.
+@pytest.mark.parametrize("V", [8, 16])
+@pytest.mark.parametrize("lens,K,N", [
+    ([1], 1, 1), ([1], 1, 3), ([1, 1], 2, 3), ([3, 0, 5], 7, 5), ([17, 32, 0, 33], 40, 49), ([33] * 5, 33, 63), ([60] * 64, 60, 65), ([460] * 64, 600, 49),
+    ([300] * 3, 301, 127)])
+def test_rows_of_an_unaligned_operand(lib, V, lens, K, N):
+    for offset in range(8):
+        ptr, col, val, rhs = operands(lens, K, V, N, 7, offset)
+        for dt in (torch.float16, torch.float32):
+            got = ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt)
+            check(got, ptr, col, val, rhs, V)
+            ops.set_kernel(ops.KERNEL_GATHER_LSU)
+            try:
+                want = ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt)
+            finally:
+                ops.set_kernel(ops.KERNEL_AUTO)
+            assert torch.equal(got, want)
