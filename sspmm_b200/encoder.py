@@ -244,7 +244,7 @@ class SparseEncoderLayer:
     def forward_grouped(self, x: torch.Tensor, batch: int, seq: int) -> torch.Tensor:
         """Same layer with the linears run as groups (sspmm_group_run) on preallocated activation buffers.  The biases of
         Q and V go into the attention, the one of O into the LayerNorm, FFN2's into the last sum.  For short sequences (fewer
-        launches, little host work); at 32 x 512 tokens, 768 wide, ``forward`` is the faster form (0.40 against 0.55 ms: products
+        launches, little host work); at 32 x 512 tokens, 768 wide, ``forward`` is the faster form (0.36 against 0.53 ms: products
         of many rows run on CTA pairs there)."""
         self._groups_for(batch * seq)
         if self.groups is None:
