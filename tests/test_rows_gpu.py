@@ -312,7 +312,7 @@ def test_batch_of_more_items_than_warps(lib):
 # several per cluster, 512 items and one more, 20 steps per warp of a full row and more), cut rows.
 @pytest.mark.parametrize("V", [8, 16])
 @pytest.mark.parametrize("lens,K,N", [
-    ([230] * 128, 4608, 72), ([0] * 127 + [2304], 2304, 48), ([2304] * 3 + [20] * 29, 2304, 800), ([4608] + [400] * 63, 4608, 56),
+    ([230] * 128, 4608, 72), ([230] * 128, 4608, 49), ([0] * 127 + [2304], 2304, 48), ([2304] * 3 + [20] * 29, 2304, 800), ([4608] + [400] * 63, 4608, 56),
     ([115, 0, 17, 1, 33, 32, 600] * 20, 2304, 200), ([25] * 512, 2048, 64), ([25] * 513, 2048, 64), ([1000] * 8, 20480, 24), ([1000] * 8, 20496, 24),
     ([1], 2048, 8), ([1900] * 10 + [30] * 500, 2000, 64)])
 def test_rows_that_may_be_long(lib, V, lens, K, N):
@@ -322,6 +322,8 @@ def test_rows_that_may_be_long(lib, V, lens, K, N):
         got = ops.sspmm(ptr, col, val, rhs, V, out_dtype=dt)
         check(got, ptr, col, val, rhs, V)
         assert torch.equal(got, ops.sspmm(ptr, col, val, rhs, V, row_indices=order, out_dtype=dt))
+    bias = torch.randn(len(lens) * V, device=DEV).half()
+    assert torch.equal(ops.sspmm_bias(ptr, col, val, rhs, V, bias, out_dtype=torch.float32), got + bias.float()[:, None])
 
 
 # Rows of B read where they lie: every offset from a 16-byte boundary, one element, row ends at the last column of a tile and of B, steps
@@ -342,3 +344,5 @@ def test_rows_of_an_unaligned_operand(lib, V, lens, K, N):
             finally:
                 ops.set_kernel(ops.KERNEL_AUTO)
             assert torch.equal(got, want)
+        bias = torch.randn(len(lens) * V, device=DEV).half()
+        assert torch.equal(ops.sspmm_bias(ptr, col, val, rhs, V, bias, out_dtype=torch.float32), got + bias.float()[:, None])
