@@ -148,7 +148,8 @@ int sspmm_f16_f16_noalloc(int m_vec, int vec_length, int N, int K, const int* ro
  *   - the block kernel takes K * m_vec*V * 2 bytes (a dense transposed copy of A), plus fp32
  *     partial tiles when it splits K, from cudaMallocAsync on `stream` and returns them with
  *     cudaFreeAsync; the row-gather kernel does the same for the partial tiles of split long rows, and
- *     either for an aligned copy of rhs when N is not a multiple of 8 or rhs not on a 16-byte boundary;
+ *     either for an aligned copy of rhs when N is not a multiple of 8 or rhs not on a 16-byte boundary (not
+ *     where rows are short and rhs is on one);
  *   - once per device the release threshold of the device's default memory pool is raised to 1 GiB
  *     so that this scratch is not returned to the system at every synchronisation.
  * Callers that must not allocate or synchronise at call time use a plan (below), or

@@ -16,7 +16,8 @@
 // 6.0 TB/s of gathers where the ring reaches 9 to 10).
 //
 // Measured (graph replays, against the former kernel that passed stages of 64 rows to tcgen05.mma): 512 x 512 at 70 %, N =
-// 256: 5.4 us (12.7); 2048 x 512 at 90 %, V = 16, N = 256: 8.0 (16.6); 512 x 4608 at 90 %, N = 64: 7.5 (26.3).
+// 256: 5.4 us (12.7); 2048 x 512 at 90 %, V = 16, N = 256: 8.0 (16.6); 512 x 4608 at 90 %, N = 64: 7.5 (26.3), with clusters by
+// what a full row would take (route) N = 56 4.7.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
